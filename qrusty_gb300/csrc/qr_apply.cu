@@ -18,99 +18,20 @@
 //
 // Diagonal factor per group: D_g(r) = (-1)^popc(r & z0) * T_g[pi(r)], with
 // pi(r) the parities of r against a GF(2) basis of the group's z
-// differences (rank d <= kDMax, table of 2^d entries precomputed in FP64 on
-// the host).  The parities split into a per-thread constant and a per-m part
-// read from a 32-entry Walsh table, so the common case costs one sign select
-// per amplitude.  The x = 0 group with a large z span is a precomputed
+// differences.  The x = 0 group with a large z span is a precomputed
 // diagonal vector (FP64 Walsh-Hadamard transform per tile, diag_wht below).
 //
-// Precision.  QR_C128: double2 amplitudes, FP64 arithmetic.  QR_C64C: float2
-// amplitudes, FP32 products, each block's contributions summed in FP32 and
-// folded into the row's running sum with a two-sum (error-free transform):
-// the running value is an unevaluated (hi + lo) pair per component.
+// Precision.  These are the QR_C64C kernels (complex128 products are in
+// qr_apply_rows.cu): float2 amplitudes, FP32 products, each block's
+// contributions summed in FP32 and folded into the row's running sum with a
+// two-sum (error-free transform): the running value is an unevaluated
+// (hi + lo) pair per component.
 #include "qr_common.cuh"
+#include "qr_device.cuh"
 
 namespace qr {
 
-// Walsh words: bit m of walsh_word(v) is popc(m & v) & 1, for m, v < 32.
-constexpr uint32_t walsh_word(uint32_t v) {
-    uint32_t w = 0;
-    for (uint32_t m = 0; m < 32; ++m) {
-        uint32_t x = m & v, p = 0;
-        while (x) { p ^= x & 1u; x >>= 1; }
-        if (p) w |= 1u << m;
-    }
-    return w;
-}
-__constant__ uint32_t c_walsh[32] = {
-    walsh_word(0),  walsh_word(1),  walsh_word(2),  walsh_word(3),  walsh_word(4),
-    walsh_word(5),  walsh_word(6),  walsh_word(7),  walsh_word(8),  walsh_word(9),
-    walsh_word(10), walsh_word(11), walsh_word(12), walsh_word(13), walsh_word(14),
-    walsh_word(15), walsh_word(16), walsh_word(17), walsh_word(18), walsh_word(19),
-    walsh_word(20), walsh_word(21), walsh_word(22), walsh_word(23), walsh_word(24),
-    walsh_word(25), walsh_word(26), walsh_word(27), walsh_word(28), walsh_word(29),
-    walsh_word(30), walsh_word(31)};
-
-// ---------------------------------------------------------------- PTX helpers
-__device__ __forceinline__ uint32_t saddr(const void *p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_fence_init() {
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(bar)),
-                 "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes,
-                                         uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-            "r"(saddr(dst)),
-        "l"(src), "r"(bytes), "r"(saddr(bar))
-        : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(saddr(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ uint64_t gtimer_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-// Bounded wait: gives up after ~limit_ns and reports false.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity,
-                                                  uint64_t limit_ns) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = gtimer_ns();
-    while (!mbar_try_wait(bar, parity)) {
-        if (gtimer_ns() - t0 > limit_ns) return false;
-    }
-    return true;
-}
-
-constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s per stage
-constexpr int kMaxStages = 4;
-
 // ---------------------------------------------------------------- arithmetic
-template <typename Real>
-__device__ __forceinline__ void cmac(Cplx<Real> &acc, const Cplx<Real> &d, const Cplx<Real> &p) {
-    acc.re = fma(d.re, p.re, fma(-d.im, p.im, acc.re));
-    acc.im = fma(d.re, p.im, fma(d.im, p.re, acc.im));
-}
 __device__ __forceinline__ void two_sum_into(float &hi, float &lo, float b) {
     const float s = __fadd_rn(hi, b);
     const float bb = __fsub_rn(s, hi);
@@ -140,227 +61,6 @@ __device__ __forceinline__ float2 two_sum_carry2(float2 &hi, float2 b) {
     hi = s;
     return e;
 }
-template <typename Real>
-__device__ __forceinline__ Cplx<Real> cneg_if(const Cplx<Real> &d, uint32_t s) {
-    Cplx<Real> r;
-    r.re = s ? -d.re : d.re;
-    r.im = s ? -d.im : d.im;
-    return r;
-}
-
-// ---------------------------------------------------------------- c128 kernel
-// Plain complex128: AMPS amplitudes per thread, one (amplitude, group) = 4
-// DFMA.  Warps run decoupled, as in the compensated-c64 kernels: each waits on
-// the stage's full mbarrier, applies the block's groups, and counts itself
-// out on a per-stage counter; the last warp out refills the stage with the
-// partner tile a ring length ahead.  No CTA-wide barrier sits between
-// partner blocks, so the FP64 pipe does not drain at every block.
-template <int AMPS>
-__global__ void __launch_bounds__(512, 1) apply_c128(const ApplyArgs a, int stages) {
-    using C = Cplx<double>;
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    const uint32_t threads = blockDim.x;
-    const uint32_t nwarps = threads >> 5;
-    const uint32_t t = threadIdx.x;
-    const uint32_t lane = t & 31;
-    const uint32_t tile = 1u << a.b;
-    const uint32_t tile_bytes = tile * (uint32_t)sizeof(C);
-    C *bufs = reinterpret_cast<C *>(smem_raw);
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem_raw + (size_t)stages * tile_bytes);
-    uint32_t *cnt = reinterpret_cast<uint32_t *>(full + kMaxStages);
-    volatile uint32_t *s_abort = cnt + kMaxStages;
-    uint32_t *s_iss = cnt + kMaxStages + 1;  // copies issued per stage (drain)
-
-    const C *psi = static_cast<const C *>(a.psi);
-    C *y = static_cast<C *>(a.y);
-    const C *tables = static_cast<const C *>(a.tables);
-    const C *fat_c = static_cast<const C *>(a.fat_c);
-    const C *diag = static_cast<const C *>(a.diag);
-    const uint32_t nb = a.nblocks;
-
-    const uint64_t first = blockIdx.x;
-    const uint64_t my_items =
-        a.nitems > first ? (a.nitems - first + gridDim.x - 1) / gridDim.x : 0;
-    const uint64_t total = my_items * nb;
-    if (total == 0) return;
-
-    auto issue = [&](uint64_t L) {
-        const uint64_t k = L / nb;
-        const uint32_t j = (uint32_t)(L - k * nb);
-        const uint64_t item = first + k * gridDim.x;
-        const uint64_t st = item / a.ntiles;
-        const uint64_t q = item - st * a.ntiles;
-        const C *src = psi + st * a.N + ((q ^ a.blk_hi[j]) << a.b);
-        const int s = (int)(L % (uint64_t)stages);
-        if (blockIdx.x == 0 && (int64_t)L == a.withhold) return;  // test hook: never issued
-        ++s_iss[s];
-        mbar_expect_tx(&full[s], tile_bytes);
-        bulk_g2s(bufs + (size_t)s * tile, src, tile_bytes, &full[s]);
-    };
-    if (t == 0) {
-        for (int s = 0; s < stages; ++s) {
-            mbar_init(&full[s], 1);
-            cnt[s] = 0;
-            s_iss[s] = 0;
-        }
-        *s_abort = 0;
-        mbar_fence_init();
-        const uint64_t pro = total < (uint64_t)stages ? total : (uint64_t)stages;
-        for (uint64_t L = 0; L < pro; ++L) issue(L);
-    }
-    __syncthreads();
-
-    C acc[AMPS];
-    const uint32_t amask = AMPS - 1;
-    uint32_t j = 0, s = 0, par = 0;
-    uint64_t st = first / a.ntiles;
-    uint64_t q = first - st * a.ntiles;
-
-    for (uint64_t L = 0; L < total; ++L) {
-        const uint64_t rbase = (q << a.b) | t;
-        if (j == 0) {
-#pragma unroll
-            for (int m = 0; m < AMPS; ++m) acc[m].re = acc[m].im = 0.0;
-        }
-        // an expired wait sets the abort flag; from then on every warp skips
-        // waits and work
-        bool skip = *s_abort != 0;
-        if (!skip && !mbar_wait_bounded(&full[s], par, a.wait_ns)) {
-            if (lane == 0) {
-                atomicExch(a.err, kErrMbarTimeout);
-                *s_abort = 1;
-            }
-            skip = true;
-        }
-        skip = __any_sync(0xffffffffu, skip);
-        const C *buf = bufs + (size_t)s * tile;
-
-        if (!skip && (int)j == a.diag_block && diag != nullptr) {
-            const C *dg = diag + (q << a.b);
-#pragma unroll
-            for (int m = 0; m < AMPS; ++m) {
-                const uint32_t rl = t + threads * (uint32_t)m;
-                cmac(acc[m], dg[rl], buf[rl]);
-            }
-        }
-
-        const uint32_t g1 = skip ? 0u : a.blk_g0[j + 1];
-        for (uint32_t g = a.blk_g0[j]; g < g1; ++g) {
-            const GroupDesc gd = a.groups[g];
-            const uint32_t lo_t = gd.lo & (threads - 1);
-            const uint32_t lo_m = gd.lo >> a.tb;
-            const C *src = buf + (t ^ lo_t);
-            if (gd.d != kFat) {
-                const uint32_t s0 = (uint32_t)__popcll(rbase & gd.z0) & 1u;
-                const uint32_t W0 = c_walsh[(gd.z0 >> a.tb) & amask];
-                uint32_t u = 0, anyW = 0;
-                uint32_t W[kDMax];
-#pragma unroll
-                for (int i = 0; i < kDMax; ++i) {
-                    W[i] = 0;
-                    if (i < (int)gd.d) {
-                        u |= ((uint32_t)__popcll(rbase & gd.beta[i]) & 1u) << i;
-                        W[i] = c_walsh[(gd.beta[i] >> a.tb) & amask];
-                        anyW |= W[i];
-                    }
-                }
-                if (anyW == 0) {
-                    const C D = tables[gd.off + u];
-                    C Dn;
-                    Dn.re = -D.re;
-                    Dn.im = -D.im;
-#pragma unroll
-                    for (int m = 0; m < AMPS; ++m) {
-                        const C p = src[((uint32_t)m ^ lo_m) << a.tb];
-                        const uint32_t sg = ((W0 >> m) ^ s0) & 1u;
-                        C Dm;
-                        Dm.re = sg ? Dn.re : D.re;
-                        Dm.im = sg ? Dn.im : D.im;
-                        cmac(acc[m], Dm, p);
-                    }
-                } else {
-#pragma unroll
-                    for (int m = 0; m < AMPS; ++m) {
-                        uint32_t um = u;
-#pragma unroll
-                        for (int i = 0; i < kDMax; ++i) um ^= ((W[i] >> m) & 1u) << i;
-                        const C D = tables[gd.off + um];
-                        const C p = src[((uint32_t)m ^ lo_m) << a.tb];
-                        const uint32_t sg = ((W0 >> m) ^ s0) & 1u;
-                        cmac(acc[m], cneg_if(D, sg), p);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int m = 0; m < AMPS; ++m) {
-                    const uint64_t r = rbase | ((uint64_t)m << a.tb);
-                    C D;
-                    D.re = D.im = 0.0;
-                    for (uint32_t kk = 0; kk < gd.cnt; ++kk) {
-                        const uint64_t zk = a.fat_z[gd.off + kk];
-                        const C ck = fat_c[gd.off + kk];
-                        const uint32_t sg = (uint32_t)__popcll(r & zk) & 1u;
-                        D.re += sg ? -ck.re : ck.re;
-                        D.im += sg ? -ck.im : ck.im;
-                    }
-                    const C p = src[((uint32_t)m ^ lo_m) << a.tb];
-                    cmac(acc[m], D, p);
-                }
-            }
-        }
-
-        if (j == nb - 1) {
-            C *yo = y + st * a.N + (q << a.b);
-#pragma unroll
-            for (int m = 0; m < AMPS; ++m) {
-                C o = acc[m];
-                const uint32_t rl = t + threads * (uint32_t)m;
-                if (a.v != nullptr) {  // fused y = alpha (H psi) + beta v
-                    const double2 vv = static_cast<const double2 *>(a.v)[st * a.N + (q << a.b) + rl];
-                    const double2 r = cx_axpby(a.ar, a.ai, make_double2(o.re, o.im), a.br, a.bi, vv);
-                    o.re = r.x;
-                    o.im = r.y;
-                }
-                yo[rl] = o;
-            }
-        }
-
-        __syncwarp();
-        if (lane == 0) {
-            __threadfence_block();
-            const uint32_t old = atomicAdd(&cnt[s], 1u);
-            if (old == nwarps - 1) {
-                cnt[s] = 0;
-                if (L + (uint64_t)stages < total && *s_abort == 0) {
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    issue(L + (uint64_t)stages);
-                }
-            }
-        }
-        if (++s == (uint32_t)stages) {
-            s = 0;
-            par ^= 1u;
-        }
-        if (++j == nb) {
-            j = 0;
-            q += gridDim.x;
-            while (q >= a.ntiles) {
-                q -= a.ntiles;
-                ++st;
-            }
-        }
-    }
-    // After an expired wait: every warp has left the loop (no copy is issued
-    // after the abort flag is set), then a bounded wait -- with the full 2 s,
-    // whatever a test set for the waits -- for the last copy issued into
-    // each stage, whose phase parity is (issues - 1) & 1.
-    __syncthreads();
-    if (t == 0 && *s_abort) {
-        for (int k = 0; k < stages; ++k)
-            if (s_iss[k] != 0) mbar_wait_bounded(&full[k], (s_iss[k] - 1u) & 1u, kWaitLimitNs);
-    }
-}
-
 // ---------------------------------------------------------------- c64c kernels
 // Compensated complex64 path.  A 4096-amplitude tile is held by T = 512
 // threads x AMPS = 8 amplitudes (single-operator and batched kernels);
@@ -1439,39 +1139,9 @@ cudaError_t launch_batch_c64c(const BatchArgs &a, int nsm, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-template <int AMPS>
-static cudaError_t launch_one(const ApplyArgs &a, int threads, int nsm, cudaStream_t st) {
-    const uint32_t tile_bytes = (1u << a.b) * (uint32_t)sizeof(Cplx<double>);
-    int stages = (int)((200u * 1024u) / tile_bytes);
-    if (stages > kMaxStages) stages = kMaxStages;
-    if (stages < 2) stages = 2;
-    // stages, then full barriers, stage counters, the abort flag and issue counts
-    const size_t smem = (size_t)stages * tile_bytes + kMaxStages * (sizeof(uint64_t) + 8u) + 8u;
-    auto kern = apply_c128<AMPS>;
-    cudaError_t e = ensure_dyn_smem(reinterpret_cast<const void *>(kern), smem);
-    if (e != cudaSuccess) return e;
-    uint64_t grid = a.nitems < (uint64_t)nsm ? a.nitems : (uint64_t)nsm;
-    if (grid == 0) return cudaSuccess;
-    kern<<<(unsigned)grid, threads, smem, st>>>(a, stages);
-    count_launch();
-    return cudaGetLastError();
-}
-
-static cudaError_t dispatch_amps(const ApplyArgs &a, int amps, int threads, int nsm,
-                                 cudaStream_t st) {
-    switch (amps) {
-        case 1: return launch_one<1>(a, threads, nsm, st);
-        case 2: return launch_one<2>(a, threads, nsm, st);
-        case 4: return launch_one<4>(a, threads, nsm, st);
-        case 8: return launch_one<8>(a, threads, nsm, st);
-        case 16: return launch_one<16>(a, threads, nsm, st);
-        default: return cudaErrorInvalidValue;
-    }
-}
-
 cudaError_t launch_apply(int dtype, const ApplyArgs &a, int amps, int threads, int nsm,
                          cudaStream_t st) {
-    if (dtype == 0) return dispatch_amps(a, amps, threads, nsm, st);
+    if (dtype == 0) return launch_c128_rows(a, st);
     if (amps >= 2 && a.tb != kTb) return cudaErrorInvalidValue;
     switch (amps) {
         case 1: return launch_c64c<1>(a, threads, nsm, st);

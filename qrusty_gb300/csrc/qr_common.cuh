@@ -12,7 +12,7 @@ namespace qr {
 constexpr int kDMax = 4;
 constexpr uint32_t kFat = 0xffffffffu;
 
-// One x-group of the apply plan.  All terms of the group share the x mask;
+// One x-group of the complex128 apply plan.  All terms of the group share the x mask;
 // their z masks are z0 ^ delta_k with delta_k in span(beta[0..d)).  The
 // group's diagonal factor at row r is
 //   D(r) = (-1)^popc(r & z0) * table[off + pi(r)],  pi(r)_i = popc(r & beta_i) & 1.
@@ -20,11 +20,13 @@ constexpr uint32_t kFat = 0xffffffffu;
 struct alignas(16) GroupDesc {
     uint64_t z0;
     uint64_t beta[kDMax];
-    uint32_t lo;    // x & (tile - 1): XOR partner inside the partner tile
+    uint64_t x;
     uint32_t d;     // rank, or kFat
     uint32_t off;   // table offset (entries) or fat-term offset
     uint32_t cnt;   // fat-term count
+    uint32_t pad;
 };
+static_assert(sizeof(GroupDesc) == 64, "GroupDesc layout");
 
 template <typename Real> struct Cplx;
 template <> struct alignas(8) Cplx<float> { float re, im; };
@@ -49,11 +51,11 @@ struct ApplyArgs {
     uint64_t ntiles;        // N >> b
     uint64_t nitems;        // nstates * ntiles
     const GroupDesc *groups;
+    uint32_t ngroups;
     const void *tables;     // Cplx<Real>
     const uint64_t *fat_z;
     const void *fat_c;      // Cplx<Real>
     const uint64_t *blk_hi; // partner-tile XOR per block
-    const uint32_t *blk_g0; // groups of block j: [blk_g0[j], blk_g0[j+1])
     uint32_t nblocks;
     const void *diag;       // Cplx<Real>[N] or null (only read in block hi == 0)
     int diag_block;         // index of the hi == 0 block, or -1
@@ -202,6 +204,8 @@ cudaError_t ensure_dyn_smem(const void *fn, size_t bytes);
 // Kernel launchers (qr_apply.cu / qr_csr.cu).
 cudaError_t launch_apply(int dtype, const ApplyArgs &a, int amps, int threads, int nsm,
                          cudaStream_t st);
+// qr_apply_rows.cu
+cudaError_t launch_c128_rows(const ApplyArgs &a, cudaStream_t st);
 cudaError_t launch_diag(int dtype, int n, int db, uint64_t ntiles, const uint64_t *bin_zlo,
                         const uint32_t *bin_off, uint32_t nbins, const uint64_t *tz,
                         const double *tc, void *out, cudaStream_t st);

@@ -116,7 +116,7 @@ struct Plan {
     uint64_t ngroups = 0, nfat = 0;
     int diag_block = -1;
     bool has_diag = false;
-    DevBuf groups, tables, fat_z, fat_c, blk_hi, blk_g0, diag;
+    DevBuf groups, tables, fat_z, fat_c, blk_hi, diag;
     // compensated-c64 kernel tables
     uint32_t nsub = 0, nruns = 0, nchunks = 0, npairs = 0;
     DevBuf tdesc, tdata, blk_r0, run_g0, run_key, chunks;
@@ -672,7 +672,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
         GroupDesc d;
         memset(&d, 0, sizeof(d));
         d.z0 = sg.z0;
-        d.lo = sg.lo;
+        d.x = (sg.hi << pl.b) | sg.lo;
         d.d = sg.d;
         for (int q = 0; q < kDMax; ++q) d.beta[q] = sg.beta[q];
         if (sg.d != kFat) {
@@ -809,7 +809,6 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
         }
     }
     QR_CUDA(pl.blk_hi.upload(bhi), "upload blocks");
-    QR_CUDA(pl.blk_g0.upload(bg0), "upload block groups");
 
     if (pl.has_diag) {
         const int db = std::min(n, 12);
@@ -1185,11 +1184,11 @@ static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *ps
     a.ntiles = op->N >> pl.b;
     a.nitems = (uint64_t)nstates * a.ntiles;
     a.groups = pl.groups.as<GroupDesc>();
+    a.ngroups = (uint32_t)pl.ngroups;
     a.tables = pl.tables.p;
     a.fat_z = pl.fat_z.as<uint64_t>();
     a.fat_c = pl.fat_c.p;
     a.blk_hi = pl.blk_hi.as<uint64_t>();
-    a.blk_g0 = pl.blk_g0.as<uint32_t>();
     a.nblocks = pl.nblocks;
     a.diag = pl.has_diag ? pl.diag.p : nullptr;
     a.diag_block = pl.diag_block;
