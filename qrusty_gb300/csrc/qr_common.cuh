@@ -40,6 +40,16 @@ struct alignas(16) TileDataC64 {
 };
 static_assert(sizeof(TileDataC64) == 64, "TileDataC64 is read as four 16-byte words");
 
+// String plans: consumer threads, strings per block, CTAs per cluster at most.
+constexpr uint32_t kStrThreads = 512, kStrEntCap = 255, kStrMaxSplit = 8;
+
+// qubits from which a block holds two partner tiles and tiles are not split
+constexpr int kStrPairN = 19;
+struct StrSplit {
+    uint32_t nblk = 0, nstr = 0, tpb = 1;  // blocks, strings, partner tiles per block
+    uint32_t part[kStrMaxSplit][kStrMaxSplit + 1] = {};
+};
+
 struct ApplyArgs {
     const void *psi;
     void *y;
@@ -82,6 +92,13 @@ struct ApplyArgs {
     // > 0: partner blocks visited in pairs (blocks 2p, 2p+1 in one ring slot
     // of two stages); blk_r0 then indexes pairs and tdesc bit 15 is the half
     uint32_t npairs;
+    // string plans (qr_apply_strings.cu): nsblk blocks of one or two partner
+    // tiles, {XOR of tile 0, of tile 1 (or ~0), first 16-byte entry, strings};
+    // a block's entries are a header {strings, diagonal flag} and one per
+    // string; rank r of a cluster takes blocks [part[r], part[r + 1])
+    const uint4 *ent, *sblk;
+    uint32_t nsblk;
+    uint32_t part[kStrMaxSplit + 1];
     // fused epilogue y = alpha * (H psi) + beta * v when v != nullptr
     const void *v;
     double ar, ai, br, bi;
@@ -204,6 +221,10 @@ cudaError_t ensure_dyn_smem(const void *fn, size_t bytes);
 // Kernel launchers (qr_apply.cu / qr_csr.cu).
 cudaError_t launch_apply(int dtype, const ApplyArgs &a, int amps, int threads, int nsm,
                          cudaStream_t st);
+// qr_apply_strings.cu
+// call_items: output tiles of the caller's whole call
+cudaError_t launch_c64c_strings(const ApplyArgs &a, const StrSplit &sp, uint64_t call_items,
+                                int nsm, cudaStream_t st);
 // qr_apply_rows.cu
 cudaError_t launch_c128_rows(const ApplyArgs &a, cudaStream_t st);
 cudaError_t launch_diag(int dtype, int n, int db, uint64_t ntiles, const uint64_t *bin_zlo,

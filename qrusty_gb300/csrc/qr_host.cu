@@ -120,6 +120,10 @@ struct Plan {
     // compensated-c64 kernel tables
     uint32_t nsub = 0, nruns = 0, nchunks = 0, npairs = 0;
     DevBuf tdesc, tdata, blk_r0, run_g0, run_key, chunks;
+    // string plans: see ApplyArgs; str.part[k - 1] are the parts of a split in k
+    bool strings = false;
+    StrSplit str;
+    DevBuf ent, sblk;
     // what the plan was built for, and its coefficient program: the slots
     // that qr_op_set_coeffs_device recomputes on the device, with the
     // diagonal's term list kept so that diag_wht can run again
@@ -318,6 +322,95 @@ struct SubGroup {
     std::vector<uint8_t> coord;
 };
 
+// Entry lists of a string plan (qr_apply_strings.cu): the merged strings
+// outside the diagonal by partner tile, in blocks, and the parts of about
+// equal work that the CTAs of a cluster of 1 ... kStrMaxSplit take.
+template <typename AddSlot>
+int build_strings(qr_op *op, Plan &pl, const std::vector<cd> &c,
+                  const std::vector<size_t> &diag_terms, AddSlot &&add_slot) {
+    const size_t M = op->mx.size();
+    std::vector<char> diag(M, 0);
+    for (size_t k : diag_terms) diag[k] = 1;
+    std::vector<uint32_t> ord;
+    for (size_t k = 0; k < M; ++k)
+        if (!diag[k]) ord.push_back((uint32_t)k);
+    std::stable_sort(ord.begin(), ord.end(), [&](uint32_t a, uint32_t b) {
+        return (op->mx[a] >> 12) < (op->mx[b] >> 12);
+    });
+    StrSplit &sp = pl.str;
+    sp.nstr = (uint32_t)ord.size();
+    // states of 2^19 amplitudes and more fill the SMs with whole tiles: two
+    // partner tiles per block halve the ring's bookkeeping.  Below, tiles are
+    // split over clusters and a block holds at most a 32nd of the strings, so
+    // that parts balance
+    sp.tpb = op->n >= kStrPairN ? 2 : 1;
+    const uint32_t cap =
+        sp.tpb > 1 ? kStrEntCap
+                   : std::min(kStrEntCap, std::max(16u, (sp.nstr + 31u) / 32u));
+    std::vector<uint4> ent, blk;
+    std::vector<uint32_t> mem;  // entry -> merged string (0xffffffff: header)
+    auto open = [&](uint64_t hi, bool dg) {
+        blk.push_back(make_uint4((uint32_t)hi, 0xffffffffu, (uint32_t)ent.size(), 0));
+        ent.push_back(make_uint4(0, dg ? 1u : 0u, 0, 0));
+        mem.push_back(0xffffffffu);
+    };
+    bool has_diag = !diag_terms.empty();
+    if (has_diag && (ord.empty() || (op->mx[ord[0]] >> 12) != 0)) {
+        open(0, true);
+        has_diag = false;
+    }
+    for (size_t i = 0; i < ord.size(); ++i) {
+        const uint64_t x = op->mx[ord[i]], z = op->mz[ord[i]], h = x >> 12;
+        if (i == 0 || (op->mx[ord[i - 1]] >> 12) != h || blk.back().w >= cap) {
+            // a tile's strings stay together where they fit a block
+            size_t j = i;
+            while (j < ord.size() && (op->mx[ord[j]] >> 12) == h && j - i < cap) ++j;
+            if (sp.tpb > 1 && !blk.empty() && blk.back().y == 0xffffffffu &&
+                blk.back().x != (uint32_t)h && blk.back().w + (j - i) <= cap) {
+                blk.back().y = (uint32_t)h;
+            } else {
+                open(h, has_diag && h == 0);
+                if (h == 0) has_diag = false;
+            }
+        }
+        uint4 &bl = blk.back();
+        ++bl.w;
+        ++ent[bl.z].x;
+        const uint32_t half = bl.x != (uint32_t)h ? 1u : 0u;
+        const uint32_t w = (uint32_t)(x & 1u) | ((uint32_t)(x >> 1) & 511u) << 4 |
+                           ((uint32_t)(x >> 10) & 3u) << 13 | half << 15 | (uint32_t)(z & 1u) << 16 |
+                           ((uint32_t)(z >> 10) & 3u) << 17 | (uint32_t)(z >> 32) << 24;
+        const float fr = (float)c[ord[i]].re, fi = (float)c[ord[i]].im;
+        uint32_t br, bi;
+        memcpy(&br, &fr, 4);
+        memcpy(&bi, &fi, 4);
+        ent.push_back(make_uint4(w, (uint32_t)z & ~0xc01u, br, bi));
+        mem.push_back(ord[i]);
+    }
+    // a block costs about two strings beside its own
+    std::vector<uint64_t> upto(blk.size() + 1, 0);
+    for (size_t j = 0; j < blk.size(); ++j) upto[j + 1] = upto[j] + 2 + blk[j].w;
+    for (uint32_t k = 1; k <= kStrMaxSplit; ++k) {
+        uint32_t *part = sp.part[k - 1];
+        uint32_t j = 0;
+        part[0] = 0;
+        for (uint32_t r = 1; r <= k; ++r) {
+            const uint64_t end = upto.back() * r / k;
+            // the boundary nearest to the r-th share
+            while (j < blk.size() && upto[j + 1] + upto[j] <= 2 * end) ++j;
+            if (r == k) j = (uint32_t)blk.size();
+            part[r] = j;
+        }
+    }
+    sp.nblk = (uint32_t)blk.size();
+    QR_CUDA(pl.ent.upload(ent), "upload string entries");
+    QR_CUDA(pl.sblk.upload(blk), "upload string blocks");
+    for (size_t i = 0; i < mem.size(); ++i)
+        if (mem[i] != 0xffffffffu)
+            add_slot((uint64_t)pl.ent.p + i * sizeof(uint4) + 8, &mem[i], nullptr, 1, 0, 0);
+    return QR_OK;
+}
+
 int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     Plan &pl = tile_bits < 0 ? op->plans[dtype][adjoint] : op->bplans[tile_bits];
     if (pl.built) return QR_OK;
@@ -479,6 +572,14 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
         }
     }
     pl.has_diag = !diag_terms.empty();
+    // One entry per string where an x group holds about one: a string costs
+    // 0.6 of a sub-group of the per-tile table kernel (n = 20, 2,000 random
+    // strings: 735 against 1,231 us) and, at up to 512 sub-groups, the paired
+    // kernel's advantage on several strings per group meets it at a third more
+    // strings than sub-groups (chain n = 22, 64 strings in 47: 111 against 109).
+    const size_t nstr = M - diag_terms.size();
+    const double most = (subs.size() <= (size_t)kTabCap ? 1.3 : 1.6) * (double)subs.size();
+    pl.strings = f32 && tile_bits < 0 && n >= 12 && nstr > 0 && (double)nstr <= most;
     // order: partner tile ascending, then (c64c) run key zm with fat last
     std::vector<size_t> ord(subs.size());
     for (size_t i = 0; i < ord.size(); ++i) ord[i] = i;
@@ -787,6 +888,10 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
         QR_CUDA(pl.run_key.upload(rkey), "upload run keys");
         pl.nruns = (uint32_t)rkey.size();
         pl.nsub = (uint32_t)ord.size();
+    }
+    if (pl.strings) {
+        const int rc = build_strings(op, pl, c, diag_terms, add_slot);
+        if (rc) return rc;
     }
     if (!f32) {  // the complex128 kernel's group descriptors, tables, term lists
         if (descs.empty()) descs.push_back(GroupDesc{});  // keep a valid pointer
@@ -1144,9 +1249,11 @@ int qr_csr_build(qr_op *op, uint64_t *indptr, uint64_t *indices, double *data, i
     return check_kernel_error(op);
 }
 
+// call_states: states of the caller's whole call, of which these nstates are
+// a part (the same work split, and so the same bits, for each of them)
 static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *psi, void *y,
-                      int32_t nstates, int32_t adjoint, void *stream, const void *v,
-                      const double *alpha, const double *beta) {
+                      int32_t nstates, int32_t call_states, int32_t adjoint, void *stream,
+                      const void *v, const double *alpha, const double *beta) {
     if (!op || !psi || !y) return fail(QR_EINVAL, "%s: null argument", name);
     if (dtype != QR_C128 && dtype != QR_C64C)
         return fail(QR_EINVAL, "%s: dtype must be QR_C128 or QR_C64C", name);
@@ -1203,6 +1310,8 @@ static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *ps
     a.chunks = pl.chunks.as<uint4>();
     a.nchunks = pl.nchunks;
     a.npairs = pl.npairs;
+    a.ent = pl.ent.as<uint4>();
+    a.sblk = pl.sblk.as<uint4>();
     a.wait_ns = op->test_wait_ns ? op->test_wait_ns : kDefaultWaitNs;
     a.withhold = op->test_withhold;
     a.wide = op->test_wide;
@@ -1218,22 +1327,26 @@ static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *ps
         QR_CUDA(cudaMemsetAsync(y, 0, bytes, static_cast<cudaStream_t>(stream)), "zero y");
         return QR_OK;
     }
-    QR_CUDA(launch_apply(dtype, a, pl.amps, pl.threads, op->nsm,
-                         static_cast<cudaStream_t>(stream)),
-            "apply launch");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (pl.strings)
+        QR_CUDA(launch_c64c_strings(a, pl.str, (uint64_t)call_states * a.ntiles, op->nsm, st),
+                "apply launch");
+    else
+        QR_CUDA(launch_apply(dtype, a, pl.amps, pl.threads, op->nsm, st), "apply launch");
     return QR_OK;
 }
 
 int qr_apply(qr_op *op, int32_t dtype, const void *psi, void *y, int32_t nstates, int32_t adjoint,
              void *stream) {
-    return apply_impl("qr_apply", op, dtype, psi, y, nstates, adjoint, stream, nullptr, nullptr,
-                      nullptr);
+    return apply_impl("qr_apply", op, dtype, psi, y, nstates, nstates, adjoint, stream, nullptr,
+                      nullptr, nullptr);
 }
 
 int qr_apply_axpby(qr_op *op, int32_t dtype, const double *alpha, const void *psi,
                    const double *beta, const void *v, void *y, int32_t nstates, void *stream) {
     if (!alpha || !beta || !v) return fail(QR_EINVAL, "qr_apply_axpby: null argument");
-    return apply_impl("qr_apply_axpby", op, dtype, psi, y, nstates, 0, stream, v, alpha, beta);
+    return apply_impl("qr_apply_axpby", op, dtype, psi, y, nstates, nstates, 0, stream, v, alpha,
+                      beta);
 }
 
 int qr_apply_host(qr_op *op, int32_t dtype, const void *psi_host, void *y_host, int32_t nstates,
@@ -1279,7 +1392,8 @@ int qr_apply_host(qr_op *op, int32_t dtype, const void *psi_host, void *y_host, 
                     "copy psi to device");
             QR_CUDA(cudaEventRecord(op->cev, op->cstream), "record copy");
             QR_CUDA(cudaStreamWaitEvent(op->hstream, op->cev, 0), "order apply after copy");
-            rc = qr_apply(op, dtype, in + st * b1, out + st * b1, 1, adjoint, op->hstream);
+            rc = apply_impl("qr_apply_host", op, dtype, in + st * b1, out + st * b1, 1, nstates,
+                            adjoint, op->hstream, nullptr, nullptr, nullptr);
             if (rc) return rc;
             if (!y_dev)
                 QR_CUDA(cudaMemcpyAsync(yb + st * b1, out + st * b1, b1, cudaMemcpyDeviceToHost,
@@ -1735,7 +1849,7 @@ int capture_graph(qr_batch *bt, cudaGraph_t *graph) {
     for (size_t i = 0; i < bt->ops.size() && e == cudaSuccess && !rc; ++i) {
         if (bt->sel[i]) continue;
         rc = apply_impl("qr_batch_apply", bt->ops[i], QR_C64C, bt->cur_psi[i], bt->cur_y[i],
-                        bt->nstates[i], 0, bt->fork[first + (k++ % nbr)], nullptr, nullptr,
+                        bt->nstates[i], bt->nstates[i], 0, bt->fork[first + (k++ % nbr)], nullptr, nullptr,
                         nullptr);
     }
     for (int f = 0; f < qr_batch::kForks && e == cudaSuccess; ++f) {
