@@ -21,6 +21,7 @@
 // classes) -- the same additions in the same order as make_row, hence the
 // same bits -- and the kernel reads the row's class from that table.
 #include "qr_common.cuh"
+#include "qr_device.cuh"
 
 namespace qr {
 
@@ -543,12 +544,56 @@ cudaError_t launch_csr_fill(const CsrArgs &a, int nsm, cudaStream_t st) {
     return launch_csr_fold(b, nsm, st);
 }
 
-// y = A v, complex128.  S lanes per row, U entries per lane per step with
-// the step's tail predicated, so that a row of up to S * U entries costs one
-// round of dependent loads (index, then the gathered v); the lanes' partial
-// sums meet in a butterfly over the S lanes.  The GB300's FP64 rate is the
-// bound: a step whose S * U slots match the row length wastes no DFMA slot.
-// Replaces spmat_dot_densevec (qrusty/src/accel.rs:338-370).
+// y = A v, complex128.  Replaces spmat_dot_densevec (qrusty/src/accel.rs:338-370).
+// S lanes per row, U entries per lane in flight with the step's tail
+// predicated; the lanes' sums meet in a butterfly.  What bounds it: the
+// matrix, read once (24 bytes per entry: 78 % of the measured HBM copy rate
+// on the chains n = 20 and 22), with the FP64 pipe next (two multiply-adds
+// per real entry, four lanes' butterfly: 0.7 of the time).  Hence one
+// accumulator per part and few lanes per row, and 4 CTAs of 256 threads per
+// SM (64 registers) rather than deeper steps: chain n = 22, 44 entries a row,
+// steps of 2 / 3 / 4 / 5 / 6 entries 1,090 / 1,030 / 979 / 890 / 839 us (all
+// four multiply-adds, 11 entries in flight: 1,436).
+// Partial sum of row [j0, j1) over this lane's entries.
+template <int S, int U>
+__device__ __forceinline__ double2 spmv_lane(uint64_t j0, uint64_t j1, uint64_t ncols,
+                                             const uint64_t *__restrict__ indices,
+                                             const double2 *__restrict__ data,
+                                             const double2 *__restrict__ v) {
+    double sr = 0.0, si = 0.0;
+    for (uint64_t j = j0 + (threadIdx.x & (S - 1)); j < j1; j += (uint64_t)U * S) {
+        uint64_t c[U];
+        double2 d[U], x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {  // the matrix streams once: evict-first loads
+            const bool ok = j + (uint64_t)u * S < j1;
+            c[u] = ok ? __ldcs(indices + j + u * S) : ncols;
+            d[u] = ok ? __ldcs(data + j + u * S) : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            x[u] = c[u] < ncols ? __ldg(v + c[u]) : make_double2(0.0, 0.0);
+        // real (or imaginary) entries take 2 of the 4 multiply-adds, where the
+        // gathered value is not infinite or NaN
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (c[u] >= ncols) continue;  // out-of-range columns (and the tail) are skipped
+            const bool fin = max(exp_bits(x[u].x), exp_bits(x[u].y)) != 0x7ff00000u;
+            if (fin && mag_bits(d[u].y) == 0) {
+                sr = fma(d[u].x, x[u].x, sr);
+                si = fma(d[u].x, x[u].y, si);
+            } else if (fin && mag_bits(d[u].x) == 0) {
+                sr = fma(-d[u].y, x[u].y, sr);
+                si = fma(d[u].y, x[u].x, si);
+            } else {
+                sr = fma(d[u].x, x[u].x, fma(-d[u].y, x[u].y, sr));
+                si = fma(d[u].x, x[u].y, fma(d[u].y, x[u].x, si));
+            }
+        }
+    }
+    return make_double2(sr, si);
+}
+
 template <int S, int U>
 __device__ __forceinline__ void spmv_rows(uint64_t nrows, uint64_t ncols,
                                           const uint64_t *__restrict__ indptr,
@@ -559,62 +604,36 @@ __device__ __forceinline__ void spmv_rows(uint64_t nrows, uint64_t ncols,
     const uint64_t groups = (uint64_t)gridDim.x * (blockDim.x / S);
     for (uint64_t r = blockIdx.x * (uint64_t)(blockDim.x / S) + (threadIdx.x / S); r < nrows;
          r += groups) {
-        const uint64_t j0 = indptr[r], j1 = indptr[r + 1];
-        double sr = 0.0, si = 0.0, tr = 0.0, ti = 0.0;
-        for (uint64_t j = j0 + sl; j < j1; j += (uint64_t)U * S) {
-            uint64_t c[U];
-            double2 d[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {  // the matrix streams once: evict-first loads
-                const bool ok = j + (uint64_t)u * S < j1;
-                c[u] = ok ? __ldcs(indices + j + u * S) : ncols;
-                d[u] = ok ? __ldcs(data + j + u * S) : make_double2(0.0, 0.0);
-            }
-            double2 x[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                x[u] = c[u] < ncols ? __ldg(v + c[u]) : make_double2(0.0, 0.0);
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                if (c[u] >= ncols) continue;  // out-of-range columns (and the tail) are skipped
-                double &ar = (u & 1) ? tr : sr, &ai = (u & 1) ? ti : si;
-                ar = fma(d[u].x, x[u].x, fma(-d[u].y, x[u].y, ar));
-                ai = fma(d[u].x, x[u].y, fma(d[u].y, x[u].x, ai));
-            }
-        }
-        sr += tr;
-        si += ti;
+        double2 q = spmv_lane<S, U>(indptr[r], indptr[r + 1], ncols, indices, data, v);
+        const uint32_t mask = ((1u << S) - 1u) << (threadIdx.x & 31u & ~(S - 1u));
 #pragma unroll
         for (int o = S / 2; o > 0; o >>= 1) {
-            sr += __shfl_xor_sync(0xffffffffu, sr, o, S);
-            si += __shfl_xor_sync(0xffffffffu, si, o, S);
+            q.x += __shfl_xor_sync(mask, q.x, o, S);
+            q.y += __shfl_xor_sync(mask, q.y, o, S);
         }
-        if (sl == 0) y[r] = make_double2(sr, si);
+        if (sl == 0) y[r] = q;
     }
 }
 
-constexpr int kSpmvLanes = 4;   // lanes per row
-constexpr int kSpmvMaxStep = 16;  // entries per lane per step, at most
+constexpr int kSpmvMaxStep = 6;  // entries per lane in flight, at most
 
-// The step depth U is chosen from the first row's length (every row of a
-// Pauli-sum CSR holds G entries; any CSR is handled at any depth).
-__global__ void __launch_bounds__(256) csr_spmv_kernel(uint64_t nrows, uint64_t ncols,
-                                                       const uint64_t *__restrict__ indptr,
-                                                       const uint64_t *__restrict__ indices,
-                                                       const double2 *__restrict__ data,
-                                                       const double2 *__restrict__ v,
-                                                       double2 *__restrict__ y) {
-    constexpr int S = kSpmvLanes;
-    const uint64_t len0 = indptr[1] - indptr[0];
-    const uint64_t want = (len0 + S - 1) / S;
-    const int u = want < 1 ? 1 : (want > (uint64_t)kSpmvMaxStep ? kSpmvMaxStep : (int)want);
+// The step depth is chosen from the first row's length, so that equal steps
+// cover it (every row of a Pauli-sum CSR holds G entries; any CSR is handled
+// at any depth).
+template <int S>
+__global__ void __launch_bounds__(256, 4) csr_spmv_kernel(uint64_t nrows, uint64_t ncols,
+                                                          const uint64_t *__restrict__ indptr,
+                                                          const uint64_t *__restrict__ indices,
+                                                          const double2 *__restrict__ data,
+                                                          const double2 *__restrict__ v,
+                                                          double2 *__restrict__ y) {
+    const uint64_t want = (indptr[1] - indptr[0] + S - 1) / S;
+    const uint64_t steps = (want + kSpmvMaxStep - 1) / kSpmvMaxStep;
+    const int u = want < 1 ? 1 : (int)((want + steps - 1) / steps);
 #define QR_SPMV_CASE(k) \
     case k: spmv_rows<S, k>(nrows, ncols, indptr, indices, data, v, y); break;
     switch (u) {
-        QR_SPMV_CASE(1) QR_SPMV_CASE(2) QR_SPMV_CASE(3) QR_SPMV_CASE(4)
-        QR_SPMV_CASE(5) QR_SPMV_CASE(6) QR_SPMV_CASE(7) QR_SPMV_CASE(8)
-        QR_SPMV_CASE(9) QR_SPMV_CASE(10) QR_SPMV_CASE(11) QR_SPMV_CASE(12)
-        QR_SPMV_CASE(13) QR_SPMV_CASE(14) QR_SPMV_CASE(15)
+        QR_SPMV_CASE(1) QR_SPMV_CASE(2) QR_SPMV_CASE(3) QR_SPMV_CASE(4) QR_SPMV_CASE(5)
         default: spmv_rows<S, kSpmvMaxStep>(nrows, ncols, indptr, indices, data, v, y); break;
     }
 #undef QR_SPMV_CASE
@@ -624,14 +643,20 @@ cudaError_t launch_csr_spmv(uint64_t nrows, uint64_t ncols, const uint64_t *indp
                             const uint64_t *indices, const double *data, const double *v,
                             double *y, int nsm, cudaStream_t st) {
     if (nrows == 0) return cudaSuccess;
-    // no host read of nnz or row lengths: the call stays asynchronous
-    const uint64_t rows_per_block = 256 / kSpmvLanes;
+    // no host read of nnz or row lengths: the call stays asynchronous.
+    // Sixteen lanes per row while the rows are too few to fill the SMs (2^12
+    // rows of 176 entries: 14.5 us against 20.8 with four); four from 2^14
+    // rows on, where a wider butterfly's additions cost more than it brings
+    // (2^14 rows of 92: 26.8 against 29.0; 2^20 of 40: 188 against 439)
+    const int lanes = nrows < (1ull << 14) ? 16 : 4;
+    const uint64_t rows_per_block = 256 / (uint64_t)lanes;
     uint64_t g = (nrows + rows_per_block - 1) / rows_per_block;
     if (g > (uint64_t)nsm * 16) g = (uint64_t)nsm * 16;
-    csr_spmv_kernel<<<(unsigned)g, 256, 0, st>>>(nrows, ncols, indptr, indices,
-                                                 reinterpret_cast<const double2 *>(data),
-                                                 reinterpret_cast<const double2 *>(v),
-                                                 reinterpret_cast<double2 *>(y));
+    auto kern = lanes == 16 ? csr_spmv_kernel<16> : csr_spmv_kernel<4>;
+    kern<<<(unsigned)g, 256, 0, st>>>(nrows, ncols, indptr, indices,
+                                      reinterpret_cast<const double2 *>(data),
+                                      reinterpret_cast<const double2 *>(v),
+                                      reinterpret_cast<double2 *>(y));
     count_launch();
     return cudaGetLastError();
 }
