@@ -17,11 +17,18 @@
 //   a / b = ((ar br + ai bi) / (br^2 + bi^2), (ai br - ar bi) / (br^2 + bi^2))
 // complex64 runs the same sequence in FP32 with the scalars rounded to float.
 //
-// All element-wise kernels are HBM-bound streams: grid-stride over 16-byte
+// The complex128 forms are bound by the FP64 pipe (2 operations per SM and
+// cycle): real scalars and real pivots, the rule for a Hermitian operator,
+// leave out the products of their zero part, and precond2 calls hypot only
+// near tol (2^20 elements: axpby with real scalars 34 -> 16 us, precond2 with
+// a real diagonal 92 -> 54, most of it the two divisions).
+//
+// All element-wise kernels are streams: grid-stride over 16-byte
 // elements (one complex128 or two complex64), four elements in flight per
 // thread, grid = 8 CTAs of 256 threads per SM.
 #include "../../include/qrusty_gpu.h"
 #include "qr_common.cuh"
+#include "qr_device.cuh"
 
 namespace qr {
 
@@ -55,6 +62,28 @@ template <> struct C2<float> {
     static __device__ __forceinline__ float norm(float a, float b) { return hypotf(a, b); }
 };
 
+__device__ __forceinline__ bool finite2(double2 v) {
+    return max(exp_bits(v.x), exp_bits(v.y)) != 0x7ff00000u;
+}
+__device__ __forceinline__ uint64_t abs_bits(double d) {
+    return (uint64_t)__double_as_longlong(d) & 0x7fffffffffffffffull;
+}
+
+// What the host knows of a scalar: general, real (im = +-0), or +1.  The
+// product of a real scalar's zero part with a finite x is +-0, which changes
+// no nonzero result; zero products and infinite or NaN operands take the full
+// form.
+enum ScalarKind { kGeneral = 0, kReal = 1, kOne = 2 };
+
+template <int K>
+__device__ __forceinline__ double2 mul_real(double ar, double2 x) {
+    return K == kOne ? x : make_double2(__dmul_rn(ar, x.x), __dmul_rn(ar, x.y));
+}
+// every part nonzero, x finite: the full product's value
+__device__ __forceinline__ bool plain(double2 u, double2 x) {
+    return finite2(x) && mag_bits(u.x) != 0 && mag_bits(u.y) != 0;
+}
+
 template <typename R>
 __device__ __forceinline__ typename C2<R>::T cmul(R ar, R ai, typename C2<R>::T x) {
     using O = C2<R>;
@@ -64,9 +93,22 @@ __device__ __forceinline__ typename C2<R>::T cmul(R ar, R ai, typename C2<R>::T 
     return r;
 }
 
-template <typename R, int OP>
+template <typename R, int OP, int KA = kGeneral, int KB = kGeneral>
 __device__ __forceinline__ typename C2<R>::T vec_elem(typename C2<R>::T x, typename C2<R>::T y,
                                                       R ar, R ai, R br, R bi, R tol) {
+    if constexpr (sizeof(R) == 8 && KA != kGeneral && OP == kAx) {
+        const double2 u = mul_real<KA>(ar, x);
+        if (plain(u, x)) return u;
+    }
+    if constexpr (sizeof(R) == 8 && KA != kGeneral && OP == kAxpy) {
+        const double2 u = mul_real<KA>(ar, x);
+        if (plain(u, x)) return make_double2(__dadd_rn(u.x, y.x), __dadd_rn(u.y, y.y));
+    }
+    if constexpr (sizeof(R) == 8 && KA != kGeneral && KB != kGeneral && OP == kAxpby) {
+        const double2 u = mul_real<KA>(ar, x), v = mul_real<KB>(br, y);
+        if (plain(u, x) && plain(v, y))
+            return make_double2(__dadd_rn(u.x, v.x), __dadd_rn(u.y, v.y));
+    }
     using O = C2<R>;
     typename C2<R>::T r;
     if (OP == kAx) return cmul<R>(ar, ai, x);
@@ -84,9 +126,29 @@ __device__ __forceinline__ typename C2<R>::T vec_elem(typename C2<R>::T x, typen
     }
     // precond: x = diag, y = dx, (ar, ai) = e
     R dr = O::sub(x.x, ar), di = O::sub(x.y, ai);
-    if (O::norm(dr, di) < tol) {
+    bool small;
+    if constexpr (sizeof(R) == 8) {
+        // hypot only where it can be below tol: a part of 2 tol or more (as
+        // integers, a NaN being more) puts it above
+        const uint64_t far = abs_bits(2.0 * tol);
+        small = tol > 0.0 && abs_bits(dr) < far && abs_bits(di) < far && O::norm(dr, di) < tol;
+    } else {
+        small = O::norm(dr, di) < tol;
+    }
+    if (small) {
         dr = tol;
         di = R(0);
+    }
+    if constexpr (sizeof(R) == 8) {
+        // a real pivot and nonzero products: the same values without the
+        // products of its zero part (see ScalarKind)
+        if (mag_bits(di) == 0 && finite2(y)) {
+            const double2 u = make_double2(__dmul_rn(y.x, dr), __dmul_rn(y.y, dr));
+            if (mag_bits(u.x) != 0 && mag_bits(u.y) != 0) {
+                const double ns = __dmul_rn(dr, dr);
+                return make_double2(__ddiv_rn(u.x, ns), __ddiv_rn(u.y, ns));
+            }
+        }
     }
     const R ns = O::add(O::mul(dr, dr), O::mul(di, di));
     r.x = O::div(O::add(O::mul(y.x, dr), O::mul(y.y, di)), ns);
@@ -95,7 +157,7 @@ __device__ __forceinline__ typename C2<R>::T vec_elem(typename C2<R>::T x, typen
 }
 
 // complex128: one element per 16-byte word.
-template <int OP>
+template <int OP, int KA, int KB>
 __global__ void __launch_bounds__(kVecThreads) vec_c128(uint64_t len, const double2 *__restrict__ x,
                                                         const double2 *__restrict__ y,
                                                         double2 *z, VecScalars s) {
@@ -112,11 +174,11 @@ __global__ void __launch_bounds__(kVecThreads) vec_c128(uint64_t len, const doub
 #pragma unroll
         for (int u = 0; u < kVecUnroll; ++u)
             __stcs(z + i + u * stride,
-                   vec_elem<double, OP>(xv[u], yv[u], s.ar, s.ai, s.br, s.bi, s.tol));
+                   vec_elem<double, OP, KA, KB>(xv[u], yv[u], s.ar, s.ai, s.br, s.bi, s.tol));
     }
     for (; i < len; i += stride) {
         const double2 yv = Y ? y[i] : make_double2(0.0, 0.0);
-        z[i] = vec_elem<double, OP>(x[i], yv, s.ar, s.ai, s.br, s.bi, s.tol);
+        z[i] = vec_elem<double, OP, KA, KB>(x[i], yv, s.ar, s.ai, s.br, s.bi, s.tol);
     }
 }
 
@@ -160,12 +222,34 @@ unsigned vec_grid(uint64_t units, int nsm) {
     return (unsigned)(want < cap ? (want ? want : 1) : cap);
 }
 
+using VecC128 = void (*)(uint64_t, const double2 *, const double2 *, double2 *, VecScalars);
+
+int scalar_kind(double re, double im) {
+    return im != 0.0 || im != im ? kGeneral : (re == 1.0 ? kOne : kReal);
+}
+
+// ax / axpy by the kind of a, axpby by both (one general scalar: both are)
+template <int OP>
+VecC128 vec_c128_for(const VecScalars &s) {
+    const int ka = scalar_kind(s.ar, s.ai), kb = scalar_kind(s.br, s.bi);
+    if constexpr (OP == kPrecond) return vec_c128<OP, kGeneral, kGeneral>;
+    if constexpr (OP == kAx || OP == kAxpy)
+        return ka == kOne    ? vec_c128<OP, kOne, kGeneral>
+               : ka == kReal ? vec_c128<OP, kReal, kGeneral>
+                             : vec_c128<OP, kGeneral, kGeneral>;
+    if constexpr (OP == kAxpby) {
+        if (ka == kGeneral || kb == kGeneral) return vec_c128<OP, kGeneral, kGeneral>;
+        if (ka == kOne) return kb == kOne ? vec_c128<OP, kOne, kOne> : vec_c128<OP, kOne, kReal>;
+        return kb == kOne ? vec_c128<OP, kReal, kOne> : vec_c128<OP, kReal, kReal>;
+    }
+}
+
 template <int OP>
 cudaError_t launch_vec(int f32, uint64_t len, const void *x, const void *y, void *z,
                        const VecScalars &s, int nsm, cudaStream_t st) {
     if (len == 0) return cudaSuccess;
     if (!f32) {
-        vec_c128<OP><<<vec_grid(len, nsm), kVecThreads, 0, st>>>(
+        vec_c128_for<OP>(s)<<<vec_grid(len, nsm), kVecThreads, 0, st>>>(
             len, static_cast<const double2 *>(x), static_cast<const double2 *>(y),
             static_cast<double2 *>(z), s);
     } else {
