@@ -39,27 +39,12 @@ __device__ __forceinline__ void two_sum_into(float &hi, float &lo, float b) {
     hi = s;
     lo = __fadd_rn(lo, e);
 }
-// The same error-free transformation on (re, im) at once with packed FP32
-// operations; x - y is formed as fma(y, -1, x) (y * -1 is exact, so the one
-// rounding is that of x - y): bit-identical to two_sum_into per component.
-__device__ __forceinline__ float2 sub2_rn(float2 x, float2 y) {
-    return __ffma2_rn(y, make_float2(-1.f, -1.f), x);
-}
 __device__ __forceinline__ void two_sum_into2(float2 &hi, float2 &lo, float2 b) {
     const float2 s = __fadd2_rn(hi, b);
     const float2 bb = sub2_rn(s, hi);
     const float2 e = __fadd2_rn(sub2_rn(hi, sub2_rn(s, bb)), sub2_rn(b, bb));
     hi = s;
     lo = __fadd2_rn(lo, e);
-}
-// hi += b with the same error-free transformation; returns the error term
-// instead of accumulating it
-__device__ __forceinline__ float2 two_sum_carry2(float2 &hi, float2 b) {
-    const float2 s = __fadd2_rn(hi, b);
-    const float2 bb = sub2_rn(s, hi);
-    const float2 e = __fadd2_rn(sub2_rn(hi, sub2_rn(s, bb)), sub2_rn(b, bb));
-    hi = s;
-    return e;
 }
 // ---------------------------------------------------------------- c64c kernels
 // Compensated complex64 path.  A 4096-amplitude tile is held by T = 512
@@ -1139,9 +1124,8 @@ cudaError_t launch_batch_c64c(const BatchArgs &a, int nsm, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_apply(int dtype, const ApplyArgs &a, int amps, int threads, int nsm,
+cudaError_t launch_apply(const ApplyArgs &a, int amps, int threads, int nsm,
                          cudaStream_t st) {
-    if (dtype == 0) return launch_c128_rows(a, st);
     if (amps >= 2 && a.tb != kTb) return cudaErrorInvalidValue;
     switch (amps) {
         case 1: return launch_c64c<1>(a, threads, nsm, st);

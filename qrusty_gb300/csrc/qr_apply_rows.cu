@@ -1,11 +1,12 @@
-// qr_apply_rows.cu -- matrix-free Pauli-sum product y = H psi in complex128.
+// qr_apply_rows.cu -- matrix-free Pauli-sum product y = H psi over rows:
+// complex128, and complex64 calls of few rows.
 //
 //     y[r] = sum_g D_g(r) psi[r ^ x_g],
 //     D_g(r) = (-1)^popc(r & z0) T_g[pi(r)],  pi(r)_i = popc(r & beta_i) & 1
 // (row semantics of qrusty/src/accel.rs:171-210; replaces CSR build plus
 // spmat_dot_densevec, :338-370).
 //
-// What bounds it: the FP64 pipe, 2 multiply-adds per SM and cycle on GB300,
+// What bounds complex128: the FP64 pipe, 2 multiply-adds per SM and cycle on GB300,
 // one 64th of the FP32 rate.  Everything else is nearly free beside it, so
 // the design spends integer operations and L2 reads to save FP64 ones:
 //   * a factor that is real (or imaginary) throughout a warp takes 2
@@ -30,6 +31,14 @@
 //     multiply-adds: 1.15 of 1.26 TFLOP/s, the FP64 peak at 2,070 MHz)
 //   Jordan-Wigner n = 24, 4,000 terms 30,960 -> 29,940  (all factors complex:
 //     98 % of the FP64 peak)
+//
+// complex64 takes the same route while a call has few rows (one tile of 4,096
+// amplitudes is one SM's work in the tile kernels), with FP32 products, a
+// compensated fold every 16 groups of a slice (Kahan: the error opens the next
+// window) and the slices' compensated sums added in order.  Bound by latency
+// and, from 2^16 rows on, by L2 reads.  Measured (us, tiles -> rows): random
+// letters n = 10, 400 terms 28 -> 9.5; n = 11, 500 52 -> 12; Jordan-Wigner
+// n = 14, 1,400 25 -> 7.6; n = 16, 1,600 33 -> 18; chain n = 16 13 -> 6.
 #include <type_traits>
 
 #include "qr_common.cuh"
@@ -80,16 +89,30 @@ __device__ __forceinline__ void mac_rows(double2 (&acc)[AMPS], const double2 (&D
     }
 }
 
+template <int AMPS>
+__device__ __forceinline__ void mac_rows(float2 (&acc)[AMPS], const float2 (&D)[AMPS],
+                                         const float2 (&p)[AMPS], uint32_t, uint32_t, uint32_t) {
+#pragma unroll
+    for (int m = 0; m < AMPS; ++m) {
+        acc[m].x = fmaf(D[m].x, p[m].x, fmaf(-D[m].y, p[m].y, acc[m].x));
+        acc[m].y = fmaf(D[m].x, p[m].y, fmaf(D[m].y, p[m].x, acc[m].y));
+    }
+}
+
 // A CTA holds 2^lrw warps of 32 * AMPS consecutive rows (lane + 32 m) and as
 // many slices of them as its warps allow: slice s takes groups s, s + slices,
 // ... of each descriptor chunk.
-template <int AMPS, bool WIDE>
-__global__ void __launch_bounds__(kRowsThreads) apply_c128_rows(const ApplyArgs a, int lrw) {
+template <typename Real, int AMPS, bool WIDE>
+__global__ void __launch_bounds__(kRowsThreads) apply_rows(const ApplyArgs a, int lrw) {
     using W = typename std::conditional<WIDE, uint64_t, uint32_t>::type;
+    constexpr bool F32 = sizeof(Real) == 4;
+    using V = typename std::conditional<F32, float2, double2>::type;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(128) GroupDesc s_desc[kRowsStages][kRowsChunk];
     __shared__ uint64_t full[kRowsStages];
-    double2 *part = reinterpret_cast<double2 *>(smem_raw);
+    // a slice's sums: double2, or (sum, error) of the compensated float2
+    using P = typename std::conditional<F32, float4, double2>::type;
+    P *part = reinterpret_cast<P *>(smem_raw);
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t rw = warp & ((1u << lrw) - 1u), sl = warp >> lrw,
                    nsl = (blockDim.x >> 5) >> lrw;
@@ -97,10 +120,10 @@ __global__ void __launch_bounds__(kRowsThreads) apply_c128_rows(const ApplyArgs 
     const uint64_t per_state = (a.N + cta_rows - 1) / cta_rows;
     const uint64_t st = blockIdx.x / per_state;
     const uint64_t r0 = (blockIdx.x - st * per_state) * cta_rows + (uint64_t)rw * (32u * AMPS) + lane;
-    const double2 *psi = static_cast<const double2 *>(a.psi) + st * a.N;
-    const double2 *tables = static_cast<const double2 *>(a.tables);
+    const V *psi = static_cast<const V *>(a.psi) + st * a.N;
+    const V *tables = static_cast<const V *>(a.tables);
     const double2 *fat_c = static_cast<const double2 *>(a.fat_c);
-    const double2 *diag = static_cast<const double2 *>(a.diag);
+    const V *diag = static_cast<const V *>(a.diag);
     const W nmask = (W)(a.N - 1);
     const uint32_t nchunk = (a.ngroups + kRowsChunk - 1) / kRowsChunk;
 
@@ -122,27 +145,30 @@ __global__ void __launch_bounds__(kRowsThreads) apply_c128_rows(const ApplyArgs 
     }
 
     W row[AMPS];
-    double2 acc[AMPS];
+    V acc[AMPS], hi[AMPS];  // hi: complex64 only
 #pragma unroll
     for (int m = 0; m < AMPS; ++m) {
         row[m] = (W)(r0 + 32u * m) & nmask;  // n < 7: the spare lanes repeat rows
-        acc[m] = make_double2(0.0, 0.0);
+        acc[m].x = acc[m].y = hi[m].x = hi[m].y = Real(0);
     }
     if (diag != nullptr && sl == 0) {
-        double2 p[AMPS], D[AMPS];
+        V p[AMPS], D[AMPS];
         uint32_t re = 0, im = 0, big = 0;
 #pragma unroll
         for (int m = 0; m < AMPS; ++m) {
             D[m] = diag[row[m]];
             p[m] = psi[row[m]];
-            re |= mag_bits(D[m].x);
-            im |= mag_bits(D[m].y);
-            big = max(big, max(exp_bits(p[m].x), exp_bits(p[m].y)));
+            if constexpr (!F32) {
+                re |= mag_bits(D[m].x);
+                im |= mag_bits(D[m].y);
+                big = max(big, max(exp_bits(p[m].x), exp_bits(p[m].y)));
+            }
         }
         mac_rows<AMPS>(acc, D, p, re, im, big);
     }
     __syncthreads();
     bool ok = true;
+    uint32_t win = 0;
     for (uint32_t c = 0; c < nchunk; ++c) {
         const uint32_t s = c % kRowsStages;
         // an expired wait (the warp's vote) skips the chunk and ends the CTA
@@ -155,7 +181,7 @@ __global__ void __launch_bounds__(kRowsThreads) apply_c128_rows(const ApplyArgs 
             const GroupDesc &gd = s_desc[s][g];
             const W x = (W)gd.x, z0 = (W)gd.z0;
             const uint32_t d = gd.d, off = gd.off;
-            double2 p[AMPS], D[AMPS];
+            V p[AMPS], D[AMPS];
 #pragma unroll
             for (int m = 0; m < AMPS; ++m) p[m] = __ldg(psi + (row[m] ^ x));
             const uint32_t s0 = par(row[0] & z0), zb = (uint32_t)(z0 >> 5);
@@ -168,13 +194,16 @@ __global__ void __launch_bounds__(kRowsThreads) apply_c128_rows(const ApplyArgs 
                     any |= (uint32_t)(b >> 5);
                 }
                 if ((any & (AMPS - 1)) == 0) {
-                    const double2 e = __ldg(tables + off + u);
-                    re = mag_bits(e.x);
-                    im = mag_bits(e.y);
+                    const V e = __ldg(tables + off + u);
+                    if constexpr (!F32) {
+                        re = mag_bits(e.x);
+                        im = mag_bits(e.y);
+                    }
 #pragma unroll
                     for (int m = 0; m < AMPS; ++m) {
                         const uint32_t sg = s0 ^ par2(m, zb);
-                        D[m] = make_double2(flip(e.x, sg), flip(e.y, sg));
+                        D[m].x = flip(e.x, sg);
+                        D[m].y = flip(e.y, sg);
                     }
                 } else {
 #pragma unroll
@@ -182,14 +211,17 @@ __global__ void __launch_bounds__(kRowsThreads) apply_c128_rows(const ApplyArgs 
                         uint32_t um = u;
                         for (uint32_t i = 0; i < d; ++i)
                             um ^= par2(m, (uint32_t)((W)gd.beta[i] >> 5)) << i;
-                        const double2 e = __ldg(tables + off + um);
+                        const V e = __ldg(tables + off + um);
                         const uint32_t sg = s0 ^ par2(m, zb);
-                        D[m] = make_double2(flip(e.x, sg), flip(e.y, sg));
-                        re |= mag_bits(e.x);
-                        im |= mag_bits(e.y);
+                        D[m].x = flip(e.x, sg);
+                        D[m].y = flip(e.y, sg);
+                        if constexpr (!F32) {
+                            re |= mag_bits(e.x);
+                            im |= mag_bits(e.y);
+                        }
                     }
                 }
-            } else {
+            } else if constexpr (!F32) {  // complex64 plans have no rank above 4
                 const uint32_t cnt = gd.cnt;
 #pragma unroll
                 for (int m = 0; m < AMPS; ++m) D[m] = make_double2(0.0, 0.0);
@@ -209,10 +241,20 @@ __global__ void __launch_bounds__(kRowsThreads) apply_c128_rows(const ApplyArgs 
                     im |= mag_bits(D[m].y);
                 }
             }
+            if constexpr (!F32) {
 #pragma unroll
-            for (int m = 0; m < AMPS; ++m)
-                big = max(big, max(exp_bits(p[m].x), exp_bits(p[m].y)));
+                for (int m = 0; m < AMPS; ++m)
+                    big = max(big, max(exp_bits(p[m].x), exp_bits(p[m].y)));
+            }
             mac_rows<AMPS>(acc, D, p, re, im, big);
+        }
+        if constexpr (F32) {  // fold every 16 groups of the slice or more
+            win += ng;
+            if (win >= 16u * nsl) {
+                win = 0;
+#pragma unroll
+                for (int m = 0; m < AMPS; ++m) acc[m] = two_sum_carry2(hi[m], acc[m]);
+            }
         }
         // every warp is done with stage s
         if (__syncthreads_or(late)) {
@@ -234,67 +276,97 @@ __global__ void __launch_bounds__(kRowsThreads) apply_c128_rows(const ApplyArgs 
         }
         return;
     }
+    if constexpr (F32) {
+#pragma unroll
+        for (int m = 0; m < AMPS; ++m) acc[m] = two_sum_carry2(hi[m], acc[m]);
+    }
     if (nsl > 1) {
         // slice s > 0 hands its sums to slice 0, added there in slice order
         const uint32_t at = rw * (32u * AMPS) + lane;
         if (sl > 0) {
 #pragma unroll
-            for (int m = 0; m < AMPS; ++m)
-                part[(size_t)(sl - 1) * cta_rows + at + 32u * m] = acc[m];
+            for (int m = 0; m < AMPS; ++m) {
+                P &q = part[(size_t)(sl - 1) * cta_rows + at + 32u * m];
+                if constexpr (F32) q = make_float4(hi[m].x, hi[m].y, acc[m].x, acc[m].y);
+                else q = acc[m];
+            }
         }
         __syncthreads();
         if (sl > 0) return;
         for (uint32_t s = 0; s + 1 < nsl; ++s) {
 #pragma unroll
             for (int m = 0; m < AMPS; ++m) {
-                const double2 q = part[(size_t)s * cta_rows + at + 32u * m];
-                acc[m].x += q.x;
-                acc[m].y += q.y;
+                const P q = part[(size_t)s * cta_rows + at + 32u * m];
+                if constexpr (F32) {
+                    const float2 e = two_sum_carry2(hi[m], make_float2(q.x, q.y));
+                    acc[m] = __fadd2_rn(acc[m], __fadd2_rn(e, make_float2(q.z, q.w)));
+                } else {
+                    acc[m].x += q.x;
+                    acc[m].y += q.y;
+                }
             }
         }
     }
-    double2 *y = static_cast<double2 *>(a.y) + st * a.N;
-    const double2 *v = a.v ? static_cast<const double2 *>(a.v) + st * a.N : nullptr;
+    V *y = static_cast<V *>(a.y) + st * a.N;
+    const V *v = a.v ? static_cast<const V *>(a.v) + st * a.N : nullptr;
 #pragma unroll
     for (int m = 0; m < AMPS; ++m) {
         const uint64_t r = r0 + 32u * m;
         if (r >= a.N) continue;
-        double2 o = acc[m];
-        if (v) o = cx_axpby(a.ar, a.ai, o, a.br, a.bi, v[r]);
+        V o = acc[m];
+        if constexpr (F32) {
+            o = __fadd2_rn(hi[m], o);
+            if (v) o = cx_axpby((float)a.ar, (float)a.ai, o, (float)a.br, (float)a.bi, v[r]);
+        } else {
+            if (v) o = cx_axpby(a.ar, a.ai, o, a.br, a.bi, v[r]);
+        }
         y[r] = o;
     }
 }
 
-// Slices by the size of a state alone, so that a state's sums are formed in
-// the same order however many states are passed: 16 warps share a row while
-// the rows give too few warps to hide the L2 reads (n = 14, 500 random terms:
-// 16 / 8 / 4 slices 50 / 58 / 83 us; n = 16 Jordan-Wigner: 98 / 73 / 72;
-// n = 18: 4 slices 471 against 564 without), none from n = 21 on (chain
-// n = 22: 637 us against 722 with 4), where the sums through shared memory
-// cost more.  Rows per thread by the number of rows of all states: four share
-// the parity and table work (1 or 2 are bound by the instruction issue
-// instead of FP64: Jordan-Wigner n = 24, 49.9 ms against 29.9), so they are
-// given up only below 2^14 rows, where fewer than 128 CTAs would be left, or
-// where a state has fewer rows than a warp would hold.
-cudaError_t launch_c128_rows(const ApplyArgs &a, cudaStream_t st) {
-    const uint64_t rows = a.N * (uint64_t)a.nstates;
-    int amps = rows < (1ull << 13) ? 1 : (rows < (1ull << 14) ? 2 : 4);
+template <typename Real>
+static cudaError_t launch_split(const ApplyArgs &a, int amps, int nsl, cudaStream_t st) {
     while (amps > 1 && 32ull * amps > a.N) amps >>= 1;
-    const int nsl = a.n < 15 ? 16 : (a.n < 16 ? 8 : (a.n < 21 ? 4 : 1));
     const int lrw = nsl == 1 ? 2 : 0;
     const int warps = nsl << lrw;
     const uint64_t cta_rows = (32ull * amps) << lrw;
     const uint64_t per_state = (a.N + cta_rows - 1) / cta_rows;
     const uint64_t grid = per_state * (uint64_t)a.nstates;
     if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
-    const size_t smem = (size_t)(nsl - 1) * cta_rows * sizeof(double2);
+    const size_t smem = (size_t)(nsl - 1) * cta_rows * 16;
     const bool wide = a.n > 32 || a.wide;
-    auto kern = amps == 4 ? (wide ? apply_c128_rows<4, true> : apply_c128_rows<4, false>)
-                : amps == 2 ? (wide ? apply_c128_rows<2, true> : apply_c128_rows<2, false>)
-                            : (wide ? apply_c128_rows<1, true> : apply_c128_rows<1, false>);
+    auto kern = amps == 4   ? (wide ? apply_rows<Real, 4, true> : apply_rows<Real, 4, false>)
+                : amps == 2 ? (wide ? apply_rows<Real, 2, true> : apply_rows<Real, 2, false>)
+                            : (wide ? apply_rows<Real, 1, true> : apply_rows<Real, 1, false>);
     kern<<<(unsigned)grid, warps * 32, smem, st>>>(a, lrw);
     count_launch();
     return cudaGetLastError();
+}
+
+cudaError_t launch_rows(int dtype, const ApplyArgs &a, uint64_t call_rows, cudaStream_t st) {
+    if (dtype == 0) {
+        // Slices by the size of a state: 16 warps share a row while the rows
+        // give too few warps to hide the L2 reads (n = 14, 500 random terms:
+        // 16 / 8 / 4 slices 50 / 58 / 83 us; n = 16 Jordan-Wigner: 98 / 73 /
+        // 72; n = 18: 4 slices 471 against 564 without), none from n = 21 on
+        // (chain n = 22: 637 us against 722 with 4), where the sums through
+        // shared memory cost more.  Rows per thread by the number of rows of
+        // all states: four share the parity and table work (1 or 2 are bound
+        // by the instruction issue instead of FP64: Jordan-Wigner n = 24,
+        // 49.9 ms against 29.9), so they are given up only below 2^14 rows,
+        // where fewer than 128 CTAs would be left.
+        const uint64_t rows = a.N * (uint64_t)a.nstates;
+        return launch_split<double>(a, rows < (1ull << 13) ? 1 : (rows < (1ull << 14) ? 2 : 4),
+                                    a.n < 15 ? 16 : (a.n < 16 ? 8 : (a.n < 21 ? 4 : 1)), st);
+    }
+    // complex64: slices and rows per thread by the rows of the call (best of
+    // 1, 2, 4 rows x 1 ... 16 slices on random, chain and Jordan-Wigner
+    // operators of 8-18 qubits, one and four states)
+    if (call_rows <= (1ull << 13)) return launch_split<float>(a, 1, 16, st);
+    if (call_rows <= (1ull << 14)) return launch_split<float>(a, 2, 16, st);
+    if (call_rows <= (1ull << 15)) return launch_split<float>(a, 2, 8, st);
+    if (call_rows <= (1ull << 16)) return launch_split<float>(a, 2, 4, st);
+    return launch_split<float>(a, 4, 4, st);
 }
 
 }  // namespace qr

@@ -54,16 +54,6 @@ constexpr uint32_t kSFold = 24;  // strings per compensated fold, at least
 
 __device__ __forceinline__ float signed_f(uint32_t f, uint32_t s) { return __uint_as_float(f ^ s); }
 
-// hi += b error-free; returns the error
-__device__ __forceinline__ float2 fold(float2 &hi, float2 b) {
-    const float2 m1 = make_float2(-1.f, -1.f);
-    const float2 s = __fadd2_rn(hi, b);
-    const float2 bb = __ffma2_rn(hi, m1, s);
-    const float2 e = __fadd2_rn(__ffma2_rn(__ffma2_rn(bb, m1, s), m1, hi), __ffma2_rn(bb, m1, b));
-    hi = s;
-    return e;
-}
-
 // partner amplitudes of one string: p[j] holds register indices 2 j, 2 j + 1
 __device__ __forceinline__ void str_load(float4 (&p)[4], const unsigned char *sm, uint32_t base,
                                          uint32_t w) {
@@ -344,7 +334,7 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
                     if (win >= kSFold) {
                         win = 0;
 #pragma unroll
-                        for (int m = 0; m < 8; ++m) y[m] = fold(hi[m], y[m]);
+                        for (int m = 0; m < 8; ++m) y[m] = two_sum_carry2(hi[m], y[m]);
                     }
                 }
                 __syncwarp();
@@ -355,7 +345,7 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
                 }
             }
 #pragma unroll
-            for (int m = 0; m < 8; ++m) y[m] = fold(hi[m], y[m]);
+            for (int m = 0; m < 8; ++m) y[m] = two_sum_carry2(hi[m], y[m]);
 
             float2 *yo = static_cast<float2 *>(a.y) + st * a.N + (q << 12);
             const float2 *vo = a.v ? static_cast<const float2 *>(a.v) + st * a.N + (q << 12) : nullptr;
@@ -407,7 +397,7 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
                         float2 h = make_float2(v.x, v.y), l = make_float2(v.z, v.w);
                         for (uint32_t r = 1; r < ks; ++r) {
                             v = ld_cluster(mapa(at, r));
-                            const float2 e = fold(h, make_float2(v.x, v.y));
+                            const float2 e = two_sum_carry2(h, make_float2(v.x, v.y));
                             l = __fadd2_rn(l, __fadd2_rn(e, make_float2(v.z, v.w)));
                         }
                         store(m, h, l);

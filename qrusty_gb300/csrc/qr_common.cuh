@@ -12,7 +12,7 @@ namespace qr {
 constexpr int kDMax = 4;
 constexpr uint32_t kFat = 0xffffffffu;
 
-// One x-group of the complex128 apply plan.  All terms of the group share the x mask;
+// One x-group (or a piece of one) of a rows plan (qr_apply_rows.cu).  All terms of the group share the x mask;
 // their z masks are z0 ^ delta_k with delta_k in span(beta[0..d)).  The
 // group's diagonal factor at row r is
 //   D(r) = (-1)^popc(r & z0) * table[off + pi(r)],  pi(r)_i = popc(r & beta_i) & 1.
@@ -219,14 +219,15 @@ void count_launch(uint64_t k = 1);
 cudaError_t ensure_dyn_smem(const void *fn, size_t bytes);
 
 // Kernel launchers (qr_apply.cu / qr_csr.cu).
-cudaError_t launch_apply(int dtype, const ApplyArgs &a, int amps, int threads, int nsm,
+cudaError_t launch_apply(const ApplyArgs &a, int amps, int threads, int nsm,
                          cudaStream_t st);
 // qr_apply_strings.cu
 // call_items: output tiles of the caller's whole call
 cudaError_t launch_c64c_strings(const ApplyArgs &a, const StrSplit &sp, uint64_t call_items,
                                 int nsm, cudaStream_t st);
 // qr_apply_rows.cu
-cudaError_t launch_c128_rows(const ApplyArgs &a, cudaStream_t st);
+// call_rows: rows of the caller's whole call (complex64 splits by them)
+cudaError_t launch_rows(int dtype, const ApplyArgs &a, uint64_t call_rows, cudaStream_t st);
 cudaError_t launch_diag(int dtype, int n, int db, uint64_t ntiles, const uint64_t *bin_zlo,
                         const uint32_t *bin_off, uint32_t nbins, const uint64_t *tz,
                         const double *tc, void *out, cudaStream_t st);

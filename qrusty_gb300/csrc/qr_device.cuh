@@ -58,6 +58,24 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
 
 constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s per stage
 
+// Error-free addition on (re, im) at once with packed FP32
+// operations; x - y is formed as fma(y, -1, x) (y * -1 is exact, so the one
+// rounding is that of x - y).
+__device__ __forceinline__ float2 sub2_rn(float2 x, float2 y) {
+    return __ffma2_rn(y, make_float2(-1.f, -1.f), x);
+}
+// hi += b with an error-free transformation; returns the error term
+// instead of accumulating it
+__device__ __forceinline__ float2 two_sum_carry2(float2 &hi, float2 b) {
+    const float2 s = __fadd2_rn(hi, b);
+    const float2 bb = sub2_rn(s, hi);
+    const float2 e = __fadd2_rn(sub2_rn(hi, sub2_rn(s, bb)), sub2_rn(b, bb));
+    hi = s;
+    return e;
+}
+__device__ __forceinline__ float flip(float d, uint32_t s) {
+    return __uint_as_float(__float_as_uint(d) ^ (s << 31));
+}
 // d with the sign bit flipped when s == 1; bits that are zero iff d is +0 or
 // -0; the exponent bits (all ones: infinite or NaN).  Integer pipe.
 __device__ __forceinline__ double flip(double d, uint32_t s) {

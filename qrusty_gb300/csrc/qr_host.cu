@@ -123,6 +123,7 @@ struct Plan {
     // string plans: see ApplyArgs; str.part[k - 1] are the parts of a split in k
     bool strings = false;
     StrSplit str;
+    bool rows = false;  // qr_apply_rows.cu: complex128, and complex64 of few rows
     DevBuf ent, sblk;
     // what the plan was built for, and its coefficient program: the slots
     // that qr_op_set_coeffs_device recomputes on the device, with the
@@ -171,6 +172,7 @@ struct qr_op {
     DevBuf d_tg_x, d_tg_z, d_tg_perm, d_tg_bat;
     DevBuf expect_y;                    // H psi buffer of qr_expect
     Plan plans[2][2];  // [dtype][adjoint]
+    Plan rplans[2];    // complex64 over rows, for calls of few rows [adjoint]
     Plan bplans[13];   // compensated-c64 plans with an explicit tile width (batched launches)
     DevBuf d_err;
     // host-call staging
@@ -322,6 +324,113 @@ struct SubGroup {
     std::vector<uint8_t> coord;
 };
 
+// Group descriptors and tables of a rows plan (qr_apply_rows.cu), x groups by
+// x >> 12 in first-occurrence order.  A z span of rank > 4 is folded term by
+// term per row in complex128; in complex64 the group is split until every
+// piece has rank <= 4, so that all factors are FP64 sums rounded once.
+template <typename Real, typename AddSlot>
+int build_rows(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vector<uint64_t> &gxs,
+               const std::vector<std::vector<size_t>> &members, bool skip_zero,
+               AddSlot &&add_slot) {
+    constexpr bool f32 = sizeof(Real) == 4;
+    std::vector<size_t> ord(gxs.size());
+    for (size_t g = 0; g < ord.size(); ++g) ord[g] = g;
+    std::stable_sort(ord.begin(), ord.end(),
+                     [&](size_t a, size_t b) { return (gxs[a] >> 12) < (gxs[b] >> 12); });
+    std::vector<GroupDesc> descs;
+    std::vector<unsigned char> tab, fc;
+    std::vector<uint64_t> fz;
+    struct Piece {
+        std::vector<uint32_t> mem;
+        std::vector<uint8_t> coord;
+        bool fat;
+    };
+    std::vector<Piece> pieces;  // of descs, for the coefficient program
+    uint32_t ntab = 0;
+    auto masks = [&](const std::vector<size_t> &part) {
+        std::vector<uint64_t> zs;
+        for (size_t k : part) zs.push_back(op->mz[k]);
+        return zs;
+    };
+    auto push = [&](uint64_t x, const std::vector<size_t> &part, const Span &sp, bool fat) {
+        GroupDesc d;
+        memset(&d, 0, sizeof(d));
+        d.z0 = op->mz[part[0]];
+        d.x = x;
+        Piece pc;
+        pc.fat = fat;
+        for (size_t kk = 0; kk < part.size(); ++kk) {
+            pc.mem.push_back((uint32_t)part[kk]);
+            pc.coord.push_back(fat ? 0 : (uint8_t)sp.coord[kk]);
+        }
+        if (fat) {
+            d.d = kFat;
+            d.off = (uint32_t)fz.size();
+            d.cnt = (uint32_t)part.size();
+            for (size_t k : part) {
+                fz.push_back(op->mz[k]);
+                push_cplx<Real>(fc, c[k]);
+            }
+            pl.nfat++;
+        } else {
+            d.d = (uint32_t)sp.basis.size();
+            d.off = ntab;
+            for (size_t i = 0; i < sp.basis.size(); ++i) d.beta[i] = sp.basis[i];
+            for (uint32_t u = 0; u < 1u << d.d; ++u) {
+                cd acc{0.0, 0.0};
+                for (size_t kk = 0; kk < part.size(); ++kk) {
+                    const cd v = c[part[kk]];
+                    if (__builtin_popcountll(u & sp.coord[kk]) & 1) {
+                        acc.re -= v.re;
+                        acc.im -= v.im;
+                    } else {
+                        acc.re += v.re;
+                        acc.im += v.im;
+                    }
+                }
+                push_cplx<Real>(tab, acc);
+            }
+            ntab += 1u << d.d;
+        }
+        descs.push_back(d);
+        pieces.push_back(std::move(pc));
+    };
+    for (size_t g : ord) {
+        if (skip_zero && gxs[g] == 0) continue;
+        const std::vector<uint64_t> zs = masks(members[g]);
+        const Span sp = gf2_span(zs, kDMax);
+        if (!sp.overflow || !f32) {
+            push(gxs[g], members[g], sp, sp.overflow);
+            continue;
+        }
+        const Span full = gf2_span(zs, 64);
+        std::map<uint64_t, std::vector<size_t>> parts;
+        for (size_t kk = 0; kk < members[g].size(); ++kk)
+            parts[full.coord[kk] >> kDMax].push_back(members[g][kk]);
+        for (const auto &pt : parts) push(gxs[g], pt.second, gf2_span(masks(pt.second), kDMax), false);
+    }
+    pl.ngroups = descs.size();
+    if (descs.empty()) descs.push_back(GroupDesc{});  // keep a valid pointer
+    QR_CUDA(pl.groups.upload(descs), "upload groups");
+    QR_CUDA(pl.tables.upload(tab), "upload tables");
+    QR_CUDA(pl.fat_z.upload(fz), "upload fat z");
+    QR_CUDA(pl.fat_c.upload(fc), "upload fat c");
+    for (size_t i = 0; i < pieces.size(); ++i) {
+        const Piece &pc = pieces[i];
+        const GroupDesc &d = descs[i];
+        if (!pc.fat) {
+            if (pc.mem.size() > 0xffff) return fail(QR_EINVAL, "plan: group too large");
+            add_slot((uint64_t)pl.tables.p + (uint64_t)d.off * sizeof(Cplx<Real>), pc.mem.data(),
+                     pc.coord.data(), pc.mem.size(), d.d, f32 ? 0 : 1);
+        } else {
+            for (size_t kk = 0; kk < pc.mem.size(); ++kk)
+                add_slot((uint64_t)pl.fat_c.p + (uint64_t)(d.off + kk) * sizeof(Cplx<Real>),
+                         &pc.mem[kk], nullptr, 1, 0, 2);
+        }
+    }
+    return QR_OK;
+}
+
 // Entry lists of a string plan (qr_apply_strings.cu): the merged strings
 // outside the diagonal by partner tile, in blocks, and the parts of about
 // equal work that the CTAs of a cluster of 1 ... kStrMaxSplit take.
@@ -411,8 +520,10 @@ int build_strings(qr_op *op, Plan &pl, const std::vector<cd> &c,
     return QR_OK;
 }
 
-int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
-    Plan &pl = tile_bits < 0 ? op->plans[dtype][adjoint] : op->bplans[tile_bits];
+int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows = false) {
+    Plan &pl = tile_bits >= 0 ? op->bplans[tile_bits]
+               : rows && dtype == QR_C64C ? op->rplans[adjoint]
+                                          : op->plans[dtype][adjoint];
     if (pl.built) return QR_OK;
     {
         const int rc = sync_host_coeffs(op);
@@ -474,6 +585,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     // each x-group by its terms' z bits there.  The c128 kernel does not split.
     int abits = 0;
     while ((1 << abits) < pl.amps) ++abits;
+    pl.rows = !f32 || rows;
     const uint64_t mmask = f32 ? (((1ull << abits) - 1) << pl.tb) : 0;
     std::vector<size_t> diag_terms;
     std::vector<SubGroup> subs;
@@ -486,6 +598,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
                 continue;
             }
         }
+        if (pl.rows) continue;  // whole groups (build_rows)
         std::vector<uint64_t> pkeys;
         std::vector<std::vector<size_t>> parts;
         for (size_t k : members[g]) {
@@ -502,10 +615,6 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
         // z differences agree beyond the first two basis vectors)
         std::vector<std::vector<size_t>> pieces;
         for (const auto &part : parts) {
-            if (!f32) {
-                pieces.push_back(part);
-                continue;
-            }
             std::vector<uint64_t> zs;
             for (size_t k : part) zs.push_back(op->mz[k]);
             Span full = gf2_span(zs, 64);
@@ -579,7 +688,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     // strings than sub-groups (chain n = 22, 64 strings in 47: 111 against 109).
     const size_t nstr = M - diag_terms.size();
     const double most = (subs.size() <= (size_t)kTabCap ? 1.3 : 1.6) * (double)subs.size();
-    pl.strings = f32 && tile_bits < 0 && n >= 12 && nstr > 0 && (double)nstr <= most;
+    pl.strings = !pl.rows && tile_bits < 0 && n >= 12 && nstr > 0 && (double)nstr <= most;
     // order: partner tile ascending, then (c64c) run key zm with fat last
     std::vector<size_t> ord(subs.size());
     for (size_t i = 0; i < ord.size(); ++i) ord[i] = i;
@@ -763,40 +872,18 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
         pl.npairs = np;
     }
 
-    std::vector<unsigned char> tab, fc;
-    std::vector<uint64_t> fz;
-    uint32_t ntab = 0, nfat_terms = 0;
-    std::vector<GroupDesc> descs;           // c128 kernel
     pl.nfat = 0;
-    for (size_t i = 0; i < ord.size(); ++i) {
-        const SubGroup &sg = subs[ord[i]];
-        GroupDesc d;
-        memset(&d, 0, sizeof(d));
-        d.z0 = sg.z0;
-        d.x = (sg.hi << pl.b) | sg.lo;
-        d.d = sg.d;
-        for (int q = 0; q < kDMax; ++q) d.beta[q] = sg.beta[q];
-        if (sg.d != kFat) {
-            d.off = ntab;
-            for (const cd &v : sg.table) {
-                if (f32) push_cplx<float>(tab, v);
-                else push_cplx<double>(tab, v);
-            }
-            ntab += (uint32_t)sg.table.size();
-        } else {
-            d.off = nfat_terms;
-            d.cnt = (uint32_t)sg.fz.size();
-            for (size_t k = 0; k < sg.fz.size(); ++k) {
-                fz.push_back(sg.fz[k]);
-                if (f32) push_cplx<float>(fc, sg.fc[k]);
-                else push_cplx<double>(fc, sg.fc[k]);
-            }
-            nfat_terms += d.cnt;
-            pl.nfat++;
-        }
-        descs.push_back(d);
+    if (pl.rows) {
+        const int rc = f32 ? build_rows<float>(op, pl, c, gxs, members, pl.has_diag, add_slot)
+                           : build_rows<double>(op, pl, c, gxs, members, pl.has_diag, add_slot);
+        if (rc) return rc;
     }
-    if (f32) {
+    if (pl.strings) {
+        const int rc = build_strings(op, pl, c, diag_terms, add_slot);
+        if (rc) return rc;
+    }
+    pl.nsub = (uint32_t)ord.size();
+    if (!pl.rows && !pl.strings) {
         // per-tile-table kernel arrays
         std::vector<uint4> td;
         std::vector<TileDataC64> tdd;
@@ -887,33 +974,8 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
         QR_CUDA(pl.run_g0.upload(rg0), "upload runs");
         QR_CUDA(pl.run_key.upload(rkey), "upload run keys");
         pl.nruns = (uint32_t)rkey.size();
-        pl.nsub = (uint32_t)ord.size();
+        QR_CUDA(pl.blk_hi.upload(bhi), "upload blocks");
     }
-    if (pl.strings) {
-        const int rc = build_strings(op, pl, c, diag_terms, add_slot);
-        if (rc) return rc;
-    }
-    if (!f32) {  // the complex128 kernel's group descriptors, tables, term lists
-        if (descs.empty()) descs.push_back(GroupDesc{});  // keep a valid pointer
-        QR_CUDA(pl.groups.upload(descs), "upload groups");
-        QR_CUDA(pl.tables.upload(tab), "upload tables");
-        QR_CUDA(pl.fat_z.upload(fz), "upload fat z");
-        QR_CUDA(pl.fat_c.upload(fc), "upload fat c");
-        for (size_t i = 0; i < ord.size(); ++i) {
-            const SubGroup &sg = subs[ord[i]];
-            const GroupDesc &d = descs[i];
-            if (sg.d != kFat) {
-                if (sg.mem.size() > 0xffff) return fail(QR_EINVAL, "plan: group too large");
-                add_slot((uint64_t)pl.tables.p + (uint64_t)d.off * sizeof(Cplx<double>),
-                         sg.mem.data(), sg.coord.data(), sg.mem.size(), sg.d, 1);
-            } else {
-                for (size_t kk = 0; kk < sg.mem.size(); ++kk)
-                    add_slot((uint64_t)pl.fat_c.p + (uint64_t)(d.off + kk) * sizeof(Cplx<double>),
-                             &sg.mem[kk], nullptr, 1, 0, 2);
-            }
-        }
-    }
-    QR_CUDA(pl.blk_hi.upload(bhi), "upload blocks");
 
     if (pl.has_diag) {
         const int db = std::min(n, 12);
@@ -961,6 +1023,27 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     pl.nslots = cmem.empty() ? 0u : (uint32_t)slots.size();
     pl.built = true;
     return QR_OK;
+}
+
+// The plan that a call of this many states takes, built on first use.
+// complex64 runs over rows (qr_apply_rows.cu) while the call has few: a tile
+// kernel takes one SM per 4,096 rows.  Measured (us, tiles against rows),
+// 1,000 random strings, where a tile's strings are split over a cluster:
+// 2^12 rows 21 / 15 (600 strings), 2^13 23 / 18 (700), 2^14 27 / 24 and, from
+// four states, 21 / 18, 2^15 23 / 33; Jordan-Wigner 2^14 25 / 8, 2^16 33 / 18,
+// 2^17 36 / 33, 2^18 40 / 66; chain 2^17 13.4 / 8.8, 2^18 14.4 / 15.2.
+// Below 12 qubits a tile is smaller and costs 0.05-0.1 us per x group:
+// n = 11, 500 groups, 52 against 12 (one state), even at 2^15-2^16 rows.
+int apply_plan(qr_op *op, int dtype, int adjoint, int32_t call_states, Plan **out) {
+    bool rows = dtype == QR_C128;
+    if (!rows) {
+        const uint64_t r = op->N * (uint64_t)call_states;
+        const bool strings = op->n >= 12 && (double)op->M <= 1.3 * (double)op->Ga;
+        rows = r <= (strings ? 1ull << 13 : op->n >= 12 ? 1ull << 17 : 1ull << 15);
+    }
+    const int rc = build_plan(op, dtype, adjoint, -1, rows);
+    *out = rows && dtype == QR_C64C ? &op->rplans[adjoint] : &op->plans[dtype][adjoint];
+    return rc;
 }
 
 // bound of every mbarrier wait of the apply kernels
@@ -1277,9 +1360,10 @@ static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *ps
     }
     int rc = check_device(op);
     if (rc) return rc;
-    rc = build_plan(op, dtype, adjoint);
+    Plan *plan = nullptr;
+    rc = apply_plan(op, dtype, adjoint, call_states, &plan);
     if (rc) return rc;
-    const Plan &pl = op->plans[dtype][adjoint];
+    const Plan &pl = *plan;
     ApplyArgs a{};
     a.psi = psi;
     a.y = y;
@@ -1322,17 +1406,14 @@ static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *ps
         a.br = beta[0];
         a.bi = beta[1];
     }
-    if (pl.nblocks == 0 && !v) {
-        // operator without terms reachable here cannot happen (T >= 1); keep y defined
-        QR_CUDA(cudaMemsetAsync(y, 0, bytes, static_cast<cudaStream_t>(stream)), "zero y");
-        return QR_OK;
-    }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (pl.strings)
+    if (pl.rows)
+        QR_CUDA(launch_rows(dtype, a, (uint64_t)call_states * op->N, st), "apply launch");
+    else if (pl.strings)
         QR_CUDA(launch_c64c_strings(a, pl.str, (uint64_t)call_states * a.ntiles, op->nsm, st),
                 "apply launch");
     else
-        QR_CUDA(launch_apply(dtype, a, pl.amps, pl.threads, op->nsm, st), "apply launch");
+        QR_CUDA(launch_apply(a, pl.amps, pl.threads, op->nsm, st), "apply launch");
     return QR_OK;
 }
 
@@ -1525,6 +1606,7 @@ int qr_op_set_coeffs(qr_op *op, const double *coeff) {
     op->host_coef_stale = true;  // plans built below fetch the new merged sums
     for (int d = 0; d < 2; ++d)
         for (int j = 0; j < 2; ++j) op->plans[d][j].built = false;
+    for (Plan &rp : op->rplans) rp.built = false;
     // plans are rebuilt on next use into the buffers they already hold
     for (Plan &bp : op->bplans) bp.built = false;
     ++op->coef_gen;
@@ -1559,6 +1641,10 @@ int qr_op_set_coeffs_device(qr_op *op, const double *coeff, void *stream) {
             rc = refresh(op->plans[d][j]);
             if (rc) return rc;
         }
+    for (Plan &rp : op->rplans) {
+        rc = refresh(rp);
+        if (rc) return rc;
+    }
     for (Plan &bp : op->bplans) {
         rc = refresh(bp);
         if (rc) return rc;
@@ -1879,7 +1965,8 @@ int instantiate_mode(qr_batch *bt, int mode) {
         bt->sel[i] = mode == 0 ? 1 : (mode == 1 ? 0 : bt->small[i]);
     int rc = batch_build(bt, kBatchTileBits);
     for (size_t i = 0; i < bt->ops.size() && !rc; ++i)
-        if (!bt->sel[i]) rc = build_plan(bt->ops[i], QR_C64C, 0);
+        if (Plan *pl = nullptr; !bt->sel[i])
+            rc = apply_plan(bt->ops[i], QR_C64C, 0, bt->nstates[i], &pl);
     if (!rc) rc = capture_graph(bt, &bt->graph);
     if (rc) return rc;
     QR_CUDA(cudaGraphInstantiate(&bt->exec, bt->graph, 0), "graph instantiate");
