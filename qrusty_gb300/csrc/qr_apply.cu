@@ -1148,6 +1148,10 @@ __global__ void __launch_bounds__(256) diag_wht(int db, uint64_t ntiles, const u
     extern __shared__ __align__(128) unsigned char smem_raw[];
     double2 *W = reinterpret_cast<double2 *>(smem_raw);
     const uint32_t sz = 1u << db;
+    // real coefficients (the rule on Z strings): the imaginary half stays 0
+    bool im = false;
+    for (uint32_t k = threadIdx.x; k < bin_off[nbins]; k += blockDim.x) im |= !(tc[2 * k + 1] == 0.0);
+    im = __syncthreads_or(im);
     for (uint64_t q = blockIdx.x; q < ntiles; q += gridDim.x) {
         for (uint32_t i = threadIdx.x; i < sz; i += blockDim.x) W[i] = make_double2(0.0, 0.0);
         __syncthreads();
@@ -1155,15 +1159,10 @@ __global__ void __launch_bounds__(256) diag_wht(int db, uint64_t ntiles, const u
         for (uint32_t bi = threadIdx.x; bi < nbins; bi += blockDim.x) {
             double wr = 0.0, wi = 0.0;
             for (uint32_t k = bin_off[bi]; k < bin_off[bi + 1]; ++k) {
-                const bool neg = (__popcll(qhi & tz[k]) & 1) != 0;
-                const double cr = tc[2 * k], ci = tc[2 * k + 1];
-                if (k == bin_off[bi]) {
-                    wr = neg ? -cr : cr;
-                    wi = neg ? -ci : ci;
-                } else {
-                    wr = neg ? wr - cr : wr + cr;
-                    wi = neg ? wi - ci : wi + ci;
-                }
+                const uint32_t neg = (uint32_t)__popcll(qhi & tz[k]) & 1u;
+                const double cr = flip(tc[2 * k], neg), ci = flip(tc[2 * k + 1], neg);
+                wr = k == bin_off[bi] ? cr : wr + cr;
+                if (im) wi = k == bin_off[bi] ? ci : wi + ci;
             }
             W[bin_zlo[bi]] = make_double2(wr, wi);
         }
@@ -1174,8 +1173,13 @@ __global__ void __launch_bounds__(256) diag_wht(int db, uint64_t ntiles, const u
                 const uint32_t ia = ((i >> l) << (l + 1)) | (i & (h - 1));
                 const uint32_t ib = ia | h;
                 const double2 u = W[ia], v = W[ib];
-                W[ia] = make_double2(u.x + v.x, u.y + v.y);
-                W[ib] = make_double2(u.x - v.x, u.y - v.y);
+                if (im) {
+                    W[ia] = make_double2(u.x + v.x, u.y + v.y);
+                    W[ib] = make_double2(u.x - v.x, u.y - v.y);
+                } else {
+                    W[ia].x = u.x + v.x;
+                    W[ib].x = u.x - v.x;
+                }
             }
             __syncthreads();
         }

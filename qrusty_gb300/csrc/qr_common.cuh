@@ -337,20 +337,38 @@ cudaError_t launch_op_diag(uint64_t N, uint32_t nt, const uint64_t *tz, const do
 uint32_t vdot_blocks(uint64_t N, int nsm);
 cudaError_t launch_vdot(int dtype, uint64_t N, const void *a, const void *b, int nstates,
                         double2 *partial, uint32_t nblk, double2 *out, cudaStream_t st);
-cudaError_t launch_term_grad(int dtype, uint64_t N, int nstates, const uint64_t *sx,
-                             const uint64_t *sz, uint32_t nstr, const void *psi, const void *g,
-                             double2 *partial, uint32_t nchunk, uint64_t chunk, double2 *R,
-                             uint64_t T, const uint32_t *map, const uint8_t *phase, double2 *out,
-                             cudaStream_t st);
-// Tiled complex64 term gradients (n >= 12): strings sorted by partner tile
-// x >> 12 (sx, sz; perm = merged index of each), batches of <= 8 strings of
-// one partner tile as (first, count), largest first; partial holds nstr x
-// nchunk entries; counter: 8 bytes of device scratch (the work counter).
-cudaError_t launch_term_grad_tiles(uint64_t N, int nstates, const uint64_t *sx, const uint64_t *sz,
-                                   const uint32_t *perm, const uint2 *batches, uint32_t nbatch,
-                                   uint32_t nstr, const void *psi, const void *g,
-                                   double2 *partial, uint32_t nchunk, double2 *R, uint64_t T,
-                                   const uint32_t *map, const uint8_t *phase, double2 *out,
+// Term gradients.  Strings of x groups of kGradWhtMin or more go through a
+// Walsh-Hadamard transform per 256 rows (wht: batches of up to kGradWhtBatch
+// strings of one x), the others one by one (direct: by partner tile x >> 12 for
+// the tiled complex64 kernel, n >= 12).  perm: merged index of each; partial
+// sums: direct.count x direct.nchunk, then wht.count x wht.nchunk.
+constexpr uint32_t kGradWhtMin = 8, kGradWhtBatch = 256;
+struct GradBatch {
+    uint64_t x;
+    uint32_t first, count;
+};
+struct GradStrings {
+    const uint32_t *perm;
+    uint32_t count, nchunk;
+};
+struct GradPlanArgs {
+    GradStrings direct, wht;
+    const uint64_t *sx, *sz;  // direct strings
+    const uint2 *batches;     // tiled kernel: <= 8 strings of one partner tile (first, count)
+    uint32_t nbatch;
+    const uint64_t *wz;       // wht strings
+    const GradBatch *wbatches;
+    uint32_t nwbatch;
+};
+cudaError_t launch_term_grad(int dtype, uint64_t N, int nstates, const GradPlanArgs &p,
+                             const void *psi, const void *g, double2 *partial,
+                             const uint32_t *mm_off, const uint32_t *mm_terms,
+                             const uint8_t *phase, double2 *out, cudaStream_t st);
+// complex64, n >= 12.  counter: 8 bytes of device scratch (the work counter)
+cudaError_t launch_term_grad_tiles(uint64_t N, int nstates, const GradPlanArgs &p,
+                                   const void *psi, const void *g, double2 *partial,
+                                   const uint32_t *mm_off, const uint32_t *mm_terms,
+                                   const uint8_t *phase, double2 *out,
                                    unsigned long long *counter, int nsm, cudaStream_t st);
 
 }  // namespace qr

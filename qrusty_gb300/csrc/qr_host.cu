@@ -165,11 +165,10 @@ struct qr_op {
     bool csr_ready = false;
     uint32_t nfold = 0, nctab = 0;
     DevBuf d_tc, d_pmask, d_sig, d_grp, d_coord, d_ctab, d_fold, d_pbeta, d_ptab, d_fv;
-    // term-gradient batches (complex64, n >= 12): merged strings sorted by
-    // partner tile x >> 12, batches of <= 8 strings of one partner tile
+    // term-gradient strings (see GradPlanArgs), built on first use
     bool tg_ready = false;
-    uint32_t tg_nbatch = 0;
-    DevBuf d_tg_x, d_tg_z, d_tg_perm, d_tg_bat;
+    uint32_t tg_ndirect = 0, tg_nbatch = 0, tg_nwht = 0, tg_nwbatch = 0;
+    DevBuf d_tg_x, d_tg_z, d_tg_perm, d_tg_bat, d_tg_wz, d_tg_wperm, d_tg_wbat;
     DevBuf expect_y;                    // H psi buffer of qr_expect
     Plan plans[2][2];  // [dtype][adjoint]
     Plan rplans[2];    // complex64 over rows, for calls of few rows [adjoint]
@@ -978,7 +977,9 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
     }
 
     if (pl.has_diag) {
-        const int db = std::min(n, 12);
+        // tiles of 2^12 rows, smaller ones below 2^21 rows so that at least 512
+        // CTAs share the transforms (n = 15: 8 tiles took 38 us)
+        const int db = std::min(n, std::min(12, std::max(5, n - 9)));
         const uint64_t dmask = (1ull << db) - 1;
         std::vector<size_t> dt = diag_terms;
         std::stable_sort(dt.begin(), dt.end(), [&](size_t a, size_t b) {
@@ -1715,75 +1716,95 @@ int qr_term_grad(qr_op *op, int32_t dtype, const void *psi, const void *g, int32
     int rc = check_device(op);
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const uint32_t nstr = (uint32_t)op->M;
-    if (dtype == QR_C64C && op->n >= 12) {
-        if (!op->tg_ready) {
-            // strings by partner tile, input order kept within one; batches
-            // of <= 8 never span two partner tiles, largest first
-            std::vector<uint32_t> ord(nstr);
-            for (uint32_t i = 0; i < nstr; ++i) ord[i] = i;
-            std::stable_sort(ord.begin(), ord.end(), [&](uint32_t a, uint32_t b) {
-                return (op->mx[a] >> 12) < (op->mx[b] >> 12);
-            });
-            std::vector<uint64_t> sx(nstr), sz(nstr);
-            for (uint32_t i = 0; i < nstr; ++i) {
-                sx[i] = op->mx[ord[i]];
-                sz[i] = op->mz[ord[i]];
+    if (!op->tg_ready) {
+        // x groups of many strings to the transform, the others in order of
+        // partner tile, input order kept within one; batches of <= 8 never
+        // span two partner tiles, largest first
+        std::vector<uint32_t> ord, word;
+        std::vector<GradBatch> wb;
+        for (size_t g = 0; g < op->Ga; ++g) {
+            const uint32_t a0 = op->ag_off[g], a1 = op->ag_off[g + 1];
+            if (a1 - a0 < kGradWhtMin) {
+                ord.insert(ord.end(), op->ag_mem.begin() + a0, op->ag_mem.begin() + a1);
+                continue;
             }
-            std::vector<uint2> bat;
-            for (uint32_t i = 0; i < nstr;) {
-                uint32_t j = i + 1;
-                while (j < nstr && j - i < 8 && (sx[j] >> 12) == (sx[i] >> 12)) ++j;
-                bat.push_back(make_uint2(i, j - i));
-                i = j;
+            for (uint32_t k = a0; k < a1; k += kGradWhtBatch) {
+                const uint32_t cnt = std::min(kGradWhtBatch, a1 - k);
+                wb.push_back(GradBatch{op->mx[op->ag_mem[k]], (uint32_t)word.size(), cnt});
+                word.insert(word.end(), op->ag_mem.begin() + k, op->ag_mem.begin() + k + cnt);
             }
-            std::stable_sort(bat.begin(), bat.end(),
-                             [](const uint2 &a, const uint2 &b) { return a.y > b.y; });
-            QR_CUDA(op->d_tg_x.upload(sx), "upload gradient strings");
-            QR_CUDA(op->d_tg_z.upload(sz), "upload gradient strings");
-            QR_CUDA(op->d_tg_perm.upload(ord), "upload gradient order");
-            QR_CUDA(op->d_tg_bat.upload(bat), "upload gradient batches");
-            op->tg_nbatch = (uint32_t)bat.size();
-            op->tg_ready = true;
         }
-        // about 8 work items per SM, chunks of at least 16 tiles
-        const uint64_t TT = (op->N >> 12) * (uint64_t)nstates;
-        uint64_t nchunk = ((uint64_t)op->nsm * 8 + op->tg_nbatch - 1) / op->tg_nbatch;
-        if (nchunk > TT / 16) nchunk = TT / 16;
-        if (nchunk < 1) nchunk = 1;
-        void *scratch = nullptr;
-        const size_t pbytes = (size_t)nstr * nchunk * sizeof(double2);
-        QR_CUDA(cudaMallocAsync(&scratch, pbytes + (size_t)nstr * sizeof(double2) + 16, st),
-                "term-grad scratch");
-        double2 *partial = static_cast<double2 *>(scratch);
-        double2 *R = partial + (size_t)nstr * nchunk;
-        auto *counter = reinterpret_cast<unsigned long long *>(R + nstr);
-        cudaError_t e = launch_term_grad_tiles(
-            op->N, nstates, op->d_tg_x.as<uint64_t>(), op->d_tg_z.as<uint64_t>(),
-            op->d_tg_perm.as<uint32_t>(), op->d_tg_bat.as<uint2>(), op->tg_nbatch, nstr, psi, g,
-            partial, (uint32_t)nchunk, R, op->T, op->d_mmap.as<uint32_t>(), op->d_ph.as<uint8_t>(),
-            reinterpret_cast<double2 *>(out), counter, op->nsm, st);
-        cudaFreeAsync(scratch, st);
-        if (e != cudaSuccess) return cuda_fail(e, "term-grad launch");
-        return QR_OK;
+        std::sort(ord.begin(), ord.end());
+        std::stable_sort(ord.begin(), ord.end(), [&](uint32_t a, uint32_t b) {
+            return (op->mx[a] >> 12) < (op->mx[b] >> 12);
+        });
+        const uint32_t nd = (uint32_t)ord.size();
+        std::vector<uint64_t> sx(nd), sz(nd), wz;
+        for (uint32_t i = 0; i < nd; ++i) {
+            sx[i] = op->mx[ord[i]];
+            sz[i] = op->mz[ord[i]];
+        }
+        for (uint32_t k : word) wz.push_back(op->mz[k]);
+        std::vector<uint2> bat;
+        for (uint32_t i = 0; i < nd;) {
+            uint32_t j = i + 1;
+            while (j < nd && j - i < 8 && (sx[j] >> 12) == (sx[i] >> 12)) ++j;
+            bat.push_back(make_uint2(i, j - i));
+            i = j;
+        }
+        std::stable_sort(bat.begin(), bat.end(),
+                         [](const uint2 &a, const uint2 &b) { return a.y > b.y; });
+        QR_CUDA(op->d_tg_x.upload(sx), "upload gradient strings");
+        QR_CUDA(op->d_tg_z.upload(sz), "upload gradient strings");
+        QR_CUDA(op->d_tg_perm.upload(ord), "upload gradient order");
+        QR_CUDA(op->d_tg_bat.upload(bat), "upload gradient batches");
+        QR_CUDA(op->d_tg_wz.upload(wz), "upload gradient strings");
+        QR_CUDA(op->d_tg_wperm.upload(word), "upload gradient order");
+        QR_CUDA(op->d_tg_wbat.upload(wb), "upload gradient batches");
+        op->tg_ndirect = nd;
+        op->tg_nbatch = (uint32_t)bat.size();
+        op->tg_nwht = (uint32_t)word.size();
+        op->tg_nwbatch = (uint32_t)wb.size();
+        op->tg_ready = true;
     }
-    // blocks take 4 strings each: enough chunks for ~8 blocks per SM
-    const uint64_t nbatch = (nstr + 3) / 4;
-    uint64_t nchunk = ((uint64_t)op->nsm * 8 + nbatch - 1) / nbatch;
-    const uint64_t maxc = op->N >= 4096 ? op->N / 4096 : 1;
-    if (nchunk > maxc) nchunk = maxc;
-    if (nchunk < 1) nchunk = 1;
-    const uint64_t chunk = (op->N + nchunk - 1) / nchunk;
+    GradPlanArgs p{};
+    p.sx = op->d_tg_x.as<uint64_t>();
+    p.sz = op->d_tg_z.as<uint64_t>();
+    p.batches = op->d_tg_bat.as<uint2>();
+    p.nbatch = op->tg_nbatch;
+    p.wz = op->d_tg_wz.as<uint64_t>();
+    p.wbatches = op->d_tg_wbat.as<GradBatch>();
+    p.nwbatch = op->tg_nwbatch;
+    const bool tiles = dtype == QR_C64C && op->n >= 12;
+    uint64_t nchunk = 1, nwchunk = 1;
+    if (op->tg_ndirect > 0) {
+        // about 8 work items (4 strings each, or a batch of the tiled kernel)
+        // per SM, chunks of at least 16 tiles or 4,096 rows
+        const uint64_t items = tiles ? op->tg_nbatch : (op->tg_ndirect + 3) / 4;
+        const uint64_t most = tiles ? (op->N >> 12) * (uint64_t)nstates / 16 : op->N / 4096;
+        nchunk = std::min(((uint64_t)op->nsm * 8 + items - 1) / items, most);
+        if (nchunk < 1) nchunk = 1;
+    }
+    if (op->tg_nwbatch > 0) {
+        // about 4 CTAs per SM, each of at least 8 blocks of 256 rows
+        const uint64_t blocks = std::max<uint64_t>(op->N / 256, 1) * (uint64_t)nstates;
+        nwchunk = std::min(((uint64_t)op->nsm * 4 + op->tg_nwbatch - 1) / op->tg_nwbatch,
+                           (blocks + 7) / 8);
+    }
+    p.direct = GradStrings{op->d_tg_perm.as<uint32_t>(), op->tg_ndirect, (uint32_t)nchunk};
+    p.wht = GradStrings{op->d_tg_wperm.as<uint32_t>(), op->tg_nwht, (uint32_t)nwchunk};
     void *scratch = nullptr;
-    const size_t pbytes = (size_t)nstr * nchunk * sizeof(double2);
-    QR_CUDA(cudaMallocAsync(&scratch, pbytes + (size_t)nstr * sizeof(double2), st),
-            "term-grad scratch");
+    const size_t np = (size_t)op->tg_ndirect * nchunk + (size_t)op->tg_nwht * nwchunk;
+    QR_CUDA(cudaMallocAsync(&scratch, np * sizeof(double2) + 16, st), "term-grad scratch");
     double2 *partial = static_cast<double2 *>(scratch);
-    double2 *R = partial + (size_t)nstr * nchunk;
-    cudaError_t e = launch_term_grad(dtype, op->N, nstates, op->d_mx.as<uint64_t>(),
-                                     op->d_mz.as<uint64_t>(), nstr, psi, g, partial,
-                                     (uint32_t)nchunk, chunk, R, op->T, op->d_mmap.as<uint32_t>(),
-                                     op->d_ph.as<uint8_t>(), reinterpret_cast<double2 *>(out), st);
+    auto *counter = reinterpret_cast<unsigned long long *>(partial + np);
+    const uint32_t *mo = op->d_mm_off.as<uint32_t>(), *mt = op->d_mm_terms.as<uint32_t>();
+    double2 *o = reinterpret_cast<double2 *>(out);
+    const cudaError_t e =
+        tiles ? launch_term_grad_tiles(op->N, nstates, p, psi, g, partial, mo, mt,
+                                       op->d_ph.as<uint8_t>(), o, counter, op->nsm, st)
+              : launch_term_grad(dtype, op->N, nstates, p, psi, g, partial, mo, mt,
+                                 op->d_ph.as<uint8_t>(), o, st);
     cudaFreeAsync(scratch, st);
     if (e != cudaSuccess) return cuda_fail(e, "term-grad launch");
     return QR_OK;

@@ -10,6 +10,7 @@
 
 #include "../../include/qrusty_gpu.h"
 #include "qr_common.cuh"
+#include "qr_device.cuh"
 
 namespace qr {
 
@@ -123,13 +124,13 @@ template <> struct GradT<false> {
     using A = double;
 };
 
-// Accumulate (-1)^popc(r & z) conj(p) g into (ar, ai).
+// Accumulate (-1)^popc(r & z) conj(p) g into (ar, ai): four multiply-adds, the
+// sign on p's bits (FP64 is the bound of the complex128 form).
 template <typename A, typename V>
 __device__ __forceinline__ void grad_acc(A &ar, A &ai, V p, V gg, bool neg) {
-    A pr = p.x * gg.x + p.y * gg.y;
-    A pi = p.x * gg.y - p.y * gg.x;
-    ar += neg ? -pr : pr;
-    ai += neg ? -pi : pi;
+    const A px = flip(p.x, neg), py = flip(p.y, neg);
+    ar = fma(px, gg.x, fma(py, gg.y, ar));
+    ai = fma(px, gg.y, fma(-py, gg.x, ai));
 }
 
 // partial[m * gridDim.x + blockIdx.x] = the chunk's sum over rows r and states
@@ -212,23 +213,170 @@ __global__ void __launch_bounds__(kRedThreads) term_grad_partial_kernel(
     }
 }
 
-__global__ void __launch_bounds__(kRedThreads) term_grad_scatter_kernel(uint64_t T,
-                                                                        const uint32_t *map,
-                                                                        const uint8_t *phase,
-                                                                        const double2 *R,
-                                                                        double2 *out) {
-    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < T;
-         k += (uint64_t)gridDim.x * blockDim.x) {
-        const double2 v = R[map[k]];
-        double2 o;
-        switch (phase[k] & 3) {
-            case 0: o = v; break;                                   // conj(1) = 1
-            case 1: o = make_double2(-v.y, v.x); break;             // conj(-i) = i
-            case 2: o = make_double2(-v.x, -v.y); break;            // -1
-            default: o = make_double2(v.y, -v.x); break;            // conj(i) = -i
+// Gradients of the input terms: one warp per string sums its partials in a
+// fixed order (lane-strided, then a butterfly) and writes every term merged
+// into the string, with the conjugate of the term's unit.
+__global__ void __launch_bounds__(kRedThreads) term_grad_finish_kernel(
+    GradStrings d, GradStrings w, const double2 *partial, const uint32_t *mm_off,
+    const uint32_t *mm_terms, const uint8_t *phase, double2 *out) {
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t i = blockIdx.x * (kRedThreads / 32) + (threadIdx.x >> 5); i < d.count + w.count;
+         i += gridDim.x * (kRedThreads / 32)) {
+        const bool first = i < d.count;
+        const uint32_t k = first ? i : i - d.count, nchunk = first ? d.nchunk : w.nchunk;
+        const uint32_t m = first ? d.perm[k] : w.perm[k];
+        const double2 *p = partial + (first ? 0 : (size_t)d.count * d.nchunk) + (size_t)k * nchunk;
+        double re = 0.0, im = 0.0;
+        for (uint32_t c = lane; c < nchunk; c += 32) {
+            re += p[c].x;
+            im += p[c].y;
         }
-        out[k] = o;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            re += __shfl_xor_sync(0xffffffffu, re, o);
+            im += __shfl_xor_sync(0xffffffffu, im, o);
+        }
+        for (uint32_t t = mm_off[m] + lane; t < mm_off[m + 1]; t += 32) {
+            const uint32_t q = mm_terms[t];
+            double2 o;
+            switch (phase[q] & 3) {
+                case 0: o = make_double2(re, im); break;    // conj(1) = 1
+                case 1: o = make_double2(-im, re); break;   // conj(-i) = i
+                case 2: o = make_double2(-re, -im); break;  // -1
+                default: o = make_double2(im, -re); break;  // conj(i) = -i
+            }
+            out[q] = o;
+        }
     }
+}
+
+// ---------------------------------------------------------------- term grads, Walsh
+// x groups of many strings: the products h(r) = conj(psi[r ^ x]) g[r] of 256
+// consecutive rows go through one Walsh-Hadamard transform (three levels in
+// registers, five across the lanes), after which string z's sum over the rows
+// is coefficient z & 255 up to the sign (-1)^popc(base & z).  A group of k
+// strings costs 4 + 16 operations per row and 2 k per 256 rows instead of 4 k
+// per row; complex128 is FP64-bound, so groups from kGradWhtMin strings take
+// this kernel (Jordan-Wigner n = 15, 500 terms, 95 of them on x = 0).
+// complex64: FP32 products and transform, FP64 sums.
+constexpr int kWhtPerLane = 8;  // strings per lane
+static_assert(kGradWhtBatch == 32 * kWhtPerLane, "strings of a batch");
+
+template <bool F32, bool WIDE>
+__global__ void __launch_bounds__(kRedThreads) term_grad_wht_kernel(
+    uint64_t N, int nstates, const GradBatch *batches, uint32_t nbatch, const uint64_t *sz,
+    const void *psi_, const void *g_, double2 *partial) {
+    using W = typename std::conditional<WIDE, uint64_t, uint32_t>::type;
+    using V = typename GradT<F32>::V;
+    constexpr int kWarps = kRedThreads / 32;
+    __shared__ double2 s_red[kWarps][kGradWhtBatch];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    V *coef = reinterpret_cast<V *>(s_red[warp]);  // 256 coefficients of this warp
+    const uint64_t per_state = N >= 256 ? N / 256 : 1, nblk = per_state * (uint64_t)nstates;
+    for (uint32_t bi = blockIdx.y; bi < nbatch; bi += gridDim.y) {
+        const GradBatch bt = batches[bi];
+        const W x = (W)bt.x;
+        W z[kWhtPerLane];
+        double2 acc[kWhtPerLane];
+#pragma unroll
+        for (int j = 0; j < kWhtPerLane; ++j) {
+            const uint32_t k = lane + 32u * j;
+            z[j] = k < bt.count ? (W)sz[bt.first + k] : (W)0;
+            acc[j] = make_double2(0.0, 0.0);
+        }
+        for (uint64_t b = (uint64_t)blockIdx.x * kWarps + warp; b < nblk;
+             b += (uint64_t)gridDim.x * kWarps) {
+            const uint64_t st = b / per_state;
+            const W base = (W)((b - st * per_state) * 256);
+            const V *psi = static_cast<const V *>(psi_) + st * N;
+            const V *g = static_cast<const V *>(g_) + st * N;
+            V h[8];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                const W r = base + lane + 32u * m;
+                h[m].x = h[m].y = 0;
+                if ((uint64_t)r < N) {
+                    const V p = psi[r ^ x], v = g[r];
+                    h[m].x = fma(p.x, v.x, p.y * v.y);
+                    h[m].y = fma(p.x, v.y, -p.y * v.x);
+                }
+            }
+#pragma unroll
+            for (int l = 1; l < 8; l <<= 1) {
+#pragma unroll
+                for (int m = 0; m < 8; ++m) {
+                    if (m & l) continue;
+                    const V u = h[m], v = h[m | l];
+                    h[m].x = u.x + v.x;
+                    h[m].y = u.y + v.y;
+                    h[m | l].x = u.x - v.x;
+                    h[m | l].y = u.y - v.y;
+                }
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const bool up = (lane & o) != 0;
+#pragma unroll
+                for (int m = 0; m < 8; ++m) {
+                    const auto px = __shfl_xor_sync(0xffffffffu, h[m].x, o);
+                    const auto py = __shfl_xor_sync(0xffffffffu, h[m].y, o);
+                    h[m].x = px + flip(h[m].x, up);
+                    h[m].y = py + flip(h[m].y, up);
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < 8; ++m) coef[lane + 32 * m] = h[m];
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < kWhtPerLane; ++j) {
+                if (32u * j >= bt.count) break;
+                const V c = coef[(uint32_t)z[j] & 255u];
+                const uint32_t neg = parity_of((W)(base & z[j])) ? 1u : 0u;
+                acc[j].x += (double)flip(c.x, neg);
+                acc[j].y += (double)flip(c.y, neg);
+            }
+        }
+        __syncthreads();  // every warp is done with its coefficients
+#pragma unroll
+        for (int j = 0; j < kWhtPerLane; ++j) s_red[warp][lane + 32 * j] = acc[j];
+        __syncthreads();
+        if (threadIdx.x < bt.count) {
+            double2 v = make_double2(0.0, 0.0);
+            for (int w = 0; w < kWarps; ++w) {
+                v.x += s_red[w][threadIdx.x].x;
+                v.y += s_red[w][threadIdx.x].y;
+            }
+            partial[(size_t)(bt.first + threadIdx.x) * gridDim.x + blockIdx.x] = v;
+        }
+        __syncthreads();  // s_red is the next batch's coefficients
+    }
+}
+
+static cudaError_t launch_wht_finish(int dtype, uint64_t N, int nstates, const GradPlanArgs &p,
+                                     const void *psi, const void *g, double2 *partial,
+                                     const uint32_t *mm_off, const uint32_t *mm_terms,
+                                     const uint8_t *phase, double2 *out, cudaStream_t st) {
+    if (p.nwbatch > 0) {
+        double2 *wp = partial + (size_t)p.direct.count * p.direct.nchunk;
+        const dim3 grid(p.wht.nchunk, p.nwbatch < 65535u ? p.nwbatch : 65535u);
+        const bool wide = N >= (1ull << 32);
+        auto kern = dtype == 1 ? (wide ? term_grad_wht_kernel<true, true>
+                                       : term_grad_wht_kernel<true, false>)
+                               : (wide ? term_grad_wht_kernel<false, true>
+                                       : term_grad_wht_kernel<false, false>);
+        kern<<<grid, kRedThreads, 0, st>>>(N, nstates, p.wbatches, p.nwbatch, p.wz, psi, g, wp);
+        count_launch();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    const uint32_t n = p.direct.count + p.wht.count;
+    uint32_t gb = (n + kRedThreads / 32 - 1) / (kRedThreads / 32);
+    if (gb > 4096) gb = 4096;
+    term_grad_finish_kernel<<<gb, kRedThreads, 0, st>>>(p.direct, p.wht, partial, mm_off, mm_terms,
+                                                        phase, out);
+    count_launch();
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------- term grads, tiled (complex64)
@@ -349,8 +497,7 @@ __device__ __forceinline__ float tg_transpose_reduce(float (&v)[16]) {
 
 __global__ void __launch_bounds__(kTgThreads, 1) term_grad_tiles_kernel(
     uint64_t ntiles, int tbits, int nstates, const uint64_t *sx, const uint64_t *sz,
-    const uint32_t *perm, const uint2 *batches, uint32_t nbatch, const float2 *psi,
-    const float2 *g, uint32_t nchunk, uint64_t chunk_tiles, double *partial,
+    const uint2 *batches, uint32_t nbatch, const float2 *psi, const float2 *g, uint32_t nchunk, uint64_t chunk_tiles, double *partial,
     unsigned long long *next_item) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ uint64_t s_x[kTgB], s_z[kTgB];
@@ -486,83 +633,64 @@ __global__ void __launch_bounds__(kTgThreads, 1) term_grad_tiles_kernel(
             double v = 0.0;
             for (int w = 0; w < kTgThreads / 32; ++w) v += s_red[w][tid];
             const uint32_t k = (uint32_t)tid >> 1;
-            if (k < kv) partial[2 * ((uint64_t)perm[bt.x + k] * nchunk + c) + (tid & 1)] = v;
+            if (k < kv) partial[2 * ((uint64_t)(bt.x + k) * nchunk + c) + (tid & 1)] = v;
         }
         __syncthreads();  // s_x, s_z, s_red and the stages are reused by the next item
     }
 }
 
-cudaError_t launch_term_grad_tiles(uint64_t N, int nstates, const uint64_t *sx, const uint64_t *sz,
-                                   const uint32_t *perm, const uint2 *batches, uint32_t nbatch,
-                                   uint32_t nstr, const void *psi, const void *g,
-                                   double2 *partial, uint32_t nchunk, double2 *R, uint64_t T,
-                                   const uint32_t *map, const uint8_t *phase, double2 *out,
+cudaError_t launch_term_grad_tiles(uint64_t N, int nstates, const GradPlanArgs &p,
+                                   const void *psi, const void *g, double2 *partial,
+                                   const uint32_t *mm_off, const uint32_t *mm_terms,
+                                   const uint8_t *phase, double2 *out,
                                    unsigned long long *counter, int nsm, cudaStream_t st) {
-    const uint64_t ntiles = N >> 12;
-    int tbits = 0;
-    while ((1ull << tbits) < ntiles) ++tbits;
-    const uint64_t TT = ntiles * (uint64_t)nstates;
-    const uint64_t chunk = (TT + nchunk - 1) / nchunk;
-    cudaError_t e = ensure_dyn_smem(reinterpret_cast<const void *>(term_grad_tiles_kernel), kTgSmem);
-    if (e != cudaSuccess) return e;
-    const uint64_t nitems = (uint64_t)nbatch * nchunk;
-    const unsigned grid = (unsigned)(nitems < (uint64_t)nsm ? nitems : (uint64_t)nsm);
-    e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
-    if (e != cudaSuccess) return e;
-    term_grad_tiles_kernel<<<grid, kTgThreads, kTgSmem, st>>>(
-        ntiles, tbits, nstates, sx, sz, perm, batches, nbatch, static_cast<const float2 *>(psi),
-        static_cast<const float2 *>(g), nchunk, chunk, reinterpret_cast<double *>(partial),
-        counter);
-    count_launch();
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    sum_partials_kernel<<<nstr, kRedThreads, 0, st>>>(partial, nchunk, R);
-    count_launch();
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    uint64_t gb = (T + kRedThreads - 1) / kRedThreads;
-    if (gb > 4096) gb = 4096;
-    term_grad_scatter_kernel<<<(unsigned)gb, kRedThreads, 0, st>>>(T, map, phase, R, out);
-    count_launch();
-    return cudaGetLastError();
+    if (p.direct.count > 0) {
+        const uint64_t ntiles = N >> 12;
+        int tbits = 0;
+        while ((1ull << tbits) < ntiles) ++tbits;
+        const uint32_t nchunk = p.direct.nchunk;
+        const uint64_t TT = ntiles * (uint64_t)nstates;
+        const uint64_t chunk = (TT + nchunk - 1) / nchunk;
+        cudaError_t e =
+            ensure_dyn_smem(reinterpret_cast<const void *>(term_grad_tiles_kernel), kTgSmem);
+        if (e != cudaSuccess) return e;
+        const uint64_t nitems = (uint64_t)p.nbatch * nchunk;
+        const unsigned grid = (unsigned)(nitems < (uint64_t)nsm ? nitems : (uint64_t)nsm);
+        e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
+        if (e != cudaSuccess) return e;
+        term_grad_tiles_kernel<<<grid, kTgThreads, kTgSmem, st>>>(
+            ntiles, tbits, nstates, p.sx, p.sz, p.batches, p.nbatch,
+            static_cast<const float2 *>(psi), static_cast<const float2 *>(g), nchunk, chunk,
+            reinterpret_cast<double *>(partial), counter);
+        count_launch();
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return launch_wht_finish(1, N, nstates, p, psi, g, partial, mm_off, mm_terms, phase, out, st);
 }
 
-cudaError_t launch_term_grad(int dtype, uint64_t N, int nstates, const uint64_t *sx,
-                             const uint64_t *sz, uint32_t nstr, const void *psi, const void *g,
-                             double2 *partial, uint32_t nchunk, uint64_t chunk, double2 *R,
-                             uint64_t T, const uint32_t *map, const uint8_t *phase, double2 *out,
-                             cudaStream_t st) {
-    const uint32_t nbatch = (nstr + kGradK - 1) / kGradK;
-    const unsigned gy = nbatch < 65535u ? nbatch : 65535u;
-    const dim3 grid(nchunk, gy);
-    const bool wide = N >= (1ull << 32);  // 32-bit rows need r + 2 * 256 < 2^32
-    if (dtype == 1) {
-        if (wide)
-            term_grad_partial_kernel<true, true><<<grid, kRedThreads, 0, st>>>(
-                N, nstates, sx, sz, nstr, psi, g, chunk, nchunk, partial);
-        else
-            term_grad_partial_kernel<true, false><<<grid, kRedThreads, 0, st>>>(
-                N, nstates, sx, sz, nstr, psi, g, chunk, nchunk, partial);
-    } else {
-        if (wide)
-            term_grad_partial_kernel<false, true><<<grid, kRedThreads, 0, st>>>(
-                N, nstates, sx, sz, nstr, psi, g, chunk, nchunk, partial);
-        else
-            term_grad_partial_kernel<false, false><<<grid, kRedThreads, 0, st>>>(
-                N, nstates, sx, sz, nstr, psi, g, chunk, nchunk, partial);
+cudaError_t launch_term_grad(int dtype, uint64_t N, int nstates, const GradPlanArgs &p,
+                             const void *psi, const void *g, double2 *partial,
+                             const uint32_t *mm_off, const uint32_t *mm_terms,
+                             const uint8_t *phase, double2 *out, cudaStream_t st) {
+    if (p.direct.count > 0) {
+        const uint32_t nstr = p.direct.count, nchunk = p.direct.nchunk;
+        const uint64_t chunk = (N + nchunk - 1) / nchunk;
+        const uint32_t nbatch = (nstr + kGradK - 1) / kGradK;
+        const dim3 grid(nchunk, nbatch < 65535u ? nbatch : 65535u);
+        const bool wide = N >= (1ull << 32);  // 32-bit rows need r + 2 * 256 < 2^32
+        auto kern = dtype == 1 ? (wide ? term_grad_partial_kernel<true, true>
+                                       : term_grad_partial_kernel<true, false>)
+                               : (wide ? term_grad_partial_kernel<false, true>
+                                       : term_grad_partial_kernel<false, false>);
+        kern<<<grid, kRedThreads, 0, st>>>(N, nstates, p.sx, p.sz, nstr, psi, g, chunk, nchunk,
+                                           partial);
+        count_launch();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
     }
-    count_launch();
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    sum_partials_kernel<<<nstr, kRedThreads, 0, st>>>(partial, nchunk, R);
-    count_launch();
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    uint64_t gb = (T + kRedThreads - 1) / kRedThreads;
-    if (gb > 4096) gb = 4096;
-    term_grad_scatter_kernel<<<(unsigned)gb, kRedThreads, 0, st>>>(T, map, phase, R, out);
-    count_launch();
-    return cudaGetLastError();
+    return launch_wht_finish(dtype, N, nstates, p, psi, g, partial, mm_off, mm_terms, phase, out,
+                             st);
 }
 
 }  // namespace qr
