@@ -100,13 +100,6 @@ constexpr uint32_t kTabBhiCap = 1024;  // partner blocks whose XORs are staged i
 // aligned
 constexpr size_t kTabBarBytes = ((size_t)kTabStages * 16u + 4u + 15u) & ~(size_t)15u;
 static_assert(kTabBarBytes % 16 == 0, "thread descriptors need 16-byte alignment");
-// paired kernel: up to three ring slots of two partner tiles; barriers,
-// counters, the abort flag and issue counts in 64 bytes
-constexpr uint32_t kMaxPairSlots = 3;
-constexpr size_t kPairBarBytes = 64;
-static_assert(kMaxPairSlots * 8 + kMaxPairSlots * 4 + 4 + kMaxPairSlots * 4 <= kPairBarBytes,
-              "pair barrier block");
-
 template <int AMPS, int ZM, bool XM, bool TV>
 __device__ __forceinline__ void sub_tab_one(float2 (&A)[AMPS], float2 (&B)[AMPS],
                                             const unsigned char *sm, uint32_t soff,
@@ -132,7 +125,7 @@ __device__ __forceinline__ void sub_tab_one(float2 (&A)[AMPS], float2 (&B)[AMPS]
         }
         // partner byte offset: the XOR part (thread and register bits of lo) is
         // precomputed per sub-group; the stage offset occupies higher bits
-        const uint32_t off = soff | (t8 ^ (d.x & 0xffffu));  // bit 15: pair half
+        const uint32_t off = soff | (t8 ^ (d.x & 0xffffu));
         float2 p[AMPS];
 #pragma unroll
         for (int m = 0; m < AMPS; ++m) {
@@ -168,103 +161,6 @@ __device__ __forceinline__ void run_tab(float2 (&A)[AMPS], float2 (&B)[AMPS],
     if (g < g1) sub_tab_one<AMPS, ZM, XM, TV>(A, B, sm, soff, s_tab, tdesc, g, t, t8);
 }
 
-// A pair of key-0 sub-groups g, g+1 in halves 0 and 1 of the slot whose x
-// masks leave the partner tiles unpermuted: each has one factor for every
-// thread and amplitude (table entry u = 0), and amplitude m of thread t sits
-// at a fixed offset from t * 8 in its half -- no descriptor, no address
-// arithmetic.  Same products in the same order as two sub_tab_one calls.
-template <int AMPS>
-__device__ __forceinline__ void cheap_pair_lo0(float2 (&A)[AMPS], float2 (&B)[AMPS],
-                                               const unsigned char *sm, uint32_t base,
-                                               const float4 *s_tab, uint32_t g) {
-    const float4 Ta = s_tab[g * 4], Tb = s_tab[(g + 1) * 4];
-    const unsigned char *h0 = sm + base;
-    const unsigned char *h1 = h0 + 32768u;
-    float2 p[AMPS];
-#pragma unroll
-    for (int m = 0; m < AMPS; ++m) p[m] = *reinterpret_cast<const float2 *>(h0 + ((uint32_t)m << kMsh));
-#pragma unroll
-    for (int m = 0; m < AMPS; ++m) {
-        A[m] = __ffma2_rn(make_float2(Ta.x, Ta.y), p[m], A[m]);
-        B[m] = __ffma2_rn(make_float2(Ta.z, Ta.w), p[m], B[m]);
-    }
-#pragma unroll
-    for (int m = 0; m < AMPS; ++m) p[m] = *reinterpret_cast<const float2 *>(h1 + ((uint32_t)m << kMsh));
-#pragma unroll
-    for (int m = 0; m < AMPS; ++m) {
-        A[m] = __ffma2_rn(make_float2(Tb.x, Tb.y), p[m], A[m]);
-        B[m] = __ffma2_rn(make_float2(Tb.z, Tb.w), p[m], B[m]);
-    }
-}
-
-// Two sub-groups g, g+1 of one x group (same partner amplitudes) whose
-// register-bit sign patterns are ZM and ZM ^ (1 << BB): an x group split
-// because its terms' z differ on one register bit.  One set of partner loads
-// serves both; the factor at register index m is
-//   (-1)^popc(m & ZM) * (F_g + (-1)^(m_BB) F_{g+1}),
-// with F the thread-signed table entries, so the pair costs the packed FMAs
-// of a single sub-group plus four packed adds.
-template <int AMPS, int ZM, int BB, bool XM, bool TV>
-__device__ __forceinline__ void sub_tab_fused(float2 (&A)[AMPS], float2 (&B)[AMPS],
-                                              const unsigned char *sm, uint32_t soff,
-                                              const float4 *s_tab, const uint4 *tdesc, uint32_t g,
-                                              uint32_t t, uint32_t t8) {
-    const uint4 da = tdesc[g], db = tdesc[g + 1];
-    uint32_t ua = 0, sa = 0, ub = 0, sb = 0;
-    if constexpr (TV) {
-        sa = (uint32_t)__popc(t & da.y) & 1u;
-        ua = ((uint32_t)__popc(t & da.z) & 1u) | (((uint32_t)__popc(t & da.w) & 1u) << 1);
-        sb = (uint32_t)__popc(t & db.y) & 1u;
-        ub = ((uint32_t)__popc(t & db.z) & 1u) | (((uint32_t)__popc(t & db.w) & 1u) << 1);
-    }
-    const float4 Ta = s_tab[g * 4 + ua];
-    const float4 Tb = s_tab[(g + 1) * 4 + ub];
-    const float sva = __uint_as_float(0x3f800000u | (sa << 31));
-    const float svb = __uint_as_float(0x3f800000u | (sb << 31));
-    float2 apa = make_float2(Ta.x, Ta.y), bpa = make_float2(Ta.z, Ta.w);
-    if constexpr (TV) {
-        apa = __fmul2_rn(apa, make_float2(sva, sva));
-        bpa = __fmul2_rn(bpa, make_float2(sva, sva));
-    }
-    // F_a + F_b and F_a - F_b: one rounding each (the sign products are exact)
-    const float2 a0 = __ffma2_rn(make_float2(Tb.x, Tb.y), make_float2(svb, svb), apa);
-    const float2 b0 = __ffma2_rn(make_float2(Tb.z, Tb.w), make_float2(svb, svb), bpa);
-    const float2 a1 = __ffma2_rn(make_float2(Tb.x, Tb.y), make_float2(-svb, -svb), apa);
-    const float2 b1 = __ffma2_rn(make_float2(Tb.z, Tb.w), make_float2(-svb, -svb), bpa);
-    const uint32_t off = soff | (t8 ^ (da.x & 0xffffu));
-    float2 p[AMPS];
-#pragma unroll
-    for (int m = 0; m < AMPS; ++m) {
-        const uint32_t o = XM ? (off ^ ((uint32_t)m << kMsh)) : (off + ((uint32_t)m << kMsh));
-        p[m] = *reinterpret_cast<const float2 *>(sm + o);
-    }
-    float2 na0 = a0, nb0 = b0, na1 = a1, nb1 = b1;
-    if constexpr (ZM != 0) {
-        na0 = __fmul2_rn(a0, make_float2(-1.f, -1.f));
-        nb0 = __fmul2_rn(b0, make_float2(-1.f, -1.f));
-        na1 = __fmul2_rn(a1, make_float2(-1.f, -1.f));
-        nb1 = __fmul2_rn(b1, make_float2(-1.f, -1.f));
-    }
-#pragma unroll
-    for (int m = 0; m < AMPS; ++m) {
-        const bool neg = (__builtin_popcount((unsigned)(m & ZM)) & 1) != 0;
-        const bool sel = ((m >> BB) & 1) != 0;
-        const float2 fa = neg ? (sel ? na1 : na0) : (sel ? a1 : a0);
-        const float2 fb = neg ? (sel ? nb1 : nb0) : (sel ? b1 : b0);
-        A[m] = __ffma2_rn(fa, p[m], A[m]);
-        B[m] = __ffma2_rn(fb, p[m], B[m]);
-    }
-}
-
-template <int AMPS, int ZM, int BB, bool XM, bool TV>
-__device__ __forceinline__ void run_fused(float2 (&A)[AMPS], float2 (&B)[AMPS],
-                                          const unsigned char *sm, uint32_t soff,
-                                          const float4 *s_tab, const uint4 *tdesc, uint32_t g0,
-                                          uint32_t g1, uint32_t t, uint32_t t8) {
-    for (uint32_t g = g0; g + 1 < g1; g += 2)
-        sub_tab_fused<AMPS, ZM, BB, XM, TV>(A, B, sm, soff, s_tab, tdesc, g, t, t8);
-}
-
 template <int AMPS>
 __device__ __forceinline__ void run_tab_dispatch(uint32_t key, float2 (&A)[AMPS],
                                                  float2 (&B)[AMPS], const unsigned char *sm,
@@ -286,38 +182,6 @@ __device__ __forceinline__ void run_tab_dispatch(uint32_t key, float2 (&A)[AMPS]
     }
 #undef QR_RUN_CASE8
 #undef QR_RUN_CASE
-}
-
-// Pair-plan runs: keys below 64 as run_tab_dispatch; 64 + (ZM | BB << 3 |
-// XM << 5 | TV << 6) is a run of fused sub-group pairs (sub_tab_fused).
-template <int AMPS>
-__device__ __forceinline__ void run_pair_dispatch(uint32_t key, float2 (&A)[AMPS],
-                                                  float2 (&B)[AMPS], const unsigned char *sm,
-                                                  uint32_t soff, const float4 *s_tab,
-                                                  const uint4 *tdesc, uint32_t g0, uint32_t g1,
-                                                  uint32_t t, uint32_t t8) {
-    if (key < 64u) {
-        run_tab_dispatch<AMPS>(key, A, B, sm, soff, s_tab, tdesc, g0, g1, t, t8);
-        return;
-    }
-#define QR_FUSED_CASE(k)                                                                  \
-    case k:                                                                               \
-        if constexpr ((k & 7) < AMPS && (1 << ((k >> 3) & 3)) < AMPS)                     \
-            run_fused<AMPS, (k & 7), ((k >> 3) & 3), ((k >> 5) & 1) != 0, ((k >> 6) & 1) != 0>( \
-                A, B, sm, soff, s_tab, tdesc, g0, g1, t, t8);                             \
-        break;
-#define QR_FUSED_CASE8(k) QR_FUSED_CASE(k) QR_FUSED_CASE(k + 1) QR_FUSED_CASE(k + 2) \
-    QR_FUSED_CASE(k + 3) QR_FUSED_CASE(k + 4) QR_FUSED_CASE(k + 5) QR_FUSED_CASE(k + 6) \
-    QR_FUSED_CASE(k + 7)
-    switch (key - 64u) {
-        QR_FUSED_CASE8(0) QR_FUSED_CASE8(8) QR_FUSED_CASE8(16)
-        QR_FUSED_CASE8(32) QR_FUSED_CASE8(40) QR_FUSED_CASE8(48)
-        QR_FUSED_CASE8(64) QR_FUSED_CASE8(72) QR_FUSED_CASE8(80)
-        QR_FUSED_CASE8(96) QR_FUSED_CASE8(104) QR_FUSED_CASE8(112)
-        default: break;
-    }
-#undef QR_FUSED_CASE8
-#undef QR_FUSED_CASE
 }
 
 template <int AMPS, bool WIDE, bool MULTI>
@@ -564,248 +428,6 @@ __global__ void __launch_bounds__(kC64Threads, 1) apply_c64c_tab(const ApplyArgs
     }
 }
 
-// Single-chunk kernel with partner blocks visited in pairs: blocks 2p and
-// 2p+1 are loaded into the two stages of one ring slot behind one barrier,
-// and the pair's sub-groups (merged, sorted by run key, bit 15 of the
-// descriptor's offset selecting the stage) run as one list.  Most partner
-// blocks of pair-structured operators hold a single sub-group, for which the
-// per-block ring wait, run lookup, dispatch and stage release cost more than
-// the sub-group itself.
-template <int AMPS, bool WIDE>
-__global__ void __launch_bounds__(kC64Threads, 1) apply_c64c_pair(const ApplyArgs a) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    const uint32_t threads = blockDim.x;
-    const uint32_t nwarps = threads >> 5;
-    const uint32_t t = threadIdx.x;
-    const uint32_t lane = t & 31;
-    const uint32_t tile_bytes = (1u << a.b) * 8u;
-    // layout (pair_smem_bytes): ring of nsl slots of two tiles, factor table,
-    // barriers / counters (64 bytes), thread descriptors, run list, pair list
-    const uint32_t nsl = a.pair_slots;
-    const uint32_t tabn = a.nsub;  // a pair plan has at most kTabCap sub-groups
-    float4 *s_tab = reinterpret_cast<float4 *>(smem_raw + (size_t)nsl * 2u * tile_bytes);
-    uint64_t *full = reinterpret_cast<uint64_t *>(s_tab + kTabEnt * (size_t)tabn);
-    uint32_t *cnt = reinterpret_cast<uint32_t *>(full + kMaxPairSlots);
-    volatile uint32_t *s_abort = cnt + kMaxPairSlots;
-    // copies issued into each slot: the drain after an expired wait waits
-    // for the last one's phase, so no copy is in flight when the CTA exits
-    uint32_t *s_iss = cnt + kMaxPairSlots + 1;
-    uint4 *s_td = reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(full) + kPairBarBytes);
-    uint32_t *s_run = reinterpret_cast<uint32_t *>(s_td + tabn);
-    uint32_t *s_blk = s_run + a.nruns + 1;
-    const uint32_t np = a.npairs, nb = a.nblocks;
-    uint64_t *s_bhi = reinterpret_cast<uint64_t *>(
-        (reinterpret_cast<uintptr_t>(s_blk + np + 1) + 7u) & ~(uintptr_t)7u);
-    for (uint32_t i = t; i < a.nsub; i += threads) s_td[i] = a.tdesc[i];
-    for (uint32_t i = t; i <= a.nruns; i += threads)
-        s_run[i] = a.run_g0[i] | (i < a.nruns ? a.run_key[i] << 16 : 0u);
-    for (uint32_t i = t; i <= np; i += threads) s_blk[i] = a.blk_r0[i];
-    for (uint32_t i = t; i < nb; i += threads) s_bhi[i] = a.blk_hi[i];
-    __syncthreads();  // the prologue reads s_bhi
-    const uint4 *tdesc = s_td;
-
-    const float2 *psi = static_cast<const float2 *>(a.psi);
-    float2 *y = static_cast<float2 *>(a.y);
-    const float2 *diag = static_cast<const float2 *>(a.diag);
-    const uint32_t t8 = t << 3;
-    const uint32_t slot_bytes = 2u * tile_bytes;
-    const int diag_pair = a.diag_block >= 0 ? (a.diag_block >> 1) : -1;
-    const uint32_t diag_half = a.diag_block >= 0 ? ((uint32_t)a.diag_block & 1u) : 0u;
-
-    const uint64_t first = blockIdx.x;
-    const uint64_t my_items =
-        a.nitems > first ? (a.nitems - first + gridDim.x - 1) / gridDim.x : 0;
-    const uint64_t total = my_items * np;
-    if (total == 0) return;
-
-    // load pair p of tile (st, q) into slot s: one or two partner tiles
-    auto issue_pair = [&](uint64_t L, uint32_t s, uint32_t p, uint64_t st, uint64_t q) {
-        if (blockIdx.x == 0 && (int64_t)L == a.withhold) return;  // test hook: never issued
-        const uint32_t j0 = 2u * p;
-        const uint32_t ntl = j0 + 1 < nb ? 2u : 1u;
-        ++s_iss[s];
-        mbar_expect_tx(&full[s], ntl * tile_bytes);
-        for (uint32_t h = 0; h < ntl; ++h) {
-            const float2 *src = psi + st * a.N + ((q ^ s_bhi[j0 + h]) << a.b);
-            bulk_g2s(smem_raw + (size_t)s * slot_bytes + (size_t)h * tile_bytes, src, tile_bytes,
-                     &full[s]);
-        }
-    };
-    uint64_t st = first / a.ntiles;
-    uint64_t q = first - st * a.ntiles;
-    if (t == 0) {
-        for (uint32_t s = 0; s < nsl; ++s) {
-            mbar_init(&full[s], 1);
-            cnt[s] = 0;
-            s_iss[s] = 0;
-        }
-        *s_abort = 0;
-        mbar_fence_init();
-        // prologue: steps 0 .. nsl - 1
-        uint32_t p1 = 0;
-        uint64_t q1 = q, st1 = st;
-        for (uint64_t L = 0; L < total && L < nsl; ++L) {
-            issue_pair(L, (uint32_t)L, p1, st1, q1);
-            if (++p1 == np) {
-                p1 = 0;
-                q1 += gridDim.x;
-                while (q1 >= a.ntiles) {
-                    q1 -= a.ntiles;
-                    ++st1;
-                }
-            }
-        }
-    }
-    __syncthreads();
-
-    // y = A + iB is the FP32 sum of the current window of pairs; every 16
-    // pairs it is folded into hi with an error-free two-sum, and the error of
-    // that addition is carried into the next window (A starts from it: the
-    // compensated summation of Kahan, with no separate low word to keep);
-    // the last fold's error is added at the store
-    float2 A[AMPS], B[AMPS], hi[AMPS];
-    uint32_t p = 0, s = 0, par = 0;
-    constexpr uint32_t kFlushPairs = 16;
-
-    for (uint64_t L = 0; L < total; ++L) {
-        if (p == 0) {
-#pragma unroll
-            for (int m = 0; m < AMPS; ++m) A[m] = B[m] = hi[m] = make_float2(0.f, 0.f);
-            // table of the new output tile: every warp has finished the last one
-            __syncthreads();
-            for (uint32_t gi = t; gi < a.nsub; gi += threads) {
-                const TileDataC64 &d = a.tdata[gi];
-                const uint32_t uq = parity<WIDE>(q, d.b0h) | (parity<WIDE>(q, d.b1h) << 1);
-                const float sq = parity<WIDE>(q, d.z0h) ? -1.f : 1.f;
-#pragma unroll
-                for (uint32_t u = 0; u < 4; ++u) {
-                    const float2 v = d.T[u ^ uq];
-                    s_tab[gi * 4 + u] = make_float4(sq * v.x, sq * v.x, sq * v.y, sq * v.y);
-                }
-            }
-            __syncthreads();
-        }
-        // fast path: the stage is complete for the whole warp; otherwise the
-        // bounded wait, which also honours another warp's abort
-        bool skip = false;
-        if (!__all_sync(0xffffffffu, mbar_try_wait(&full[s], par))) {
-            skip = *s_abort != 0;
-            if (!skip && !mbar_wait_bounded(&full[s], par, a.wait_ns)) {
-                if (lane == 0) {
-                    atomicExch(a.err, kErrMbarTimeout);
-                    *s_abort = 1;
-                }
-                skip = true;
-            }
-            skip = __any_sync(0xffffffffu, skip);
-        }
-        const uint32_t soff = s * slot_bytes;
-
-        if (!skip && (int)p == diag_pair && diag != nullptr) {
-            const float2 *dg = diag + (q << a.b);
-            const uint32_t doff = soff + diag_half * tile_bytes;
-#pragma unroll
-            for (int m = 0; m < AMPS; ++m) {
-                const uint32_t rl = t + threads * (uint32_t)m;
-                const float2 d = dg[rl];
-                const float2 pv = *reinterpret_cast<const float2 *>(smem_raw + doff + rl * 8u);
-                A[m] = __ffma2_rn(make_float2(d.x, d.x), pv, A[m]);
-                B[m] = __ffma2_rn(make_float2(d.y, d.y), pv, B[m]);
-            }
-        }
-
-        // bit 31 of a pair's first run: exactly two sub-groups of key 0; bit
-        // 30: in halves 0 and 1, partner tiles unpermuted
-        const uint32_t bw = s_blk[p];
-        const uint32_t rb = bw & 0x3fffffffu;
-        if (!skip && (bw >> 31) != 0) {
-            const uint32_t g0 = s_run[rb] & 0xffffu;
-            if ((bw >> 30) & 1u) {
-                cheap_pair_lo0<AMPS>(A, B, smem_raw, soff | t8, s_tab, g0);
-            } else {
-                sub_tab_one<AMPS, 0, false, false>(A, B, smem_raw, soff, s_tab, tdesc, g0, t, t8);
-                sub_tab_one<AMPS, 0, false, false>(A, B, smem_raw, soff, s_tab, tdesc, g0 + 1, t,
-                                                   t8);
-            }
-        } else {
-            const uint32_t r1 = skip ? 0u : (s_blk[p + 1] & 0x3fffffffu);
-            uint32_t rw = s_run[rb];
-            for (uint32_t r = rb; r < r1; ++r) {
-                const uint32_t rn = s_run[r + 1];
-                run_pair_dispatch<AMPS>(rw >> 16, A, B, smem_raw, soff, s_tab, tdesc,
-                                        rw & 0xffffu, rn & 0xffffu, t, t8);
-                rw = rn;
-            }
-        }
-
-        const bool last = (p == np - 1);
-        if (last || (p % kFlushPairs) == kFlushPairs - 1) {
-#pragma unroll
-            for (int m = 0; m < AMPS; ++m) {
-                const float2 yv =
-                    make_float2(__fsub_rn(A[m].x, B[m].y), __fadd_rn(A[m].y, B[m].x));
-                A[m] = two_sum_carry2(hi[m], yv);  // the error opens the next window
-                B[m] = make_float2(0.f, 0.f);
-            }
-        }
-        if (last) {
-            float2 *yo = y + st * a.N + (q << a.b);
-            const float2 *vo = a.v ? static_cast<const float2 *>(a.v) + st * a.N + (q << a.b)
-                                   : nullptr;
-#pragma unroll
-            for (int m = 0; m < AMPS; ++m) {
-                const uint32_t rl = t + threads * (uint32_t)m;
-                float2 o = make_float2(__fadd_rn(hi[m].x, A[m].x), __fadd_rn(hi[m].y, A[m].y));
-                if (vo)  // fused y = alpha (H psi) + beta v, in FP32
-                    o = cx_axpby((float)a.ar, (float)a.ai, o, (float)a.br, (float)a.bi, vo[rl]);
-                yo[rl] = o;
-            }
-        }
-
-        __syncwarp();
-        if (lane == 0) {
-            __threadfence_block();
-            const uint32_t old = atomicAdd(&cnt[s], 1u);
-            if (old == nwarps - 1) {
-                cnt[s] = 0;
-                if (L + nsl < total && *s_abort == 0) {
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    // nsl pairs ahead of (st, q, p), stepped with adds
-                    uint32_t p2 = p + nsl;
-                    uint64_t q2 = q, st2 = st;
-                    while (p2 >= np) {
-                        p2 -= np;
-                        q2 += gridDim.x;
-                        while (q2 >= a.ntiles) {
-                            q2 -= a.ntiles;
-                            ++st2;
-                        }
-                    }
-                    issue_pair(L + nsl, s, p2, st2, q2);
-                }
-            }
-        }
-        if (++s == nsl) {
-            s = 0;
-            par ^= 1u;
-        }
-        if (++p == np) {
-            p = 0;
-            q += gridDim.x;
-            while (q >= a.ntiles) {
-                q -= a.ntiles;
-                ++st;
-            }
-        }
-    }
-    // drain after an expired wait, as in apply_c64c_tab
-    __syncthreads();
-    if (t == 0 && *s_abort) {
-        for (uint32_t k = 0; k < nsl; ++k)
-            if (s_iss[k] != 0) mbar_wait_bounded(&full[k], (s_iss[k] - 1u) & 1u, kWaitLimitNs);
-    }
-}
-
 template <int AMPS>
 static size_t tab_smem_bytes(const ApplyArgs &a, int threads) {
     const uint32_t tile_bytes = (1u << a.b) * 8u;
@@ -816,29 +438,11 @@ static size_t tab_smem_bytes(const ApplyArgs &a, int threads) {
            (a.nblocks <= kTabBhiCap ? (size_t)a.nblocks * 8u : 0u);
 }
 
-// shared memory of the paired kernel with nsl ring slots (exact sizes of the
-// table, descriptors and lists of this plan)
-static size_t pair_smem_bytes(const ApplyArgs &a, uint32_t nsl) {
-    const size_t tile_bytes = ((size_t)1 << a.b) * 8u;
-    return (size_t)nsl * 2u * tile_bytes + (size_t)a.nsub * 16u * kTabEnt + kPairBarBytes +
-           (size_t)a.nsub * sizeof(uint4) + ((size_t)a.nruns + 1 + a.npairs + 1) * 4u + 8u +
-           (size_t)a.nblocks * 8u;
-}
-
 template <int AMPS, bool WIDE>
-static cudaError_t launch_c64c_tab(const ApplyArgs &a_in, int threads, int nsm, cudaStream_t st) {
-    ApplyArgs a = a_in;
-    size_t smem = tab_smem_bytes<AMPS>(a, threads);
-    // one chunk (operators of up to 512 sub-groups): no chunk bookkeeping;
-    // with a pair plan, partner blocks two at a time, in a ring of three
-    // slots when the plan's tables leave room for it, else two
+static cudaError_t launch_c64c_tab(const ApplyArgs &a, int threads, int nsm, cudaStream_t st) {
+    const size_t smem = tab_smem_bytes<AMPS>(a, threads);
+    // one chunk (operators of up to 512 sub-groups): no chunk bookkeeping
     auto kern = a.nchunks > 1 ? apply_c64c_tab<AMPS, WIDE, true> : apply_c64c_tab<AMPS, WIDE, false>;
-    if constexpr (AMPS == 8)
-        if (a.npairs > 0 && a.nchunks <= 1) {
-            kern = apply_c64c_pair<AMPS, WIDE>;
-            a.pair_slots = pair_smem_bytes(a, kMaxPairSlots) <= kMaxSmemPerBlock ? kMaxPairSlots : 2u;
-            smem = pair_smem_bytes(a, a.pair_slots);
-        }
     cudaError_t e = ensure_dyn_smem(reinterpret_cast<const void *>(kern), smem);
     if (e != cudaSuccess) return e;
     uint64_t grid = a.nitems < (uint64_t)nsm ? a.nitems : (uint64_t)nsm;

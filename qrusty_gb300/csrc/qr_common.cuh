@@ -35,9 +35,11 @@ template <> struct alignas(16) Cplx<double> { double re, im; };
 // Per-sub-group data of the per-tile table of the compensated-c64 kernel:
 // the masks' tile-index parts (>> b) and the FP32 table T[u] of the factor.
 struct alignas(16) TileDataC64 {
-    uint64_t z0h, b0h, b1h, pad;
+    uint64_t z0h, b0h, b1h;
+    uint64_t role;  // coset plans: 0, or a merged pair's (kMerged...)
     float2 T[4];
 };
+enum : uint64_t { kMergedBasis = 1, kMergedSign = 2, kMergedSecond = 3 };
 static_assert(sizeof(TileDataC64) == 64, "TileDataC64 is read as four 16-byte words");
 
 // String plans: consumer threads, strings per block, CTAs per cluster at most.
@@ -73,25 +75,19 @@ struct ApplyArgs {
     // compensated-c64 plan: sub-groups (see qr_apply.cu)
     uint32_t nsub;
     // per-tile-table kernel: per sub-group a 16-byte thread descriptor
-    // {partner byte-offset XOR | pair half << 15 | tvar << 31, z0_t, beta0_t,
-    //  beta1_t} (the thread-bit parts of z0 and of the basis) and its
-    // TileDataC64; sub-groups of a block (or pair of blocks) in runs of
-    // equal key
+    // {partner byte-offset XOR | tvar << 31, z0_t, beta0_t, beta1_t} (the
+    // thread-bit parts of z0 and of the basis) and its TileDataC64;
+    // sub-groups of a block in runs of equal key
     const uint4 *tdesc;
     const TileDataC64 *tdata;
-    const uint32_t *blk_r0;   // runs of block (pair) j: [blk_r0[j], blk_r0[j+1])
+    const uint32_t *blk_r0;   // runs of block j: [blk_r0[j], blk_r0[j+1])
     const uint32_t *run_g0;   // sub-groups of run r: [run_g0[r], run_g0[r+1])
-    const uint32_t *run_key;  // key = zm | xm << 4 | tv << 5 (factor depends on the thread);
-                              // pair plans: 64 + (zm | bb << 3 | xm << 5 | tv << 6) for
-                              // runs of fused sub-group pairs
+    const uint32_t *run_key;  // key = zm | xm << 4 | tv << 5 (factor depends on the thread)
     uint32_t nruns;
     // chunks of consecutive blocks with at most kTabCap sub-groups:
     // {first sub-group, first run, first block, 0}, nchunks + 1 entries
     const uint4 *chunks;
     uint32_t nchunks;
-    // > 0: partner blocks visited in pairs (blocks 2p, 2p+1 in one ring slot
-    // of two stages); blk_r0 then indexes pairs and tdesc bit 15 is the half
-    uint32_t npairs;
     // string plans (qr_apply_strings.cu): nsblk blocks of one or two partner
     // tiles, {XOR of tile 0, of tile 1 (or ~0), first 16-byte entry, strings};
     // a block's entries are a header {strings, diagonal flag} and one per
@@ -99,6 +95,14 @@ struct ApplyArgs {
     const uint4 *ent, *sblk;
     uint32_t nsblk;
     uint32_t part[kStrMaxSplit + 1];
+    // coset plans (qr_apply_cosets.cu): blocks {XOR of tile 0, of tile 1 (or
+    // ~0), first sub-group | lone uniform ones << 10 | cheap << 30 | diagonal
+    // << 31, lone ones by thread | quads << 10 | others << 16}; per sub-group
+    // {partner offset within the slot | new loads << 16 | key << 17 | merged
+    // pair << 24, thread parts of z0, beta0, beta1} and its tile data
+    const uint4 *cblk, *ctdesc;
+    const TileDataC64 *ctdata;
+    uint32_t ncblk, ncsub;
     // fused epilogue y = alpha * (H psi) + beta * v when v != nullptr
     const void *v;
     double ar, ai, br, bi;
@@ -109,15 +113,12 @@ struct ApplyArgs {
     int64_t withhold;
     // 64-bit row words (the n > 32 instantiations) forced at any n (test hook)
     int wide;
-    // paired kernel: ring slots of two partner tiles (set by the launcher)
-    uint32_t pair_slots;
 };
 
 
 
 // One operator of a batched compensated-c64 launch (device copy): the
-// per-tile-table plan of the operator (no partner-tile pairs) and its tile
-// geometry.
+// per-tile-table plan of the operator and its tile geometry.
 struct BatchOp {
     uint64_t N, ntiles;
     int32_t b, mcount, tact, diag_block;  // tile bits, amplitudes / threads used, x = 0 block
@@ -225,6 +226,10 @@ cudaError_t launch_apply(const ApplyArgs &a, int amps, int threads, int nsm,
 // call_items: output tiles of the caller's whole call
 cudaError_t launch_c64c_strings(const ApplyArgs &a, const StrSplit &sp, uint64_t call_items,
                                 int nsm, cudaStream_t st);
+// qr_apply_cosets.cu
+constexpr size_t kCosetSmem = 227u * 1024u - 256u;  // dynamic shared memory, at most
+size_t coset_smem_bytes(uint32_t nsub, uint32_t nblk, uint32_t slots, uint32_t ntab);
+cudaError_t launch_c64c_cosets(const ApplyArgs &a, int nsm, cudaStream_t st);
 // qr_apply_rows.cu
 // call_rows: rows of the caller's whole call (complex64 splits by them)
 cudaError_t launch_rows(int dtype, const ApplyArgs &a, uint64_t call_rows, cudaStream_t st);

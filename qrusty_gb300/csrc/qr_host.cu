@@ -118,11 +118,14 @@ struct Plan {
     bool has_diag = false;
     DevBuf groups, tables, fat_z, fat_c, blk_hi, diag;
     // compensated-c64 kernel tables
-    uint32_t nsub = 0, nruns = 0, nchunks = 0, npairs = 0;
+    uint32_t nsub = 0, nruns = 0, nchunks = 0;
     DevBuf tdesc, tdata, blk_r0, run_g0, run_key, chunks;
     // string plans: see ApplyArgs; str.part[k - 1] are the parts of a split in k
     bool strings = false;
     StrSplit str;
+    bool cosets = false;  // qr_apply_cosets.cu
+    uint32_t ncblk = 0, ncsub = 0;
+    DevBuf cblk, ctdesc, ctdata;
     bool rows = false;  // qr_apply_rows.cu: complex128, and complex64 of few rows
     DevBuf ent, sblk;
     // what the plan was built for, and its coefficient program: the slots
@@ -519,6 +522,291 @@ int build_strings(qr_op *op, Plan &pl, const std::vector<cd> &c,
     return QR_OK;
 }
 
+// Sub-groups of a coset plan (qr_apply_cosets.cu), blocks and tables; *fits is
+// false, and nothing is made, when they do not fit the kernel's shared memory.
+//
+// A thread's rows are t' + 512 m, t' = t ^ 256 for odd popc(m): the coset of
+// the even-weight subsets of row bits 8 ... 11.  Within a tile, x = (xt, xm),
+// xm its bits 9-11, moves the coset by c = xt ^ (256 for odd popc(xm)) and m by
+// xm; a string's sign is (-1)^(popc(t & z) + popc(m & zm)), zm = its bits 9-11,
+// complemented when bit 8 is set.  A sub-group holds the strings of one x with
+// one zm, their z differences (bits 9-11 aside) of rank <= 2.
+template <typename AddSlot>
+int build_cosets(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vector<uint64_t> &gxs,
+                 const std::vector<std::vector<size_t>> &members, bool has_diag, bool *fits,
+                 AddSlot &&add_slot) {
+    struct Sub {
+        uint64_t hi, x;
+        uint32_t off, xm, zm;
+        uint64_t z0;
+        Span sp;
+        std::vector<size_t> part;
+        bool fused_next = false;
+    };
+    auto zm_of = [&](size_t k) {
+        const uint32_t z = (uint32_t)(op->mz[k] >> 8) & 15u;
+        return (z >> 1) ^ ((z & 1u) ? 7u : 0u);
+    };
+    auto masked = [&](const std::vector<size_t> &part) {
+        std::vector<uint64_t> zs;
+        for (size_t k : part) zs.push_back(op->mz[k] & ~0xe00ull);
+        return zs;
+    };
+    std::vector<Sub> subs;
+    for (size_t g = 0; g < gxs.size(); ++g) {
+        if (has_diag && gxs[g] == 0) continue;
+        const uint32_t lo = (uint32_t)(gxs[g] & 4095u), xm = lo >> 9;
+        const uint32_t off = ((lo & 511u) ^ ((__builtin_popcount(xm) & 1) ? 256u : 0u)) << 3;
+        std::vector<std::vector<size_t>> byzm(8);
+        for (size_t k : members[g]) byzm[zm_of(k)].push_back(k);
+        for (uint32_t zm = 0; zm < 8; ++zm) {
+            if (byzm[zm].empty()) continue;
+            std::vector<std::vector<size_t>> pieces;
+            const Span full = gf2_span(masked(byzm[zm]), 64);
+            if (full.basis.size() <= 2) {
+                pieces.push_back(byzm[zm]);
+            } else {
+                std::map<uint64_t, std::vector<size_t>> parts;
+                for (size_t kk = 0; kk < byzm[zm].size(); ++kk)
+                    parts[full.coord[kk] >> 2].push_back(byzm[zm][kk]);
+                for (auto &pt : parts) pieces.push_back(std::move(pt.second));
+            }
+            for (auto &part : pieces) {
+                Sub sg;
+                sg.hi = gxs[g] >> 12;
+                sg.x = gxs[g];
+                sg.off = off;
+                sg.xm = xm;
+                sg.zm = zm;
+                const std::vector<uint64_t> zs = masked(part);
+                sg.z0 = zs[0];
+                sg.sp = gf2_span(zs, 2);
+                sg.part = std::move(part);
+                subs.push_back(std::move(sg));
+            }
+        }
+    }
+    *fits = !subs.empty() && subs.size() <= (size_t)kTabCap;
+    if (!*fits) return QR_OK;
+    std::stable_sort(subs.begin(), subs.end(), [](const Sub &a, const Sub &b) {
+        return a.hi != b.hi ? a.hi < b.hi : a.off < b.off;
+    });
+    // partner tiles and their sub-groups
+    struct Tile {
+        uint64_t hi;
+        uint32_t g0, g1;
+    };
+    std::vector<Tile> tiles;
+    if (has_diag && subs[0].hi != 0) tiles.push_back({0, 0, 0});
+    for (uint32_t i = 0; i < subs.size(); ++i) {
+        if (tiles.empty() || tiles.back().hi != subs[i].hi) tiles.push_back({subs[i].hi, i, i});
+        tiles.back().g1 = i + 1;
+    }
+    // Tiles in pairs, heavy with heavy and light (one sub-group) with light, the
+    // heavy pairs spread evenly among the light ones, each closing a run of
+    // them: a ring of three pairs does not hide its refill behind a run of light
+    // pairs, and the tile's last pair is heavy, so the ring refills across the
+    // table rebuild.  The diagonal's tile is tile 0 of its pair.
+    std::vector<uint32_t> heavy, light;
+    for (uint32_t j = 0; j < tiles.size(); ++j)
+        ((tiles[j].g1 - tiles[j].g0 > 1 || tiles[j].hi == 0) ? heavy : light).push_back(j);
+    std::vector<std::pair<uint32_t, uint32_t>> hp, lp, seq;
+    constexpr uint32_t none = 0xffffffffu;
+    size_t l0 = 0;
+    for (size_t i = 0; i < heavy.size(); i += 2) {
+        if (i + 1 < heavy.size()) hp.push_back({heavy[i], heavy[i + 1]});
+        else if (!light.empty()) hp.push_back({heavy[i], light[l0++]});
+        else hp.push_back({heavy[i], none});
+    }
+    for (size_t i = l0; i < light.size(); i += 2)
+        lp.push_back({light[i], i + 1 < light.size() ? light[i + 1] : none});
+    size_t ih = 0, il = 0;
+    const size_t tot = hp.size() + lp.size();
+    for (size_t k = 0; k < tot; ++k) {
+        if (ih < hp.size() && (il >= lp.size() || k >= (ih + 1) * tot / hp.size() - 1))
+            seq.push_back(hp[ih++]);
+        else seq.push_back(lp[il++]);
+    }
+    std::vector<uint4> blk, td;
+    std::vector<TileDataC64> data;
+    std::vector<const Sub *> placed;
+    auto thread_var = [](const Sub &g) {
+        uint64_t m = g.z0;
+        for (uint64_t b : g.sp.basis) m |= b;
+        return (m & 511u) != 0;
+    };
+    // role and masks of a merged pair: one table index and sign for both
+    struct Merge {
+        uint64_t role = 0;
+        uint32_t b0t = 0, b1t = 0;
+    };
+    auto merge_of = [](const Sub &a, const Sub &b) {
+        Merge m;
+        auto bt = [](const Sub &s, size_t i) {
+            return i < s.sp.basis.size() ? (uint32_t)s.sp.basis[i] & 511u : 0u;
+        };
+        const uint32_t mu = (uint32_t)(a.z0 ^ b.z0) & 511u;
+        if (mu == 0 && bt(a, 0) == bt(b, 0) && bt(a, 1) == bt(b, 1) &&
+            a.sp.basis.size() == b.sp.basis.size()) {
+            m = {kMergedBasis, bt(a, 0), bt(a, 1)};
+        } else if (a.sp.basis.size() <= 1 && b.sp.basis.size() <= 1 &&
+                   (a.sp.basis.empty() || b.sp.basis.empty() || bt(a, 0) == bt(b, 0))) {
+            m = {kMergedSign, bt(a.sp.basis.empty() ? b : a, 0), mu};
+        }
+        return m;
+    };
+    std::vector<uint32_t> rank;  // of placed, as its table is filled
+    auto push = [&](const Sub &g, uint32_t half, bool load, uint32_t key, uint64_t role = 0,
+                    Merge m = Merge()) {
+        const uint64_t b0 = g.sp.basis.size() > 0 ? g.sp.basis[0] : 0,
+                       b1 = g.sp.basis.size() > 1 ? g.sp.basis[1] : 0;
+        const uint32_t b0t = m.role ? m.b0t : (uint32_t)b0 & 511u,
+                       b1t = m.role ? m.b1t : (uint32_t)b1 & 511u;
+        td.push_back(make_uint4(g.off | half << 15 | (load ? 1u << 16 : 0u) | key << 17 |
+                                    (m.role && role != kMergedSecond ? 1u << 24 : 0u),
+                                (uint32_t)g.z0 & 511u, b0t, b1t));
+        TileDataC64 d;
+        memset(&d, 0, sizeof(d));
+        d.z0h = g.z0 >> 12;
+        d.b0h = b0 >> 12;
+        d.b1h = b1 >> 12;
+        d.role = role;
+        // a rank-0 table beside a rank-1 one repeats its entry
+        const uint32_t rk = m.role == kMergedSign ? 1u : (uint32_t)g.sp.basis.size();
+        for (uint32_t u = 0; u < 1u << rk; ++u) {
+            cd acc{0.0, 0.0};
+            for (size_t kk = 0; kk < g.part.size(); ++kk) {
+                const cd v = c[g.part[kk]];
+                if (__builtin_popcountll(u & g.sp.coord[kk]) & 1) {
+                    acc.re -= v.re;
+                    acc.im -= v.im;
+                } else {
+                    acc.re += v.re;
+                    acc.im += v.im;
+                }
+            }
+            d.T[u] = make_float2((float)acc.re, (float)acc.im);
+        }
+        data.push_back(d);
+        placed.push_back(&g);
+        rank.push_back(rk);
+    };
+    for (const auto &pr : seq) {
+        struct Item {
+            uint32_t first, half;  // coset: sub-groups [first, last)
+            uint32_t last;
+        };
+        std::vector<Item> uniform, bythread, others;
+        const uint32_t two[2] = {pr.first, pr.second};
+        for (uint32_t h = 0; h < 2; ++h) {
+            if (two[h] == none) continue;
+            const Tile &tl = tiles[two[h]];
+            for (uint32_t i = tl.g0; i < tl.g1;) {
+                uint32_t j = i + 1;
+                while (j < tl.g1 && subs[j].off == subs[i].off) ++j;
+                const bool lone = j == i + 1 && subs[i].xm == 0 && subs[i].zm == 0;
+                (lone ? (thread_var(subs[i]) ? bythread : uniform) : others).push_back({i, h, j});
+                i = j;
+            }
+        }
+        const uint32_t g0 = (uint32_t)td.size();
+        for (const Item &it : uniform) push(subs[it.first], it.half, true, 0);
+        for (const Item &it : bythread) push(subs[it.first], it.half, true, 0);
+        // cosets of several: pairs of one x whose patterns differ by DL(xm); four
+        // merged pairs with a Jordan-Wigner hop's patterns make a quad
+        struct Placed {
+            uint32_t a, b;  // sub-groups, b == none: alone
+            uint32_t key;
+            Merge m;
+        };
+        static const uint32_t quad_zm[4] = {0, 7, 6, 4};
+        uint32_t nquad = 0;
+        std::vector<std::pair<uint32_t, std::vector<Placed>>> rest;  // half, sub-groups
+        for (const Item &it : others) {
+            std::vector<char> used(it.last - it.first, 0);
+            std::vector<Placed> out;
+            for (uint32_t i = it.first; i < it.last; ++i) {
+                if (used[i - it.first]) continue;
+                const Sub &a = subs[i];
+                const uint32_t f =
+                    a.xm == 0 ? 0u : a.xm == 1 ? 1u : a.xm == 2 ? 2u : a.xm == 4 ? 3u : 4u;
+                const uint32_t dl = f == 0 ? 7u : a.xm;
+                uint32_t mate = none;
+                for (uint32_t j = i + 1; j < it.last && f < 4 && mate == none; ++j)
+                    if (!used[j - it.first] && subs[j].x == a.x && (subs[j].zm ^ a.zm) == dl)
+                        mate = j;
+                if (mate == none) {
+                    out.push_back({i, none, a.xm | a.zm << 3, Merge()});
+                    continue;
+                }
+                used[mate - it.first] = 1;
+                uint32_t p0 = i, p1 = mate;
+                if (subs[p1].zm == quad_zm[f]) std::swap(p0, p1);
+                const Merge m = merge_of(subs[p0], subs[p1]);
+                if (m.role == 0) {  // no common table: two sub-groups on one set of loads
+                    out.push_back({i, none, a.xm | a.zm << 3, Merge()});
+                    out.push_back({mate, none, a.xm | subs[mate].zm << 3, Merge()});
+                } else {
+                    out.push_back({p0, p1, 64u + (f | subs[p0].zm << 2), m});
+                }
+            }
+            std::vector<Placed> q(4, Placed{none, none, 0, Merge()});
+            bool quad = out.size() == 4 && nquad < 63;
+            for (const Placed &o : out) {
+                const uint32_t f = o.key & 3u;
+                quad = quad && o.key >= 64u && q[f].a == none && subs[o.a].zm == quad_zm[f];
+                if (quad) q[f] = o;
+            }
+            if (!quad) {
+                rest.push_back({it.half, out});
+                continue;
+            }
+            ++nquad;
+            for (uint32_t f = 0; f < 4; ++f) {
+                push(subs[q[f].a], it.half, f == 0, q[f].key, q[f].m.role, q[f].m);
+                push(subs[q[f].b], it.half, false, 0, kMergedSecond, q[f].m);
+            }
+        }
+        for (const auto &r : rest) {
+            bool load = true;
+            for (const Placed &o : r.second) {
+                push(subs[o.a], r.first, load, o.key, o.m.role, o.m);
+                if (o.b != none) push(subs[o.b], r.first, false, 0, kMergedSecond, o.m);
+                load = false;
+            }
+        }
+        const bool dg = has_diag && tiles[pr.first].hi == 0;
+        const bool cheap = uniform.size() == 2 && bythread.empty() && others.empty() &&
+                           uniform[0].half != uniform[1].half &&
+                           subs[uniform[0].first].off == 0 && subs[uniform[1].first].off == 0;
+        blk.push_back(make_uint4((uint32_t)tiles[pr.first].hi,
+                                 pr.second == none ? none : (uint32_t)tiles[pr.second].hi,
+                                 g0 | (uint32_t)uniform.size() << 10 | (cheap ? 1u << 30 : 0u) |
+                                     (dg ? 1u << 31 : 0u),
+                                 (uint32_t)bythread.size() | nquad << 10 |
+                                     ((uint32_t)td.size() - g0 - (uint32_t)uniform.size() -
+                                      (uint32_t)bythread.size() - 8 * nquad)
+                                         << 16));
+    }
+    *fits = coset_smem_bytes((uint32_t)td.size(), (uint32_t)blk.size(), 2, 1) <=
+            kCosetSmem;
+    if (!*fits) return QR_OK;
+    pl.ncblk = (uint32_t)blk.size();
+    pl.ncsub = (uint32_t)td.size();
+    QR_CUDA(pl.cblk.upload(blk), "upload coset blocks");
+    QR_CUDA(pl.ctdesc.upload(td), "upload coset descriptors");
+    QR_CUDA(pl.ctdata.upload(data), "upload coset tile data");
+    for (size_t i = 0; i < placed.size(); ++i) {
+        const Sub &g = *placed[i];
+        if (g.part.size() > 0xffff) return fail(QR_EINVAL, "plan: sub-group too large");
+        std::vector<uint32_t> mem(g.part.begin(), g.part.end());
+        std::vector<uint8_t> coord(g.sp.coord.begin(), g.sp.coord.end());
+        add_slot((uint64_t)pl.ctdata.p + i * sizeof(TileDataC64) + offsetof(TileDataC64, T),
+                 mem.data(), coord.data(), mem.size(), rank[i], 0);
+    }
+    return QR_OK;
+}
+
 int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows = false) {
     Plan &pl = tile_bits >= 0 ? op->bplans[tile_bits]
                : rows && dtype == QR_C64C ? op->rplans[adjoint]
@@ -682,9 +970,9 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
     pl.has_diag = !diag_terms.empty();
     // One entry per string where an x group holds about one: a string costs
     // 0.6 of a sub-group of the per-tile table kernel (n = 20, 2,000 random
-    // strings: 735 against 1,231 us) and, at up to 512 sub-groups, the paired
-    // kernel's advantage on several strings per group meets it at a third more
-    // strings than sub-groups (chain n = 22, 64 strings in 47: 111 against 109).
+    // strings: 735 against 1,231 us) and, at up to 512 sub-groups, the coset
+    // kernel is the better one from a third more strings than sub-groups on
+    // (chain n = 22, 64 strings in 47: 111 against 93).
     const size_t nstr = M - diag_terms.size();
     const double most = (subs.size() <= (size_t)kTabCap ? 1.3 : 1.6) * (double)subs.size();
     pl.strings = !pl.rows && tile_bits < 0 && n >= 12 && nstr > 0 && (double)nstr <= most;
@@ -735,141 +1023,11 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
         bhi.swap(vh);
         bg0.swap(vg);
     }
-    // pair plans: partner blocks with one sub-group are cheap to consume and
-    // a ring of three pairs cannot hide the refill behind a run of them, so
-    // the blocks are paired heavy with heavy and light with light and the
-    // heavy pairs are spread evenly among the light ones, each closing a run
-    // of light pairs (the tile's last pair is heavy, so the ring refills
-    // across the table rebuild and the next tile starts on light pairs); the
-    // same order for every output tile
-    if (f32 && tile_bits < 0 && ord.size() <= (size_t)kTabCap && bhi.size() >= 4 &&
-        pl.amps == 8) {
-        const size_t nbk = bhi.size();
-        std::vector<uint32_t> heavy, light;
-        for (uint32_t j = 0; j < nbk; ++j)
-            ((bg0[j + 1] - bg0[j] > 1 || bhi[j] == 0) ? heavy : light).push_back(j);
-        std::vector<std::vector<uint32_t>> hp, lp;
-        for (size_t i = 0; i < heavy.size(); i += 2)
-            hp.push_back(i + 1 < heavy.size() ? std::vector<uint32_t>{heavy[i], heavy[i + 1]}
-                                              : std::vector<uint32_t>{heavy[i]});
-        // an odd heavy block takes a light partner
-        size_t l0 = 0;
-        if (!hp.empty() && hp.back().size() == 1 && !light.empty()) hp.back().push_back(light[l0++]);
-        for (size_t i = l0; i < light.size(); i += 2)
-            lp.push_back(i + 1 < light.size() ? std::vector<uint32_t>{light[i], light[i + 1]}
-                                              : std::vector<uint32_t>{light[i]});
-        // a single-block pair can only be the last one
-        std::vector<uint32_t> tail;
-        if (!lp.empty() && lp.back().size() == 1) {
-            tail = lp.back();
-            lp.pop_back();
-        } else if (!hp.empty() && hp.back().size() == 1) {
-            tail = hp.back();
-            hp.pop_back();
-        }
-        std::vector<std::vector<uint32_t>> seq;
-        const size_t nh = hp.size(), tot = hp.size() + lp.size();
-        size_t ih = 0, il = 0;
-        for (size_t k = 0; k < tot; ++k) {
-            // heavy pair ih goes at position floor((ih + 1) * tot / nh) - 1
-            if (ih < nh && (il >= lp.size() || k >= (ih + 1) * tot / nh - 1))
-                seq.push_back(hp[ih++]);
-            else seq.push_back(lp[il++]);
-        }
-        if (!tail.empty()) seq.push_back(tail);
-        std::vector<size_t> nord;
-        std::vector<uint64_t> nbhi;
-        std::vector<uint32_t> nbg0;
-        for (const auto &pr : seq)
-            for (uint32_t j : pr) {
-                nbhi.push_back(bhi[j]);
-                nbg0.push_back((uint32_t)nord.size());
-                for (uint32_t g = bg0[j]; g < bg0[j + 1]; ++g) nord.push_back(ord[g]);
-            }
-        nbg0.push_back((uint32_t)nord.size());
-        ord.swap(nord);
-        bhi.swap(nbhi);
-        bg0.swap(nbg0);
-    }
     pl.nblocks = (uint32_t)bhi.size();
     pl.ngroups = ord.size();
     pl.diag_block = -1;
     for (size_t j = 0; j < bhi.size(); ++j)
         if (bhi[j] == 0 && pl.diag_block < 0) pl.diag_block = (int)j;
-
-    // single-chunk c64c plans: partner blocks are visited in pairs (two
-    // stages behind one barrier, one ring slot); each pair's sub-groups are
-    // merged and sorted by run key, their block recorded as the half
-    std::vector<uint32_t> half(ord.size(), 0u), pg0, pkey;
-    pl.npairs = 0;
-    if (f32 && tile_bits < 0 && ord.size() <= (size_t)kTabCap && pl.nblocks >= 2 &&
-        pl.amps == 8) {
-        const uint32_t np = (pl.nblocks + 1) / 2;
-        std::vector<size_t> ord2;
-        std::vector<uint32_t> half2;
-        ord2.reserve(ord.size());
-        const uint64_t tm = (uint64_t)pl.threads - 1;
-        auto small = [&](const SubGroup &g) { return g.d != kFat && g.d <= 2; };
-        auto thread_var = [&](const SubGroup &g) -> uint32_t {
-            const uint64_t b0 = g.d > 0 ? g.beta[0] : 0, b1 = g.d > 1 ? g.beta[1] : 0;
-            return ((g.z0 | b0 | b1) & tm) != 0 ? 1u : 0u;
-        };
-        for (uint32_t p = 0; p < np; ++p) {
-            pg0.push_back((uint32_t)ord2.size());
-            const uint32_t ga = bg0[2 * p], gm = bg0[std::min(2 * p + 1, pl.nblocks)],
-                           gb = bg0[std::min(2 * p + 2, pl.nblocks)];
-            // fused pairs: two sub-groups of one x group (same partner
-            // amplitudes) whose register-bit sign patterns differ in one bit
-            std::vector<uint32_t> items;
-            std::vector<char> used(gb - ga, 0);
-            struct Fused { uint32_t key, a, b; };
-            std::vector<Fused> fused;
-            for (uint32_t i = ga; i < gb; ++i) {
-                const SubGroup &si = subs[ord[i]];
-                if (used[i - ga]) continue;
-                for (uint32_t j = i + 1; j < gb && small(si); ++j) {
-                    const SubGroup &sj = subs[ord[j]];
-                    if (used[j - ga] || !small(sj) || si.hi != sj.hi || si.lo != sj.lo ||
-                        (i >= gm) != (j >= gm))
-                        continue;
-                    const uint32_t diff = si.zm ^ sj.zm;
-                    if (__builtin_popcount(diff) != 1) continue;
-                    const uint32_t a = si.zm < sj.zm ? i : j, b = si.zm < sj.zm ? j : i;
-                    const uint32_t bb = (uint32_t)__builtin_ctz(diff);
-                    const uint32_t xm = (si.lo >> pl.tb) != 0 ? 1u : 0u;
-                    const uint32_t tv = thread_var(si) | thread_var(sj);
-                    // key 64 + (ZM | BB << 3 | XM << 5 | TV << 6): 64..191
-                    fused.push_back({64u + ((subs[ord[a]].zm & 7u) | (bb << 3) | (xm << 5) |
-                                            (tv << 6)),
-                                     a, b});
-                    used[i - ga] = used[j - ga] = 1;
-                    break;
-                }
-                if (!used[i - ga]) items.push_back(i);
-            }
-            std::stable_sort(items.begin(), items.end(), [&](uint32_t x, uint32_t y) {
-                return runkey(subs[ord[x]]) < runkey(subs[ord[y]]);
-            });
-            std::stable_sort(fused.begin(), fused.end(),
-                             [](const Fused &x, const Fused &y) { return x.key < y.key; });
-            for (uint32_t i : items) {
-                ord2.push_back(ord[i]);
-                half2.push_back(i >= gm ? 1u : 0u);
-                pkey.push_back(runkey(subs[ord[i]]) & 63u);
-            }
-            for (const Fused &f : fused) {
-                for (uint32_t i : {f.a, f.b}) {
-                    ord2.push_back(ord[i]);
-                    half2.push_back(i >= gm ? 1u : 0u);
-                    pkey.push_back(f.key);
-                }
-            }
-        }
-        pg0.push_back((uint32_t)ord2.size());
-        ord.swap(ord2);
-        half.swap(half2);
-        pl.npairs = np;
-    }
 
     pl.nfat = 0;
     if (pl.rows) {
@@ -881,8 +1039,13 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
         const int rc = build_strings(op, pl, c, diag_terms, add_slot);
         if (rc) return rc;
     }
+    pl.cosets = false;
+    if (f32 && !pl.rows && !pl.strings && tile_bits < 0 && n >= 12) {
+        const int rc = build_cosets(op, pl, c, gxs, members, pl.has_diag, &pl.cosets, add_slot);
+        if (rc) return rc;
+    }
     pl.nsub = (uint32_t)ord.size();
-    if (!pl.rows && !pl.strings) {
+    if (!pl.rows && !pl.strings && !pl.cosets) {
         // per-tile-table kernel arrays
         std::vector<uint4> td;
         std::vector<TileDataC64> tdd;
@@ -900,7 +1063,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
             // threads == 1 << kC64ThreadBits whenever lo has register bits
             const uint32_t lt = (uint32_t)(sg.lo & tmask_t), lm = sg.lo >> pl.tb;
             const uint32_t dx = (lt << 3) | (lm << (pl.tb + 3));
-            td.push_back(make_uint4(dx | (half[i] << 15) | (tvar << 31), zt, bt0, bt1));
+            td.push_back(make_uint4(dx | (tvar << 31), zt, bt0, bt1));
             TileDataC64 d;
             memset(&d, 0, sizeof(d));
             d.z0h = sg.z0 >> pl.b;
@@ -910,15 +1073,12 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
                 d.T[u] = make_float2((float)sg.table[u].re, (float)sg.table[u].im);
             tdd.push_back(d);
         }
-        // runs per block, or per pair of blocks
-        const std::vector<uint32_t> &rng = pl.npairs ? pg0 : bg0;
-        const uint32_t nunits = pl.npairs ? pl.npairs : pl.nblocks;
-        for (uint32_t j = 0; j < nunits; ++j) {
+        // runs per block
+        for (uint32_t j = 0; j < pl.nblocks; ++j) {
             r0v.push_back((uint32_t)rkey.size());
-            for (uint32_t g = rng[j]; g < rng[j + 1]; ++g) {
-                // pair plans: per-position keys (fused pairs carry keys >= 64)
-                const uint32_t k = pl.npairs ? pkey[g] : (runkey(subs[ord[g]]) & 63u);
-                if (g == rng[j] || k != rkey.back()) {
+            for (uint32_t g = bg0[j]; g < bg0[j + 1]; ++g) {
+                const uint32_t k = runkey(subs[ord[g]]) & 63u;
+                if (g == bg0[j] || k != rkey.back()) {
                     rkey.push_back(k);
                     rg0.push_back(g);
                 }
@@ -951,23 +1111,6 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
                 return fail(QR_EINVAL, "plan: sub-group of rank > 2 in a complex64 plan");
             add_slot((uint64_t)pl.tdata.p + i * sizeof(TileDataC64) + offsetof(TileDataC64, T),
                      sg.mem.data(), sg.coord.data(), sg.mem.size(), sg.d, 0);
-        }
-        // pair plans: bit 31 of a pair's first run marks a pair of exactly two
-        // sub-groups with key 0 (no sign pattern, no register-bit XOR, factor
-        // constant over the threads), which the kernel runs without the run
-        // list; bit 30 in addition when the two sit in halves 0 and 1 and
-        // neither permutes the partner tile (x & (tile - 1) == 0), so that
-        // their partner offsets are known at compile time
-        if (pl.npairs) {
-            for (uint32_t j = 0; j < pl.npairs; ++j) {
-                const uint32_t a0 = pg0[j], a1 = pg0[j] + 1;
-                if (pg0[j + 1] - pg0[j] == 2 && pkey[a0] == 0 && pkey[a1] == 0) {
-                    r0v[j] |= 0x80000000u;
-                    if (subs[ord[a0]].lo == 0 && subs[ord[a1]].lo == 0 && half[a0] == 0 &&
-                        half[a1] == 1)
-                        r0v[j] |= 0x40000000u;
-                }
-            }
         }
         QR_CUDA(pl.blk_r0.upload(r0v), "upload block runs");
         QR_CUDA(pl.run_g0.upload(rg0), "upload runs");
@@ -1394,7 +1537,11 @@ static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *ps
     a.nruns = pl.nruns;
     a.chunks = pl.chunks.as<uint4>();
     a.nchunks = pl.nchunks;
-    a.npairs = pl.npairs;
+    a.cblk = pl.cblk.as<uint4>();
+    a.ctdesc = pl.ctdesc.as<uint4>();
+    a.ctdata = pl.ctdata.as<TileDataC64>();
+    a.ncblk = pl.ncblk;
+    a.ncsub = pl.ncsub;
     a.ent = pl.ent.as<uint4>();
     a.sblk = pl.sblk.as<uint4>();
     a.wait_ns = op->test_wait_ns ? op->test_wait_ns : kDefaultWaitNs;
@@ -1413,6 +1560,8 @@ static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *ps
     else if (pl.strings)
         QR_CUDA(launch_c64c_strings(a, pl.str, (uint64_t)call_states * a.ntiles, op->nsm, st),
                 "apply launch");
+    else if (pl.cosets)
+        QR_CUDA(launch_c64c_cosets(a, op->nsm, st), "apply launch");
     else
         QR_CUDA(launch_apply(a, pl.amps, pl.threads, op->nsm, st), "apply launch");
     return QR_OK;
