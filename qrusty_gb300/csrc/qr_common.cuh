@@ -342,7 +342,7 @@ cudaError_t launch_op_diag(uint64_t N, uint32_t nt, const uint64_t *tz, const do
 uint32_t vdot_blocks(uint64_t N, int nsm);
 cudaError_t launch_vdot(int dtype, uint64_t N, const void *a, const void *b, int nstates,
                         double2 *partial, uint32_t nblk, double2 *out, cudaStream_t st);
-// Term gradients.  Strings of x groups of kGradWhtMin or more go through a
+// Term gradients.  complex128 strings of x groups of kGradWhtMin or more go through a
 // Walsh-Hadamard transform per 256 rows (wht: batches of up to kGradWhtBatch
 // strings of one x), the others one by one (direct: by partner tile x >> 12 for
 // the tiled complex64 kernel, n >= 12).  perm: merged index of each; partial

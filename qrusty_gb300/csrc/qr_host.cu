@@ -168,10 +168,12 @@ struct qr_op {
     bool csr_ready = false;
     uint32_t nfold = 0, nctab = 0;
     DevBuf d_tc, d_pmask, d_sig, d_grp, d_coord, d_ctab, d_fold, d_pbeta, d_ptab, d_fv;
-    // term-gradient strings (see GradPlanArgs), built on first use
-    bool tg_ready = false;
-    uint32_t tg_ndirect = 0, tg_nbatch = 0, tg_nwht = 0, tg_nwbatch = 0;
-    DevBuf d_tg_x, d_tg_z, d_tg_perm, d_tg_bat, d_tg_wz, d_tg_wperm, d_tg_wbat;
+    // term-gradient strings (see GradPlanArgs) per dtype, built on first use
+    struct GradPlan {
+        bool ready = false;
+        uint32_t ndirect = 0, nbatch = 0, nwht = 0, nwbatch = 0;
+        DevBuf x, z, perm, bat, wz, wperm, wbat;
+    } tg[2];
     DevBuf expect_y;                    // H psi buffer of qr_expect
     Plan plans[2][2];  // [dtype][adjoint]
     Plan rplans[2];    // complex64 over rows, for calls of few rows [adjoint]
@@ -1865,15 +1867,16 @@ int qr_term_grad(qr_op *op, int32_t dtype, const void *psi, const void *g, int32
     int rc = check_device(op);
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (!op->tg_ready) {
-        // x groups of many strings to the transform, the others in order of
+    qr_op::GradPlan &tg = op->tg[dtype];
+    if (!tg.ready) {
+        // complex128: x groups of many strings to the transform; the others in order of
         // partner tile, input order kept within one; batches of <= 8 never
         // span two partner tiles, largest first
         std::vector<uint32_t> ord, word;
         std::vector<GradBatch> wb;
         for (size_t g = 0; g < op->Ga; ++g) {
             const uint32_t a0 = op->ag_off[g], a1 = op->ag_off[g + 1];
-            if (a1 - a0 < kGradWhtMin) {
+            if (dtype != QR_C128 || a1 - a0 < kGradWhtMin) {
                 ord.insert(ord.end(), op->ag_mem.begin() + a0, op->ag_mem.begin() + a1);
                 continue;
             }
@@ -1903,47 +1906,47 @@ int qr_term_grad(qr_op *op, int32_t dtype, const void *psi, const void *g, int32
         }
         std::stable_sort(bat.begin(), bat.end(),
                          [](const uint2 &a, const uint2 &b) { return a.y > b.y; });
-        QR_CUDA(op->d_tg_x.upload(sx), "upload gradient strings");
-        QR_CUDA(op->d_tg_z.upload(sz), "upload gradient strings");
-        QR_CUDA(op->d_tg_perm.upload(ord), "upload gradient order");
-        QR_CUDA(op->d_tg_bat.upload(bat), "upload gradient batches");
-        QR_CUDA(op->d_tg_wz.upload(wz), "upload gradient strings");
-        QR_CUDA(op->d_tg_wperm.upload(word), "upload gradient order");
-        QR_CUDA(op->d_tg_wbat.upload(wb), "upload gradient batches");
-        op->tg_ndirect = nd;
-        op->tg_nbatch = (uint32_t)bat.size();
-        op->tg_nwht = (uint32_t)word.size();
-        op->tg_nwbatch = (uint32_t)wb.size();
-        op->tg_ready = true;
+        QR_CUDA(tg.x.upload(sx), "upload gradient strings");
+        QR_CUDA(tg.z.upload(sz), "upload gradient strings");
+        QR_CUDA(tg.perm.upload(ord), "upload gradient order");
+        QR_CUDA(tg.bat.upload(bat), "upload gradient batches");
+        QR_CUDA(tg.wz.upload(wz), "upload gradient strings");
+        QR_CUDA(tg.wperm.upload(word), "upload gradient order");
+        QR_CUDA(tg.wbat.upload(wb), "upload gradient batches");
+        tg.ndirect = nd;
+        tg.nbatch = (uint32_t)bat.size();
+        tg.nwht = (uint32_t)word.size();
+        tg.nwbatch = (uint32_t)wb.size();
+        tg.ready = true;
     }
     GradPlanArgs p{};
-    p.sx = op->d_tg_x.as<uint64_t>();
-    p.sz = op->d_tg_z.as<uint64_t>();
-    p.batches = op->d_tg_bat.as<uint2>();
-    p.nbatch = op->tg_nbatch;
-    p.wz = op->d_tg_wz.as<uint64_t>();
-    p.wbatches = op->d_tg_wbat.as<GradBatch>();
-    p.nwbatch = op->tg_nwbatch;
+    p.sx = tg.x.as<uint64_t>();
+    p.sz = tg.z.as<uint64_t>();
+    p.batches = tg.bat.as<uint2>();
+    p.nbatch = tg.nbatch;
+    p.wz = tg.wz.as<uint64_t>();
+    p.wbatches = tg.wbat.as<GradBatch>();
+    p.nwbatch = tg.nwbatch;
     const bool tiles = dtype == QR_C64C && op->n >= 12;
     uint64_t nchunk = 1, nwchunk = 1;
-    if (op->tg_ndirect > 0) {
+    if (tg.ndirect > 0) {
         // about 8 work items (4 strings each, or a batch of the tiled kernel)
         // per SM, chunks of at least 16 tiles or 4,096 rows
-        const uint64_t items = tiles ? op->tg_nbatch : (op->tg_ndirect + 3) / 4;
+        const uint64_t items = tiles ? tg.nbatch : (tg.ndirect + 3) / 4;
         const uint64_t most = tiles ? (op->N >> 12) * (uint64_t)nstates / 16 : op->N / 4096;
         nchunk = std::min(((uint64_t)op->nsm * 8 + items - 1) / items, most);
         if (nchunk < 1) nchunk = 1;
     }
-    if (op->tg_nwbatch > 0) {
+    if (tg.nwbatch > 0) {
         // about 4 CTAs per SM, each of at least 8 blocks of 256 rows
         const uint64_t blocks = std::max<uint64_t>(op->N / 256, 1) * (uint64_t)nstates;
-        nwchunk = std::min(((uint64_t)op->nsm * 4 + op->tg_nwbatch - 1) / op->tg_nwbatch,
+        nwchunk = std::min(((uint64_t)op->nsm * 4 + tg.nwbatch - 1) / tg.nwbatch,
                            (blocks + 7) / 8);
     }
-    p.direct = GradStrings{op->d_tg_perm.as<uint32_t>(), op->tg_ndirect, (uint32_t)nchunk};
-    p.wht = GradStrings{op->d_tg_wperm.as<uint32_t>(), op->tg_nwht, (uint32_t)nwchunk};
+    p.direct = GradStrings{tg.perm.as<uint32_t>(), tg.ndirect, (uint32_t)nchunk};
+    p.wht = GradStrings{tg.wperm.as<uint32_t>(), tg.nwht, (uint32_t)nwchunk};
     void *scratch = nullptr;
-    const size_t np = (size_t)op->tg_ndirect * nchunk + (size_t)op->tg_nwht * nwchunk;
+    const size_t np = (size_t)tg.ndirect * nchunk + (size_t)tg.nwht * nwchunk;
     QR_CUDA(cudaMallocAsync(&scratch, np * sizeof(double2) + 16, st), "term-grad scratch");
     double2 *partial = static_cast<double2 *>(scratch);
     auto *counter = reinterpret_cast<unsigned long long *>(partial + np);

@@ -124,13 +124,19 @@ template <> struct GradT<false> {
     using A = double;
 };
 
-// Accumulate (-1)^popc(r & z) conj(p) g into (ar, ai): four multiply-adds, the
-// sign on p's bits (FP64 is the bound of the complex128 form).
-template <typename A, typename V>
-__device__ __forceinline__ void grad_acc(A &ar, A &ai, V p, V gg, bool neg) {
-    const A px = flip(p.x, neg), py = flip(p.y, neg);
+// Accumulate (-1)^popc(r & z) conj(p) g into (ar, ai).  complex128, bound by
+// FP64: four multiply-adds, the sign on p's bits.  complex64: the product
+// rounded to FP32, then added.
+__device__ __forceinline__ void grad_acc(double &ar, double &ai, double2 p, double2 gg, bool neg) {
+    const double px = flip(p.x, neg), py = flip(p.y, neg);
     ar = fma(px, gg.x, fma(py, gg.y, ar));
     ai = fma(px, gg.y, fma(-py, gg.x, ai));
+}
+__device__ __forceinline__ void grad_acc(float &ar, float &ai, float2 p, float2 gg, bool neg) {
+    const float pr = p.x * gg.x + p.y * gg.y;
+    const float pi = p.x * gg.y - p.y * gg.x;
+    ar += neg ? -pr : pr;
+    ai += neg ? -pi : pi;
 }
 
 // partial[m * gridDim.x + blockIdx.x] = the chunk's sum over rows r and states
@@ -176,8 +182,8 @@ __global__ void __launch_bounds__(kRedThreads) term_grad_partial_kernel(
                     for (int k = 0; k < kGradK; ++k) {
                         if ((uint32_t)k < kv) {
                             const V p1 = psi[r ^ x[k]], p2 = psi[r2 ^ x[k]];
-                            grad_acc<A, V>(fr[k], fi[k], p1, g1, parity_of(r & z[k]));
-                            grad_acc<A, V>(fr[k], fi[k], p2, g2, parity_of(r2 & z[k]));
+                            grad_acc(fr[k], fi[k], p1, g1, parity_of(r & z[k]));
+                            grad_acc(fr[k], fi[k], p2, g2, parity_of(r2 & z[k]));
                         }
                     }
                     if (F32 && ++cnt == kGradPerThread / 2) {  // 2 rows per step
@@ -195,7 +201,7 @@ __global__ void __launch_bounds__(kRedThreads) term_grad_partial_kernel(
 #pragma unroll
                     for (int k = 0; k < kGradK; ++k)
                         if ((uint32_t)k < kv)
-                            grad_acc<A, V>(fr[k], fi[k], psi[r ^ x[k]], g1, parity_of(r & z[k]));
+                            grad_acc(fr[k], fi[k], psi[r ^ x[k]], g1, parity_of(r & z[k]));
                 }
 #pragma unroll
                 for (int k = 0; k < kGradK; ++k) {
@@ -262,16 +268,15 @@ __global__ void __launch_bounds__(kRedThreads) term_grad_finish_kernel(
 constexpr int kWhtPerLane = 8;  // strings per lane
 static_assert(kGradWhtBatch == 32 * kWhtPerLane, "strings of a batch");
 
-template <bool F32, bool WIDE>
+template <bool WIDE>
 __global__ void __launch_bounds__(kRedThreads) term_grad_wht_kernel(
     uint64_t N, int nstates, const GradBatch *batches, uint32_t nbatch, const uint64_t *sz,
-    const void *psi_, const void *g_, double2 *partial) {
+    const double2 *psi_, const double2 *g_, double2 *partial) {
     using W = typename std::conditional<WIDE, uint64_t, uint32_t>::type;
-    using V = typename GradT<F32>::V;
     constexpr int kWarps = kRedThreads / 32;
     __shared__ double2 s_red[kWarps][kGradWhtBatch];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    V *coef = reinterpret_cast<V *>(s_red[warp]);  // 256 coefficients of this warp
+    double2 *coef = s_red[warp];  // 256 coefficients of this warp
     const uint64_t per_state = N >= 256 ? N / 256 : 1, nblk = per_state * (uint64_t)nstates;
     for (uint32_t bi = blockIdx.y; bi < nbatch; bi += gridDim.y) {
         const GradBatch bt = batches[bi];
@@ -288,15 +293,15 @@ __global__ void __launch_bounds__(kRedThreads) term_grad_wht_kernel(
              b += (uint64_t)gridDim.x * kWarps) {
             const uint64_t st = b / per_state;
             const W base = (W)((b - st * per_state) * 256);
-            const V *psi = static_cast<const V *>(psi_) + st * N;
-            const V *g = static_cast<const V *>(g_) + st * N;
-            V h[8];
+            const double2 *psi = psi_ + st * N;
+            const double2 *g = g_ + st * N;
+            double2 h[8];
 #pragma unroll
             for (int m = 0; m < 8; ++m) {
                 const W r = base + lane + 32u * m;
-                h[m].x = h[m].y = 0;
+                h[m].x = h[m].y = 0.0;
                 if ((uint64_t)r < N) {
-                    const V p = psi[r ^ x], v = g[r];
+                    const double2 p = psi[r ^ x], v = g[r];
                     h[m].x = fma(p.x, v.x, p.y * v.y);
                     h[m].y = fma(p.x, v.y, -p.y * v.x);
                 }
@@ -306,7 +311,7 @@ __global__ void __launch_bounds__(kRedThreads) term_grad_wht_kernel(
 #pragma unroll
                 for (int m = 0; m < 8; ++m) {
                     if (m & l) continue;
-                    const V u = h[m], v = h[m | l];
+                    const double2 u = h[m], v = h[m | l];
                     h[m].x = u.x + v.x;
                     h[m].y = u.y + v.y;
                     h[m | l].x = u.x - v.x;
@@ -318,8 +323,8 @@ __global__ void __launch_bounds__(kRedThreads) term_grad_wht_kernel(
                 const bool up = (lane & o) != 0;
 #pragma unroll
                 for (int m = 0; m < 8; ++m) {
-                    const auto px = __shfl_xor_sync(0xffffffffu, h[m].x, o);
-                    const auto py = __shfl_xor_sync(0xffffffffu, h[m].y, o);
+                    const double px = __shfl_xor_sync(0xffffffffu, h[m].x, o);
+                    const double py = __shfl_xor_sync(0xffffffffu, h[m].y, o);
                     h[m].x = px + flip(h[m].x, up);
                     h[m].y = py + flip(h[m].y, up);
                 }
@@ -331,10 +336,10 @@ __global__ void __launch_bounds__(kRedThreads) term_grad_wht_kernel(
 #pragma unroll
             for (int j = 0; j < kWhtPerLane; ++j) {
                 if (32u * j >= bt.count) break;
-                const V c = coef[(uint32_t)z[j] & 255u];
+                const double2 c = coef[(uint32_t)z[j] & 255u];
                 const uint32_t neg = parity_of((W)(base & z[j])) ? 1u : 0u;
-                acc[j].x += (double)flip(c.x, neg);
-                acc[j].y += (double)flip(c.y, neg);
+                acc[j].x += flip(c.x, neg);
+                acc[j].y += flip(c.y, neg);
             }
         }
         __syncthreads();  // every warp is done with its coefficients
@@ -353,7 +358,7 @@ __global__ void __launch_bounds__(kRedThreads) term_grad_wht_kernel(
     }
 }
 
-static cudaError_t launch_wht_finish(int dtype, uint64_t N, int nstates, const GradPlanArgs &p,
+static cudaError_t launch_wht_finish(uint64_t N, int nstates, const GradPlanArgs &p,
                                      const void *psi, const void *g, double2 *partial,
                                      const uint32_t *mm_off, const uint32_t *mm_terms,
                                      const uint8_t *phase, double2 *out, cudaStream_t st) {
@@ -361,11 +366,10 @@ static cudaError_t launch_wht_finish(int dtype, uint64_t N, int nstates, const G
         double2 *wp = partial + (size_t)p.direct.count * p.direct.nchunk;
         const dim3 grid(p.wht.nchunk, p.nwbatch < 65535u ? p.nwbatch : 65535u);
         const bool wide = N >= (1ull << 32);
-        auto kern = dtype == 1 ? (wide ? term_grad_wht_kernel<true, true>
-                                       : term_grad_wht_kernel<true, false>)
-                               : (wide ? term_grad_wht_kernel<false, true>
-                                       : term_grad_wht_kernel<false, false>);
-        kern<<<grid, kRedThreads, 0, st>>>(N, nstates, p.wbatches, p.nwbatch, p.wz, psi, g, wp);
+        auto kern = wide ? term_grad_wht_kernel<true> : term_grad_wht_kernel<false>;
+        kern<<<grid, kRedThreads, 0, st>>>(N, nstates, p.wbatches, p.nwbatch, p.wz,
+                                           static_cast<const double2 *>(psi),
+                                           static_cast<const double2 *>(g), wp);
         count_launch();
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
@@ -666,7 +670,7 @@ cudaError_t launch_term_grad_tiles(uint64_t N, int nstates, const GradPlanArgs &
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    return launch_wht_finish(1, N, nstates, p, psi, g, partial, mm_off, mm_terms, phase, out, st);
+    return launch_wht_finish(N, nstates, p, psi, g, partial, mm_off, mm_terms, phase, out, st);
 }
 
 cudaError_t launch_term_grad(int dtype, uint64_t N, int nstates, const GradPlanArgs &p,
@@ -689,8 +693,7 @@ cudaError_t launch_term_grad(int dtype, uint64_t N, int nstates, const GradPlanA
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    return launch_wht_finish(dtype, N, nstates, p, psi, g, partial, mm_off, mm_terms, phase, out,
-                             st);
+    return launch_wht_finish(N, nstates, p, psi, g, partial, mm_off, mm_terms, phase, out, st);
 }
 
 }  // namespace qr
