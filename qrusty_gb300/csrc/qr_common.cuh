@@ -266,6 +266,7 @@ struct CsrArgs {
     const CsrGroup *grp;      // G
     const uint64_t *pmask;    // G: bits b with a nonzero sigma_{g,b}
     const int32_t *sig;       // G x n: sigma_{g,b} (0 where b is not in pmask)
+    const uint16_t *tables;   // position and class terms by row bits (G <= 256)
     const uint32_t *fold;     // groups in fold mode
     uint32_t nfold;
     const double2 *ctab;      // class tables
@@ -275,6 +276,7 @@ struct CsrArgs {
     const uint64_t *pbeta;    // nfold x kCsrPrefixRank: prefix span bases (fold mode)
     const double2 *ptab;      // prefix class tables (fold mode)
     double2 *fvals;           // nfold x nrows fold-mode values, or null (written in place)
+    int inline_fold;          // fold-mode entries folded by the staged fill (fvals null)
     uint64_t *indptr, *indices;
     double *data;
     uint64_t row0, nrows;     // rows to fill
@@ -282,6 +284,12 @@ struct CsrArgs {
     int wide;                 // 64-bit row words (the n > 32 kernels) forced (test hook)
 };
 cudaError_t launch_csr_fill(const CsrArgs &a, int nsm, cudaStream_t st);
+// Whether the staged fill folds nfold fold-mode groups of at most fold_rem
+// terms past their prefix itself (no value buffer).
+bool csr_inline_fold(uint64_t G, int n, uint32_t nfold, uint32_t fold_rem);
+// The staged fill's mask tables (a.tables, csr_tables_bytes), once per operator.
+size_t csr_tables_bytes(uint64_t G, int n);
+cudaError_t launch_csr_tables(const CsrArgs &a, cudaStream_t st);
 
 // qr_group.cu: term grouping on the device.  Buffers sized for T terms (the
 // group counts are bounded by T).
@@ -316,6 +324,7 @@ struct CsrStructOut {
 struct CsrStructCounts {
     uint64_t nctab = 0, nptab = 0;
     uint32_t nfold = 0;
+    uint32_t fold_rem = 0;  // fold-mode groups: most terms past the prefix
 };
 // Mask-only CSR tables; synchronises st and returns the table sizes.
 cudaError_t csr_structure(int n, uint64_t G, const uint64_t *gx, const uint32_t *goff,

@@ -225,208 +225,552 @@ __device__ __forceinline__ double2 csr_fold_row(const CsrArgs &a, uint64_t r, co
     return make_double2(vr, vi);
 }
 
+__device__ __forceinline__ double2 csr_fold_entry(const CsrArgs &a, uint64_t r, const CsrGroup &d,
+                                                  uint32_t f) {
+    switch (d.zparts & 3u) {  // warp-uniform
+        case 1: return csr_fold_row<true, false>(a, r, d, f);
+        case 2: return csr_fold_row<false, true>(a, r, d, f);
+        case 3: return csr_fold_row<true, true>(a, r, d, f);
+        default: return csr_fold_row<false, false>(a, r, d, f);
+    }
+}
+
 // ------------------------------------------------------------ staged fill
 // Rows are assembled in shared memory and leave the SM as contiguous TMA
 // bulk stores (cp.async.bulk shared -> global): a warp's entries of one row
 // land at permuted positions, which as direct global stores become many
-// partial-line L2 writes.  Two staging buffers of R rows (R a power of two
-// dividing the 2^L-row chunk) alternate, so the bulk store of one overlaps
-// the assembly of the next.  Fold-mode groups (per-row FP64 folds) are
-// computed first by csr_fold_kernel<true> into a row-major value buffer and
-// copied into the stage here: folded inside the staged pass, their serial
-// chains would hold every warp of the block at the sub-chunk barrier, and
-// stored in place after it, each entry becomes a DRAM read-modify-write of
-// a line the bulk store has already evicted.  Without a value buffer the
-// fold entries are left unset and stored afterwards by csr_fold_kernel<false>.
-constexpr size_t kCsrStageBytes = 24u * 1024u;  // one buffer: R rows x G x (8 + 16) bytes
-constexpr uint32_t kCsrFvSlots = 4;              // fold-value ring depth (sub-chunks)
+// partial-line L2 writes.  Three staging buffers of R rows: one barrier per
+// stage, and a buffer's bulk store has a whole stage to finish reading it.
+// Eight warps assemble class-table entries; a ninth issues the bulk stores
+// and folds the entries of a short fold-mode group (csr_inline_fold).  Other
+// folds are computed first by csr_fold_kernel<true> into a row-major value
+// buffer and placed from there: their serial chains would hold the block at
+// the barrier, and stored in place after the fill each entry becomes a DRAM
+// read-modify-write of a line the bulk store has already evicted.  Without a
+// value buffer they are left unset and stored afterwards by
+// csr_fold_kernel<false>.  Which of these a launch needs is a template
+// argument: the code of all three in one body costs 10 %.
+//
+// Bound by the write stream (2.11 GB at chain n = 21, 42 groups: 271 us at
+// the rate of a device fill), so the order of the writes counts: blocks that
+// stride or halve the rows by a fixed rule finish unevenly and reach
+// 6.6 TB/s with any stage size, blocks that take the next piece of rows as
+// they get free 7.7.  Hence one block per unit of about 128 KB, and a resident
+// block goes on with the next unit that has not started
+// (clusterlaunchcontrol), which keeps its tables.  What is left above the
+// write stream's time is a stage's barrier, stores and bookkeeping: chain
+// n = 21 takes 336 us (two-buffer stages over fixed strides, per-chunk sums
+// in every thread and a fold kernel before it: 487), random strings n = 16,
+// 200 groups, 55 us (67).
+constexpr uint32_t kCsrBufs = 3;  // staging buffers
+constexpr int kCsrStageThreads = kCsrThreads + 32;
+constexpr size_t kCsrStageBytes = 16896u;  // one buffer, at most: R rows x G x (8 + 16) bytes
+constexpr size_t kCsrUnitBytes = 131072u;   // output of one unit, about
+constexpr size_t kCsrLowBytes = 9u * 1024u, kCsrTableBytes = 26u * 1024u;
+constexpr int kCsrChunkBits = 6;        // chunk rows of the inline fold: two per lane of its warp
+constexpr uint32_t kCsrRingItems = 256;  // value-buffer entries of a chunk kept ahead, at most
+constexpr uint32_t kCsrInlineRem = 64;  // its terms past the prefix, at most
 
-__host__ __device__ inline int csr_stage_rows(uint32_t G, int L) {
-    int R = 1 << L;
-    while (R > 2 && (size_t)R * G * 24u > kCsrStageBytes) R >>= 1;
-    return R;
+// Chunk and stage of the staged fill.  A chunk is 2^L rows.  What a row's bits
+// add to a group's position and class comes from tables of one 16-bit word
+// per (group, bits): position term (11 bits, signed) and class term (5 bits),
+// rows padded to an odd number of 32-bit words; one table for the low L bits
+// and `up` tables for U bits each above them (bits above those are summed per
+// chunk).  For the inline fold the same split holds the parities that pick
+// prefix class and term signs.  The tables depend on masks only and are
+// written once per operator (csr_tables_kernel).  A stage holds R rows (even,
+// so that bulk stores are whole 16-byte units), the chunk in equal parts.
+struct CsrStage {
+    int L, U, up;
+    uint32_t R, lsz, usz;  // lsz, usz: 16-bit words of a group's table row
+    uint32_t ups, ups_sz;  // first upper table, words of one
+    uint32_t cls, sgn, bytes;  // byte offsets of the inline folds' classes and signs; table bytes
+    // byte offsets in shared memory (class table: 0 where it stays in global memory)
+    uint32_t ctab, tc, bufs, buf_bytes, fold, fphi, fval, total;
+    bool ring;  // value-buffer entries pass through shared memory
+};
+__host__ __device__ inline uint32_t csr_align(size_t b, uint32_t to) {
+    return ((uint32_t)b + to - 1u) & ~(to - 1u);
+}
+__host__ __device__ inline CsrStage csr_stage(uint32_t G, int n, uint32_t nctab, uint32_t nfv) {
+    CsrStage s;
+    // 64 rows where they fill a stage
+    s.L = (size_t)G * 24u << kCsrChunkBits >= kCsrStageBytes ? kCsrChunkBits : 8;
+    while (s.L > 1 && (size_t)G * ((1u << s.L) + 2) * 2u > kCsrLowBytes) --s.L;
+    s.U = s.L > 1 ? s.L - 1 : 1;
+    s.lsz = (1u << s.L) + 2;
+    s.usz = (1u << s.U) + 2;
+    s.ups = csr_align((size_t)G * s.lsz, 8);
+    s.ups_sz = csr_align((size_t)G * s.usz, 8);
+    s.up = 0;
+    while (s.L + s.up * s.U < n &&
+           ((size_t)s.ups + (size_t)(s.up + 1) * s.ups_sz) * 2u <= kCsrTableBytes)
+        ++s.up;
+    const uint32_t words = (1u << s.L) + (uint32_t)s.up * (1u << s.U);
+    s.cls = (s.ups + (uint32_t)s.up * s.ups_sz) * 2u;
+    s.sgn = csr_align(s.cls + words * 2u, 16);
+    s.bytes = csr_align(s.sgn + words * 8u, 16);
+    const uint32_t rows = 1u << s.L;
+    uint32_t most = (uint32_t)(kCsrStageBytes / ((size_t)G * 24u)) & ~1u;
+    if (most < 2) most = 2;
+    const uint32_t parts = (rows + most - 1) / most;
+    s.R = ((rows + parts - 1) / parts + 1u) & ~1u;
+    const bool ct = nctab <= kCsrSmemCtab;
+    s.ctab = ct ? s.bytes : 0u;
+    s.tc = s.bytes + (ct ? nctab * (uint32_t)sizeof(double2) : 0u);
+    s.bufs = csr_align(s.tc + kCsrInlineRem * sizeof(double2), 128);
+    s.buf_bytes = csr_align((size_t)s.R * G * 24u, 128);
+    // value buffer: the groups' x and index, and for two chunks their position
+    // terms and values
+    s.fold = s.bufs + kCsrBufs * s.buf_bytes;
+    s.fphi = s.fold + nfv * 12u;
+    s.fval = csr_align(s.fphi + 2u * nfv * sizeof(int32_t), 16);
+    s.ring = nfv > 0 && (nfv << s.L) <= kCsrRingItems;
+    s.total = s.fval + (s.ring ? 2u * (nfv << s.L) * (uint32_t)sizeof(double2) : 0u);
+    return s;
+}
+// Chunks of one unit: about kCsrUnitBytes of output, fewer where the rows
+// would leave SMs idle.
+__host__ __device__ inline uint32_t csr_unit_chunks(uint32_t G, int L, uint64_t nchunk, int nsm) {
+    uint64_t q = kCsrUnitBytes / (((size_t)G * 24u) << L);
+    if (q > nchunk / (2u * (uint32_t)nsm)) q = nchunk / (2u * (uint32_t)nsm);
+    return q < 1 ? 1u : (uint32_t)q;
 }
 
-__device__ __forceinline__ uint32_t csr_saddr(const void *p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
+// A fold-mode group inside the staged fill: one warp per CTA folds a chunk's
+// rows, two per lane, in about 130 clocks a term past the prefix; the block's
+// share of the write stream takes about (G << L) * 2.8 clocks a chunk.  Folded
+// here while the fold is a third of that at most (chain n = 21, 9 terms and
+// 2,688 entries a chunk: 338 us against 370 through the value buffer; an
+// operator of 94 groups, 26 terms and chunks of 16 rows: 195 against 158).  One group (the
+// diagonal of a spin chain); all row bits have to be in the tables.
+bool csr_inline_fold(uint64_t G, int n, uint32_t nfold, uint32_t fold_rem) {
+    if (G > (uint64_t)kCsrThreads || nfold != 1 || fold_rem > kCsrInlineRem) return false;
+    const CsrStage s = csr_stage((uint32_t)G, n, 0, 0);
+    return s.L <= kCsrChunkBits && s.L + s.up * s.U >= n &&
+           fold_rem * 128u <= (uint32_t)G << s.L;
 }
+size_t csr_tables_bytes(uint64_t G, int n) {
+    return G <= (uint64_t)kCsrThreads ? csr_stage((uint32_t)G, n, 0, 0).bytes : 0;
+}
+
+__global__ void __launch_bounds__(kCsrThreads) csr_tables_kernel(const CsrArgs a) {
+    const uint32_t G = (uint32_t)a.G;
+    const CsrStage cs = csr_stage(G, a.n, a.nctab, 0);
+    uint16_t *const w16 = const_cast<uint16_t *>(a.tables);
+    const uint32_t nlow = G << cs.L, nup = G << cs.U, ntab = nlow + (uint32_t)cs.up * nup;
+    const uint32_t per = (1u << cs.L) + (uint32_t)cs.up * (1u << cs.U);
+    const uint32_t step = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ntab + (a.inline_fold ? per : 0u);
+         i += step) {
+        if (i < ntab) {
+            const uint32_t lev = i < nlow ? 0u : 1u + (i - nlow) / nup;
+            const uint32_t j = lev ? (i - nlow) % nup : i;
+            const int b = lev ? cs.U : cs.L;
+            const uint32_t g = j >> b, v = j & ((1u << b) - 1u);
+            const uint64_t z = (uint64_t)v << (lev ? cs.L + (int)(lev - 1u) * cs.U : 0);
+            const CsrGroup dg = a.grp[g];
+            uint32_t w = (uint32_t)sigma_sum<uint64_t>(z & a.pmask[g],
+                                                       a.sig + (size_t)g * (uint32_t)a.n) & 0x7ffu;
+            if (dg.d != kCsrFold) w |= csr_class<uint64_t>(dg, z) << 11;
+            w16[lev ? cs.ups + (lev - 1u) * cs.ups_sz + g * cs.usz + v : g * cs.lsz + v] =
+                (uint16_t)w;
+        } else {
+            const uint32_t j = i - ntab;
+            const uint32_t lo = 1u << cs.L;
+            const uint32_t lev = j < lo ? 0u : 1u + (j - lo) / (1u << cs.U);
+            const uint32_t v = lev ? (j - lo) & ((1u << cs.U) - 1u) : j;
+            const uint64_t z = (uint64_t)v << (lev ? cs.L + (int)(lev - 1u) * cs.U : 0);
+            const CsrGroup d = a.grp[a.fold[0]];
+            const uint32_t m = d.pre & 0xffffffu, dp = d.pre >> 24;
+            uint32_t c = parity<uint64_t>(z & d.z0);
+            for (uint32_t q = 0; q < dp; ++q) c |= parity<uint64_t>(z & a.pbeta[q]) << (q + 1);
+            uint64_t sg = 0;
+            for (uint32_t q = 0; d.k0 + m + q < d.k1; ++q)
+                sg |= (uint64_t)parity<uint64_t>(z & a.tz[d.k0 + m + q]) << q;
+            w16[cs.cls / 2u + j] = (uint16_t)c;
+            reinterpret_cast<uint64_t *>(w16 + cs.sgn / 2u)[j] = sg;
+        }
+    }
+}
+
+cudaError_t launch_csr_tables(const CsrArgs &a, cudaStream_t st) {
+    if (a.G > (uint64_t)kCsrThreads) return cudaSuccess;
+    const CsrStage cs = csr_stage((uint32_t)a.G, a.n, a.nctab, 0);
+    cudaError_t e = cudaMemsetAsync(const_cast<uint16_t *>(a.tables), 0, cs.bytes, st);
+    if (e != cudaSuccess) return e;
+    const uint32_t n = ((uint32_t)a.G << cs.L) + (uint32_t)cs.up * ((uint32_t)a.G << cs.U);
+    csr_tables_kernel<<<(n + kCsrThreads - 1) / kCsrThreads, kCsrThreads, 0, st>>>(a);
+    count_launch();
+    return cudaGetLastError();
+}
+
 __device__ __forceinline__ void csr_bulk_s2g(void *dst, const void *src, uint32_t bytes) {
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
-                 "r"(csr_saddr(src)), "r"(bytes)
+                 "r"(saddr(src)), "r"(bytes)
                  : "memory");
 }
+// Ask for the next block of the grid that has not started; the answer (16
+// bytes) arrives on the barrier.
+__device__ __forceinline__ void next_block_ask(void *resp, uint64_t *bar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], 16;" ::"r"(saddr(bar))
+                 : "memory");
+    asm volatile(
+        "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 "
+        "[%0], [%1];" ::"r"(saddr(resp)),
+        "r"(saddr(bar))
+        : "memory");
+}
+// Block index of the answer, or kCsrNoUnit.
+constexpr uint32_t kCsrNoUnit = 0xffffffffu;
+__device__ __forceinline__ uint32_t next_block_answer(const void *resp) {
+    uint32_t x;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b128 v;\n\tld.shared.b128 v, [%1];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, v;\n\t"
+        "mov.u32 %0, 0xffffffff;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, v;\n\t}"
+        : "=r"(x)
+        : "r"(saddr(resp))
+        : "memory");
+    return x;
+}
+__device__ __forceinline__ uint32_t hi_word(double v) { return (uint32_t)__double2hiint(v); }
+// term << 31 of a sign mask onto a value
+__device__ __forceinline__ double sign_by(double v, uint32_t bit) {
+    return __hiloint2double((int)(hi_word(v) ^ (bit << 31)), __double2loint(v));
+}
 
-template <bool WIDE>
-__global__ void __launch_bounds__(kCsrThreads) csr_fill_staged_kernel(const CsrArgs a) {
+// The inline fold's group.
+struct FoldDesc {
+    uint64_t x;
+    uint32_t g, tab, m, rem, zparts;
+};
+// The terms after the prefix folded onto the values of a lane's two rows
+// (csr_fold_row's additions and signs of zero), together: a dependent addition
+// takes about 100 clocks.
+template <bool RE, bool IM>
+__device__ __forceinline__ void fold_rest(const FoldDesc &fd, const double2 *tc,
+                                          const uint64_t (&sg)[2], double2 (&v)[2]) {
+    constexpr uint32_t K = 2;
+    const bool pre = fd.m != 0;
+    uint32_t nr[K], ni[K];
+#pragma unroll
+    for (uint32_t i = 0; i < K; ++i) {
+        nr[i] = pre ? hi_word(v[i].x) >> 31 : 1u;
+        ni[i] = pre ? hi_word(v[i].y) >> 31 : 1u;
+    }
+    for (uint32_t j = 0; j < fd.rem; ++j) {
+        const double2 c = tc[j];
+#pragma unroll
+        for (uint32_t i = 0; i < K; ++i) {
+            const uint32_t s1 = (uint32_t)(sg[i] >> j) & 1u;
+            const double cr = sign_by(c.x, s1), ci = sign_by(c.y, s1);
+            if constexpr (RE) v[i].x = pre || j ? __dadd_rn(v[i].x, cr) : cr;
+            else nr[i] &= hi_word(cr) >> 31;
+            if constexpr (IM) v[i].y = pre || j ? __dadd_rn(v[i].y, ci) : ci;
+            else ni[i] &= hi_word(ci) >> 31;
+        }
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < K; ++i) {
+        if constexpr (!RE) v[i].x = nr[i] ? -0.0 : 0.0;
+        if constexpr (!IM) v[i].y = ni[i] ? -0.0 : 0.0;
+    }
+}
+
+// FOLD: 0 no fold-mode group placed, 1 one folded here, 2 from the value buffer
+template <bool WIDE, int FOLD>
+__global__ void __launch_bounds__(kCsrStageThreads, 3) csr_fill_staged_kernel(const CsrArgs a,
+                                                                              uint32_t q) {
     using W = typename RowT<WIDE>::T;
     extern __shared__ __align__(128) int32_t s_dyn[];
+    __shared__ __align__(16) uint4 s_resp;
+    __shared__ __align__(8) uint64_t s_bar;
+    __shared__ FoldDesc s_fold;
+    __shared__ __align__(16) double2 s_fval[2][1 << kCsrChunkBits];
+    __shared__ uint32_t s_next[2];  // next unit, by the parity of this block's units
+    unsigned char *const s_base = reinterpret_cast<unsigned char *>(s_dyn);
     const uint32_t G = (uint32_t)a.G;
-    const int L = csr_lut_bits(G);
-    const uint32_t lsz = (1u << L) + 1;
+    const uint32_t nfv = FOLD == 2 ? a.nfold : 0u;
+    constexpr bool inl = FOLD == 1;
+    const CsrStage cs = csr_stage(G, a.n, a.nctab, nfv);
+    const int L = cs.L, U = cs.U;
+    const uint32_t lsz = cs.lsz;
     const uint32_t t = threadIdx.x;
-    for (uint32_t i = t; i < G * lsz; i += kCsrThreads) {
-        const uint32_t g = i / lsz, v = i - g * lsz;
-        const W pm = (W)a.pmask[g] & (((W)1 << L) - 1) & (W)v;
-        s_dyn[i] = v < (1u << L) ? sigma_sum<W>(pm, a.sig + (size_t)g * (uint32_t)a.n) : 0;
+    const bool helper = t >= (uint32_t)kCsrThreads;  // the ninth warp
+    const W lomask = ((W)1 << L) - 1;
+    const uint64_t nchunk = (a.nrows + lomask) >> L;
+    {
+        const uint4 *src = reinterpret_cast<const uint4 *>(a.tables);
+        uint4 *dst = reinterpret_cast<uint4 *>(s_base);
+        for (uint32_t i = t; i < cs.bytes / 16u; i += kCsrStageThreads) dst[i] = src[i];
     }
-    double2 *s_ctab = reinterpret_cast<double2 *>(s_dyn + ((G * lsz + 3u) & ~3u));
-    const bool ctab_smem = a.nctab <= kCsrSmemCtab;
+    const uint16_t *s_lut = reinterpret_cast<const uint16_t *>(s_base);
+    const bool ctab_smem = cs.ctab != 0;
+    double2 *s_ctab = reinterpret_cast<double2 *>(s_base + cs.ctab);
     if (ctab_smem)
-        for (uint32_t i = t; i < a.nctab; i += kCsrThreads) s_ctab[i] = a.ctab[i];
-    // staging buffers, 128-byte aligned: per buffer R*G indices then R*G values
-    const uint32_t R = (uint32_t)csr_stage_rows(G, L);
-    const uint32_t ent = R * G;
-    const size_t head = ((size_t)((G * lsz + 3u) & ~3u) * 4u +
-                         (ctab_smem ? (size_t)a.nctab * sizeof(double2) : 0u) + 127u) &
-                        ~(size_t)127u;
-    unsigned char *stage = reinterpret_cast<unsigned char *>(s_dyn) + head;
-    const size_t buf_bytes = ((size_t)ent * 24u + 127u) & ~(size_t)127u;
-    // with precomputed fold values: high-bit position term of each fold-mode
-    // group for the current chunk
-    int32_t *s_phi = reinterpret_cast<int32_t *>(stage + 2 * buf_bytes);
-    const uint32_t nfv = a.fvals ? a.nfold : 0u;
+        for (uint32_t i = t; i < a.nctab; i += kCsrStageThreads) s_ctab[i] = a.ctab[i];
+    double2 *s_tc = reinterpret_cast<double2 *>(s_base + cs.tc);
+    if (inl) {
+        const CsrGroup &df = a.grp[a.fold[0]];
+        const uint32_t m = df.pre & 0xffffffu, k = df.k0 + m, rem = df.k1 - k;
+        if (t == 0) s_fold = {a.gx[a.fold[0]], a.fold[0], df.tab, m, rem, df.zparts & 3u};
+        for (uint32_t i = t; i < rem && i < kCsrInlineRem; i += kCsrStageThreads)
+            s_tc[i] = make_double2(a.tc[2 * (size_t)(k + i)], a.tc[2 * (size_t)(k + i) + 1]);
+    }
+    // groups of the value buffer
+    uint64_t *s_fx = reinterpret_cast<uint64_t *>(s_base + cs.fold);
+    uint32_t *s_fg = reinterpret_cast<uint32_t *>(s_fx + nfv);
+    for (uint32_t f = t; f < nfv; f += kCsrStageThreads) {
+        s_fg[f] = a.fold[f];
+        s_fx[f] = a.gx[a.fold[f]];
+    }
+    if (t == (uint32_t)kCsrThreads) {
+        mbar_init(&s_bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
     __syncthreads();
 
+    const uint32_t R = cs.R;
     const uint32_t rpp = kCsrThreads / G;
     const uint32_t rs = t / G, g = t - rs * G;
-    const bool lane_on = t < rpp * G;  // idle threads still take every barrier
     CsrGroup d{};
-    W xg = 0, pm = 0;
-    const int32_t *sg = a.sig;
+    W xg = 0;
     bool active = false;
-    if (lane_on) {
+    if (t < rpp * G) {  // idle threads still take every barrier
         d = a.grp[g];
         active = d.d != kCsrFold;
         xg = (W)a.gx[g];
-        pm = (W)a.pmask[g];
-        sg = a.sig + (size_t)g * (uint32_t)a.n;
     }
-    const W lomask = ((W)1 << L) - 1;
-    const int32_t *lut = s_dyn + (lane_on ? g : 0u) * lsz;
+    const uint16_t *lut = s_lut + (active ? g : 0u) * lsz;
     const double2 *tab = (ctab_smem ? s_ctab : a.ctab) + d.tab;
-    const uint64_t nchunk = (a.nrows + lomask) >> L;
-    // fold-mode entries: with nfold * R <= threads, the highest nfold * R
-    // threads (idle in the class-table pass whenever rpp * G < threads) own
-    // one item (f, rl) of every sub-chunk each and copy its value into a
-    // kCsrFvSlots-deep shared ring, kCsrFvSlots - 1 sub-chunks ahead
-    // (cp.async: no register waits on the load; the values come from DRAM,
-    // the fill's write stream having evicted them from L2)
-    const bool ring = nfv > 0 && nfv * R <= (uint32_t)kCsrThreads;
-    const uint32_t base_it = ring ? (uint32_t)kCsrThreads - nfv * R : (uint32_t)kCsrThreads;
-    const bool own = ring && t >= base_it;
-    const uint32_t i_it = own ? t - base_it : 0u;
-    const uint32_t f_it = i_it / R, rl_it = i_it - (i_it / R) * R;
-    const uint32_t g_it = own ? a.fold[f_it] : 0u;
-    const uint64_t x_it = own ? a.gx[g_it] : 0ull;
-    double2 *s_fv = reinterpret_cast<double2 *>(s_phi + ((nfv + 3u) & ~3u));  // slots x nfold*R
-    auto next_sub = [&](uint64_t &c, uint64_t &s0) {
-        const uint64_t e = min((c << L) + ((uint64_t)1 << L), a.nrows);
-        s0 += R;
-        if (s0 >= e) {
-            c += gridDim.x;
-            s0 = c << L;
-        }
-    };
-    auto prefetch = [&](uint64_t c, uint64_t s0, uint32_t slot) {
-        if (own && c < nchunk) {
-            const uint32_t rows = (uint32_t)min((uint64_t)R, min((c << L) + ((uint64_t)1 << L),
-                                                                   a.nrows) - s0);
-            if (rl_it < rows) {
-                const double2 *src = a.fvals + (size_t)f_it * a.nrows + s0 + rl_it;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                                 csr_saddr(s_fv + (size_t)slot * nfv * R + i_it)),
-                             "l"(src)
-                             : "memory");
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    uint32_t k = 0;  // sub-chunks issued by this block: buffer k & 1, ring slot k % kCsrFvSlots
-    uint64_t ch = blockIdx.x, sc = ch << L;
-    uint64_t chP = ch, scP = sc;  // prefetch cursor: sub-chunk k + kCsrFvSlots - 1
-    if (ring)
-        for (uint32_t q = 0; q + 1 < kCsrFvSlots; ++q) {
-            prefetch(chP, scP, q);
-            next_sub(chP, scP);
-        }
-    int32_t phi = 0;
-    while (ch < nchunk) {
-        const uint64_t rr0 = ch << L;
-        const uint64_t rend = min(rr0 + ((uint64_t)1 << L), a.nrows);
-        const uint32_t rows = (uint32_t)min((uint64_t)R, rend - sc);
-        unsigned char *buf = stage + (size_t)(k & 1u) * buf_bytes;
-        uint64_t *s_idx = reinterpret_cast<uint64_t *>(buf);
-        double2 *s_val = reinterpret_cast<double2 *>(buf + (size_t)ent * 8u);
-        // the bulk store that last read this buffer (two sub-chunks ago) has
-        // finished reading it
-        if (t == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        if (sc == rr0) {  // chunk start: high-bit position terms
-            phi = active ? (int32_t)g + sigma_sum<W>((W)(a.row0 + rr0) & pm & ~lomask, sg) : 0;
-            // (the previous sub-chunk's barrier has retired every reader of s_phi)
-            for (uint32_t f = t; f < nfv; f += kCsrThreads) {
-                const uint32_t gf = a.fold[f];
-                s_phi[f] = (int32_t)gf + sigma_sum<W>((W)(a.row0 + rr0) & (W)a.pmask[gf] & ~lomask,
-                                                      a.sig + (size_t)gf * (uint32_t)a.n);
-            }
-        }
-        __syncthreads();
-        if (ring) {
-            prefetch(chP, scP, (k + kCsrFvSlots - 1) % kCsrFvSlots);
-            next_sub(chP, scP);
-        }
-        if (active) {
-#pragma unroll 2
-            for (uint32_t rl = rs; rl < rows; rl += rpp) {
-                const W r = (W)(a.row0 + sc + rl);
-                const double2 v =
-                    ctab_smem ? s_ctab[d.tab + csr_class<W>(d, r)] : tab[csr_class<W>(d, r)];
-                const int32_t pos = phi + lut[(uint32_t)(r & lomask)];
-                if (pos < 0 || (uint32_t)pos >= G) {  // cannot happen for a valid trie table
-                    atomicExch(a.err, kErrCsrPos);
-                    continue;
-                }
-                s_idx[rl * G + (uint32_t)pos] = (uint64_t)(r ^ xg);
-                s_val[rl * G + (uint32_t)pos] = v;
-            }
-        }
-        // fold-mode entries from the values the fold pass wrote
-        auto place = [&](uint32_t f, uint32_t rl, uint32_t gf, uint64_t xf, double2 v) {
-            const W r = (W)(a.row0 + sc + rl);
-            const int32_t pos = s_phi[f] + s_dyn[gf * lsz + (uint32_t)(r & lomask)];
-            if (pos < 0 || (uint32_t)pos >= G) {
-                atomicExch(a.err, kErrCsrPos);
-                return;
-            }
-            s_idx[rl * G + (uint32_t)pos] = (uint64_t)r ^ xf;
-            s_val[rl * G + (uint32_t)pos] = v;
+    // Groups of span rank 0 and 1 (2 and 4 classes) keep their values in
+    // registers: the entries of classes 0 and 2, and for each part whether
+    // the class with bit 0 set (every term's sign flipped) has it negated
+    // (not so where the sum cancels to zero).  Lanes reading the table at
+    // their rows' classes conflict on its banks.
+    double2 e0 = make_double2(0.0, 0.0), e1 = e0;
+    uint32_t neg = 0;  // bits 0, 1: parts of e0; bits 2, 3: of e1
+    bool held = active && d.d <= 1;
+    if (held) {
+        e0 = tab[0];
+        e1 = d.d ? tab[2] : e0;
+        const double2 f0 = tab[1], f1 = d.d ? tab[3] : f0;
+        auto flip_of = [&](double p, double r, uint32_t bit) {
+            const uint64_t x = (uint64_t)(__double_as_longlong(p) ^ __double_as_longlong(r));
+            if (x == 1ull << 63) neg |= 1u << bit;
+            else if (x != 0) held = false;
         };
-        const uint32_t nitem = nfv * rows;
-        if (ring) {
-            // this thread's copy for sub-chunk k has landed (newer ones pending)
-            asm volatile("cp.async.wait_group %0;" ::"n"(kCsrFvSlots - 1) : "memory");
-            if (own && rl_it < rows)
-                place(f_it, rl_it, g_it, x_it,
-                      s_fv[(size_t)(k % kCsrFvSlots) * nfv * R + i_it]);
-        } else {
-            for (uint32_t i = t; i < nitem; i += kCsrThreads) {
-                const uint32_t f = i / rows, rl = i - f * rows;
-                const uint32_t gf = a.fold[f];
-                place(f, rl, gf, a.gx[gf], a.fvals[(size_t)f * a.nrows + sc + rl]);
-            }
-        }
-        // shared writes visible to the bulk-copy (async) proxy
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (t == 0) {
-            csr_bulk_s2g(a.indices + sc * G, s_idx, rows * G * 8u);
-            csr_bulk_s2g(a.data + 2 * sc * G, s_val, rows * G * 16u);
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
-        next_sub(ch, sc);
-        ++k;
+        flip_of(e0.x, f0.x, 0);
+        flip_of(e0.y, f0.y, 1);
+        flip_of(e1.x, f1.x, 2);
+        flip_of(e1.y, f1.y, 3);
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    if (t == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    auto pos_of = [](uint32_t w) { return (int32_t)(w << 21) >> 21; };
+    // position (from gq on) and class terms of a chunk's high bits
+    auto high_terms = [&](uint32_t gq, W hi, bool fold, int32_t *ph, uint32_t *cl) {
+        int32_t p = (int32_t)gq;
+        uint32_t c = 0;
+        const uint16_t *row = s_lut + cs.ups + gq * cs.usz;
+        W rest = hi >> L;
+        for (int l = 0; l < cs.up; ++l, row += cs.ups_sz) {
+            const uint32_t w = row[(uint32_t)rest & ((1u << U) - 1u)];
+            p += pos_of(w);
+            c ^= w >> 11;
+            rest >>= U;
+        }
+        if (rest) {  // bits above the tables
+            const W top = rest << (L + cs.up * U);
+            p += sigma_sum<W>(top & (W)a.pmask[gq], a.sig + (size_t)gq * (uint32_t)a.n);
+            if (!fold) c ^= csr_class<W>(a.grp[gq], top);
+        }
+        *ph = p;
+        *cl = c;
+    };
+    uint32_t b = 0;  // staging buffer
+    uint32_t par = 0, ask = 0;
+    uint32_t unit = blockIdx.x;
+    int32_t phi = 0;
+    uint32_t cls = 0;
+    auto answer = [&]() {
+        if (mbar_wait_bounded(&s_bar, ask, kWaitLimitNs)) return next_block_answer(&s_resp);
+        atomicExch(a.err, kErrMbarTimeout);
+        return kCsrNoUnit;
+    };
+    // Inline fold, a chunk ahead of the stages: at a chunk's first stage the
+    // helper's lanes read the next chunk's prefix values (on their way while
+    // the stages pass), at its last stage they add the other terms and leave
+    // the values in shared memory, by the parity of this block's chunks.
+    const uint32_t lane = t & 31u;
+    const uint16_t *s_cls = reinterpret_cast<const uint16_t *>(s_base + cs.cls);
+    const uint64_t *s_sgn = reinterpret_cast<const uint64_t *>(s_base + cs.sgn);
+    double2 it_v[2];   // rows lane and lane + 32 of the next chunk
+    uint64_t it_s[2];
+    auto fold_fetch = [&](uint64_t ch) {
+        W rest = (W)(a.row0 + (ch << L)) >> L;
+        uint32_t c = 0;
+        uint64_t sg = 0;
+        for (uint32_t j = 1u << L, l = 0; l < (uint32_t)cs.up; ++l, j += 1u << U, rest >>= U) {
+            const uint32_t i = j + ((uint32_t)rest & ((1u << U) - 1u));
+            c ^= s_cls[i];
+            sg ^= s_sgn[i];
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 2; ++i) {
+            const uint32_t rl = (lane + 32u * i) & ((1u << L) - 1u);
+            it_s[i] = sg ^ s_sgn[rl];
+            it_v[i] = s_fold.m ? a.ptab[s_fold.tab + (c ^ s_cls[rl])] : make_double2(0.0, 0.0);
+        }
+    };
+    auto fold_finish = [&](uint32_t to) {
+        switch (s_fold.zparts) {
+            case 1: fold_rest<false, true>(s_fold, s_tc, it_s, it_v); break;
+            case 2: fold_rest<true, false>(s_fold, s_tc, it_s, it_v); break;
+            case 3: fold_rest<false, false>(s_fold, s_tc, it_s, it_v); break;
+            default: fold_rest<true, true>(s_fold, s_tc, it_s, it_v); break;
+        }
+        s_fval[to][lane] = it_v[0];
+        s_fval[to][lane + 32u] = it_v[1];
+        __syncwarp();
+    };
+    // Value buffer, a chunk ahead as well: position terms of the groups'
+    // entries, and the values on their way to shared memory (from DRAM, the
+    // fill's write stream having evicted them from L2).
+    int32_t *s_fphi = reinterpret_cast<int32_t *>(s_base + cs.fphi);
+    double2 *s_fv = reinterpret_cast<double2 *>(s_base + cs.fval);
+    auto buffer_ahead = [&](uint64_t ch, uint32_t to) {
+        const uint64_t rr0 = ch << L;
+        const uint32_t rows = (uint32_t)min((uint64_t)1 << L, a.nrows - rr0);
+        for (uint32_t f = lane; f < nfv; f += 32) {
+            uint32_t cl;
+            high_terms(s_fg[f], (W)(a.row0 + rr0), true, &s_fphi[to * nfv + f], &cl);
+        }
+        if (!cs.ring) return;
+        for (uint32_t i = lane; i < nfv << L; i += 32) {
+            const uint32_t f = i >> L, rl = i & ((1u << L) - 1u);
+            if (rl < rows)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                 saddr(s_fv + (to * nfv << L) + i)),
+                             "l"(a.fvals + (size_t)f * a.nrows + rr0 + rl)
+                             : "memory");
+        }
+    };
+    if (helper && nfv > 0) {
+        buffer_ahead((uint64_t)unit * q, 0);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    // the unit after this block's first: asked for now, and each later one
+    // while the unit before the last known is filled
+    uint32_t after = kCsrNoUnit;
+    if (t == (uint32_t)kCsrThreads) {
+        next_block_ask(&s_resp, &s_bar);
+        s_next[1] = answer();
+    }
+    if (helper && inl) {
+        fold_fetch((uint64_t)unit * q);
+        fold_finish(0);
+    }
+    __syncthreads();
+    after = s_next[1];
+    ask = 1;
+    uint32_t cpar = 0;  // parity of this block's chunks
+    while (unit != kCsrNoUnit) {
+        if (t == (uint32_t)kCsrThreads && after != kCsrNoUnit) {
+            // the last answer has been read: its buffer goes back to the async proxy
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            next_block_ask(&s_resp, &s_bar);
+        }
+        const uint64_t ch1 = min((uint64_t)(unit + 1ull) * q, nchunk);
+        for (uint64_t ch = (uint64_t)unit * q; ch < ch1; ++ch) {
+            const uint64_t rr0 = ch << L;
+            const uint32_t crows = (uint32_t)min((uint64_t)1 << L, a.nrows - rr0);
+            const W hi = (W)(a.row0 + rr0);
+            if (active) high_terms(g, hi, false, &phi, &cls);
+            for (uint32_t low = 0; low < crows; low += R) {
+                const uint32_t rows = min(R, crows - low);
+                const W r0 = hi + low;
+                unsigned char *buf = s_base + cs.bufs + b * cs.buf_bytes;
+                uint64_t *s_idx = reinterpret_cast<uint64_t *>(buf);
+                double2 *s_val = reinterpret_cast<double2 *>(buf + R * G * 8u);
+                auto put = [&](uint32_t rl, int32_t pos, W x, double2 v) {
+                    if ((uint32_t)pos >= G) {  // cannot happen for a valid trie table
+                        atomicExch(a.err, kErrCsrPos);
+                        return;
+                    }
+                    s_idx[rl * G + (uint32_t)pos] = (uint64_t)((r0 + rl) ^ x);
+                    s_val[rl * G + (uint32_t)pos] = v;
+                };
+                if (active) {
+#pragma unroll 2
+                    for (uint32_t rl = rs; rl < rows; rl += rpp) {
+                        const uint32_t w = lut[low + rl];
+                        const uint32_t c = cls ^ (w >> 11);
+                        double2 v;
+                        if (held) {
+                            v = c & 2u ? e1 : e0;
+                            const uint32_t m = neg >> (c & 2u);
+                            v.x = sign_by(v.x, m & c);
+                            v.y = sign_by(v.y, (m >> 1) & c);
+                        } else {
+                            v = ctab_smem ? s_ctab[d.tab + c] : tab[c];
+                        }
+                        put(rl, phi + pos_of(w), xg, v);
+                    }
+                }
+                // entries of the value buffer
+                if (nfv > 0 && !helper) {
+                    const uint32_t nitem = nfv * rows;
+                    for (uint32_t i = (uint32_t)kCsrThreads - 1u - t; i < nitem; i += kCsrThreads) {
+                        const uint32_t f = i / rows, rl = i - f * rows;
+                        const double2 v = cs.ring
+                                              ? s_fv[((cpar * nfv + f) << L) + low + rl]
+                                              : a.fvals[(size_t)f * a.nrows + rr0 + low + rl];
+                        put(rl, s_fphi[cpar * nfv + f] + pos_of(s_lut[s_fg[f] * lsz + low + rl]),
+                            (W)s_fx[f], v);
+                    }
+                }
+                const bool last = low + R >= crows;  // the chunk's last stage
+                const uint64_t chn = ch + 1 < ch1 ? ch + 1 : (uint64_t)after * q;
+                const bool more = ch + 1 < ch1 || after != kCsrNoUnit;
+                if (helper && nfv > 0) {
+                    if (low == 0 && more) buffer_ahead(chn, cpar ^ 1u);
+                    if (last) asm volatile("cp.async.wait_all;" ::: "memory");
+                }
+                if (helper && inl) {
+                    if (low == 0 && more) fold_fetch(chn);
+                    if (low == 0) high_terms(s_fold.g, hi, true, &phi, &cls);
+                    for (uint32_t rl = lane; rl < rows; rl += 32)
+                        put(rl, phi + pos_of(s_lut[s_fold.g * lsz + low + rl]), (W)s_fold.x,
+                            s_fval[cpar][low + rl]);
+                    if (last && more) fold_finish(cpar ^ 1u);
+                }
+                if (last && ch + 1 == ch1 && t == (uint32_t)kCsrThreads)
+                    s_next[par] = after != kCsrNoUnit ? answer() : kCsrNoUnit;
+                __syncthreads();
+                if (t == (uint32_t)kCsrThreads) {
+                    // the block's shared writes, ordered before this by the
+                    // barrier, made visible to the bulk copies (one fence
+                    // instead of every thread's: 5 % of the whole)
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    const uint64_t o = (rr0 + low) * G;
+                    csr_bulk_s2g(a.indices + o, s_idx, rows * G * 8u);
+                    csr_bulk_s2g(a.data + 2 * o, s_val, rows * G * 16u);
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    // the previous stage's buffer is read: stage k + 2 takes it, past
+                    // the next barrier, at which this thread arrives after this wait
+                    asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                }
+                b = b + 1 == kCsrBufs ? 0u : b + 1;
+            }
+            cpar ^= 1u;
+        }
+        unit = after;
+        after = s_next[par];  // written before the last barrier; the other half is written next
+        par ^= 1u;
+        ask ^= 1u;
+    }
+    if (t == (uint32_t)kCsrThreads) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // VALS: write the values row-major per fold group into a.fvals (coalesced),
@@ -441,13 +785,7 @@ __global__ void __launch_bounds__(kCsrThreads) csr_fold_kernel(const CsrArgs a) 
         for (uint64_t rr = blockIdx.x * (uint64_t)kCsrThreads + threadIdx.x; rr < a.nrows;
              rr += (uint64_t)gridDim.x * kCsrThreads) {
             const uint64_t r = a.row0 + rr;
-            double2 v;
-            switch (d.zparts & 3u) {  // warp-uniform
-                case 1: v = csr_fold_row<true, false>(a, r, d, f); break;
-                case 2: v = csr_fold_row<false, true>(a, r, d, f); break;
-                case 3: v = csr_fold_row<true, true>(a, r, d, f); break;
-                default: v = csr_fold_row<false, false>(a, r, d, f); break;
-            }
+            const double2 v = csr_fold_entry(a, r, d, f);
             if constexpr (VALS)
                 a.fvals[(size_t)f * a.nrows + rr] = v;
             else
@@ -493,31 +831,28 @@ cudaError_t launch_csr_fill(const CsrArgs &a, int nsm, cudaStream_t st) {
         // staged path: every bulk store a whole number of 16-byte units
         // (even row counts) from 16-byte aligned outputs
         if (aligned && L >= 1 && a.nrows % 2 == 0) {
-            const uint32_t R = (uint32_t)csr_stage_rows((uint32_t)a.G, L);
-            const size_t buf = ((size_t)R * a.G * 24u + 127u) & ~(size_t)127u;
-            size_t sm = ((smem + 127u) & ~(size_t)127u) + 2 * buf;
-            if (a.fvals && a.nfold > 0) {  // chunk positions, then the value ring
-                sm += (((size_t)a.nfold + 3u) & ~(size_t)3u) * 4u;
-                if ((size_t)a.nfold * R <= (size_t)kCsrThreads)
-                    sm += (size_t)kCsrFvSlots * a.nfold * R * 16u;
-            }
-            auto kern = (a.n > 32 || a.wide) ? csr_fill_staged_kernel<true> : csr_fill_staged_kernel<false>;
+            const CsrStage cs = csr_stage((uint32_t)a.G, a.n, a.nctab, a.fvals ? a.nfold : 0u);
+            const uint64_t nchunk = (a.nrows + (1u << cs.L) - 1) >> cs.L;
+            const uint32_t q = csr_unit_chunks((uint32_t)a.G, cs.L, nchunk, nsm);
+            g = (nchunk + q - 1) / q;
+            if (g > 0x7fffffffull) return cudaErrorInvalidValue;
+            const size_t sm = cs.total;
+            const bool wide = a.n > 32 || a.wide;
+            auto kern = a.inline_fold ? (wide ? csr_fill_staged_kernel<true, 1> : csr_fill_staged_kernel<false, 1>)
+                        : a.fvals && a.nfold
+                            ? (wide ? csr_fill_staged_kernel<true, 2> : csr_fill_staged_kernel<false, 2>)
+                            : (wide ? csr_fill_staged_kernel<true, 0> : csr_fill_staged_kernel<false, 0>);
             cudaError_t e0 =
                 cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             if (e0 != cudaSuccess) return e0;
-            int per_sm = 0;
-            e0 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCsrThreads, sm);
-            if (e0 != cudaSuccess) return e0;
-            if (per_sm < 1) per_sm = 1;
-            if (g > (uint64_t)nsm * per_sm) g = (uint64_t)nsm * per_sm;
             if (a.fvals) {  // fold values first; the staged pass places them
                 cudaError_t e = launch_csr_fold(a, nsm, st);
                 if (e != cudaSuccess) return e;
             }
-            kern<<<(unsigned)g, kCsrThreads, sm, st>>>(a);
+            kern<<<(unsigned)g, kCsrStageThreads, sm, st>>>(a, q);
             count_launch();
             cudaError_t e = cudaGetLastError();
-            if (e != cudaSuccess || a.fvals) return e;
+            if (e != cudaSuccess || a.fvals || a.inline_fold) return e;
             return launch_csr_fold(a, nsm, st);
         }
     } else {

@@ -541,7 +541,7 @@ __device__ int group_span(const uint64_t *tz, uint32_t k0, uint32_t k1, uint64_t
 // class (prefix table).  tab and zparts are filled later.
 __global__ void csr_span_kernel(uint32_t G, const uint32_t *goff, const uint64_t *tz,
                                 CsrGroup *grp, uint16_t *coord, uint64_t *ctsz, uint64_t *ptsz,
-                                uint32_t *isfold, uint64_t *gbeta) {
+                                uint32_t *isfold, uint64_t *gbeta, uint32_t *fold_rem) {
     GRID_STRIDE(g, G) {
         CsrGroup d;
         d.k0 = goff[g];
@@ -576,6 +576,7 @@ __global__ void csr_span_kernel(uint32_t G, const uint32_t *goff, const uint64_t
                 gbeta[g * (uint64_t)kCsrPrefixRank + j] = j < nb ? basis[j] : 0ull;
             ctsz[g] = 0;
             isfold[g] = 1;
+            atomicMax(fold_rem, d.k1 - d.k0 - (d.pre & 0xffffffu));
         }
         grp[g] = d;
     }
@@ -605,13 +606,14 @@ cudaError_t csr_structure(int n, uint64_t G, const uint64_t *gx, const uint32_t 
     if (G == 0 || G > 0xffffffffull) return cudaErrorInvalidValue;
     Scratch sc{st};
     uint64_t *ctsz = sc.get<uint64_t>(G + 1), *ptsz = sc.get<uint64_t>(G + 1);
-    uint32_t *foff = sc.get<uint32_t>(G + 1);
+    uint32_t *foff = sc.get<uint32_t>(G + 2);  // fold flags' scan, then the longest remainder
     uint64_t *gbeta = sc.get<uint64_t>(G * kCsrPrefixRank);
     GR_TRY(sc.e);
+    GR_TRY(cudaMemsetAsync(foff + G + 1, 0, sizeof(uint32_t), st));
     csr_trie_kernel<<<grid_of(G), 256, 0, st>>>(gx, (uint32_t)G, n, o.pmask, o.sig);
     GR_LAUNCH();
     csr_span_kernel<<<grid_of(G, 128), 128, 0, st>>>((uint32_t)G, goff, tz, o.grp, o.coord, ctsz,
-                                                     ptsz, foff, gbeta);
+                                                     ptsz, foff, gbeta, foff + G + 1);
     GR_LAUNCH();
     GR_TRY(scan_excl<uint64_t>(ctsz, ctsz, G, st));
     GR_TRY(scan_excl<uint64_t>(ptsz, ptsz, G, st));
@@ -620,14 +622,15 @@ cudaError_t csr_structure(int n, uint64_t G, const uint64_t *gx, const uint32_t 
                                                 o.fold, o.pbeta);
     GR_LAUNCH();
     uint64_t tot[2] = {0, 0};
-    uint32_t nfold = 0;
+    uint32_t fold[2] = {0, 0};
     GR_TRY(cudaMemcpyAsync(&tot[0], ctsz + G, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     GR_TRY(cudaMemcpyAsync(&tot[1], ptsz + G, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    GR_TRY(cudaMemcpyAsync(&nfold, foff + G, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    GR_TRY(cudaMemcpyAsync(fold, foff + G, sizeof(fold), cudaMemcpyDeviceToHost, st));
     GR_TRY(cudaStreamSynchronize(st));
     cnt->nctab = tot[0];
     cnt->nptab = tot[1];
-    cnt->nfold = nfold;
+    cnt->nfold = fold[0];
+    cnt->fold_rem = fold[1];
     return cudaSuccess;
 }
 

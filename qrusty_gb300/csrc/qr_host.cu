@@ -166,7 +166,8 @@ struct qr_op {
     // CSR tables, built on the device on first use; their coefficient parts
     // follow every coefficient update on the device
     bool csr_ready = false;
-    uint32_t nfold = 0, nctab = 0;
+    uint32_t nfold = 0, nctab = 0, fold_rem = 0;
+    size_t csr_tables = 0;  // byte offset of the staged fill's tables in d_sig
     DevBuf d_tc, d_pmask, d_sig, d_grp, d_coord, d_ctab, d_fold, d_pbeta, d_ptab, d_fv;
     // term-gradient strings (see GradPlanArgs) per dtype, built on first use
     struct GradPlan {
@@ -230,6 +231,31 @@ int refresh_csr_values(qr_op *op, cudaStream_t st) {
     return QR_OK;
 }
 
+// The operator's CSR tables as kernel arguments (no rows, no outputs yet).
+CsrArgs csr_args(qr_op *op) {
+    CsrArgs a{};
+    a.N = op->N;
+    a.G = op->G;
+    a.gx = op->d_gx.as<uint64_t>();
+    a.n = op->n;
+    a.grp = op->d_grp.as<CsrGroup>();
+    a.pmask = op->d_pmask.as<uint64_t>();
+    a.sig = op->d_sig.as<int32_t>();
+    a.tables = reinterpret_cast<const uint16_t *>(op->d_sig.as<unsigned char>() + op->csr_tables);
+    a.fold = op->d_fold.as<uint32_t>();
+    a.nfold = op->nfold;
+    a.ctab = op->d_ctab.as<double2>();
+    a.pbeta = op->d_pbeta.as<uint64_t>();
+    a.ptab = op->d_ptab.as<double2>();
+    a.nctab = op->nctab;
+    a.tz = op->d_tz.as<uint64_t>();
+    a.tc = op->d_tc.as<double>();
+    a.err = op->d_err.as<int>();
+    a.wide = op->test_wide;
+    a.inline_fold = csr_inline_fold(op->G, op->n, op->nfold, op->fold_rem) ? 1 : 0;
+    return a;
+}
+
 // CSR tables on the device, once per operator (qr_group.cu): the position
 // trie, group spans and descriptors, then the coefficient parts.
 int upload_csr_tables(qr_op *op) {
@@ -238,7 +264,9 @@ int upload_csr_tables(qr_op *op) {
     QR_CUDA(cudaDeviceSynchronize(), "CSR tables: sync");
     const uint64_t G = op->G, T = op->T;
     QR_CUDA(op->d_pmask.alloc(G * sizeof(uint64_t)), "alloc position masks");
-    QR_CUDA(op->d_sig.alloc(G * op->n * sizeof(int32_t)), "alloc position table");
+    // position terms by bit, then the staged fill's tables (16-byte aligned)
+    op->csr_tables = (G * op->n * sizeof(int32_t) + 15u) & ~(size_t)15u;
+    QR_CUDA(op->d_sig.alloc(op->csr_tables + csr_tables_bytes(G, op->n)), "alloc position tables");
     QR_CUDA(op->d_grp.alloc(G * sizeof(CsrGroup)), "alloc group descriptors");
     QR_CUDA(op->d_coord.alloc(T * sizeof(uint16_t)), "alloc span coordinates");
     QR_CUDA(op->d_fold.alloc(G * sizeof(uint32_t)), "alloc fold groups");
@@ -257,6 +285,8 @@ int upload_csr_tables(qr_op *op) {
     QR_CUDA(op->d_ptab.alloc(cnt.nptab * sizeof(cd)), "alloc prefix tables");
     op->nctab = (uint32_t)cnt.nctab;
     op->nfold = cnt.nfold;
+    op->fold_rem = cnt.fold_rem;
+    QR_CUDA(launch_csr_tables(csr_args(op), nullptr), "CSR row-bit tables");
     int rc = refresh_csr_values(op, nullptr);
     if (rc) return rc;
     QR_CUDA(cudaStreamSynchronize(nullptr), "CSR tables: sync");
@@ -1406,30 +1436,12 @@ int qr_csr_build(qr_op *op, uint64_t *indptr, uint64_t *indices, double *data, i
     rc = upload_csr_tables(op);
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    CsrArgs a;
-    a.N = op->N;
-    a.G = op->G;
-    a.gx = op->d_gx.as<uint64_t>();
-    a.n = op->n;
-    a.grp = op->d_grp.as<CsrGroup>();
-    a.pmask = op->d_pmask.as<uint64_t>();
-    a.sig = op->d_sig.as<int32_t>();
-    a.fold = op->d_fold.as<uint32_t>();
-    a.nfold = op->nfold;
-    a.ctab = op->d_ctab.as<double2>();
-    a.pbeta = op->d_pbeta.as<uint64_t>();
-    a.ptab = op->d_ptab.as<double2>();
-    a.nctab = op->nctab;
-    a.tz = op->d_tz.as<uint64_t>();
-    a.tc = op->d_tc.as<double>();
-    a.err = op->d_err.as<int>();
-    a.wide = op->test_wide;
-    a.fvals = nullptr;
+    CsrArgs a = csr_args(op);
     // fold-mode values buffer (nfold x rows) for the staged fill; without
     // it the fold entries are stored in place after the fill
     auto fold_buffer = [&](uint64_t rows) {
         a.fvals = nullptr;
-        if (op->nfold == 0 || op->G > 256) return;
+        if (op->nfold == 0 || op->G > 256 || a.inline_fold) return;
         if (op->d_fv.alloc((size_t)op->nfold * rows * sizeof(double2)) == cudaSuccess)
             a.fvals = op->d_fv.as<double2>();
         else
