@@ -334,7 +334,7 @@ cudaError_t csr_structure(int n, uint64_t G, const uint64_t *gx, const uint32_t 
 // tables) from the raw coefficients: stream-ordered, no synchronisation.
 cudaError_t csr_values(uint64_t G, uint64_t T, const uint32_t *order, const double2 *coef,
                        const uint8_t *phase, double2 *tc, CsrGroup *grp, const uint16_t *coord,
-                       double2 *ctab, double2 *ptab, cudaStream_t st);
+                       double2 *ctab, double2 *ptab, bool has_fold, cudaStream_t st);
 cudaError_t launch_csr_spmv(uint64_t nrows, uint64_t ncols, const uint64_t *indptr,
                             const uint64_t *indices, const double *data, const double *v,
                             double *y, int nsm, cudaStream_t st);

@@ -392,8 +392,144 @@ static cudaError_t group_runs(const uint32_t *P, const uint64_t *ka, const uint6
     return cudaSuccess;
 }
 
+// Grouping of short term lists by counting: what a term's place in every
+// table depends on is how many terms compare less, equal or earlier, so two
+// kernels over all pairs replace the sorts, scans and run searches above
+// (about 55 launches and three host waits, 0.3 ms whatever the length; two
+// launches and one wait here).  Bound by launch latency up to a few hundred
+// terms, then by the pairs, as a thread compares one term against all: an
+// operator of 200 terms is created in 379 us (779 by the sorts), of 4,096 in
+// 590 (931); the pairs' share grows with the length, so the sorts take over
+// there.
+constexpr uint64_t kSmallTerms = 4096;
+constexpr int kSmallThreads = 128;
+constexpr uint32_t kSmallTile = 1024;
+
+// Per term i: lt terms of smaller x, eqb earlier terms of equal x, lx the
+// first term of equal x; ld the first term equal in x and z, eb the earlier
+// ones.  cnt: distinct x, distinct (x, z).
+struct SmallClass {
+    uint32_t lt, eqb, lx, ld, eb;
+};
+
+__global__ void __launch_bounds__(kSmallThreads) small_classes_kernel(uint32_t T,
+                                                                      const uint64_t *x,
+                                                                      const uint64_t *z,
+                                                                      SmallClass *cls,
+                                                                      uint32_t *cnt) {
+    __shared__ uint64_t sx[kSmallTile], sz[kSmallTile];
+    const uint32_t i = blockIdx.x * kSmallThreads + threadIdx.x;
+    const uint64_t xi = i < T ? x[i] : 0, zi = i < T ? z[i] : 0;
+    SmallClass c{0, 0, 0xffffffffu, 0xffffffffu, 0};
+    for (uint32_t base = 0; base < T; base += kSmallTile) {
+        const uint32_t m = min(kSmallTile, T - base);
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < m; j += kSmallThreads) {
+            sx[j] = x[base + j];
+            sz[j] = z[base + j];
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t j = 0; j < m; ++j) {
+            const uint32_t k = base + j;
+            const bool same = sx[j] == xi, both = same && sz[j] == zi;
+            c.lt += sx[j] < xi;
+            c.eqb += same && k < i;
+            c.eb += both && k < i;
+            if (same) c.lx = min(c.lx, k);
+            if (both) c.ld = min(c.ld, k);
+        }
+    }
+    if (i >= T) return;
+    cls[i] = c;
+    if (c.lx == i) atomicAdd(&cnt[0], 1u);
+    if (c.ld == i) atomicAdd(&cnt[1], 1u);
+}
+
+__global__ void __launch_bounds__(kSmallThreads) small_tables_kernel(uint32_t T, const uint64_t *x,
+                                                                     const uint64_t *z,
+                                                                     const SmallClass *cls,
+                                                                     const uint32_t *cnt,
+                                                                     TermGroupsOut o) {
+    __shared__ uint32_t s_lt[kSmallTile], s_lx[kSmallTile], s_ld[kSmallTile];
+    const uint32_t i = blockIdx.x * kSmallThreads + threadIdx.x;
+    const SmallClass c = i < T ? cls[i] : SmallClass{};
+    uint32_t g = 0;      // CSR group: first terms of a smaller x
+    uint32_t m = 0;      // merged string: strings that occur first
+    uint32_t moff = 0;   // terms of those strings
+    uint32_t ga = 0;     // x group in order of first occurrence
+    uint32_t aoff = 0;   // strings of the groups before it
+    uint32_t arank = 0;  // strings of this group before term i
+    for (uint32_t base = 0; base < T; base += kSmallTile) {
+        const uint32_t n = min(kSmallTile, T - base);
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < n; j += kSmallThreads) {
+            const SmallClass k = cls[base + j];
+            s_lt[j] = k.lt;
+            s_lx[j] = k.lx;
+            s_ld[j] = k.ld;
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t j = 0; j < n; ++j) {
+            const uint32_t k = base + j;
+            const bool fx = s_lx[j] == k, fs = s_ld[j] == k;
+            g += fx && s_lt[j] < c.lt;
+            m += fs && k < c.ld;
+            moff += s_ld[j] < c.ld;
+            ga += fx && k < c.lx;
+            aoff += fs && s_lx[j] < c.lx;
+            arank += fs && s_lx[j] == c.lx && k < i;
+        }
+    }
+    if (i >= T) return;
+    const uint64_t xi = x[i], zi = z[i];
+    o.order[c.lt + c.eqb] = i;
+    o.tz[c.lt + c.eqb] = zi;
+    o.mmap[i] = m;
+    o.mm_terms[moff + c.eb] = i;
+    if (c.lx == i) {
+        o.gx[g] = xi;
+        o.goff[g] = c.lt;
+        o.ag_off[ga] = aoff;
+    }
+    if (c.ld == i) {
+        o.mm_off[m] = moff;
+        o.mx[m] = xi;
+        o.mz[m] = zi;
+        o.madj[m] = (uint8_t)(__popcll(xi & zi) & 1);
+        o.ag_mem[aoff + arank] = m;
+    }
+    if (i == 0) {
+        o.goff[cnt[0]] = T;
+        o.mm_off[cnt[1]] = T;
+        o.ag_off[cnt[0]] = cnt[1];
+    }
+}
+
+static cudaError_t group_small(uint32_t T, const uint64_t *x, const uint64_t *z,
+                               const TermGroupsOut &o, TermGroupCounts *cnt, cudaStream_t st) {
+    Scratch sc{st};
+    SmallClass *cls = sc.get<SmallClass>(T + 1);  // the counts after the classes
+    GR_TRY(sc.e);
+    uint32_t *dc = reinterpret_cast<uint32_t *>(cls + T);
+    GR_TRY(cudaMemsetAsync(dc, 0, 2 * sizeof(uint32_t), st));
+    const unsigned g = (T + kSmallThreads - 1) / kSmallThreads;
+    small_classes_kernel<<<g, kSmallThreads, 0, st>>>(T, x, z, cls, dc);
+    GR_LAUNCH();
+    small_tables_kernel<<<g, kSmallThreads, 0, st>>>(T, x, z, cls, dc, o);
+    GR_LAUNCH();
+    uint32_t h[2] = {0, 0};
+    GR_TRY(cudaMemcpyAsync(h, dc, sizeof(h), cudaMemcpyDeviceToHost, st));
+    GR_TRY(cudaStreamSynchronize(st));
+    cnt->G = cnt->Ga = h[0];
+    cnt->M = h[1];
+    return cudaSuccess;
+}
+
 cudaError_t group_terms(int n, uint64_t T, const uint64_t *x, const uint64_t *z,
                         const TermGroupsOut &o, TermGroupCounts *cnt, cudaStream_t st) {
+    if (T <= kSmallTerms) return group_small((uint32_t)T, x, z, o, cnt, st);
     Scratch sc{st};
     uint64_t *ka = sc.get<uint64_t>(T), *kb = sc.get<uint64_t>(T);
     uint32_t *va = sc.get<uint32_t>(T), *vb = sc.get<uint32_t>(T);
@@ -470,25 +606,28 @@ __device__ __forceinline__ uint32_t lower_bound_u64(const uint64_t *a, uint32_t 
 // Position trie over the ascending x masks: at bit b, the groups sharing x_g's
 // bits above b form a range; where bit b splits it, sigma_{g,b} is the size of
 // the other side (+ when x_g is on the 0-side, - on the 1-side).
+__device__ void csr_trie(const uint64_t *gx, uint32_t G, int n, uint64_t g, uint64_t *pmask,
+                         int32_t *sig) {
+    const uint64_t x = gx[g];
+    uint64_t pm = 0;
+    for (int b = n - 1; b >= 0; --b) {
+        const uint64_t pre = (x >> (b + 1)) << (b + 1);  // b + 1 <= 63
+        const uint32_t lo = lower_bound_u64(gx, 0, G, pre);
+        const uint32_t hi = lower_bound_u64(gx, lo, G, pre + (2ull << b));
+        const uint32_t mid = lower_bound_u64(gx, lo, hi, pre | (1ull << b));
+        int32_t s = 0;
+        if (mid > lo && mid < hi) {
+            pm |= 1ull << b;
+            s = ((x >> b) & 1) ? -(int32_t)(mid - lo) : (int32_t)(hi - mid);
+        }
+        sig[g * (uint64_t)n + b] = s;
+    }
+    pmask[g] = pm;
+}
+
 __global__ void csr_trie_kernel(const uint64_t *gx, uint32_t G, int n, uint64_t *pmask,
                                 int32_t *sig) {
-    GRID_STRIDE(g, G) {
-        const uint64_t x = gx[g];
-        uint64_t pm = 0;
-        for (int b = n - 1; b >= 0; --b) {
-            const uint64_t pre = (x >> (b + 1)) << (b + 1);  // b + 1 <= 63
-            const uint32_t lo = lower_bound_u64(gx, 0, G, pre);
-            const uint32_t hi = lower_bound_u64(gx, lo, G, pre + (2ull << b));
-            const uint32_t mid = lower_bound_u64(gx, lo, hi, pre | (1ull << b));
-            int32_t s = 0;
-            if (mid > lo && mid < hi) {
-                pm |= 1ull << b;
-                s = ((x >> b) & 1) ? -(int32_t)(mid - lo) : (int32_t)(hi - mid);
-            }
-            sig[g * (uint64_t)n + b] = s;
-        }
-        pmask[g] = pm;
-    }
+    GRID_STRIDE(g, G) csr_trie(gx, G, n, g, pmask, sig);
 }
 
 // GF(2) span of tz[k] ^ tz[k0] over k in [k0, k1): basis in insertion order,
@@ -539,46 +678,62 @@ __device__ int group_span(const uint64_t *tz, uint32_t k0, uint32_t k1, uint64_t
 // Per group: rank-<= kCsrMaxRank span (class table of 2^(d+1) entries) or
 // fold mode with the leading terms of span rank <= kCsrPrefixRank folded per
 // class (prefix table).  tab and zparts are filled later.
+struct CsrSpan {
+    CsrGroup d;
+    uint64_t basis[kCsrPrefixRank];  // prefix span basis (fold mode; zeros after it)
+    uint64_t ctsz, ptsz;             // class and prefix table entries
+    uint32_t isfold, rem;            // fold mode, and its terms past the prefix
+};
+__device__ void csr_span(uint32_t k0, uint32_t k1, const uint64_t *tz, uint16_t *coord,
+                         CsrSpan &s) {
+    CsrGroup &d = s.d;
+    d.k0 = k0;
+    d.k1 = k1;
+    d.z0 = tz[k0];
+    for (int j = 0; j < kCsrMaxRank; ++j) d.beta[j] = 0;
+    d.tab = 0;
+    d.zparts = 0;
+    d.pre = 0;
+    s.ctsz = s.ptsz = 0;
+    s.isfold = s.rem = 0;
+    uint32_t used;
+    int nb;
+    const int r = group_span<kCsrMaxRank>(tz, k0, k1, s.basis, coord, &used, &nb);
+    if (r >= 0) {
+        d.d = (uint32_t)r;
+        for (int j = 0; j < r; ++j) d.beta[j] = s.basis[j];
+        s.ctsz = 2ull << r;
+        return;
+    }
+    d.d = kCsrFold;
+    group_span<kCsrPrefixRank>(tz, k0, k1, s.basis, coord, &used, &nb);
+    for (int j = nb; j < kCsrPrefixRank; ++j) s.basis[j] = 0;
+    // the kernel continues the term-order fold after the prefix, so a
+    // prefix cut short of a 24-bit count gives the same additions
+    const uint32_t m = used < 0xffffffu ? used : 0xffffffu;
+    if (m >= 2) {
+        d.pre = m | ((uint32_t)nb << 24);
+        s.ptsz = 2ull << nb;
+    }
+    s.isfold = 1;
+    s.rem = k1 - k0 - (d.pre & 0xffffffu);
+}
+
 __global__ void csr_span_kernel(uint32_t G, const uint32_t *goff, const uint64_t *tz,
                                 CsrGroup *grp, uint16_t *coord, uint64_t *ctsz, uint64_t *ptsz,
                                 uint32_t *isfold, uint64_t *gbeta, uint32_t *fold_rem) {
     GRID_STRIDE(g, G) {
-        CsrGroup d;
-        d.k0 = goff[g];
-        d.k1 = goff[g + 1];
-        d.z0 = tz[d.k0];
-        for (int j = 0; j < kCsrMaxRank; ++j) d.beta[j] = 0;
-        d.tab = 0;
-        d.zparts = 0;
-        d.pre = 0;
-        uint64_t basis[kCsrPrefixRank];
-        uint32_t used;
-        int nb;
-        const int r = group_span<kCsrMaxRank>(tz, d.k0, d.k1, basis, coord, &used, &nb);
-        if (r >= 0) {
-            d.d = (uint32_t)r;
-            for (int j = 0; j < r; ++j) d.beta[j] = basis[j];
-            ctsz[g] = 2ull << r;
-            ptsz[g] = 0;
-            isfold[g] = 0;
-        } else {
-            d.d = kCsrFold;
-            group_span<kCsrPrefixRank>(tz, d.k0, d.k1, basis, coord, &used, &nb);
-            // the kernel continues the term-order fold after the prefix, so a
-            // prefix cut short of a 24-bit count gives the same additions
-            const uint32_t m = used < 0xffffffu ? used : 0xffffffu;
-            ptsz[g] = 0;
-            if (m >= 2) {
-                d.pre = m | ((uint32_t)nb << 24);
-                ptsz[g] = 2ull << nb;
-            }
+        CsrSpan s;
+        csr_span(goff[g], goff[g + 1], tz, coord, s);
+        grp[g] = s.d;
+        ctsz[g] = s.ctsz;
+        ptsz[g] = s.ptsz;
+        isfold[g] = s.isfold;
+        if (s.isfold) {
             for (int j = 0; j < kCsrPrefixRank; ++j)
-                gbeta[g * (uint64_t)kCsrPrefixRank + j] = j < nb ? basis[j] : 0ull;
-            ctsz[g] = 0;
-            isfold[g] = 1;
-            atomicMax(fold_rem, d.k1 - d.k0 - (d.pre & 0xffffffu));
+                gbeta[g * (uint64_t)kCsrPrefixRank + j] = s.basis[j];
+            atomicMax(fold_rem, s.rem);
         }
-        grp[g] = d;
     }
 }
 
@@ -600,10 +755,87 @@ __global__ void csr_desc_kernel(uint32_t G, CsrGroup *grp, const uint64_t *ctoff
     }
 }
 
+// Up to kSmallGroups groups: trie, spans, offsets and descriptors by one block,
+// a thread per group.  Launch latency bounds it: one launch and one copy of
+// totals instead of 12 and three (first CSR build of a chain n = 21: 803 us
+// with them, 687 so, prefix tables over several blocks included).
+constexpr uint32_t kSmallGroups = 512;
+
+struct CsrTotals {
+    uint64_t nctab, nptab;
+    uint32_t nfold, fold_rem;
+};
+
+__global__ void __launch_bounds__(kSmallGroups) csr_small_kernel(int n, uint32_t G,
+                                                                 const uint64_t *gx,
+                                                                 const uint32_t *goff,
+                                                                 const uint64_t *tz,
+                                                                 CsrStructOut o, CsrTotals *tot) {
+    __shared__ uint64_t s_ct[kSmallGroups], s_pt[kSmallGroups];
+    __shared__ uint32_t s_f[kSmallGroups], s_rem;
+    const uint32_t g = threadIdx.x;
+    if (g == 0) s_rem = 0;
+    if (g < G) csr_trie(gx, G, n, g, o.pmask, o.sig);
+    CsrSpan s;
+    s.ctsz = s.ptsz = 0;
+    s.isfold = s.rem = 0;
+    if (g < G) csr_span(goff[g], goff[g + 1], tz, o.coord, s);
+    s_ct[g] = s.ctsz;
+    s_pt[g] = s.ptsz;
+    s_f[g] = s.isfold;
+    __syncthreads();
+    if (s.isfold) atomicMax(&s_rem, s.rem);
+    for (uint32_t w = 1; w < blockDim.x; w <<= 1) {  // inclusive sums
+        uint64_t c = 0, p = 0;
+        uint32_t f = 0;
+        if (g >= w) {
+            c = s_ct[g - w];
+            p = s_pt[g - w];
+            f = s_f[g - w];
+        }
+        __syncthreads();
+        s_ct[g] += c;
+        s_pt[g] += p;
+        s_f[g] += f;
+        __syncthreads();
+    }
+    if (g < G) {
+        if (s.isfold) {
+            const uint32_t f = s_f[g] - 1u;
+            o.fold[f] = g;
+            s.d.tab = s.d.pre ? (uint32_t)(s_pt[g] - s.ptsz) : 0u;
+            for (int j = 0; j < kCsrPrefixRank; ++j)
+                o.pbeta[(uint64_t)f * kCsrPrefixRank + j] = s.basis[j];
+        } else {
+            s.d.tab = (uint32_t)(s_ct[g] - s.ctsz);
+        }
+        o.grp[g] = s.d;
+    }
+    if (g == G - 1u) *tot = CsrTotals{s_ct[g], s_pt[g], s_f[g], s_rem};
+}
+
+static cudaError_t csr_structure_small(int n, uint32_t G, const uint64_t *gx, const uint32_t *goff,
+                                       const uint64_t *tz, const CsrStructOut &o,
+                                       CsrStructCounts *cnt, cudaStream_t st) {
+    Scratch sc{st};
+    CsrTotals *dt = sc.get<CsrTotals>(1), h{};
+    GR_TRY(sc.e);
+    csr_small_kernel<<<1, (G + 31u) & ~31u, 0, st>>>(n, G, gx, goff, tz, o, dt);
+    GR_LAUNCH();
+    GR_TRY(cudaMemcpyAsync(&h, dt, sizeof(h), cudaMemcpyDeviceToHost, st));
+    GR_TRY(cudaStreamSynchronize(st));
+    cnt->nctab = h.nctab;
+    cnt->nptab = h.nptab;
+    cnt->nfold = h.nfold;
+    cnt->fold_rem = h.fold_rem;
+    return cudaSuccess;
+}
+
 cudaError_t csr_structure(int n, uint64_t G, const uint64_t *gx, const uint32_t *goff,
                           const uint64_t *tz, const CsrStructOut &o, CsrStructCounts *cnt,
                           cudaStream_t st) {
     if (G == 0 || G > 0xffffffffull) return cudaErrorInvalidValue;
+    if (G <= kSmallGroups) return csr_structure_small(n, (uint32_t)G, gx, goff, tz, o, cnt, st);
     Scratch sc{st};
     uint64_t *ctsz = sc.get<uint64_t>(G + 1), *ptsz = sc.get<uint64_t>(G + 1);
     uint32_t *foff = sc.get<uint32_t>(G + 2);  // fold flags' scan, then the longest remainder
@@ -663,7 +895,7 @@ __global__ void __launch_bounds__(128) csr_fold_tables_kernel(uint32_t G, CsrGro
             }
             rz = __syncthreads_and(rz);
             iz = __syncthreads_and(iz);
-            if (threadIdx.x == 0) grp[g].zparts = (rz ? 1u : 0u) | (iz ? 2u : 0u);
+            if (threadIdx.x == 0 && blockIdx.y == 0) grp[g].zparts = (rz ? 1u : 0u) | (iz ? 2u : 0u);
             m = pre & 0xffffffu;
             if (m < 2) continue;
             ncls = 2u << (pre >> 24);
@@ -673,7 +905,9 @@ __global__ void __launch_bounds__(128) csr_fold_tables_kernel(uint32_t G, CsrGro
             ncls = 2u << d;
             out = ctab + tab;
         }
-        for (uint32_t c = threadIdx.x; c < ncls; c += blockDim.x) {
+        // a prefix table's classes over the blocks of grid row g (one block: 40 us)
+        for (uint32_t c = blockIdx.y * blockDim.x + threadIdx.x; c < ncls;
+             c += gridDim.y * blockDim.x) {
             double2 v = make_double2(0.0, 0.0);
             for (uint32_t k = k0; k < k0 + m; ++k) {
                 const uint32_t sel = 1u | ((uint32_t)coord[k] << 1);
@@ -696,11 +930,12 @@ __global__ void __launch_bounds__(128) csr_fold_tables_kernel(uint32_t G, CsrGro
 
 cudaError_t csr_values(uint64_t G, uint64_t T, const uint32_t *order, const double2 *coef,
                        const uint8_t *phase, double2 *tc, CsrGroup *grp, const uint16_t *coord,
-                       double2 *ctab, double2 *ptab, cudaStream_t st) {
+                       double2 *ctab, double2 *ptab, bool has_fold, cudaStream_t st) {
     csr_tc_kernel<<<grid_of(T), 256, 0, st>>>(order, coef, phase, T, tc);
     GR_LAUNCH();
     const unsigned gb = G < 4096 ? (unsigned)(G ? G : 1) : 4096u;
-    csr_fold_tables_kernel<<<gb, 128, 0, st>>>((uint32_t)G, grp, coord, tc, ctab, ptab);
+    csr_fold_tables_kernel<<<dim3(gb, has_fold ? 16u : 1u), 128, 0, st>>>((uint32_t)G, grp, coord,
+                                                                          tc, ctab, ptab);
     GR_LAUNCH();
     return cudaSuccess;
 }

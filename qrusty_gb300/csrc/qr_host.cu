@@ -226,7 +226,7 @@ int refresh_csr_values(qr_op *op, cudaStream_t st) {
     QR_CUDA(csr_values(op->G, op->T, op->d_order.as<uint32_t>(), op->d_coef.as<double2>(),
                        op->d_ph.as<uint8_t>(), op->d_tc.as<double2>(), op->d_grp.as<CsrGroup>(),
                        op->d_coord.as<uint16_t>(), op->d_ctab.as<double2>(),
-                       op->d_ptab.as<double2>(), st),
+                       op->d_ptab.as<double2>(), op->nfold > 0, st),
             "CSR coefficient tables");
     return QR_OK;
 }
