@@ -245,9 +245,12 @@ cudaError_t launch_diag(int dtype, int n, int db, uint64_t ntiles, const uint64_
 constexpr int kCsrMaxRank = 4;
 constexpr uint32_t kCsrFold = 0xffffffffu;
 // Fold-mode groups: the longest leading run of terms whose z differences
-// span rank <= kCsrPrefixRank is folded per class on the host (table of
-// 2^(rank+1) entries); rows add only the terms after it.
-constexpr int kCsrPrefixRank = 10;
+// span rank <= kCsrPrefixRank is folded per class once (table of
+// 2^(rank+1) entries); rows add only the terms after it.  Rank 12 (128 KB per
+// fold-mode group): chain n = 21 builds in 330 us, 338 with rank 10; with rank
+// 14 a Jordan-Wigner operator of 94 groups, n = 18, takes 143 instead of 132,
+// its rows' reads missing L1.
+constexpr int kCsrPrefixRank = 12;
 struct CsrGroup {
     uint64_t z0;
     uint64_t beta[kCsrMaxRank];

@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kCsrThreads) csr_fill_kernel(const CsrArgs a) 
 // Fold-mode groups (z span wider than kCsrMaxRank): one thread per row, all
 // lanes of a warp on the same group, the group's +-c'_k folded in input-term
 // order from the first term (make_row's fold), terms read warp-uniformly.
-// The leading terms up to z-span rank kCsrPrefixRank come from the host's
+// The leading terms up to z-span rank kCsrPrefixRank come from a
 // per-class fold of them (same additions, same order); the rest are added
 // per row.  A part (re or im) whose every coefficient is +-0 takes no FP64
 // additions: under round-to-nearest a sum of signed zeros is -0 exactly when
@@ -259,7 +259,7 @@ __device__ __forceinline__ double2 csr_fold_entry(const CsrArgs &a, uint64_t r, 
 // block goes on with the next unit that has not started
 // (clusterlaunchcontrol), which keeps its tables.  What is left above the
 // write stream's time is a stage's barrier, stores and bookkeeping: chain
-// n = 21 takes 336 us (two-buffer stages over fixed strides, per-chunk sums
+// n = 21 takes 330 us (two-buffer stages over fixed strides, per-chunk sums
 // in every thread and a fold kernel before it: 487), random strings n = 16,
 // 200 groups, 55 us (67).
 constexpr uint32_t kCsrBufs = 3;  // staging buffers
@@ -342,7 +342,8 @@ __host__ __device__ inline uint32_t csr_unit_chunks(uint32_t G, int L, uint64_t 
 // share of the write stream takes about (G << L) * 2.8 clocks a chunk.  Folded
 // here while the fold is a third of that at most (chain n = 21, 9 terms and
 // 2,688 entries a chunk: 338 us against 370 through the value buffer; an
-// operator of 94 groups, 26 terms and chunks of 16 rows: 195 against 158).  One group (the
+// operator of 94 groups, 26 terms and chunks of 16 rows: 195 against 158;
+// both with prefixes of rank 10).  One group (the
 // diagonal of a spin chain); all row bits have to be in the tables.
 bool csr_inline_fold(uint64_t G, int n, uint32_t nfold, uint32_t fold_rem) {
     if (G > (uint64_t)kCsrThreads || nfold != 1 || fold_rem > kCsrInlineRem) return false;

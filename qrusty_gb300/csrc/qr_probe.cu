@@ -19,6 +19,10 @@ constexpr int kThreads = 256;
 __global__ void __launch_bounds__(kThreads) dfma_chains(int iters, double a, double b,
                                                         double *out) {
     double x[kChains];
+    // per-thread operands: kernel parameters would be read as constants by
+    // every DFMA, at 0.84 of the rate of registers
+    a -= (double)threadIdx.x * 1e-14;
+    b += (double)threadIdx.x * 1e-14;
 #pragma unroll
     for (int k = 0; k < kChains; ++k) x[k] = (double)(threadIdx.x + k) * 1e-3;
     for (int i = 0; i < iters; ++i) {

@@ -34,7 +34,7 @@ def test_stage_sizes(cuda, oracle, n, groups):
 
 # one wide diagonal group of m terms among narrow ones: prefix only, a few and
 # the most terms after it that are folded in the pass, and one more
-@pytest.mark.parametrize("m", [6, 11, 12, 19, 40, 74, 75, 76, 90])
+@pytest.mark.parametrize("m", [6, 12, 13, 14, 19, 29, 30, 31, 40, 76, 77, 78, 90])
 @pytest.mark.parametrize("kind", ["real", "imag", "complex", "zeros"])
 def test_one_wide_group(cuda, oracle, m, kind):
     n, groups = 14, 70
