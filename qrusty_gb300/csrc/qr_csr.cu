@@ -11,13 +11,13 @@
 //     pos_r(g) = g + sum_{b : bit b of r set} sigma_{g,b},
 // where sigma_{g,b} = +S (x_g has 0 at b) or -S (x_g has 1 at b) and S is
 // the size of g's sibling subtree at bit b of the binary trie of the x
-// masks (nonzero only at the trie's branching bits).  The host precomputes
-// the (b, sigma) lists; each thread places one (row, group) entry directly.
+// masks (nonzero only at the trie's branching bits).  qr_group.cu computes
+// the sigmas; each thread places one (row, group) entry directly.
 //
 // Values without a per-row fold: a group's value in row r depends on r only
 // through the parities of r against the group's z masks, i.e. against z0 and
-// a GF(2) basis beta_1..beta_d of the differences z_k ^ z0.  For d <= 4 the
-// host folds the group's +-c'_k in input order once per class (2^(d+1)
+// a GF(2) basis beta_1..beta_d of the differences z_k ^ z0.  For d <= 4
+// the group's +-c'_k are folded in input order once per class (2^(d+1)
 // classes) -- the same additions in the same order as make_row, hence the
 // same bits -- and the kernel reads the row's class from that table.
 #include "qr_common.cuh"
@@ -83,8 +83,7 @@ constexpr uint32_t kCsrSmemCtab = 2048;  // class-table entries staged in shared
 
 // Low-bit width of the per-group position lookup table: G x (2^L + 1)
 // 32-bit entries (rows padded by one word so lanes on consecutive groups hit
-// distinct banks) within 16 KB, so that with the staging buffers four
-// 256-thread blocks fit an SM's 228 KB.  L <= 8, so 256-row launches stay aligned.
+// distinct banks) within 16 KB.  L <= 8, so 256-row launches stay aligned.
 __host__ __device__ inline int csr_lut_bits(uint32_t G) {
     int L = 8;
     while (L > 1 && (size_t)G * ((1u << L) + 1) * 4u > kCsrLutBytes) --L;
