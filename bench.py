@@ -660,7 +660,8 @@ def measure_batch(steps=3, warmup=3, per_op=True):
                        "8 complex64 states each" % (W.SEED0 + 3),
            "ms_per_step": ms_b, "value": units / (ms_b / 1e3), "unit": UNIT,
            "mode": {0: "persistent work-list kernel", 1: "graph of per-operator kernels",
-                    2: "persistent kernel for the small operators + per-operator kernels"}
+                    2: "persistent kernel for the small operators, string kernel over the random-letter "
+                       "ones, per-operator kernels for the rest"}
                    .get(b.mode, str(b.mode)),
            "mode_code": b.mode,
            "tile_bits": b.tile_bits, "gpu_launches_per_step": launches,

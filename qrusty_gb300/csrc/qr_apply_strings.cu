@@ -115,16 +115,64 @@ __device__ __forceinline__ void str_mac(float2 (&y)[8], const float4 (&p)[4], ui
     }
 }
 
+// One block of the ring: the diagonal where it is flagged, then the strings in
+// turn, one's partner loads in flight while the other's products are formed.
+template <bool WIDE>
+__device__ __forceinline__ void str_block(float2 (&y)[8], float2 (&hi)[8], uint32_t &win,
+                                          const unsigned char *sm, const uint4 *E, uint32_t base,
+                                          const float4 *dg, uint32_t t, uint32_t r0, uint32_t rhi) {
+    float4 pa[4], pb[4];
+    const uint2 head = *reinterpret_cast<const uint2 *>(E);
+    const uint32_t ne = head.x;
+    if (head.y != 0) {
+        str_load(pa, sm, base, 0);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 d = dg[t + 512u * (uint32_t)j], p = pa[j];
+            float2 &u = y[2 * j], &v = y[2 * j + 1];
+            u.x = fmaf(d.x, p.x, fmaf(-d.y, p.y, u.x));
+            u.y = fmaf(d.x, p.y, fmaf(d.y, p.x, u.y));
+            v.x = fmaf(d.z, p.z, fmaf(-d.w, p.w, v.x));
+            v.y = fmaf(d.z, p.w, fmaf(d.w, p.z, v.y));
+        }
+    }
+    uint32_t i = 1;
+    uint4 ea = E[1], eb;
+    if (ne > 0) str_load(pa, sm, base, ea.x);
+    for (; i + 1 < ne; i += 2) {
+        eb = E[i + 1];
+        str_load(pb, sm, base, eb.x);
+        str_mac<WIDE>(y, pa, ea, r0, rhi);
+        ea = E[i + 2];
+        str_load(pa, sm, base, ea.x);
+        str_mac<WIDE>(y, pb, eb, r0, rhi);
+    }
+    if (i < ne) {
+        eb = E[i + 1];
+        str_load(pb, sm, base, eb.x);
+        str_mac<WIDE>(y, pa, ea, r0, rhi);
+        str_mac<WIDE>(y, pb, eb, r0, rhi);
+    } else if (i == ne) {
+        str_mac<WIDE>(y, pa, ea, r0, rhi);
+    }
+    win += ne;
+    if (win >= kSFold) {
+        win = 0;
+#pragma unroll
+        for (int m = 0; m < 8; ++m) y[m] = two_sum_carry2(hi[m], y[m]);
+    }
+}
+
 // Row r with every product formed: what a row that met an infinite or NaN
 // amplitude must return (0 * inf included).
-__device__ __noinline__ float2 str_row(const ApplyArgs &a, uint64_t st, uint64_t r) {
-    const float2 *psi = static_cast<const float2 *>(a.psi) + st * a.N;
+__device__ __noinline__ float2 str_row(const uint4 *sblk, uint32_t nblk, const uint4 *ent,
+                                       const float2 *diag, const float2 *psi, uint64_t r) {
     float yr = 0.f, yi = 0.f;
-    for (uint32_t b = 0; b < a.nsblk; ++b) {
-        const uint4 bl = a.sblk[b];
-        const uint4 *E = a.ent + bl.z;
+    for (uint32_t b = 0; b < nblk; ++b) {
+        const uint4 bl = sblk[b];
+        const uint4 *E = ent + bl.z;
         if (E[0].y != 0) {
-            const float2 d = static_cast<const float2 *>(a.diag)[r], p = psi[r];
+            const float2 d = diag[r], p = psi[r];
             yr += d.x * p.x - d.y * p.y;
             yi += d.x * p.y + d.y * p.x;
         }
@@ -266,7 +314,6 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
         float2 y[8], hi[8];
-        float4 pa[4], pb[4];
         uint32_t s = 0, par = 0, it = 0;
         const uint32_t t16 = t << 4;
         for (uint64_t item = cl; item < a.nitems; item += ncl, ++it) {
@@ -293,49 +340,8 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
                 }
                 if (!skip) {
                     const uint4 *E = reinterpret_cast<const uint4 *>(s_ent + (size_t)s * kSEntBytes);
-                    const uint32_t base = s * slot + t16;
-                    const uint2 head = *reinterpret_cast<const uint2 *>(E);
-                    const uint32_t ne = head.x;
-                    if (head.y != 0) {
-                        const float4 *dg = reinterpret_cast<const float4 *>(a.diag) + (q << 11);
-                        str_load(pa, smem_raw, base, 0);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float4 d = dg[t + 512u * (uint32_t)j], p = pa[j];
-                            float2 &u = y[2 * j], &v = y[2 * j + 1];
-                            u.x = fmaf(d.x, p.x, fmaf(-d.y, p.y, u.x));
-                            u.y = fmaf(d.x, p.y, fmaf(d.y, p.x, u.y));
-                            v.x = fmaf(d.z, p.z, fmaf(-d.w, p.w, v.x));
-                            v.y = fmaf(d.z, p.w, fmaf(d.w, p.z, v.y));
-                        }
-                    }
-                    // two strings in turn: one's partner loads are in flight
-                    // while the other's products are formed
-                    uint32_t i = 1;
-                    uint4 ea = E[1], eb;
-                    if (ne > 0) str_load(pa, smem_raw, base, ea.x);
-                    for (; i + 1 < ne; i += 2) {
-                        eb = E[i + 1];
-                        str_load(pb, smem_raw, base, eb.x);
-                        str_mac<WIDE>(y, pa, ea, r0, rhi);
-                        ea = E[i + 2];
-                        str_load(pa, smem_raw, base, ea.x);
-                        str_mac<WIDE>(y, pb, eb, r0, rhi);
-                    }
-                    if (i < ne) {
-                        eb = E[i + 1];
-                        str_load(pb, smem_raw, base, eb.x);
-                        str_mac<WIDE>(y, pa, ea, r0, rhi);
-                        str_mac<WIDE>(y, pb, eb, r0, rhi);
-                    } else if (i == ne) {
-                        str_mac<WIDE>(y, pa, ea, r0, rhi);
-                    }
-                    win += ne;
-                    if (win >= kSFold) {
-                        win = 0;
-#pragma unroll
-                        for (int m = 0; m < 8; ++m) y[m] = two_sum_carry2(hi[m], y[m]);
-                    }
+                    str_block<WIDE>(y, hi, win, smem_raw, E, s * slot + t16,
+                                    static_cast<const float4 *>(a.diag) + (q << 11), t, r0, rhi);
                 }
                 __syncwarp();
                 if (lane == 0) arrive_local(&empty[s]);
@@ -413,7 +419,8 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
                 const uint32_t rl = row_of((uint32_t)(__ffs((int)redo) - 1));
                 redo &= redo - 1u;
                 // the compensated sum of an infinite part is NaN
-                float2 o = str_row(a, st, (q << 12) | rl);
+                float2 o = str_row(a.sblk, a.nsblk, a.ent, static_cast<const float2 *>(a.diag),
+                                   static_cast<const float2 *>(a.psi) + st * a.N, (q << 12) | rl);
                 if (!(fabsf(o.x) <= kFltMax)) o.x = __uint_as_float(0x7fc00000u);
                 if (!(fabsf(o.y) <= kFltMax)) o.y = __uint_as_float(0x7fc00000u);
                 finish(rl, o);
@@ -424,6 +431,164 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
     if (ks > 1) {  // a peer may still read this CTA's sums or arrive on its barriers
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
+}
+
+// Many operators, states and tiles in one launch: the same ring and inner loop,
+// a CTA per SM taking the next (operator, state, tile) item, largest first,
+// from a counter as it gets free.  What an operator's own launch leaves idle
+// is the SMs its tiles do not cover (four states of 2^17 amplitudes are 128
+// tiles on 152 SMs; smaller ones are split over clusters, with a round of
+// exchange per tile) and its start and end; the ring runs on from item to
+// item.  24 operators of 10 to 17 qubits, 4 states: 1,366 us (1,428 with the
+// small ones in the table kernel and a launch per large one).  A string and
+// tile cost 390 clocks of an SM, as in a full launch of one operator, of which
+// the shared-memory wavefronts are 288.  A block's item travels with it: {operator, state, tile, first | last
+// << 1 | end << 2}.
+__global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings_batch(const StrBatchArgs a) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ uint64_t full[kSMaxStages], empty[kSMaxStages];
+    __shared__ uint4 s_meta[kSMaxStages];
+    __shared__ uint32_t s_abort_;
+    volatile uint32_t *s_abort = &s_abort_;
+    constexpr uint32_t kEnd = 4u;
+    unsigned char *s_ent = smem_raw + (size_t)kSMaxStages * kSTileBytes;
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (t == 0) {
+        for (uint32_t s = 0; s < kSMaxStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], kSWarps);
+        }
+        s_abort_ = 0;
+        mbar_fence_init();
+    }
+    __syncthreads();
+
+    if (warp >= kSWarps) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+        if (warp == kSWarps && lane == 0) {
+            uint32_t s = 0, round = 0, issued = 0, last_round[kSMaxStages];
+            bool ok = true;
+            // the stage is free, or the kernel gives up
+            auto take = [&]() {
+                if (round > 0 && !mbar_wait_bounded(&empty[s], (round - 1) & 1u, a.wait_ns)) {
+                    atomicExch(a.err, kErrMbarTimeout);
+                    *s_abort = 1;
+                }
+                ok = *s_abort == 0;
+                return ok;
+            };
+            auto next = [&]() {
+                if (++s == kSMaxStages) {
+                    s = 0;
+                    ++round;
+                }
+            };
+            uint32_t i = atomicAdd(a.counter, 1u);
+            while (ok && i < a.nitems) {
+                const uint32_t ahead = atomicAdd(a.counter, 1u);
+                const BatchItem it = a.items[i];
+                const StrOp op = a.ops[it.op];
+                const float2 *src = a.psi[it.op] + (uint64_t)it.state * op.N;
+                for (uint32_t b = 0; b < op.nblk && take(); ++b, next()) {
+                    const uint4 bl = op.sblk[b];
+                    const uint32_t eb = (bl.w + 1u) * 16u;
+                    s_meta[s] = make_uint4(it.op, it.state, it.tile,
+                                           (b == 0 ? 1u : 0u) | (b + 1 == op.nblk ? 2u : 0u));
+                    mbar_expect_tx(&full[s], kSTileBytes + eb);
+                    bulk_g2s(smem_raw + (size_t)s * kSTileBytes,
+                             src + ((uint64_t)(it.tile ^ bl.x) << 12), kSTileBytes, &full[s]);
+                    bulk_g2s(s_ent + (size_t)s * kSEntBytes, op.ent + bl.z, eb, &full[s]);
+                    issued |= 1u << s;
+                    last_round[s] = round;
+                }
+                i = ahead;
+            }
+            if (ok && take()) {
+                s_meta[s] = make_uint4(0u, 0u, 0u, kEnd);
+                arrive_local(&full[s]);
+            }
+            // after an expired wait no copy is in flight when the CTA exits
+            if (!ok) {
+                for (uint32_t k = 0; k < kSMaxStages; ++k)
+                    if (issued >> k & 1u) mbar_wait_bounded(&full[k], last_round[k] & 1u, kWaitLimitNs);
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+        float2 y[8], hi[8];
+        uint32_t s = 0, par = 0, win = 0;
+        for (;;) {
+            // an expired wait sets the abort flag; every warp then leaves
+            bool skip = false;
+            if (!__all_sync(0xffffffffu, mbar_try_wait(&full[s], par))) {
+                skip = *s_abort != 0;
+                if (!skip && !mbar_wait_bounded(&full[s], par, a.wait_ns)) {
+                    if (lane == 0) {
+                        atomicExch(a.err, kErrMbarTimeout);
+                        *s_abort = 1;
+                    }
+                    skip = true;
+                }
+                skip = __any_sync(0xffffffffu, skip);
+            }
+            if (skip) break;
+            const uint4 me = s_meta[s];
+            if (me.w & kEnd) break;
+            if (me.w & 1u) {
+                win = 0;
+#pragma unroll
+                for (int m = 0; m < 8; ++m) y[m] = hi[m] = make_float2(0.f, 0.f);
+            }
+            str_block<false>(y, hi, win, smem_raw,
+                             reinterpret_cast<const uint4 *>(s_ent + (size_t)s * kSEntBytes),
+                             s * kSTileBytes + (t << 4),
+                             reinterpret_cast<const float4 *>(a.ops[me.x].diag) + ((uint64_t)me.z << 11),
+                             t, me.z << 12 | t << 1, 0u);
+            __syncwarp();
+            if (lane == 0) arrive_local(&empty[s]);
+            if (++s == kSMaxStages) {
+                s = 0;
+                par ^= 1u;
+            }
+            if (!(me.w & 2u)) continue;
+            const StrOp op = a.ops[me.x];
+            const uint64_t at = (uint64_t)me.y * op.N;
+            float2 *yo = a.y[me.x] + at + ((uint64_t)me.z << 12);
+            uint32_t redo = 0;  // register indices of rows to form anew
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                y[m] = two_sum_carry2(hi[m], y[m]);
+                const float2 o = make_float2(__fadd_rn(hi[m].x, y[m].x), __fadd_rn(hi[m].y, y[m].y));
+                if (fabsf(o.x) <= kFltMax && fabsf(o.y) <= kFltMax)
+                    yo[2u * t + (m & 1u) + 1024u * (m >> 1)] = o;
+                else
+                    redo |= 1u << m;
+            }
+            while (redo != 0) {
+                const uint32_t m = (uint32_t)(__ffs((int)redo) - 1);
+                redo &= redo - 1u;
+                const uint32_t rl = 2u * t + (m & 1u) + 1024u * (m >> 1);
+                // the compensated sum of an infinite part is NaN
+                float2 o = str_row(op.sblk, op.nblk, op.ent, op.diag, a.psi[me.x] + at,
+                                   ((uint64_t)me.z << 12) | rl);
+                if (!(fabsf(o.x) <= kFltMax)) o.x = __uint_as_float(0x7fc00000u);
+                if (!(fabsf(o.y) <= kFltMax)) o.y = __uint_as_float(0x7fc00000u);
+                yo[rl] = o;
+            }
+        }
+    }
+    __syncthreads();
+}
+
+cudaError_t launch_strings_batch(const StrBatchArgs &a, uint32_t ctas, cudaStream_t st) {
+    const size_t sm = (size_t)kSMaxStages * (kSTileBytes + kSEntBytes);
+    cudaError_t e = ensure_dyn_smem(reinterpret_cast<const void *>(apply_c64c_strings_batch), sm);
+    if (e != cudaSuccess) return e;
+    const uint32_t grid = a.nitems < ctas ? a.nitems : ctas;
+    if (grid == 0) return cudaSuccess;
+    apply_c64c_strings_batch<<<grid, kSBlockThreads, sm, st>>>(a);
+    count_launch();
+    return cudaGetLastError();
 }
 
 // Clusters of ks CTAs that run at once (a GPC's SMs need not be a multiple of

@@ -222,6 +222,27 @@ cudaError_t ensure_dyn_smem(const void *fn, size_t bytes);
 // Kernel launchers (qr_apply.cu / qr_csr.cu).
 cudaError_t launch_apply(const ApplyArgs &a, int amps, int threads, int nsm,
                          cudaStream_t st);
+// Batched string operators (apply_c64c_strings_batch): n >= 12, one partner
+// tile per block.
+struct StrOp {
+    const uint4 *sblk, *ent;
+    const float2 *diag;  // or null
+    uint64_t N;
+    uint32_t nblk;
+};
+struct StrBatchArgs {
+    const StrOp *ops;         // by operator of the batch
+    const BatchItem *items;   // largest first
+    uint32_t nitems;
+    const float2 *const *psi;
+    float2 *const *y;
+    uint32_t *counter;
+    int *err;
+    uint64_t wait_ns;
+};
+// The counter is zeroed before; launches that share it share the items.
+cudaError_t launch_strings_batch(const StrBatchArgs &a, uint32_t ctas, cudaStream_t st);
+
 // qr_apply_strings.cu
 // call_items: output tiles of the caller's whole call
 cudaError_t launch_c64c_strings(const ApplyArgs &a, const StrSplit &sp, uint64_t call_items,

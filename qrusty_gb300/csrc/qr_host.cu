@@ -1986,14 +1986,17 @@ struct qr_batch {
     std::vector<int32_t> nstates;
     int tile_bits = 0;
     // 0: one persistent work-list kernel, 1: graph of per-operator kernels,
-    // 2: both in one graph -- the persistent kernel for the small operators
-    // (fewer work items than half the SMs), one kernel per large operator
+    // 2: one graph of the persistent kernel for the small operators (fewer
+    // work items than half the SMs), the string kernel's batch for those that
+    // their own launch would give to it, and one kernel per other operator
     int mode = 0;
     int force_mode = -1;  // -1: the autotuner chooses
     std::vector<char> sel;    // operators in the persistent kernel's work list
     std::vector<char> small;  // operators with fewer items than half the SMs
+    std::vector<char> str;    // operators in the string batch's work list
     DevBuf d_ops, d_items, d_ptrs, d_err;
-    uint32_t nitems = 0;
+    DevBuf d_sops, d_sitems, d_sctr;  // string batch
+    uint32_t nitems = 0, nsitems = 0;
     std::vector<const void *> cur_psi;
     std::vector<void *> cur_y;
     bool ptrs_changed = false;
@@ -2062,6 +2065,56 @@ int batch_build(qr_batch *bt, int tb) {
     return QR_OK;
 }
 
+// The string batch's operator table and work list (largest items first).
+int str_batch_build(qr_batch *bt) {
+    std::vector<StrOp> so(bt->ops.size());
+    std::vector<std::pair<double, size_t>> cost;
+    for (size_t i = 0; i < bt->ops.size(); ++i) {
+        if (!bt->str[i]) continue;
+        Plan *pl = nullptr;
+        const int rc = apply_plan(bt->ops[i], QR_C64C, 0, bt->nstates[i], &pl);
+        if (rc) return rc;
+        so[i].sblk = pl->sblk.as<uint4>();
+        so[i].ent = pl->ent.as<uint4>();
+        so[i].diag = pl->has_diag ? pl->diag.as<float2>() : nullptr;
+        so[i].N = bt->ops[i]->N;
+        so[i].nblk = pl->str.nblk;
+        cost.push_back({(double)pl->str.nstr + 2.0 * pl->str.nblk, i});
+    }
+    std::stable_sort(cost.begin(), cost.end(),
+                     [](const std::pair<double, size_t> &a, const std::pair<double, size_t> &b) {
+                         return a.first > b.first;
+                     });
+    std::vector<BatchItem> items;
+    for (auto &c : cost) {
+        const size_t i = c.second;
+        for (int32_t st = 0; st < bt->nstates[i]; ++st)
+            for (uint64_t q = 0; q < bt->ops[i]->N >> 12; ++q)
+                items.push_back(BatchItem{(uint32_t)i, (uint32_t)st, (uint32_t)q, 0u});
+    }
+    // the counter runs up to two past the list per CTA
+    if (items.size() > 0xfffff000ull) return fail(QR_EINVAL, "qr_batch: work list too long");
+    bt->nsitems = (uint32_t)items.size();
+    QR_CUDA(bt->d_sops.upload(so), "upload string batch operators");
+    QR_CUDA(bt->d_sitems.upload(items), "upload string batch work list");
+    QR_CUDA(bt->d_sctr.alloc(sizeof(uint32_t)), "alloc string batch counter");
+    return QR_OK;
+}
+
+StrBatchArgs str_batch_args(qr_batch *bt) {
+    StrBatchArgs a;
+    a.ops = bt->d_sops.as<StrOp>();
+    a.items = bt->d_sitems.as<BatchItem>();
+    a.nitems = bt->nsitems;
+    float2 **pp = bt->d_ptrs.as<float2 *>();
+    a.psi = pp;
+    a.y = pp + bt->ops.size();
+    a.counter = bt->d_sctr.as<uint32_t>();
+    a.err = bt->d_err.as<int>();
+    a.wait_ns = kDefaultWaitNs;
+    return a;
+}
+
 BatchArgs batch_args(qr_batch *bt) {
     BatchArgs a;
     a.ops = bt->d_ops.as<BatchOp>();
@@ -2100,28 +2153,41 @@ int batch_upload_ptrs(qr_batch *bt, const void *const *psi, void *const *y, cuda
 }
 
 // The batch's graph on the current pointers, on kForks parallel branches:
-// the persistent work-list kernel over the selected operators (branch 0)
-// and one compensated-c64 apply per other operator (round-robin over the
-// remaining branches, or all of them when nothing is selected).  The
-// selected operators' tables and work list (batch_build) and the other
-// operators' plans must already exist.
+// the persistent work-list kernel over the selected operators (branch 0),
+// one compensated-c64 apply per other operator (round-robin over the
+// remaining branches, or all of them when nothing is selected) and, on
+// the last branch and behind the persistent kernel, the string batch, whose CTAs
+// take work until there is none.  The selected operators' tables
+// and work lists (batch_build, str_batch_build) and the other operators'
+// plans must already exist.
 int capture_graph(qr_batch *bt, cudaGraph_t *graph) {
     cudaStream_t cap = bt->cap;
     bool any_sel = false;
     for (char c : bt->sel) any_sel |= c != 0;
     QR_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeRelaxed), "begin capture");
-    cudaError_t e = cudaEventRecord(bt->fork_ev[qr_batch::kForks], cap);
+    bool any_str = false;
+    for (char c : bt->str) any_str |= c != 0;
+    cudaError_t e = cudaSuccess;
+    if (any_str) e = cudaMemsetAsync(bt->d_sctr.p, 0, sizeof(uint32_t), cap);
+    if (e == cudaSuccess) e = cudaEventRecord(bt->fork_ev[qr_batch::kForks], cap);
     for (int k = 0; k < qr_batch::kForks && e == cudaSuccess; ++k)
         e = cudaStreamWaitEvent(bt->fork[k], bt->fork_ev[qr_batch::kForks], 0);
     int rc = QR_OK;
     if (any_sel && e == cudaSuccess) e = launch_batch_c64c(batch_args(bt), bt->nsm, bt->fork[0]);
-    const int first = any_sel ? 1 : 0, nbr = qr_batch::kForks - first;
+    const int first = any_sel ? 1 : 0, nbr = qr_batch::kForks - first - (any_str ? 1 : 0);
     int k = 0;
     for (size_t i = 0; i < bt->ops.size() && e == cudaSuccess && !rc; ++i) {
-        if (bt->sel[i]) continue;
+        if (bt->sel[i] || bt->str[i]) continue;
         rc = apply_impl("qr_batch_apply", bt->ops[i], QR_C64C, bt->cur_psi[i], bt->cur_y[i],
                         bt->nstates[i], bt->nstates[i], 0, bt->fork[first + (k++ % nbr)], nullptr, nullptr,
                         nullptr);
+    }
+    if (any_str && e == cudaSuccess && !rc) {
+        // leave the persistent kernel its SMs, and take them over after it
+        const uint32_t k = any_sel ? std::min(bt->nitems, (uint32_t)bt->nsm / 2) : 0u;
+        e = launch_strings_batch(str_batch_args(bt), (uint32_t)bt->nsm - k,
+                                 bt->fork[qr_batch::kForks - 1]);
+        if (k > 0 && e == cudaSuccess) e = launch_strings_batch(str_batch_args(bt), k, bt->fork[0]);
     }
     for (int f = 0; f < qr_batch::kForks && e == cudaSuccess; ++f) {
         e = cudaEventRecord(bt->fork_ev[f], bt->fork[f]);
@@ -2146,12 +2212,16 @@ void drop_graph(qr_batch *bt) {
 // capture and instantiate it.
 int instantiate_mode(qr_batch *bt, int mode) {
     drop_graph(bt);
-    for (size_t i = 0; i < bt->ops.size(); ++i)
-        bt->sel[i] = mode == 0 ? 1 : (mode == 1 ? 0 : bt->small[i]);
-    int rc = batch_build(bt, kBatchTileBits);
-    for (size_t i = 0; i < bt->ops.size() && !rc; ++i)
-        if (Plan *pl = nullptr; !bt->sel[i])
-            rc = apply_plan(bt->ops[i], QR_C64C, 0, bt->nstates[i], &pl);
+    int rc = QR_OK;
+    for (size_t i = 0; i < bt->ops.size() && !rc; ++i) {
+        Plan *pl = nullptr;
+        bt->str[i] = 0;
+        if (mode != 0) rc = apply_plan(bt->ops[i], QR_C64C, 0, bt->nstates[i], &pl);
+        if (mode == 2 && !rc) bt->str[i] = !pl->rows && pl->strings && pl->str.tpb == 1;
+        bt->sel[i] = mode == 0 ? 1 : (mode == 1 ? 0 : bt->small[i] && !bt->str[i]);
+    }
+    if (!rc) rc = batch_build(bt, kBatchTileBits);
+    if (!rc) rc = str_batch_build(bt);
     if (!rc) rc = capture_graph(bt, &bt->graph);
     if (rc) return rc;
     QR_CUDA(cudaGraphInstantiate(&bt->exec, bt->graph, 0), "graph instantiate");
@@ -2161,12 +2231,13 @@ int instantiate_mode(qr_batch *bt, int mode) {
 
 uint64_t graph_kernels(const qr_batch *bt) {
     uint64_t k = 0;
-    bool any_sel = false;
+    bool any_sel = false, any_str = false;
     for (size_t i = 0; i < bt->ops.size(); ++i) {
         if (bt->sel[i]) any_sel = true;
+        else if (bt->str[i]) any_str = true;
         else ++k;
     }
-    return k + (any_sel ? 1 : 0);
+    return k + (any_sel ? 1 : 0) + (any_str ? (any_sel ? 2 : 1) : 0);
 }
 
 void record_gens(qr_batch *bt) {
@@ -2211,6 +2282,7 @@ int qr_batch_create(int32_t nops, qr_op *const *ops, const int32_t *nstates, qr_
     cudaError_t e = cudaDeviceGetAttribute(&bt->nsm, cudaDevAttrMultiProcessorCount, dev);
     bt->sel.assign(nops, 1);
     bt->small.assign(nops, 0);
+    bt->str.assign(nops, 0);
     for (int32_t i = 0; i < nops; ++i) {
         const int b = std::min(ops[i]->n, kBatchTileBits);
         const uint64_t items = (ops[i]->N >> b) * (uint64_t)nstates[i];
