@@ -884,8 +884,9 @@ cudaError_t launch_csr_fill(const CsrArgs &a, int nsm, cudaStream_t st) {
 // predicated; the lanes' sums meet in a butterfly.  What bounds it: the
 // matrix, read once (24 bytes per entry: 78 % of the measured HBM copy rate
 // on the chains n = 20 and 22), with the FP64 pipe next (two multiply-adds
-// per real entry, four lanes' butterfly: 0.7 of the time).  Hence one
-// accumulator per part and few lanes per row, and 4 CTAs of 256 threads per
+// per real entry, the lanes' sum: 0.7 of the time).  Hence one accumulator per
+// part, a sum in which half of the lanes take each part (n = 20: 180 us, 191
+// with both parts in every lane) and few lanes per row, and 4 CTAs of 256 threads per
 // SM (64 registers) rather than deeper steps: chain n = 22, 44 entries a row,
 // steps of 2 / 3 / 4 / 5 / 6 entries 1,090 / 1,030 / 979 / 890 / 839 us (all
 // four multiply-adds, 11 entries in flight: 1,436).
@@ -939,14 +940,14 @@ __device__ __forceinline__ void spmv_rows(uint64_t nrows, uint64_t ncols,
     const uint64_t groups = (uint64_t)gridDim.x * (blockDim.x / S);
     for (uint64_t r = blockIdx.x * (uint64_t)(blockDim.x / S) + (threadIdx.x / S); r < nrows;
          r += groups) {
-        double2 q = spmv_lane<S, U>(indptr[r], indptr[r + 1], ncols, indices, data, v);
+        const double2 q = spmv_lane<S, U>(indptr[r], indptr[r + 1], ncols, indices, data, v);
         const uint32_t mask = ((1u << S) - 1u) << (threadIdx.x & 31u & ~(S - 1u));
+        // halves of the row's lanes take a part each (one addition a step, not two)
+        const bool im = (sl & (S / 2)) != 0;
+        double p = (im ? q.y : q.x) + __shfl_xor_sync(mask, im ? q.x : q.y, S / 2, S);
 #pragma unroll
-        for (int o = S / 2; o > 0; o >>= 1) {
-            q.x += __shfl_xor_sync(mask, q.x, o, S);
-            q.y += __shfl_xor_sync(mask, q.y, o, S);
-        }
-        if (sl == 0) y[r] = q;
+        for (int o = S / 4; o > 0; o >>= 1) p += __shfl_xor_sync(mask, p, o, S);
+        if ((sl & (S / 2 - 1)) == 0) reinterpret_cast<double *>(y + r)[im ? 1 : 0] = p;
     }
 }
 
