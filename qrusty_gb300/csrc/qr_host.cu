@@ -113,10 +113,17 @@ struct Plan {
     bool built = false;
     int b = 0, tb = 0, threads = 0, amps = 0;
     uint32_t nblocks = 0;
-    uint64_t ngroups = 0, nfat = 0;
+    uint64_t nfat = 0;
     int diag_block = -1;
     bool has_diag = false;
-    DevBuf groups, tables, fat_z, fat_c, blk_hi, diag;
+    DevBuf blk_hi, diag;
+    // qr_apply_rows.cu: complex128, and complex64 calls of few rows.  A
+    // complex64 plan holds this form beside its tile form (strings, cosets or
+    // per-tile tables) where both can be reached: a call of any number of
+    // states finds its tables built and every coefficient update reaches them
+    bool rows = false;
+    uint32_t nrgroups = 0;
+    DevBuf groups, tables, fat_z, fat_c;
     // compensated-c64 kernel tables
     uint32_t nsub = 0, nruns = 0, nchunks = 0;
     DevBuf tdesc, tdata, blk_r0, run_g0, run_key, chunks;
@@ -126,7 +133,6 @@ struct Plan {
     bool cosets = false;  // qr_apply_cosets.cu
     uint32_t ncblk = 0, ncsub = 0;
     DevBuf cblk, ctdesc, ctdata;
-    bool rows = false;  // qr_apply_rows.cu: complex128, and complex64 of few rows
     DevBuf ent, sblk;
     // what the plan was built for, and its coefficient program: the slots
     // that qr_op_set_coeffs_device recomputes on the device, with the
@@ -177,7 +183,6 @@ struct qr_op {
     } tg[2];
     DevBuf expect_y;                    // H psi buffer of qr_expect
     Plan plans[2][2];  // [dtype][adjoint]
-    Plan rplans[2];    // complex64 over rows, for calls of few rows [adjoint]
     Plan bplans[13];   // compensated-c64 plans with an explicit tile width (batched launches)
     DevBuf d_err;
     // host-call staging
@@ -443,12 +448,14 @@ int build_rows(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vector<
             parts[full.coord[kk] >> kDMax].push_back(members[g][kk]);
         for (const auto &pt : parts) push(gxs[g], pt.second, gf2_span(masks(pt.second), kDMax), false);
     }
-    pl.ngroups = descs.size();
+    pl.nrgroups = (uint32_t)descs.size();
     if (descs.empty()) descs.push_back(GroupDesc{});  // keep a valid pointer
     QR_CUDA(pl.groups.upload(descs), "upload groups");
     QR_CUDA(pl.tables.upload(tab), "upload tables");
-    QR_CUDA(pl.fat_z.upload(fz), "upload fat z");
-    QR_CUDA(pl.fat_c.upload(fc), "upload fat c");
+    if constexpr (!f32) {
+        QR_CUDA(pl.fat_z.upload(fz), "upload fat z");
+        QR_CUDA(pl.fat_c.upload(fc), "upload fat c");
+    }
     for (size_t i = 0; i < pieces.size(); ++i) {
         const Piece &pc = pieces[i];
         const GroupDesc &d = descs[i];
@@ -839,10 +846,27 @@ int build_cosets(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vecto
     return QR_OK;
 }
 
-int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows = false) {
-    Plan &pl = tile_bits >= 0 ? op->bplans[tile_bits]
-               : rows && dtype == QR_C64C ? op->rplans[adjoint]
-                                          : op->plans[dtype][adjoint];
+// Rows up to which a complex64 call runs over rows: a tile kernel takes one SM
+// per 4,096 rows.  Measured (us, tiles against rows), 1,000 random strings,
+// where a tile's strings are split over a cluster: 2^12 rows 21 / 15 (600
+// strings), 2^13 23 / 18 (700), 2^14 27 / 24 and, from four states, 21 / 18,
+// 2^15 23 / 33; Jordan-Wigner 2^14 25 / 8, 2^16 33 / 18, 2^17 36 / 33, 2^18
+// 40 / 66; chain 2^17 13.4 / 8.8, 2^18 14.4 / 15.2.  Below 12 qubits a tile is
+// smaller and costs 0.05-0.1 us per x group: n = 11, 500 groups, 52 against 12
+// (one state), even at 2^15-2^16 rows.
+uint64_t c64_rows_limit(const qr_op *op) {
+    const bool strings = op->n >= 12 && (double)op->M <= 1.3 * (double)op->Ga;
+    return strings ? 1ull << 13 : op->n >= 12 ? 1ull << 17 : 1ull << 15;
+}
+
+// Whether a call of this many states runs over rows.
+bool over_rows(const qr_op *op, const Plan &pl, int32_t call_states) {
+    return pl.dtype == QR_C128 ||
+           (pl.rows && op->N * (uint64_t)call_states <= c64_rows_limit(op));
+}
+
+int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
+    Plan &pl = tile_bits >= 0 ? op->bplans[tile_bits] : op->plans[dtype][adjoint];
     if (pl.built) return QR_OK;
     {
         const int rc = sync_host_coeffs(op);
@@ -904,7 +928,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
     // each x-group by its terms' z bits there.  The c128 kernel does not split.
     int abits = 0;
     while ((1 << abits) < pl.amps) ++abits;
-    pl.rows = !f32 || rows;
+    pl.rows = !f32 || (tile_bits < 0 && op->N <= c64_rows_limit(op));
     const uint64_t mmask = f32 ? (((1ull << abits) - 1) << pl.tb) : 0;
     std::vector<size_t> diag_terms;
     std::vector<SubGroup> subs;
@@ -917,7 +941,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
                 continue;
             }
         }
-        if (pl.rows) continue;  // whole groups (build_rows)
+        if (!f32) continue;  // whole groups (build_rows)
         std::vector<uint64_t> pkeys;
         std::vector<std::vector<size_t>> parts;
         for (size_t k : members[g]) {
@@ -1007,7 +1031,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
     // (chain n = 22, 64 strings in 47: 111 against 93).
     const size_t nstr = M - diag_terms.size();
     const double most = (subs.size() <= (size_t)kTabCap ? 1.3 : 1.6) * (double)subs.size();
-    pl.strings = !pl.rows && tile_bits < 0 && n >= 12 && nstr > 0 && (double)nstr <= most;
+    pl.strings = f32 && tile_bits < 0 && n >= 12 && nstr > 0 && (double)nstr <= most;
     // order: partner tile ascending, then (c64c) run key zm with fat last
     std::vector<size_t> ord(subs.size());
     for (size_t i = 0; i < ord.size(); ++i) ord[i] = i;
@@ -1056,7 +1080,6 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
         bg0.swap(vg);
     }
     pl.nblocks = (uint32_t)bhi.size();
-    pl.ngroups = ord.size();
     pl.diag_block = -1;
     for (size_t j = 0; j < bhi.size(); ++j)
         if (bhi[j] == 0 && pl.diag_block < 0) pl.diag_block = (int)j;
@@ -1072,12 +1095,12 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
         if (rc) return rc;
     }
     pl.cosets = false;
-    if (f32 && !pl.rows && !pl.strings && tile_bits < 0 && n >= 12) {
+    if (f32 && !pl.strings && tile_bits < 0 && n >= 12) {
         const int rc = build_cosets(op, pl, c, gxs, members, pl.has_diag, &pl.cosets, add_slot);
         if (rc) return rc;
     }
     pl.nsub = (uint32_t)ord.size();
-    if (!pl.rows && !pl.strings && !pl.cosets) {
+    if (f32 && !pl.strings && !pl.cosets) {
         // per-tile-table kernel arrays
         std::vector<uint4> td;
         std::vector<TileDataC64> tdd;
@@ -1199,27 +1222,6 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1, bool rows 
     pl.nslots = cmem.empty() ? 0u : (uint32_t)slots.size();
     pl.built = true;
     return QR_OK;
-}
-
-// The plan that a call of this many states takes, built on first use.
-// complex64 runs over rows (qr_apply_rows.cu) while the call has few: a tile
-// kernel takes one SM per 4,096 rows.  Measured (us, tiles against rows),
-// 1,000 random strings, where a tile's strings are split over a cluster:
-// 2^12 rows 21 / 15 (600 strings), 2^13 23 / 18 (700), 2^14 27 / 24 and, from
-// four states, 21 / 18, 2^15 23 / 33; Jordan-Wigner 2^14 25 / 8, 2^16 33 / 18,
-// 2^17 36 / 33, 2^18 40 / 66; chain 2^17 13.4 / 8.8, 2^18 14.4 / 15.2.
-// Below 12 qubits a tile is smaller and costs 0.05-0.1 us per x group:
-// n = 11, 500 groups, 52 against 12 (one state), even at 2^15-2^16 rows.
-int apply_plan(qr_op *op, int dtype, int adjoint, int32_t call_states, Plan **out) {
-    bool rows = dtype == QR_C128;
-    if (!rows) {
-        const uint64_t r = op->N * (uint64_t)call_states;
-        const bool strings = op->n >= 12 && (double)op->M <= 1.3 * (double)op->Ga;
-        rows = r <= (strings ? 1ull << 13 : op->n >= 12 ? 1ull << 17 : 1ull << 15);
-    }
-    const int rc = build_plan(op, dtype, adjoint, -1, rows);
-    *out = rows && dtype == QR_C64C ? &op->rplans[adjoint] : &op->plans[dtype][adjoint];
-    return rc;
 }
 
 // bound of every mbarrier wait of the apply kernels
@@ -1518,10 +1520,9 @@ static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *ps
     }
     int rc = check_device(op);
     if (rc) return rc;
-    Plan *plan = nullptr;
-    rc = apply_plan(op, dtype, adjoint, call_states, &plan);
+    rc = build_plan(op, dtype, adjoint);
     if (rc) return rc;
-    const Plan &pl = *plan;
+    const Plan &pl = op->plans[dtype][adjoint];
     ApplyArgs a{};
     a.psi = psi;
     a.y = y;
@@ -1533,7 +1534,7 @@ static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *ps
     a.ntiles = op->N >> pl.b;
     a.nitems = (uint64_t)nstates * a.ntiles;
     a.groups = pl.groups.as<GroupDesc>();
-    a.ngroups = (uint32_t)pl.ngroups;
+    a.ngroups = pl.nrgroups;
     a.tables = pl.tables.p;
     a.fat_z = pl.fat_z.as<uint64_t>();
     a.fat_c = pl.fat_c.p;
@@ -1569,7 +1570,7 @@ static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *ps
         a.bi = beta[1];
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (pl.rows)
+    if (over_rows(op, pl, call_states))
         QR_CUDA(launch_rows(dtype, a, (uint64_t)call_states * op->N, st), "apply launch");
     else if (pl.strings)
         QR_CUDA(launch_c64c_strings(a, pl.str, (uint64_t)call_states * a.ntiles, op->nsm, st),
@@ -1770,7 +1771,6 @@ int qr_op_set_coeffs(qr_op *op, const double *coeff) {
     op->host_coef_stale = true;  // plans built below fetch the new merged sums
     for (int d = 0; d < 2; ++d)
         for (int j = 0; j < 2; ++j) op->plans[d][j].built = false;
-    for (Plan &rp : op->rplans) rp.built = false;
     // plans are rebuilt on next use into the buffers they already hold
     for (Plan &bp : op->bplans) bp.built = false;
     ++op->coef_gen;
@@ -1805,10 +1805,6 @@ int qr_op_set_coeffs_device(qr_op *op, const double *coeff, void *stream) {
             rc = refresh(op->plans[d][j]);
             if (rc) return rc;
         }
-    for (Plan &rp : op->rplans) {
-        rc = refresh(rp);
-        if (rc) return rc;
-    }
     for (Plan &bp : op->bplans) {
         rc = refresh(bp);
         if (rc) return rc;
@@ -2071,9 +2067,9 @@ int str_batch_build(qr_batch *bt) {
     std::vector<std::pair<double, size_t>> cost;
     for (size_t i = 0; i < bt->ops.size(); ++i) {
         if (!bt->str[i]) continue;
-        Plan *pl = nullptr;
-        const int rc = apply_plan(bt->ops[i], QR_C64C, 0, bt->nstates[i], &pl);
+        const int rc = build_plan(bt->ops[i], QR_C64C, 0);
         if (rc) return rc;
+        const Plan *pl = &bt->ops[i]->plans[QR_C64C][0];
         so[i].sblk = pl->sblk.as<uint4>();
         so[i].ent = pl->ent.as<uint4>();
         so[i].diag = pl->has_diag ? pl->diag.as<float2>() : nullptr;
@@ -2214,10 +2210,11 @@ int instantiate_mode(qr_batch *bt, int mode) {
     drop_graph(bt);
     int rc = QR_OK;
     for (size_t i = 0; i < bt->ops.size() && !rc; ++i) {
-        Plan *pl = nullptr;
         bt->str[i] = 0;
-        if (mode != 0) rc = apply_plan(bt->ops[i], QR_C64C, 0, bt->nstates[i], &pl);
-        if (mode == 2 && !rc) bt->str[i] = !pl->rows && pl->strings && pl->str.tpb == 1;
+        if (mode != 0) rc = build_plan(bt->ops[i], QR_C64C, 0);
+        const Plan &pl = bt->ops[i]->plans[QR_C64C][0];
+        if (mode == 2 && !rc)
+            bt->str[i] = pl.strings && pl.str.tpb == 1 && !over_rows(bt->ops[i], pl, bt->nstates[i]);
         bt->sel[i] = mode == 0 ? 1 : (mode == 1 ? 0 : bt->small[i] && !bt->str[i]);
     }
     if (!rc) rc = batch_build(bt, kBatchTileBits);
