@@ -1492,6 +1492,12 @@ int qr_csr_build(qr_op *op, uint64_t *indptr, uint64_t *indices, double *data, i
     return check_kernel_error(op);
 }
 
+// psi and y (bytes each) share memory
+static bool states_overlap(const void *psi, const void *y, uint64_t bytes) {
+    const char *p = static_cast<const char *>(psi), *q = static_cast<const char *>(y);
+    return p < q + bytes && q < p + bytes;
+}
+
 // call_states: states of the caller's whole call, of which these nstates are
 // a part (the same work split, and so the same bits, for each of them)
 static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *psi, void *y,
@@ -1505,8 +1511,8 @@ static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *ps
     if (op->n > 40) return fail(QR_EINVAL, "%s: n=%d too large for a state vector", name, op->n);
     const size_t esz = dtype == QR_C128 ? 16 : 8;
     const uint64_t bytes = (uint64_t)nstates * op->N * esz;
-    const char *pb = static_cast<const char *>(psi), *yb = static_cast<const char *>(y);
-    if (pb < yb + bytes && yb < pb + bytes) return fail(QR_EINVAL, "%s: psi and y overlap", name);
+    const char *yb = static_cast<const char *>(y);
+    if (states_overlap(psi, y, bytes)) return fail(QR_EINVAL, "%s: psi and y overlap", name);
     if ((reinterpret_cast<uintptr_t>(psi) | reinterpret_cast<uintptr_t>(y)) & 15)
         return fail(QR_EINVAL, "%s: psi and y must be 16-byte aligned", name);
     if (v) {
@@ -2067,6 +2073,10 @@ int str_batch_build(qr_batch *bt) {
     std::vector<std::pair<double, size_t>> cost;
     for (size_t i = 0; i < bt->ops.size(); ++i) {
         if (!bt->str[i]) continue;
+        // as a launch of its own would
+        if (states_overlap(bt->cur_psi[i], bt->cur_y[i],
+                           (uint64_t)bt->nstates[i] * bt->ops[i]->N * sizeof(float2)))
+            return fail(QR_EINVAL, "qr_batch_apply: psi and y overlap");
         const int rc = build_plan(bt->ops[i], QR_C64C, 0);
         if (rc) return rc;
         const Plan *pl = &bt->ops[i]->plans[QR_C64C][0];
