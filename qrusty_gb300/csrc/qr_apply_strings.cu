@@ -433,6 +433,14 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
     }
 }
 
+// An expired wait of the batch: its own error word and, as which items are lost
+// is not known, that of every operator in the work list
+__device__ __forceinline__ void str_batch_late(const StrBatchArgs &a) {
+    atomicExch(a.err, kErrMbarTimeout);
+    for (uint32_t i = 0; i < a.nops; ++i)
+        if (a.ops[i].err != nullptr) atomicExch(a.ops[i].err, kErrMbarTimeout);
+}
+
 // Many operators, states and tiles in one launch: the same ring and inner loop,
 // a CTA per SM taking the next (operator, state, tile) item, largest first,
 // from a counter as it gets free.  What an operator's own launch leaves idle
@@ -471,7 +479,7 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings_batch(co
             // the stage is free, or the kernel gives up
             auto take = [&]() {
                 if (round > 0 && !mbar_wait_bounded(&empty[s], (round - 1) & 1u, a.wait_ns)) {
-                    atomicExch(a.err, kErrMbarTimeout);
+                    str_batch_late(a);
                     *s_abort = 1;
                 }
                 ok = *s_abort == 0;
@@ -484,12 +492,14 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings_batch(co
                 }
             };
             uint32_t i = atomicAdd(a.counter, 1u);
+            int64_t step = blockIdx.x == 0 ? 0 : -1;  // test hook: ring step of CTA 0
             while (ok && i < a.nitems) {
                 const uint32_t ahead = atomicAdd(a.counter, 1u);
                 const BatchItem it = a.items[i];
                 const StrOp op = a.ops[it.op];
                 const float2 *src = a.psi[it.op] + (uint64_t)it.state * op.N;
                 for (uint32_t b = 0; b < op.nblk && take(); ++b, next()) {
+                    if (step >= 0 && step++ == a.withhold) continue;
                     const uint4 bl = op.sblk[b];
                     const uint32_t eb = (bl.w + 1u) * 16u;
                     s_meta[s] = make_uint4(it.op, it.state, it.tile,
@@ -524,7 +534,7 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings_batch(co
                 skip = *s_abort != 0;
                 if (!skip && !mbar_wait_bounded(&full[s], par, a.wait_ns)) {
                     if (lane == 0) {
-                        atomicExch(a.err, kErrMbarTimeout);
+                        str_batch_late(a);
                         *s_abort = 1;
                     }
                     skip = true;

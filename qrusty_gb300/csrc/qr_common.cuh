@@ -228,10 +228,12 @@ struct StrOp {
     const uint4 *sblk, *ent;
     const float2 *diag;  // or null
     uint64_t N;
+    int *err;            // the operator's error word (null: not in the work list)
     uint32_t nblk;
 };
 struct StrBatchArgs {
     const StrOp *ops;         // by operator of the batch
+    uint32_t nops;
     const BatchItem *items;   // largest first
     uint32_t nitems;
     const float2 *const *psi;
@@ -239,6 +241,7 @@ struct StrBatchArgs {
     uint32_t *counter;
     int *err;
     uint64_t wait_ns;
+    int64_t withhold;         // test hook: ring step of CTA 0 never issued, -1 = off
 };
 // The counter is zeroed before; launches that share it share the items.
 cudaError_t launch_strings_batch(const StrBatchArgs &a, uint32_t ctas, cudaStream_t st);

@@ -2069,7 +2069,7 @@ int batch_build(qr_batch *bt, int tb) {
 
 // The string batch's operator table and work list (largest items first).
 int str_batch_build(qr_batch *bt) {
-    std::vector<StrOp> so(bt->ops.size());
+    std::vector<StrOp> so(bt->ops.size(), StrOp{});
     std::vector<std::pair<double, size_t>> cost;
     for (size_t i = 0; i < bt->ops.size(); ++i) {
         if (!bt->str[i]) continue;
@@ -2084,6 +2084,7 @@ int str_batch_build(qr_batch *bt) {
         so[i].ent = pl->ent.as<uint4>();
         so[i].diag = pl->has_diag ? pl->diag.as<float2>() : nullptr;
         so[i].N = bt->ops[i]->N;
+        so[i].err = bt->ops[i]->d_err.as<int>();
         so[i].nblk = pl->str.nblk;
         cost.push_back({(double)pl->str.nstr + 2.0 * pl->str.nblk, i});
     }
@@ -2110,6 +2111,7 @@ int str_batch_build(qr_batch *bt) {
 StrBatchArgs str_batch_args(qr_batch *bt) {
     StrBatchArgs a;
     a.ops = bt->d_sops.as<StrOp>();
+    a.nops = (uint32_t)bt->ops.size();
     a.items = bt->d_sitems.as<BatchItem>();
     a.nitems = bt->nsitems;
     float2 **pp = bt->d_ptrs.as<float2 *>();
@@ -2118,6 +2120,14 @@ StrBatchArgs str_batch_args(qr_batch *bt) {
     a.counter = bt->d_sctr.as<uint32_t>();
     a.err = bt->d_err.as<int>();
     a.wait_ns = kDefaultWaitNs;
+    a.withhold = -1;
+    // test hooks of the operators, read when the graph is made (as a launch of
+    // an operator's own reads them)
+    for (size_t i = 0; i < bt->ops.size(); ++i) {
+        if (!bt->str[i]) continue;
+        if (bt->ops[i]->test_wait_ns != 0) a.wait_ns = std::min(a.wait_ns, bt->ops[i]->test_wait_ns);
+        a.withhold = std::max(a.withhold, bt->ops[i]->test_withhold);
+    }
     return a;
 }
 
