@@ -279,11 +279,10 @@ __global__ void __launch_bounds__(kCBlockThreads, 1) apply_c64c_cosets(const App
                     }
                 }
             }
-            // after an expired wait no copy is in flight when the CTA exits
-            if (*s_abort != 0) {
-                for (uint32_t k = 0; k < slots; ++k)
-                    if (issued >> k & 1u) mbar_wait_bounded(&full[k], last_round[k] & 1u, kWaitLimitNs);
-            }
+            // no copy is in flight when the CTA exits, also when the consumers'
+            // wait expires after the last one was issued
+            for (uint32_t k = 0; k < slots; ++k)
+                if (issued >> k & 1u) mbar_wait_bounded(&full[k], last_round[k] & 1u, kWaitLimitNs);
         } else if (warp > kCWarps) {
             // the other three warps: factor tables of the next tile, in turn
             // into two buffers

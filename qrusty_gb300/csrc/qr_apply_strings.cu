@@ -305,11 +305,10 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
                     }
                 }
             }
-            // after an expired wait no copy is in flight when the CTA exits
-            if (*s_abort != 0 || !ok) {
-                for (uint32_t k = 0; k < stages; ++k)
-                    if (issued >> k & 1u) mbar_wait_bounded(&full[k], last_round[k] & 1u, kWaitLimitNs);
-            }
+            // no copy is in flight when the CTA exits, also when the consumers'
+            // wait expires after the last one was issued
+            for (uint32_t k = 0; k < stages; ++k)
+                if (issued >> k & 1u) mbar_wait_bounded(&full[k], last_round[k] & 1u, kWaitLimitNs);
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
@@ -516,12 +515,13 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings_batch(co
             if (ok && take()) {
                 s_meta[s] = make_uint4(0u, 0u, 0u, kEnd);
                 arrive_local(&full[s]);
+                issued |= 1u << s;  // the stage's last phase is this one
+                last_round[s] = round;
             }
-            // after an expired wait no copy is in flight when the CTA exits
-            if (!ok) {
-                for (uint32_t k = 0; k < kSMaxStages; ++k)
-                    if (issued >> k & 1u) mbar_wait_bounded(&full[k], last_round[k] & 1u, kWaitLimitNs);
-            }
+            // no copy is in flight when the CTA exits, also when the consumers'
+            // wait expires after the last one was issued
+            for (uint32_t k = 0; k < kSMaxStages; ++k)
+                if (issued >> k & 1u) mbar_wait_bounded(&full[k], last_round[k] & 1u, kWaitLimitNs);
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
