@@ -52,8 +52,6 @@ constexpr uint32_t kSMaxStages = 4;
 constexpr float kFltMax = 3.402823466e38f;
 constexpr uint32_t kSFold = 24;  // strings per compensated fold, at least
 
-__device__ __forceinline__ float signed_f(uint32_t f, uint32_t s) { return __uint_as_float(f ^ s); }
-
 // partner amplitudes of one string: p[j] holds register indices 2 j, 2 j + 1
 __device__ __forceinline__ void str_load(float4 (&p)[4], const unsigned char *sm, uint32_t base,
                                          uint32_t w) {
@@ -115,6 +113,36 @@ __device__ __forceinline__ void str_mac(float2 (&y)[8], const float4 (&p)[4], ui
     }
 }
 
+__device__ __forceinline__ bool finite_f(float v) { return fabsf(v) <= kFltMax; }
+
+// Of the rows `left` (a mask of register indices), those with an infinite or NaN
+// partner in this block.  A string's zero part forms no product, so such a row
+// may have one finite part where 0 * inf, with every product formed, makes both
+// NaN.  Asked while the block's tiles are at hand: a state full of them costs no
+// more than a second pass over the block.
+__device__ __noinline__ uint32_t str_nonfinite(uint32_t left, const unsigned char *sm,
+                                              const uint4 *E, uint32_t ne, uint32_t base) {
+    uint32_t bad = 0;
+    for (uint32_t i = 1; i <= ne && left != 0; ++i) {
+        const uint32_t w = E[i].x, off = base ^ (w & 0xfff0u);
+        for (uint32_t r = left; r != 0; r &= r - 1u) {
+            const uint32_t m = (uint32_t)__ffs((int)r) - 1u;
+            const float2 p = *reinterpret_cast<const float2 *>(
+                sm + (off ^ ((m >> 1) << 13)) + (((m ^ w) & 1u) << 3));
+            if (!(finite_f(p.x) && finite_f(p.y))) bad |= 1u << m;
+        }
+        left &= ~bad;
+    }
+    return bad;
+}
+
+// A row's value: an infinite sum is NaN (its compensation is)
+__device__ __forceinline__ float2 str_value(float2 h, float2 l) {
+    const float nan = __uint_as_float(0x7fc00000u);
+    const float2 o = make_float2(__fadd_rn(h.x, l.x), __fadd_rn(h.y, l.y));
+    return make_float2(finite_f(o.x) ? o.x : nan, finite_f(o.y) ? o.y : nan);
+}
+
 // One block of the ring: the diagonal where it is flagged, then the strings in
 // turn, one's partner loads in flight while the other's products are formed.
 template <bool WIDE>
@@ -155,41 +183,30 @@ __device__ __forceinline__ void str_block(float2 (&y)[8], float2 (&hi)[8], uint3
     } else if (i == ne) {
         str_mac<WIDE>(y, pa, ea, r0, rhi);
     }
+    // 0 * y: NaN once a part is infinite or NaN.  Once per block, 1 % of the
+    // time (n = 20, 16 strings a block); the warp's vote and the call keep it so
+    const float2 z2 = make_float2(0.f, 0.f);
+    float2 q[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) q[m] = __ffma2_rn(y[m], z2, __fmul2_rn(y[m + 4], z2));
+    q[0] = __fadd2_rn(__fadd2_rn(q[0], q[1]), __fadd2_rn(q[2], q[3]));
+    if (__any_sync(0xffffffffu, q[0].x + q[0].y != 0.f)) {
+        uint32_t left = 0;
+#pragma unroll
+        for (int m = 0; m < 8; ++m)
+            left |= (finite_f(y[m].x) != finite_f(y[m].y) ? 1u : 0u) << m;
+        const uint32_t bad = str_nonfinite(left, sm, E, ne, base);
+        const float nan = __uint_as_float(0x7fc00000u);
+#pragma unroll
+        for (int m = 0; m < 8; ++m)
+            if (bad >> m & 1u) y[m] = make_float2(nan, nan);
+    }
     win += ne;
     if (win >= kSFold) {
         win = 0;
 #pragma unroll
         for (int m = 0; m < 8; ++m) y[m] = two_sum_carry2(hi[m], y[m]);
     }
-}
-
-// Row r with every product formed: what a row that met an infinite or NaN
-// amplitude must return (0 * inf included).
-__device__ __noinline__ float2 str_row(const uint4 *sblk, uint32_t nblk, const uint4 *ent,
-                                       const float2 *diag, const float2 *psi, uint64_t r) {
-    float yr = 0.f, yi = 0.f;
-    for (uint32_t b = 0; b < nblk; ++b) {
-        const uint4 bl = sblk[b];
-        const uint4 *E = ent + bl.z;
-        if (E[0].y != 0) {
-            const float2 d = diag[r], p = psi[r];
-            yr += d.x * p.x - d.y * p.y;
-            yi += d.x * p.y + d.y * p.x;
-        }
-        for (uint32_t i = 1; i <= bl.w; ++i) {
-            const uint4 e = E[i];
-            const uint64_t lo = (e.x & 1u) | ((e.x >> 4) & 511u) << 1 | ((e.x >> 13) & 3u) << 10;
-            const float2 p = psi[r ^ (((uint64_t)((e.x >> 15) & 1u ? bl.y : bl.x) << 12) | lo)];
-            const uint32_t zz = e.y | ((e.x >> 16) & 1u) | ((e.x >> 17) & 3u) << 10;
-            const uint32_t s = ((uint32_t)__popc((uint32_t)r & zz) +
-                                (uint32_t)__popc((uint32_t)(r >> 32) & (e.x >> 24)))
-                               << 31;
-            const float fr = signed_f(e.z, s), fi = signed_f(e.w, s);
-            yr += fr * p.x - fi * p.y;
-            yi += fr * p.y + fi * p.x;
-        }
-    }
-    return make_float2(yr, yi);
 }
 
 __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
@@ -360,17 +377,9 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
                 yo[rl] = o;
             };
             auto row_of = [&](uint32_t m) { return 2u * t + (m & 1u) + 1024u * (m >> 1); };
-            uint32_t redo = 0;  // register indices of rows to form anew
-            auto store = [&](uint32_t m, float2 h, float2 l) {
-                const float2 o = make_float2(__fadd_rn(h.x, l.x), __fadd_rn(h.y, l.y));
-                if (fabsf(o.x) <= kFltMax && fabsf(o.y) <= kFltMax)
-                    finish(row_of(m), o);
-                else
-                    redo |= 1u << m;
-            };
             if (ks == 1) {
 #pragma unroll
-                for (int m = 0; m < 8; ++m) store((uint32_t)m, hi[m], y[m]);
+                for (int m = 0; m < 8; ++m) finish(row_of((uint32_t)m), str_value(hi[m], y[m]));
             } else {
                 // the ranks' sums meet in shared memory: rank r adds rows
                 // of register index m = r, r + ks, ... of every rank, in rank order
@@ -405,7 +414,7 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
                             const float2 e = two_sum_carry2(h, make_float2(v.x, v.y));
                             l = __fadd2_rn(l, __fadd2_rn(e, make_float2(v.z, v.w)));
                         }
-                        store(m, h, l);
+                        finish(row_of(m), str_value(h, l));
                     }
                 }
                 __syncwarp();
@@ -413,16 +422,6 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
                     asm volatile("fence.acq_rel.cluster;" ::: "memory");
                     arrive_cluster(mapa(saddr(&xfree), lane));
                 }
-            }
-            while (redo != 0) {
-                const uint32_t rl = row_of((uint32_t)(__ffs((int)redo) - 1));
-                redo &= redo - 1u;
-                // the compensated sum of an infinite part is NaN
-                float2 o = str_row(a.sblk, a.nsblk, a.ent, static_cast<const float2 *>(a.diag),
-                                   static_cast<const float2 *>(a.psi) + st * a.N, (q << 12) | rl);
-                if (!(fabsf(o.x) <= kFltMax)) o.x = __uint_as_float(0x7fc00000u);
-                if (!(fabsf(o.y) <= kFltMax)) o.y = __uint_as_float(0x7fc00000u);
-                finish(rl, o);
             }
         }
     }
@@ -561,29 +560,11 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings_batch(co
                 par ^= 1u;
             }
             if (!(me.w & 2u)) continue;
-            const StrOp op = a.ops[me.x];
-            const uint64_t at = (uint64_t)me.y * op.N;
-            float2 *yo = a.y[me.x] + at + ((uint64_t)me.z << 12);
-            uint32_t redo = 0;  // register indices of rows to form anew
+            float2 *yo = a.y[me.x] + (uint64_t)me.y * a.ops[me.x].N + ((uint64_t)me.z << 12);
 #pragma unroll
             for (int m = 0; m < 8; ++m) {
                 y[m] = two_sum_carry2(hi[m], y[m]);
-                const float2 o = make_float2(__fadd_rn(hi[m].x, y[m].x), __fadd_rn(hi[m].y, y[m].y));
-                if (fabsf(o.x) <= kFltMax && fabsf(o.y) <= kFltMax)
-                    yo[2u * t + (m & 1u) + 1024u * (m >> 1)] = o;
-                else
-                    redo |= 1u << m;
-            }
-            while (redo != 0) {
-                const uint32_t m = (uint32_t)(__ffs((int)redo) - 1);
-                redo &= redo - 1u;
-                const uint32_t rl = 2u * t + (m & 1u) + 1024u * (m >> 1);
-                // the compensated sum of an infinite part is NaN
-                float2 o = str_row(op.sblk, op.nblk, op.ent, op.diag, a.psi[me.x] + at,
-                                   ((uint64_t)me.z << 12) | rl);
-                if (!(fabsf(o.x) <= kFltMax)) o.x = __uint_as_float(0x7fc00000u);
-                if (!(fabsf(o.y) <= kFltMax)) o.y = __uint_as_float(0x7fc00000u);
-                yo[rl] = o;
+                yo[2u * t + (m & 1u) + 1024u * (m >> 1)] = str_value(hi[m], y[m]);
             }
         }
     }
