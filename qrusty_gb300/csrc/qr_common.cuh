@@ -381,7 +381,8 @@ cudaError_t launch_vdot(int dtype, uint64_t N, const void *a, const void *b, int
 // Term gradients.  complex128 strings of x groups of kGradWhtMin or more go through a
 // Walsh-Hadamard transform per 256 rows (wht: batches of up to kGradWhtBatch
 // strings of one x), the others one by one (direct: by partner tile x >> 12 for
-// the tiled complex64 kernel, n >= 12).  perm: merged index of each; partial
+// the tiled complex64 kernel, n >= 12).  perm: merged index of each (null: in
+// merged order); partial
 // sums: direct.count x direct.nchunk, then wht.count x wht.nchunk.
 constexpr uint32_t kGradWhtMin = 8, kGradWhtBatch = 256;
 struct GradBatch {

@@ -1882,7 +1882,17 @@ int qr_term_grad(qr_op *op, int32_t dtype, const void *psi, const void *g, int32
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     qr_op::GradPlan &tg = op->tg[dtype];
-    if (!tg.ready) {
+    const bool tiles = dtype == QR_C64C && op->n >= 12;
+    // The first call inside a stream capture, where no plan can be uploaded:
+    // string by string from the merged masks on the device (the tiled kernel
+    // needs its batches)
+    bool unplanned = false;
+    if (!tg.ready && !tiles) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        QR_CUDA(cudaStreamIsCapturing(st, &cap), "term-grad capture status");
+        unplanned = cap == cudaStreamCaptureStatusActive;
+    }
+    if (!tg.ready && !unplanned) {
         // complex128: x groups of many strings to the transform; the others in order of
         // partner tile, input order kept within one; batches of <= 8 never
         // span two partner tiles, largest first
@@ -1934,19 +1944,19 @@ int qr_term_grad(qr_op *op, int32_t dtype, const void *psi, const void *g, int32
         tg.ready = true;
     }
     GradPlanArgs p{};
-    p.sx = tg.x.as<uint64_t>();
-    p.sz = tg.z.as<uint64_t>();
+    p.sx = unplanned ? op->d_mx.as<uint64_t>() : tg.x.as<uint64_t>();
+    p.sz = unplanned ? op->d_mz.as<uint64_t>() : tg.z.as<uint64_t>();
     p.batches = tg.bat.as<uint2>();
     p.nbatch = tg.nbatch;
     p.wz = tg.wz.as<uint64_t>();
     p.wbatches = tg.wbat.as<GradBatch>();
     p.nwbatch = tg.nwbatch;
-    const bool tiles = dtype == QR_C64C && op->n >= 12;
+    const uint32_t nd = unplanned ? (uint32_t)op->M : tg.ndirect;
     uint64_t nchunk = 1, nwchunk = 1;
-    if (tg.ndirect > 0) {
+    if (nd > 0) {
         // about 8 work items (4 strings each, or a batch of the tiled kernel)
         // per SM, chunks of at least 16 tiles or 4,096 rows
-        const uint64_t items = tiles ? tg.nbatch : (tg.ndirect + 3) / 4;
+        const uint64_t items = tiles ? tg.nbatch : (nd + 3) / 4;
         const uint64_t most = tiles ? (op->N >> 12) * (uint64_t)nstates / 16 : op->N / 4096;
         nchunk = std::min(((uint64_t)op->nsm * 8 + items - 1) / items, most);
         if (nchunk < 1) nchunk = 1;
@@ -1957,10 +1967,10 @@ int qr_term_grad(qr_op *op, int32_t dtype, const void *psi, const void *g, int32
         nwchunk = std::min(((uint64_t)op->nsm * 4 + tg.nwbatch - 1) / tg.nwbatch,
                            (blocks + 7) / 8);
     }
-    p.direct = GradStrings{tg.perm.as<uint32_t>(), tg.ndirect, (uint32_t)nchunk};
+    p.direct = GradStrings{unplanned ? nullptr : tg.perm.as<uint32_t>(), nd, (uint32_t)nchunk};
     p.wht = GradStrings{tg.wperm.as<uint32_t>(), tg.nwht, (uint32_t)nwchunk};
     void *scratch = nullptr;
-    const size_t np = (size_t)tg.ndirect * nchunk + (size_t)tg.nwht * nwchunk;
+    const size_t np = (size_t)nd * nchunk + (size_t)tg.nwht * nwchunk;
     QR_CUDA(cudaMallocAsync(&scratch, np * sizeof(double2) + 16, st), "term-grad scratch");
     double2 *partial = static_cast<double2 *>(scratch);
     auto *counter = reinterpret_cast<unsigned long long *>(partial + np);

@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kRedThreads) term_grad_finish_kernel(
          i += gridDim.x * (kRedThreads / 32)) {
         const bool first = i < d.count;
         const uint32_t k = first ? i : i - d.count, nchunk = first ? d.nchunk : w.nchunk;
-        const uint32_t m = first ? d.perm[k] : w.perm[k];
+        const uint32_t m = !first ? w.perm[k] : d.perm != nullptr ? d.perm[k] : k;
         const double2 *p = partial + (first ? 0 : (size_t)d.count * d.nchunk) + (size_t)k * nchunk;
         double re = 0.0, im = 0.0;
         for (uint32_t c = lane; c < nchunk; c += 32) {
