@@ -205,6 +205,10 @@ int qr_op_set_coeffs_device(qr_op *op, const double *coeff, void *stream);
  * Hooks stay set until changed; (0, 0, -1) restores normal operation. */
 enum { QR_TEST_FORCE_WIDE = 1 };
 int qr_op_set_test_hooks(qr_op *op, uint32_t flags, uint64_t wait_ns, int64_t withhold_step);
+/* TEST HOOK: the kernel family that qr_apply of nstates states runs on
+ * (QR_FORM_*, or a negative error code).  Builds the plan as qr_apply would. */
+enum { QR_FORM_TABLES = 0, QR_FORM_ROWS = 1, QR_FORM_STRINGS = 2, QR_FORM_COSETS = 3 };
+int qr_op_apply_form(qr_op *op, int32_t dtype, int32_t adjoint, int32_t nstates);
 
 /* out[s] = <a_s, b_s> = sum_r conj(a_s[r]) * b_s[r] for nstates states of
  * 2^n amplitudes, accumulated in FP64 (complex128 out: 2 doubles per state,

@@ -846,23 +846,25 @@ int build_cosets(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vecto
     return QR_OK;
 }
 
-// Rows up to which a complex64 call runs over rows: a tile kernel takes one SM
-// per 4,096 rows.  Measured (us, tiles against rows), 1,000 random strings,
-// where a tile's strings are split over a cluster: 2^12 rows 21 / 15 (600
-// strings), 2^13 23 / 18 (700), 2^14 27 / 24 and, from four states, 21 / 18,
-// 2^15 23 / 33; Jordan-Wigner 2^14 25 / 8, 2^16 33 / 18, 2^17 36 / 33, 2^18
-// 40 / 66; chain 2^17 13.4 / 8.8, 2^18 14.4 / 15.2.  Below 12 qubits a tile is
-// smaller and costs 0.05-0.1 us per x group: n = 11, 500 groups, 52 against 12
-// (one state), even at 2^15-2^16 rows.
-uint64_t c64_rows_limit(const qr_op *op) {
-    const bool strings = op->n >= 12 && (double)op->M <= 1.3 * (double)op->Ga;
-    return strings ? 1ull << 13 : op->n >= 12 ? 1ull << 17 : 1ull << 15;
+// Rows up to which a complex64 call runs over rows, by what it would run on
+// otherwise: a tile kernel takes one SM per 4,096 rows.  Measured (us, tiles
+// against rows).  String kernel, which splits a tile over a cluster, 2^13 rows:
+// n = 12, 1,000 strings 33 / 25, 4,000 88 / 75, n = 13, 2,000 53 / 45; 2^14:
+// n = 12, 1,000 33 / 29, n = 14, 1,000 31 / 32, 5,000 128 / 121; 2^15: n = 12,
+// 2,000 51 / 76, n = 14, 5,000 128 / 194; 2^17: n = 12, 4,000 167 / 426.  Cosets
+// and per-tile tables, 2^17 rows: Jordan-Wigner of 92 x groups 25 / 25, 121 31 /
+// 31, molecular sums of 286 173 / 127, 981 507 / 377, 1,941 900 / 597, chain 13
+// / 9; 2^18: 121 31 / 55, 286 174 / 235, 981 507 / 707, 1,941 901 / 1,108.
+// Below 12 qubits a tile is smaller and costs 0.05-0.1 us per x group: n = 11,
+// 500 groups, 52 against 12 (one state), even at 2^15-2^16 rows.
+uint64_t c64_rows_limit(int n, bool strings) {
+    return strings ? 1ull << 13 : n >= 12 ? 1ull << 17 : 1ull << 15;
 }
 
 // Whether a call of this many states runs over rows.
 bool over_rows(const qr_op *op, const Plan &pl, int32_t call_states) {
     return pl.dtype == QR_C128 ||
-           (pl.rows && op->N * (uint64_t)call_states <= c64_rows_limit(op));
+           (pl.rows && op->N * (uint64_t)call_states <= c64_rows_limit(op->n, pl.strings));
 }
 
 int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
@@ -928,7 +930,6 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     // each x-group by its terms' z bits there.  The c128 kernel does not split.
     int abits = 0;
     while ((1 << abits) < pl.amps) ++abits;
-    pl.rows = !f32 || (tile_bits < 0 && op->N <= c64_rows_limit(op));
     const uint64_t mmask = f32 ? (((1ull << abits) - 1) << pl.tb) : 0;
     std::vector<size_t> diag_terms;
     std::vector<SubGroup> subs;
@@ -1032,6 +1033,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     const size_t nstr = M - diag_terms.size();
     const double most = (subs.size() <= (size_t)kTabCap ? 1.3 : 1.6) * (double)subs.size();
     pl.strings = f32 && tile_bits < 0 && n >= 12 && nstr > 0 && (double)nstr <= most;
+    pl.rows = !f32 || (tile_bits < 0 && op->N <= c64_rows_limit(n, pl.strings));
     // order: partner tile ascending, then (c64c) run key zm with fat last
     std::vector<size_t> ord(subs.size());
     for (size_t i = 0; i < ord.size(); ++i) ord[i] = i;
@@ -1830,6 +1832,22 @@ int qr_op_set_test_hooks(qr_op *op, uint32_t flags, uint64_t wait_ns, int64_t wi
     op->test_wait_ns = wait_ns;
     op->test_withhold = withhold_step;
     return QR_OK;
+}
+
+int qr_op_apply_form(qr_op *op, int32_t dtype, int32_t adjoint, int32_t nstates) {
+    if (!op) return fail(QR_EINVAL, "qr_op_apply_form: null operator");
+    if (dtype != QR_C128 && dtype != QR_C64C) return fail(QR_EINVAL, "qr_op_apply_form: bad dtype");
+    if (adjoint != 0 && adjoint != 1) return fail(QR_EINVAL, "qr_op_apply_form: bad adjoint");
+    if (nstates < 1) return fail(QR_EINVAL, "qr_op_apply_form: nstates=%d < 1", nstates);
+    int rc = check_device(op);
+    if (rc) return rc;
+    rc = build_plan(op, dtype, adjoint);
+    if (rc) return rc;
+    const Plan &pl = op->plans[dtype][adjoint];
+    return over_rows(op, pl, nstates) ? QR_FORM_ROWS
+           : pl.strings               ? QR_FORM_STRINGS
+           : pl.cosets                ? QR_FORM_COSETS
+                                      : QR_FORM_TABLES;
 }
 
 int qr_vdot(int32_t n, int32_t dtype, const void *a, const void *b, int32_t nstates, double *out,

@@ -368,6 +368,16 @@ class PauliOperator:
         flags = _lib.QR_TEST_FORCE_WIDE if force_wide else 0
         check(_lib.load().qr_op_set_test_hooks(self._h, flags, int(wait_ns), int(withhold_step)))
 
+    def apply_form(self, dtype, nstates: int = 1, adjoint: bool = False) -> str:
+        """Test-only: the kernel family a product of ``nstates`` states of this
+        torch dtype runs on ("tables", "rows", "strings" or "cosets")."""
+        import torch
+        dt = {torch.complex64: QR_C64C, torch.complex128: QR_C128}[dtype]
+        form = _lib.load().qr_op_apply_form(self._h, dt, int(bool(adjoint)), int(nstates))
+        if form < 0:
+            check(form)
+        return ("tables", "rows", "strings", "cosets")[form]
+
 
 def _term_masks(paulis):
     """(x, z, phase, base phase) of equally long strings.  Up to 63 letters
