@@ -268,13 +268,18 @@ cudaError_t launch_diag(int dtype, int n, int db, uint64_t ntiles, const uint64_
 // span has rank > kCsrMaxRank, the term range to fold per row.
 constexpr int kCsrMaxRank = 4;
 constexpr uint32_t kCsrFold = 0xffffffffu;
-// Fold-mode groups: the longest leading run of terms whose z differences
-// span rank <= kCsrPrefixRank is folded per class once (table of
-// 2^(rank+1) entries); rows add only the terms after it.  Rank 12 (128 KB per
-// fold-mode group): chain n = 21 builds in 330 us, 338 with rank 10; with rank
-// 14 a Jordan-Wigner operator of 94 groups, n = 18, takes 143 instead of 132,
-// its rows' reads missing L1.
-constexpr int kCsrPrefixRank = 12;
+// Fold-mode groups: the longest leading run of terms whose z differences span
+// a bounded rank is folded per class once (table of 2^(rank+1) entries); rows
+// add only the terms after it.  The tables are computed anew by every
+// coefficient update, so the larger rank serves operators of few such groups
+// and rows enough to pay it back.  Measured, rank 10 / 12 (us, build and
+// coefficient update): chain n = 21 (one group) 377 / 358 and 19 / 27, n = 14
+// 11.8 / 11.8 and 20 / 31; Jordan-Wigner n = 12 (66 groups) 75 / 13 and 29 /
+// 246; 200 groups n = 16 1,174 / 1,064 and 54 / 190; 2,000 groups n = 12 656 /
+// 279 and 386 / 3,745 (first build 1,269 / 4,576, tables 64 / 256 MB).  With
+// rank 14 the chain's and a Jordan-Wigner operator's rows miss L1.
+constexpr int kCsrPrefixRank = 12, kCsrPrefixRankMany = 10;
+constexpr int kCsrDeepFolds = 8, kCsrDeepN = 16;  // at most, at least, for the larger rank
 struct CsrGroup {
     uint64_t z0;
     uint64_t beta[kCsrMaxRank];
@@ -300,7 +305,7 @@ struct CsrArgs {
     uint32_t nctab;           // class-table entries
     const uint64_t *tz;       // terms in group-stable order (fold mode)
     const double *tc;         // 2 doubles per term
-    const uint64_t *pbeta;    // nfold x kCsrPrefixRank: prefix span bases (fold mode)
+    const uint64_t *pbeta;    // nfold x kCsrPrefixRank: prefix span bases (fold mode; zeros after)
     const double2 *ptab;      // prefix class tables (fold mode)
     double2 *fvals;           // nfold x nrows fold-mode values, or null (written in place)
     int inline_fold;          // fold-mode entries folded by the staged fill (fvals null)

@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kCsrThreads) csr_fill_kernel(const CsrArgs a) 
 // Fold-mode groups (z span wider than kCsrMaxRank): one thread per row, all
 // lanes of a warp on the same group, the group's +-c'_k folded in input-term
 // order from the first term (make_row's fold), terms read warp-uniformly.
-// The leading terms up to z-span rank kCsrPrefixRank come from a
+// The leading terms up to a bounded z-span rank (kCsrPrefixRank) come from a
 // per-class fold of them (same additions, same order); the rest are added
 // per row.  A part (re or im) whose every coefficient is +-0 takes no FP64
 // additions: under round-to-nearest a sum of signed zeros is -0 exactly when

@@ -633,11 +633,11 @@ __global__ void csr_trie_kernel(const uint64_t *gx, uint32_t G, int n, uint64_t 
 // GF(2) span of tz[k] ^ tz[k0] over k in [k0, k1): basis in insertion order,
 // each difference reduced by the basis in descending pivot (msb) order;
 // coord[k] = its coordinates (bit i: basis i).  Stops at the first
-// difference that would need basis vector DMAX + 1: *used = terms spanned,
+// difference that would need basis vector dmax + 1 (dmax <= DMAX): *used = terms spanned,
 // return = -1 then, else the rank.  *nb = basis vectors found.
 template <int DMAX>
-__device__ int group_span(const uint64_t *tz, uint32_t k0, uint32_t k1, uint64_t *basis,
-                          uint16_t *coord, uint32_t *used, int *nb) {
+__device__ int group_span(const uint64_t *tz, uint32_t k0, uint32_t k1, int dmax,
+                          uint64_t *basis, uint16_t *coord, uint32_t *used, int *nb) {
     const uint64_t z0 = tz[k0];
     int cnt = 0;
     int ord[DMAX];  // basis indices by descending value (= descending pivot)
@@ -653,7 +653,7 @@ __device__ int group_span(const uint64_t *tz, uint32_t k0, uint32_t k1, uint64_t
             }
         }
         if (v != 0) {
-            if (cnt >= DMAX) {
+            if (cnt >= dmax) {
                 *used = k - k0;
                 *nb = cnt;
                 return -1;
@@ -676,7 +676,7 @@ __device__ int group_span(const uint64_t *tz, uint32_t k0, uint32_t k1, uint64_t
 }
 
 // Per group: rank-<= kCsrMaxRank span (class table of 2^(d+1) entries) or
-// fold mode with the leading terms of span rank <= kCsrPrefixRank folded per
+// fold mode with the leading terms of bounded span rank folded per
 // class (prefix table).  tab and zparts are filled later.
 struct CsrSpan {
     CsrGroup d;
@@ -698,7 +698,7 @@ __device__ void csr_span(uint32_t k0, uint32_t k1, const uint64_t *tz, uint16_t 
     s.isfold = s.rem = 0;
     uint32_t used;
     int nb;
-    const int r = group_span<kCsrMaxRank>(tz, k0, k1, s.basis, coord, &used, &nb);
+    const int r = group_span<kCsrMaxRank>(tz, k0, k1, kCsrMaxRank, s.basis, coord, &used, &nb);
     if (r >= 0) {
         d.d = (uint32_t)r;
         for (int j = 0; j < r; ++j) d.beta[j] = s.basis[j];
@@ -706,7 +706,15 @@ __device__ void csr_span(uint32_t k0, uint32_t k1, const uint64_t *tz, uint16_t 
         return;
     }
     d.d = kCsrFold;
-    group_span<kCsrPrefixRank>(tz, k0, k1, s.basis, coord, &used, &nb);
+    s.isfold = 1;
+}
+// A fold-mode group's prefix.
+__device__ void csr_prefix(const uint64_t *tz, int prank, uint16_t *coord, CsrSpan &s) {
+    CsrGroup &d = s.d;
+    const uint32_t k0 = d.k0, k1 = d.k1;
+    uint32_t used;
+    int nb;
+    group_span<kCsrPrefixRank>(tz, k0, k1, prank, s.basis, coord, &used, &nb);
     for (int j = nb; j < kCsrPrefixRank; ++j) s.basis[j] = 0;
     // the kernel continues the term-order fold after the prefix, so a
     // prefix cut short of a 24-bit count gives the same additions
@@ -715,7 +723,6 @@ __device__ void csr_span(uint32_t k0, uint32_t k1, const uint64_t *tz, uint16_t 
         d.pre = m | ((uint32_t)nb << 24);
         s.ptsz = 2ull << nb;
     }
-    s.isfold = 1;
     s.rem = k1 - k0 - (d.pre & 0xffffffu);
 }
 
@@ -725,6 +732,7 @@ __global__ void csr_span_kernel(uint32_t G, const uint32_t *goff, const uint64_t
     GRID_STRIDE(g, G) {
         CsrSpan s;
         csr_span(goff[g], goff[g + 1], tz, coord, s);
+        if (s.isfold) csr_prefix(tz, kCsrPrefixRankMany, coord, s);
         grp[g] = s.d;
         ctsz[g] = s.ctsz;
         ptsz[g] = s.ptsz;
@@ -780,6 +788,8 @@ __global__ void __launch_bounds__(kSmallGroups) csr_small_kernel(int n, uint32_t
     s.ctsz = s.ptsz = 0;
     s.isfold = s.rem = 0;
     if (g < G) csr_span(goff[g], goff[g + 1], tz, o.coord, s);
+    const bool deep = __syncthreads_count((int)s.isfold) <= kCsrDeepFolds && n >= kCsrDeepN;
+    if (s.isfold) csr_prefix(tz, deep ? kCsrPrefixRank : kCsrPrefixRankMany, o.coord, s);
     s_ct[g] = s.ctsz;
     s_pt[g] = s.ptsz;
     s_f[g] = s.isfold;
