@@ -48,43 +48,48 @@ __device__ __forceinline__ double2 plan_coef(const double2 *mc, const uint8_t *m
     return c;
 }
 
+// A thread per table entry: 2^ebits threads per slot, the widest slot's entries.
+// Bound by latency: an entry is a chain of as many FP64 additions as the slot
+// has strings, behind two dependent loads each.  (A thread per slot: 39 us for
+// 200 random strings of 8 qubits, 21 so.)
 __global__ void __launch_bounds__(256) coef_program_kernel(const CoefSlot *slots, uint32_t nslots,
+                                                           int ebits,
                                                            const uint32_t *mem,
                                                            const uint8_t *coord,
                                                            const double2 *mc, const uint8_t *madj,
                                                            int adjoint) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nslots;
-         i += gridDim.x * blockDim.x) {
-        const CoefSlot S = slots[i];
+    const uint64_t n = (uint64_t)nslots << ebits;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const CoefSlot S = slots[i >> ebits];
+        const uint32_t u = (uint32_t)i & ((1u << ebits) - 1u);
+        if (u >> S.d != 0) continue;
         if (S.kind == 2) {
             *reinterpret_cast<double2 *>(S.dst) = plan_coef(mc, madj, mem[S.m0], adjoint);
             continue;
         }
-        const uint32_t ent = 1u << S.d;
-        for (uint32_t u = 0; u < ent; ++u) {
-            double ar = 0.0, ai = 0.0;
-            for (uint32_t kk = S.m0; kk < S.m0 + S.cnt; ++kk) {
-                const double2 c = plan_coef(mc, madj, mem[kk], adjoint);
-                if (__popc(u & coord[kk]) & 1) {
-                    ar = __dsub_rn(ar, c.x);
-                    ai = __dsub_rn(ai, c.y);
-                } else {
-                    ar = __dadd_rn(ar, c.x);
-                    ai = __dadd_rn(ai, c.y);
-                }
+        double ar = 0.0, ai = 0.0;
+        for (uint32_t kk = S.m0; kk < S.m0 + S.cnt; ++kk) {
+            const double2 c = plan_coef(mc, madj, mem[kk], adjoint);
+            if (__popc(u & coord[kk]) & 1) {
+                ar = __dsub_rn(ar, c.x);
+                ai = __dsub_rn(ai, c.y);
+            } else {
+                ar = __dadd_rn(ar, c.x);
+                ai = __dadd_rn(ai, c.y);
             }
-            if (S.kind == 0)
-                reinterpret_cast<float2 *>(S.dst)[u] =
-                    make_float2(__double2float_rn(ar), __double2float_rn(ai));
-            else
-                reinterpret_cast<double2 *>(S.dst)[u] = make_double2(ar, ai);
         }
+        if (S.kind == 0)
+            reinterpret_cast<float2 *>(S.dst)[u] =
+                make_float2(__double2float_rn(ar), __double2float_rn(ai));
+        else
+            reinterpret_cast<double2 *>(S.dst)[u] = make_double2(ar, ai);
     }
 }
 
-static unsigned grid_for(uint32_t n) {
-    const uint32_t g = (n + 255u) / 256u;
-    return g == 0 ? 1u : (g > 4096u ? 4096u : g);
+static unsigned grid_for(uint64_t n) {
+    const uint64_t g = (n + 255u) / 256u;
+    return g == 0 ? 1u : (unsigned)(g > 4096u ? 4096u : g);
 }
 
 cudaError_t launch_merge_coeffs(uint32_t M, const uint32_t *mm_off, const uint32_t *mm_terms,
@@ -96,12 +101,12 @@ cudaError_t launch_merge_coeffs(uint32_t M, const uint32_t *mm_off, const uint32
     return cudaGetLastError();
 }
 
-cudaError_t launch_coef_program(const CoefSlot *slots, uint32_t nslots, const uint32_t *mem,
-                                const uint8_t *coord, const double2 *mc, const uint8_t *madj,
-                                int adjoint, cudaStream_t st) {
+cudaError_t launch_coef_program(const CoefSlot *slots, uint32_t nslots, int ebits,
+                                const uint32_t *mem, const uint8_t *coord, const double2 *mc,
+                                const uint8_t *madj, int adjoint, cudaStream_t st) {
     if (nslots == 0) return cudaSuccess;
-    coef_program_kernel<<<grid_for(nslots), 256, 0, st>>>(slots, nslots, mem, coord, mc, madj,
-                                                          adjoint);
+    coef_program_kernel<<<grid_for((uint64_t)nslots << ebits), 256, 0, st>>>(
+        slots, nslots, ebits, mem, coord, mc, madj, adjoint);
     count_launch();
     return cudaGetLastError();
 }

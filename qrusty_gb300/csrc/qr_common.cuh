@@ -163,9 +163,9 @@ static_assert(sizeof(CoefSlot) == 16, "CoefSlot layout");
 cudaError_t launch_merge_coeffs(uint32_t M, const uint32_t *mm_off, const uint32_t *mm_terms,
                                 const double2 *coeff, const uint8_t *phase, double2 *mc,
                                 cudaStream_t st);
-cudaError_t launch_coef_program(const CoefSlot *slots, uint32_t nslots, const uint32_t *mem,
-                                const uint8_t *coord, const double2 *mc, const uint8_t *madj,
-                                int adjoint, cudaStream_t st);
+cudaError_t launch_coef_program(const CoefSlot *slots, uint32_t nslots, int ebits,
+                                const uint32_t *mem, const uint8_t *coord, const double2 *mc,
+                                const uint8_t *madj, int adjoint, cudaStream_t st);
 
 // c'_k = m(phase_k) * c_k (make_params, qrusty/src/accel.rs:141-157):
 // m = (1, -i, -1, +i)[phase], num-complex's product (ar br - ai bi,

@@ -139,6 +139,7 @@ struct Plan {
     // diagonal's term list kept so that diag_wht can run again
     int dtype = 0, adjoint = 0;
     uint32_t nslots = 0;
+    int ebits = 0;  // log2 of the entries of the program's widest slot
     DevBuf cslots, cmem, ccoord;
     DevBuf dg_tz, dg_tc, dg_bz, dg_boff;
     uint32_t dg_nbins = 0;
@@ -1221,6 +1222,8 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     QR_CUDA(pl.cslots.upload(slots), "upload coefficient program");
     QR_CUDA(pl.cmem.upload(cmem), "upload coefficient program members");
     QR_CUDA(pl.ccoord.upload(ccoord), "upload coefficient program coordinates");
+    pl.ebits = 0;
+    for (const CoefSlot &sl : slots) pl.ebits = std::max(pl.ebits, (int)sl.d);
     pl.nslots = cmem.empty() ? 0u : (uint32_t)slots.size();
     pl.built = true;
     return QR_OK;
@@ -1797,7 +1800,7 @@ int qr_op_set_coeffs_device(qr_op *op, const double *coeff, void *stream) {
     if (rc) return rc;
     auto refresh = [&](Plan &pl) -> int {
         if (!pl.built) return QR_OK;
-        QR_CUDA(launch_coef_program(pl.cslots.as<CoefSlot>(), pl.nslots, pl.cmem.as<uint32_t>(),
+        QR_CUDA(launch_coef_program(pl.cslots.as<CoefSlot>(), pl.nslots, pl.ebits, pl.cmem.as<uint32_t>(),
                                     pl.ccoord.as<uint8_t>(), op->d_mc.as<double2>(),
                                     op->d_madj.as<uint8_t>(), pl.adjoint, st),
                 "coefficient program");
