@@ -1178,9 +1178,18 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     }
 
     if (pl.has_diag) {
-        // tiles of 2^12 rows, smaller ones below 2^21 rows so that at least 512
-        // CTAs share the transforms (n = 15: 8 tiles took 38 us)
-        const int db = std::min(n, std::min(12, std::max(5, n - 9)));
+        // Tile of the diagonal's transform: 2^8 rows up to n = 16, so that many
+        // CTAs share it, 2^12 from n = 20 on, where more tiles form their bins
+        // from all the terms more often; larger ones where a bin would hold
+        // many terms, which one thread adds up.  Measured, a coefficient update
+        // with tiles of 2^5 / 2^8 / 2^10 / 2^12 rows (us): n = 14, 300 terms 23 /
+        // 20 / 27 / 49, 16,000 164 / 51 / 62 / 94; n = 16, 60,000 1,251 / 173 /
+        // 151 / 192; n = 18, 300 58 / 31 / 32 / 49, 3,000 195 / 55 / 43 / 64,
+        // 200,000 14,500 / 1,558 / 555 / 500; n = 20, 30,000 8,560 / 861 / 314 /
+        // 183.
+        const size_t nd = diag_terms.size();
+        int db = std::min(n, std::min(12, std::max(8, n - (nd >= 1024 ? 8 : 9))));
+        while (db < std::min(n, 12) && nd >> db > (n < 17 ? 64u : 32u)) ++db;
         const uint64_t dmask = (1ull << db) - 1;
         std::vector<size_t> dt = diag_terms;
         std::stable_sort(dt.begin(), dt.end(), [&](size_t a, size_t b) {
