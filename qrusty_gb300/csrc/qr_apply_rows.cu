@@ -345,19 +345,26 @@ static cudaError_t launch_split(const ApplyArgs &a, int amps, int nsl, cudaStrea
 
 cudaError_t launch_rows(int dtype, const ApplyArgs &a, uint64_t call_rows, cudaStream_t st) {
     if (dtype == 0) {
-        // Slices by the size of a state: 16 warps share a row while the rows
-        // give too few warps to hide the L2 reads (n = 14, 500 random terms:
-        // 16 / 8 / 4 slices 50 / 58 / 83 us; n = 16 Jordan-Wigner: 98 / 73 /
-        // 72; n = 18: 4 slices 471 against 564 without), none from n = 21 on
-        // (chain n = 22: 637 us against 722 with 4), where the sums through
-        // shared memory cost more.  Rows per thread by the number of rows of
+        // Slices by the rows of the call: 16 warps share a row while the rows
+        // give too few warps to hide the L2 reads, none from 2^21 on, where the
+        // additions of the slices' sums are FP64 work like any other (us with
+        // 16 / 8 / 4 / 2 / 1 slices: 300 random strings 2^13 rows 25 / 25 / 37 /
+        // 60 / 107, 2^15 63 / 45 / 54 / 80 / 146, 2^17 209 / 149 / 130 / 135 /
+        // 177, 2^20 1,577 / 1,051 / 915 / 889 / 923; chain n = 13 2^19 rows 218 /
+        // 96 / 64 / 58 / 54, 2^21 856 / 361 / 234 / 199 / 189).  Without slices
+        // a CTA holds 512 rows of a state, so smaller states keep two.  Rows
+        // per thread by the number of rows of
         // all states: four share the parity and table work (1 or 2 are bound
         // by the instruction issue instead of FP64: Jordan-Wigner n = 24,
         // 49.9 ms against 29.9), so they are given up only below 2^14 rows,
         // where fewer than 128 CTAs would be left.
         const uint64_t rows = a.N * (uint64_t)a.nstates;
-        return launch_split<double>(a, rows < (1ull << 13) ? 1 : (rows < (1ull << 14) ? 2 : 4),
-                                    a.n < 15 ? 16 : (a.n < 16 ? 8 : (a.n < 21 ? 4 : 1)), st);
+        const int nsl = call_rows <= (1ull << 14)   ? 16
+                        : call_rows <= (1ull << 15) ? 8
+                        : call_rows < (1ull << 20)  ? 4
+                        : call_rows < (1ull << 21) || a.N < 512 ? 2 : 1;
+        return launch_split<double>(a, rows < (1ull << 13) ? 1 : (rows < (1ull << 14) ? 2 : 4), nsl,
+                                    st);
     }
     // complex64: slices and rows per thread by the rows of the call (best of
     // 1, 2, 4 rows x 1 ... 16 slices on random, chain and Jordan-Wigner

@@ -255,7 +255,7 @@ constexpr size_t kCosetSmem = 227u * 1024u - 256u;  // dynamic shared memory, at
 size_t coset_smem_bytes(uint32_t nsub, uint32_t nblk, uint32_t slots, uint32_t ntab);
 cudaError_t launch_c64c_cosets(const ApplyArgs &a, int nsm, cudaStream_t st);
 // qr_apply_rows.cu
-// call_rows: rows of the caller's whole call (complex64 splits by them)
+// call_rows: rows of the caller's whole call, which the split over warps follows
 cudaError_t launch_rows(int dtype, const ApplyArgs &a, uint64_t call_rows, cudaStream_t st);
 cudaError_t launch_diag(int dtype, int n, int db, uint64_t ntiles, const uint64_t *bin_zlo,
                         const uint32_t *bin_off, uint32_t nbins, const uint64_t *tz,
