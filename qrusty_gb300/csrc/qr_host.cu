@@ -859,6 +859,9 @@ int build_cosets(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vecto
 // Below 12 qubits a tile is smaller and costs 0.05-0.1 us per x group: n = 11,
 // 500 groups, 52 against 12 (one state), even at 2^15-2^16 rows.
 uint64_t c64_rows_limit(int n, bool strings) {
+    // a tile of fewer than 32 rows is less than a warp, which the per-tile-table
+    // kernel does not run on
+    if (n < 5) return ~0ull;
     return strings ? 1ull << 13 : n >= 12 ? 1ull << 17 : 1ull << 15;
 }
 
