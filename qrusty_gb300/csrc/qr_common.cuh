@@ -390,6 +390,12 @@ cudaError_t launch_vdot(int dtype, uint64_t N, const void *a, const void *b, int
 // merged order); partial
 // sums: direct.count x direct.nchunk, then wht.count x wht.nchunk.
 constexpr uint32_t kGradWhtMin = 8, kGradWhtBatch = 256;
+// Rows, passed over by each SM with four strings, that the transform has to save
+// to pay for its launch (us, all strings one by one / with the transform, one
+// state and eight): Jordan-Wigner n = 8 17 / 27 and 28 / 44, 300 Z strings n =
+// 12 (saves none: one round of blocks in both) 33 / 51 and 151 / 169, n = 13 (two
+// rounds or one) 52 / 51 and 283 / 169, H6 74 / 70 and 421 / 339.
+constexpr uint64_t kGradWhtRows = 4096;
 struct GradBatch {
     uint64_t x;
     uint32_t first, count;

@@ -1905,6 +1905,14 @@ int qr_expect(qr_op *op, int32_t dtype, const void *psi, int32_t nstates, double
     return qr_vdot(op->n, dtype, psi, op->expect_y.p, nstates, out, stream);
 }
 
+// Chunks of rows of the string-by-string gradients: about 8 work items of four
+// strings per SM, chunks of at least 4,096 rows.
+static uint64_t grad_chunks(uint64_t strings, uint64_t N, int nsm) {
+    const uint64_t items = (strings + 3) / 4;
+    if (items == 0) return 1;
+    return std::max<uint64_t>(1, std::min(((uint64_t)nsm * 8 + items - 1) / items, N / 4096));
+}
+
 int qr_term_grad(qr_op *op, int32_t dtype, const void *psi, const void *g, int32_t nstates,
                  double *out, void *stream) {
     if (!op || !psi || !g || !out) return fail(QR_EINVAL, "qr_term_grad: null argument");
@@ -1931,9 +1939,22 @@ int qr_term_grad(qr_op *op, int32_t dtype, const void *psi, const void *g, int32
         // span two partner tiles, largest first
         std::vector<uint32_t> ord, word;
         std::vector<GradBatch> wb;
+        uint64_t many = 0;  // strings that the transform could take
+        for (size_t g = 0; g < op->Ga; ++g) {
+            const uint32_t k = op->ag_off[g + 1] - op->ag_off[g];
+            if (k >= kGradWhtMin) many += k;
+        }
+        // rows that an SM passes four strings over, one by one
+        auto direct_rows = [&](uint64_t k) {
+            const uint64_t chunks = grad_chunks(k, op->N, op->nsm);
+            const uint64_t rounds = ((k + 3) / 4 * chunks + op->nsm - 1) / op->nsm;
+            return rounds * (op->N / chunks);
+        };
+        const bool wht = dtype == QR_C128 && many > 0 &&
+                         direct_rows(op->M) >= direct_rows(op->M - many) + kGradWhtRows;
         for (size_t g = 0; g < op->Ga; ++g) {
             const uint32_t a0 = op->ag_off[g], a1 = op->ag_off[g + 1];
-            if (dtype != QR_C128 || a1 - a0 < kGradWhtMin) {
+            if (!wht || a1 - a0 < kGradWhtMin) {
                 ord.insert(ord.end(), op->ag_mem.begin() + a0, op->ag_mem.begin() + a1);
                 continue;
             }
@@ -1986,12 +2007,12 @@ int qr_term_grad(qr_op *op, int32_t dtype, const void *psi, const void *g, int32
     p.nwbatch = tg.nwbatch;
     const uint32_t nd = unplanned ? (uint32_t)op->M : tg.ndirect;
     uint64_t nchunk = 1, nwchunk = 1;
-    if (nd > 0) {
-        // about 8 work items (4 strings each, or a batch of the tiled kernel)
-        // per SM, chunks of at least 16 tiles or 4,096 rows
-        const uint64_t items = tiles ? tg.nbatch : (nd + 3) / 4;
-        const uint64_t most = tiles ? (op->N >> 12) * (uint64_t)nstates / 16 : op->N / 4096;
-        nchunk = std::min(((uint64_t)op->nsm * 8 + items - 1) / items, most);
+    if (!tiles) {
+        nchunk = grad_chunks(nd, op->N, op->nsm);
+    } else if (nd > 0) {
+        // about 8 batches per SM, chunks of at least 16 tiles
+        nchunk = std::min(((uint64_t)op->nsm * 8 + tg.nbatch - 1) / tg.nbatch,
+                          (op->N >> 12) * (uint64_t)nstates / 16);
         if (nchunk < 1) nchunk = 1;
     }
     if (tg.nwbatch > 0) {
