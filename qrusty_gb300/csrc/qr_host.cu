@@ -346,18 +346,16 @@ void push_cplx(std::vector<unsigned char> &buf, cd v) {
     buf.insert(buf.end(), p, p + sizeof(c));
 }
 
-// One sub-group of the apply plan: terms sharing x (and, for the c64c
-// kernel, z on the register bits), with their FP64 table or term list.
+// One sub-group of a per-tile-table plan: merged strings sharing x and z on
+// the register bits, their z differences of rank <= 2, with their FP64 table.
 struct SubGroup {
     uint64_t hi = 0;       // partner-tile XOR (x >> b)
     uint32_t lo = 0;       // x & (tile - 1)
-    uint32_t zm = 0;       // z bits on the register bits (c64c), or kFat
+    uint32_t zm = 0;       // z bits on the register bits
     uint64_t z0 = 0;
-    uint64_t beta[kDMax] = {0, 0, 0, 0};
-    uint32_t d = 0;        // rank, or kFat
-    std::vector<cd> table; // 2^d entries
-    std::vector<uint64_t> fz;
-    std::vector<cd> fc;
+    uint64_t b0 = 0, b1 = 0;
+    uint32_t d = 0;        // rank
+    cd table[4];           // 2^d entries
     // merged strings of the sub-group in fold order, each with its coordinate
     // in the span basis (table entry u adds it with sign (-1)^popc(u & coord))
     std::vector<uint32_t> mem;
@@ -581,7 +579,6 @@ int build_cosets(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vecto
         uint64_t z0;
         Span sp;
         std::vector<size_t> part;
-        bool fused_next = false;
     };
     auto zm_of = [&](size_t k) {
         const uint32_t z = (uint32_t)(op->mz[k] >> 8) & 15u;
@@ -936,7 +933,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     while ((1 << abits) < pl.amps) ++abits;
     const uint64_t mmask = f32 ? (((1ull << abits) - 1) << pl.tb) : 0;
     std::vector<size_t> diag_terms;
-    std::vector<SubGroup> subs;
+    std::vector<std::pair<size_t, std::vector<size_t>>> pieces;  // sub-groups: x group, strings
     for (size_t g = 0; g < gxs.size(); ++g) {
         if (gxs[g] == 0) {
             std::vector<uint64_t> zs;
@@ -947,6 +944,10 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
             }
         }
         if (!f32) continue;  // whole groups (build_rows)
+        if (members[g].size() == 1) {
+            pieces.push_back({g, members[g]});
+            continue;
+        }
         std::vector<uint64_t> pkeys;
         std::vector<std::vector<size_t>> parts;
         for (size_t k : members[g]) {
@@ -959,15 +960,14 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
             }
             parts[pi].push_back(k);
         }
-        // c64c: split further until every sub-group has rank <= 2 (terms whose
-        // z differences agree beyond the first two basis vectors)
-        std::vector<std::vector<size_t>> pieces;
-        for (const auto &part : parts) {
+        // split further until every sub-group has rank <= 2 (strings whose z
+        // differences agree beyond the first two basis vectors)
+        for (auto &part : parts) {
             std::vector<uint64_t> zs;
             for (size_t k : part) zs.push_back(op->mz[k]);
             Span full = gf2_span(zs, 64);
             if (full.basis.size() <= 2) {
-                pieces.push_back(part);
+                pieces.push_back({g, std::move(part)});
                 continue;
             }
             std::vector<uint64_t> hk;
@@ -982,50 +982,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
                 }
                 hp[pi].push_back(part[kk]);
             }
-            for (auto &h : hp) pieces.push_back(std::move(h));
-        }
-        for (const auto &part : pieces) {
-            std::vector<uint64_t> zs;
-            for (size_t k : part) zs.push_back(op->mz[k]);
-            Span sp = gf2_span(zs, kDMax);
-            SubGroup sg;
-            sg.hi = gxs[g] >> pl.b;
-            sg.lo = (uint32_t)(gxs[g] & tmask);
-            sg.z0 = zs[0];
-            if (!sp.overflow) {
-                sg.d = (uint32_t)sp.basis.size();
-                sg.zm = (uint32_t)((sg.z0 & mmask) >> pl.tb);
-                for (size_t i = 0; i < sp.basis.size(); ++i) sg.beta[i] = sp.basis[i];
-                const uint32_t ent = 1u << sg.d;
-                for (size_t kk = 0; kk < part.size(); ++kk) {
-                    sg.mem.push_back((uint32_t)part[kk]);
-                    sg.coord.push_back((uint8_t)sp.coord[kk]);
-                }
-                for (uint32_t u = 0; u < ent; ++u) {
-                    cd acc{0.0, 0.0};
-                    for (size_t kk = 0; kk < part.size(); ++kk) {
-                        const cd v = c[part[kk]];
-                        if (__builtin_popcountll(u & sp.coord[kk]) & 1) {
-                            acc.re -= v.re;
-                            acc.im -= v.im;
-                        } else {
-                            acc.re += v.re;
-                            acc.im += v.im;
-                        }
-                    }
-                    sg.table.push_back(acc);
-                }
-            } else {
-                sg.d = kFat;
-                sg.zm = kFat;
-                for (size_t k : part) {
-                    sg.fz.push_back(op->mz[k]);
-                    sg.fc.push_back(c[k]);
-                    sg.mem.push_back((uint32_t)k);
-                    sg.coord.push_back(0);
-                }
-            }
-            subs.push_back(std::move(sg));
+            for (auto &h : hp) pieces.push_back({g, std::move(h)});
         }
     }
     pl.has_diag = !diag_terms.empty();
@@ -1035,60 +992,28 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     // kernel is the better one from a third more strings than sub-groups on
     // (chain n = 22, 64 strings in 47: 111 against 93).
     const size_t nstr = M - diag_terms.size();
-    const double most = (subs.size() <= (size_t)kTabCap ? 1.3 : 1.6) * (double)subs.size();
+    const double most = (pieces.size() <= (size_t)kTabCap ? 1.3 : 1.6) * (double)pieces.size();
     pl.strings = f32 && tile_bits < 0 && n >= 12 && nstr > 0 && (double)nstr <= most;
     pl.rows = !f32 || (tile_bits < 0 && op->N <= c64_rows_limit(n, pl.strings));
-    // order: partner tile ascending, then (c64c) run key zm with fat last
-    std::vector<size_t> ord(subs.size());
-    for (size_t i = 0; i < ord.size(); ++i) ord[i] = i;
-    // run key: register-bit sign pattern zm, register bits in the partner
-    // XOR (xm), and whether the factor depends on the thread index (tv)
-    auto runkey = [&](const SubGroup &g) -> uint32_t {
-        if (g.d == kFat || g.d > 2) return 0xffffffffu;
-        const uint64_t tm = (uint64_t)pl.threads - 1;
-        const uint64_t b0 = g.d > 0 ? g.beta[0] : 0, b1 = g.d > 1 ? g.beta[1] : 0;
-        const uint32_t tv = ((g.z0 | b0 | b1) & tm) != 0 ? 1u : 0u;
-        return (g.zm & 15u) | (((g.lo >> pl.tb) != 0 ? 1u : 0u) << 4) | (tv << 5);
-    };
-    std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) {
-        if (subs[a].hi != subs[b].hi) return subs[a].hi < subs[b].hi;
-        return f32 && runkey(subs[a]) < runkey(subs[b]);
-    });
+    pl.nsub = (uint32_t)pieces.size();
+    // partner tiles, one with more than kTabCap sub-groups (the per-tile table's
+    // size) visited as several consecutive blocks
+    std::vector<uint64_t> his;
+    for (const auto &pc : pieces) his.push_back(gxs[pc.first] >> pl.b);
+    std::sort(his.begin(), his.end());
     std::vector<uint64_t> bhi;
     std::vector<uint32_t> bg0;
-    if (pl.has_diag && (ord.empty() || subs[ord[0]].hi != 0)) {
+    if (pl.has_diag && (his.empty() || his[0] != 0)) {
         bhi.push_back(0);
         bg0.push_back(0);
     }
-    for (size_t i = 0; i < ord.size(); ++i) {
-        const uint64_t h = subs[ord[i]].hi;
-        if (bhi.empty() || bhi.back() != h) {
-            bhi.push_back(h);
+    for (size_t i = 0; i < his.size(); ++i)
+        if (i == 0 || his[i] != his[i - 1] || i - bg0.back() == (size_t)kTabCap) {
+            bhi.push_back(his[i]);
             bg0.push_back((uint32_t)i);
         }
-    }
-    bg0.push_back((uint32_t)ord.size());
-    if (f32) {
-        // the per-tile table holds at most kTabCap sub-groups: a partner tile
-        // with more is visited as several consecutive blocks (same partner)
-        std::vector<uint64_t> vh;
-        std::vector<uint32_t> vg;
-        for (size_t j = 0; j + 1 < bg0.size(); ++j) {
-            uint32_t g = bg0[j];
-            do {
-                vh.push_back(bhi[j]);
-                vg.push_back(g);
-                g += std::min<uint32_t>(kTabCap, bg0[j + 1] - g);
-            } while (g < bg0[j + 1]);
-        }
-        vg.push_back((uint32_t)ord.size());
-        bhi.swap(vh);
-        bg0.swap(vg);
-    }
+    bg0.push_back((uint32_t)his.size());
     pl.nblocks = (uint32_t)bhi.size();
-    pl.diag_block = -1;
-    for (size_t j = 0; j < bhi.size(); ++j)
-        if (bhi[j] == 0 && pl.diag_block < 0) pl.diag_block = (int)j;
 
     pl.nfat = 0;
     if (pl.rows) {
@@ -1105,19 +1030,68 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
         const int rc = build_cosets(op, pl, c, gxs, members, pl.has_diag, &pl.cosets, add_slot);
         if (rc) return rc;
     }
-    pl.nsub = (uint32_t)ord.size();
     if (f32 && !pl.strings && !pl.cosets) {
         // per-tile-table kernel arrays
+        pl.diag_block = -1;
+        for (size_t j = 0; j < bhi.size() && pl.diag_block < 0; ++j)
+            if (bhi[j] == 0) pl.diag_block = (int)j;
+        std::vector<SubGroup> subs;
+        for (const auto &pc : pieces) {
+            const std::vector<size_t> &part = pc.second;
+            std::vector<uint64_t> zs;
+            for (size_t k : part) zs.push_back(op->mz[k]);
+            const Span sp = gf2_span(zs, 2);
+            if (sp.overflow || part.size() > 0xffff)
+                return fail(QR_EINVAL, "plan: sub-group of rank > 2 in a complex64 plan");
+            SubGroup sg;
+            sg.hi = gxs[pc.first] >> pl.b;
+            sg.lo = (uint32_t)(gxs[pc.first] & tmask);
+            sg.z0 = zs[0];
+            sg.d = (uint32_t)sp.basis.size();
+            sg.zm = (uint32_t)((sg.z0 & mmask) >> pl.tb);
+            if (sg.d > 0) sg.b0 = sp.basis[0];
+            if (sg.d > 1) sg.b1 = sp.basis[1];
+            for (size_t kk = 0; kk < part.size(); ++kk) {
+                sg.mem.push_back((uint32_t)part[kk]);
+                sg.coord.push_back((uint8_t)sp.coord[kk]);
+            }
+            for (uint32_t u = 0; u < 1u << sg.d; ++u) {
+                cd acc{0.0, 0.0};
+                for (size_t kk = 0; kk < part.size(); ++kk) {
+                    const cd v = c[part[kk]];
+                    if (__builtin_popcountll(u & sp.coord[kk]) & 1) {
+                        acc.re -= v.re;
+                        acc.im -= v.im;
+                    } else {
+                        acc.re += v.re;
+                        acc.im += v.im;
+                    }
+                }
+                sg.table[u] = acc;
+            }
+            subs.push_back(std::move(sg));
+        }
+        const uint64_t tmask_t = (uint64_t)pl.threads - 1;
+        // run key: register-bit sign pattern zm, register bits in the partner
+        // XOR (xm), and whether the factor depends on the thread index (tv)
+        auto runkey = [&](const SubGroup &g) -> uint32_t {
+            const uint32_t tv = ((g.z0 | g.b0 | g.b1) & tmask_t) != 0 ? 1u : 0u;
+            return (g.zm & 15u) | (((g.lo >> pl.tb) != 0 ? 1u : 0u) << 4) | (tv << 5);
+        };
+        // order: partner tile ascending, then run key
+        std::vector<size_t> ord(subs.size());
+        for (size_t i = 0; i < ord.size(); ++i) ord[i] = i;
+        std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) {
+            if (subs[a].hi != subs[b].hi) return subs[a].hi < subs[b].hi;
+            return runkey(subs[a]) < runkey(subs[b]);
+        });
         std::vector<uint4> td;
         std::vector<TileDataC64> tdd;
         std::vector<uint32_t> r0v, rg0, rkey;
-        const uint64_t tmask_t = (uint64_t)pl.threads - 1;
         for (size_t i = 0; i < ord.size(); ++i) {
             const SubGroup &sg = subs[ord[i]];
-            const uint64_t b0 = sg.d > 0 && sg.d != kFat ? sg.beta[0] : 0;
-            const uint64_t b1 = sg.d > 1 && sg.d != kFat ? sg.beta[1] : 0;
-            const uint32_t zt = (uint32_t)(sg.z0 & tmask_t), bt0 = (uint32_t)(b0 & tmask_t),
-                           bt1 = (uint32_t)(b1 & tmask_t);
+            const uint32_t zt = (uint32_t)(sg.z0 & tmask_t), bt0 = (uint32_t)(sg.b0 & tmask_t),
+                           bt1 = (uint32_t)(sg.b1 & tmask_t);
             const uint32_t tvar = (zt | bt0 | bt1) != 0 ? 1u : 0u;
             // byte-offset XOR of the partner within the tile: thread bits of lo
             // (x 8 bytes) and register bits of lo (x 8 x threads); needs
@@ -1128,9 +1102,9 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
             TileDataC64 d;
             memset(&d, 0, sizeof(d));
             d.z0h = sg.z0 >> pl.b;
-            d.b0h = b0 >> pl.b;
-            d.b1h = b1 >> pl.b;
-            for (size_t u = 0; u < sg.table.size() && u < 4; ++u)
+            d.b0h = sg.b0 >> pl.b;
+            d.b1h = sg.b1 >> pl.b;
+            for (uint32_t u = 0; u < 1u << sg.d; ++u)
                 d.T[u] = make_float2((float)sg.table[u].re, (float)sg.table[u].im);
             tdd.push_back(d);
         }
@@ -1138,7 +1112,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
         for (uint32_t j = 0; j < pl.nblocks; ++j) {
             r0v.push_back((uint32_t)rkey.size());
             for (uint32_t g = bg0[j]; g < bg0[j + 1]; ++g) {
-                const uint32_t k = runkey(subs[ord[g]]) & 63u;
+                const uint32_t k = runkey(subs[ord[g]]);
                 if (g == bg0[j] || k != rkey.back()) {
                     rkey.push_back(k);
                     rg0.push_back(g);
@@ -1168,8 +1142,6 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
         QR_CUDA(pl.tdata.upload(tdd), "upload tile data");
         for (size_t i = 0; i < ord.size(); ++i) {
             const SubGroup &sg = subs[ord[i]];
-            if (sg.d == kFat || sg.d > 2 || sg.mem.size() > 0xffff)
-                return fail(QR_EINVAL, "plan: sub-group of rank > 2 in a complex64 plan");
             add_slot((uint64_t)pl.tdata.p + i * sizeof(TileDataC64) + offsetof(TileDataC64, T),
                      sg.mem.data(), sg.coord.data(), sg.mem.size(), sg.d, 0);
         }
