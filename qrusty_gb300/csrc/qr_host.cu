@@ -123,7 +123,8 @@ struct Plan {
     // states finds its tables built and every coefficient update reaches them
     bool rows = false;
     uint32_t nrgroups = 0;
-    DevBuf groups, tables, fat_z, fat_c;
+    size_t rtables = 0;  // byte offset of the factor tables behind the descriptors in groups
+    DevBuf groups, fat_z, fat_c;
     // compensated-c64 kernel tables
     uint32_t nsub = 0, nruns = 0, nchunks = 0;
     DevBuf tdesc, tdata, blk_r0, run_g0, run_key, chunks;
@@ -140,7 +141,8 @@ struct Plan {
     int dtype = 0, adjoint = 0;
     uint32_t nslots = 0;
     int ebits = 0;  // log2 of the entries of the program's widest slot
-    DevBuf cslots, cmem, ccoord;
+    DevBuf prog;            // its slots, their members and coordinates
+    size_t prog_mem = 0, prog_coord = 0;  // byte offsets of those
     DevBuf dg_tz, dg_tc, dg_bz, dg_boff;
     uint32_t dg_nbins = 0;
     int dg_db = 0;
@@ -306,15 +308,12 @@ Span gf2_span(const std::vector<uint64_t> &zs, size_t dmax) {
     Span sp;
     const uint64_t z0 = zs[0];
     sp.coord.resize(zs.size());
+    uint8_t ord[64];  // basis indices by descending pivot; the basis itself in order of insertion
     for (size_t k = 0; k < zs.size(); ++k) {
         uint64_t v = zs[k] ^ z0;
         uint64_t c = 0;
-        // basis kept in order of insertion; reduce by descending pivot
-        std::vector<size_t> ord(sp.basis.size());
-        for (size_t i = 0; i < ord.size(); ++i) ord[i] = i;
-        std::sort(ord.begin(), ord.end(),
-                  [&](size_t a, size_t b) { return sp.basis[a] > sp.basis[b]; });
-        for (size_t i : ord) {
+        for (size_t j = 0; j < sp.basis.size(); ++j) {
+            const size_t i = ord[j];
             const uint64_t bv = sp.basis[i];
             const int piv = 63 - __builtin_clzll(bv);
             if ((v >> piv) & 1ull) {
@@ -328,7 +327,10 @@ Span gf2_span(const std::vector<uint64_t> &zs, size_t dmax) {
                 sp.used = k;
                 return sp;
             }
-            c |= 1ull << sp.basis.size();
+            size_t j = sp.basis.size();
+            c |= 1ull << j;
+            for (; j > 0 && sp.basis[ord[j - 1]] < v; --j) ord[j] = ord[j - 1];
+            ord[j] = (uint8_t)sp.basis.size();
             sp.basis.push_back(v);
         }
         sp.coord[k] = c;
@@ -449,8 +451,11 @@ int build_rows(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vector<
     }
     pl.nrgroups = (uint32_t)descs.size();
     if (descs.empty()) descs.push_back(GroupDesc{});  // keep a valid pointer
-    QR_CUDA(pl.groups.upload(descs), "upload groups");
-    QR_CUDA(pl.tables.upload(tab), "upload tables");
+    pl.rtables = descs.size() * sizeof(GroupDesc);
+    std::vector<unsigned char> img(pl.rtables + tab.size());
+    memcpy(img.data(), descs.data(), pl.rtables);
+    if (!tab.empty()) memcpy(img.data() + pl.rtables, tab.data(), tab.size());
+    QR_CUDA(pl.groups.upload(img), "upload groups and tables");
     if constexpr (!f32) {
         QR_CUDA(pl.fat_z.upload(fz), "upload fat z");
         QR_CUDA(pl.fat_c.upload(fc), "upload fat c");
@@ -460,7 +465,7 @@ int build_rows(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vector<
         const GroupDesc &d = descs[i];
         if (!pc.fat) {
             if (pc.mem.size() > 0xffff) return fail(QR_EINVAL, "plan: group too large");
-            add_slot((uint64_t)pl.tables.p + (uint64_t)d.off * sizeof(Cplx<Real>), pc.mem.data(),
+            add_slot((uint64_t)pl.groups.p + pl.rtables + (uint64_t)d.off * sizeof(Cplx<Real>), pc.mem.data(),
                      pc.coord.data(), pc.mem.size(), d.d, f32 ? 0 : 1);
         } else {
             for (size_t kk = 0; kk < pc.mem.size(); ++kk)
@@ -1203,9 +1208,15 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
         QR_CUDA(cudaDeviceSynchronize(), "diagonal kernel sync");
     }
     if (slots.empty()) slots.push_back(CoefSlot{});  // keep valid pointers
-    QR_CUDA(pl.cslots.upload(slots), "upload coefficient program");
-    QR_CUDA(pl.cmem.upload(cmem), "upload coefficient program members");
-    QR_CUDA(pl.ccoord.upload(ccoord), "upload coefficient program coordinates");
+    pl.prog_mem = slots.size() * sizeof(CoefSlot);
+    pl.prog_coord = pl.prog_mem + cmem.size() * sizeof(uint32_t);
+    std::vector<unsigned char> prog(pl.prog_coord + ccoord.size());
+    memcpy(prog.data(), slots.data(), pl.prog_mem);
+    if (!cmem.empty()) {
+        memcpy(prog.data() + pl.prog_mem, cmem.data(), cmem.size() * sizeof(uint32_t));
+        memcpy(prog.data() + pl.prog_coord, ccoord.data(), ccoord.size());
+    }
+    QR_CUDA(pl.prog.upload(prog), "upload coefficient program");
     pl.ebits = 0;
     for (const CoefSlot &sl : slots) pl.ebits = std::max(pl.ebits, (int)sl.d);
     pl.nslots = cmem.empty() ? 0u : (uint32_t)slots.size();
@@ -1530,7 +1541,7 @@ static int apply_impl(const char *name, qr_op *op, int32_t dtype, const void *ps
     a.nitems = (uint64_t)nstates * a.ntiles;
     a.groups = pl.groups.as<GroupDesc>();
     a.ngroups = pl.nrgroups;
-    a.tables = pl.tables.p;
+    a.tables = pl.groups.as<unsigned char>() + pl.rtables;
     a.fat_z = pl.fat_z.as<uint64_t>();
     a.fat_c = pl.fat_c.p;
     a.blk_hi = pl.blk_hi.as<uint64_t>();
@@ -1784,8 +1795,10 @@ int qr_op_set_coeffs_device(qr_op *op, const double *coeff, void *stream) {
     if (rc) return rc;
     auto refresh = [&](Plan &pl) -> int {
         if (!pl.built) return QR_OK;
-        QR_CUDA(launch_coef_program(pl.cslots.as<CoefSlot>(), pl.nslots, pl.ebits, pl.cmem.as<uint32_t>(),
-                                    pl.ccoord.as<uint8_t>(), op->d_mc.as<double2>(),
+        const unsigned char *prog = pl.prog.as<unsigned char>();
+        QR_CUDA(launch_coef_program(pl.prog.as<CoefSlot>(), pl.nslots, pl.ebits,
+                                    reinterpret_cast<const uint32_t *>(prog + pl.prog_mem),
+                                    prog + pl.prog_coord, op->d_mc.as<double2>(),
                                     op->d_madj.as<uint8_t>(), pl.adjoint, st),
                 "coefficient program");
         if (pl.has_diag)
