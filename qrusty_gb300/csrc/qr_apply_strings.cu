@@ -115,25 +115,63 @@ __device__ __forceinline__ void str_mac(float2 (&y)[8], const float4 (&p)[4], ui
 
 __device__ __forceinline__ bool finite_f(float v) { return fabsf(v) <= kFltMax; }
 
-// Of the rows `left` (a mask of register indices), those with an infinite or NaN
-// partner in this block.  A string's zero part forms no product, so such a row
-// may have one finite part where 0 * inf, with every product formed, makes both
-// NaN.  Asked while the block's tiles are at hand: a state full of them costs no
-// more than a second pass over the block.
-__device__ __noinline__ uint32_t str_nonfinite(uint32_t left, const unsigned char *sm,
-                                              const uint4 *E, uint32_t ne, uint32_t base) {
+// Of the rows `left` (a mask of register indices; row: the first one's), those
+// with an infinite or NaN partner in blocks [b0, b1).  A string's zero part forms
+// no product, so such a row may have one finite part where 0 * inf, with every
+// product formed, makes both NaN.  Asked at each fold of its blocks, so that the
+// rows of a state full of them take no longer than the bounded waits allow.
+__device__ __forceinline__ uint32_t str_nonfinite(uint32_t left, const uint4 *sblk, uint32_t b0,
+                                                 uint32_t b1, const uint4 *ent, const float2 *psi,
+                                                 uint64_t row) {
     uint32_t bad = 0;
-    for (uint32_t i = 1; i <= ne && left != 0; ++i) {
-        const uint32_t w = E[i].x, off = base ^ (w & 0xfff0u);
-        for (uint32_t r = left; r != 0; r &= r - 1u) {
-            const uint32_t m = (uint32_t)__ffs((int)r) - 1u;
-            const float2 p = *reinterpret_cast<const float2 *>(
-                sm + (off ^ ((m >> 1) << 13)) + (((m ^ w) & 1u) << 3));
-            if (!(finite_f(p.x) && finite_f(p.y))) bad |= 1u << m;
+    for (uint32_t b = b0; b < b1 && left != 0; ++b) {
+        const uint4 bl = sblk[b];
+        for (uint32_t i = 1; i <= bl.w && left != 0; ++i) {
+            const uint32_t e = ent[bl.z + i].x;
+            const uint64_t x = (uint64_t)((e >> 15) & 1u ? bl.y : bl.x) << 12 | (e & 1u) |
+                               ((e >> 4) & 511u) << 1 | ((e >> 13) & 3u) << 10;
+            for (uint32_t r = left; r != 0; r &= r - 1u) {
+                const uint32_t m = (uint32_t)__ffs((int)r) - 1u;
+                const float2 p = psi[row ^ x ^ ((m & 1u) | (m >> 1) << 10)];
+                if (!(finite_f(p.x) && finite_f(p.y))) bad |= 1u << m;
+            }
+            left &= ~bad;
         }
-        left &= ~bad;
     }
     return bad;
+}
+
+// The same as a call: in line it costs the single kernel 2 %; the batch kernel
+// takes it in line, a call costs that one 8 %.
+__device__ __noinline__ uint32_t str_nonfinite_call(uint32_t left, const uint4 *sblk, uint32_t b0,
+                                                   uint32_t b1, const uint4 *ent,
+                                                   const float2 *psi, uint64_t row) {
+    return str_nonfinite(left, sblk, b0, b1, ent, psi, row);
+}
+
+// Fold the window's sums y into hi; the error opens the next window.  nonfinite:
+// asks str_nonfinite for the window's blocks.
+template <typename F>
+__device__ __forceinline__ void str_fold(float2 (&y)[8], float2 (&hi)[8], F &&nonfinite) {
+    // 0 * y: NaN once a part is infinite or NaN
+    const float2 z2 = make_float2(0.f, 0.f);
+    float2 q[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) q[m] = __ffma2_rn(y[m], z2, __fmul2_rn(y[m + 4], z2));
+    q[0] = __fadd2_rn(__fadd2_rn(q[0], q[1]), __fadd2_rn(q[2], q[3]));
+    if (__any_sync(0xffffffffu, q[0].x + q[0].y != 0.f)) {
+        uint32_t left = 0;
+#pragma unroll
+        for (int m = 0; m < 8; ++m)
+            left |= (finite_f(y[m].x) != finite_f(y[m].y) ? 1u : 0u) << m;
+        const uint32_t bad = nonfinite(left);
+        const float nan = __uint_as_float(0x7fc00000u);
+#pragma unroll
+        for (int m = 0; m < 8; ++m)
+            if (bad >> m & 1u) y[m] = make_float2(nan, nan);
+    }
+#pragma unroll
+    for (int m = 0; m < 8; ++m) y[m] = two_sum_carry2(hi[m], y[m]);
 }
 
 // A row's value: an infinite sum is NaN (its compensation is)
@@ -145,10 +183,11 @@ __device__ __forceinline__ float2 str_value(float2 h, float2 l) {
 
 // One block of the ring: the diagonal where it is flagged, then the strings in
 // turn, one's partner loads in flight while the other's products are formed.
+// Returns their number.
 template <bool WIDE>
-__device__ __forceinline__ void str_block(float2 (&y)[8], float2 (&hi)[8], uint32_t &win,
-                                          const unsigned char *sm, const uint4 *E, uint32_t base,
-                                          const float4 *dg, uint32_t t, uint32_t r0, uint32_t rhi) {
+__device__ __forceinline__ uint32_t str_block(float2 (&y)[8], const unsigned char *sm,
+                                              const uint4 *E, uint32_t base, const float4 *dg,
+                                              uint32_t t, uint32_t r0, uint32_t rhi) {
     float4 pa[4], pb[4];
     const uint2 head = *reinterpret_cast<const uint2 *>(E);
     const uint32_t ne = head.x;
@@ -183,30 +222,7 @@ __device__ __forceinline__ void str_block(float2 (&y)[8], float2 (&hi)[8], uint3
     } else if (i == ne) {
         str_mac<WIDE>(y, pa, ea, r0, rhi);
     }
-    // 0 * y: NaN once a part is infinite or NaN.  Once per block, 1 % of the
-    // time (n = 20, 16 strings a block); the warp's vote and the call keep it so
-    const float2 z2 = make_float2(0.f, 0.f);
-    float2 q[4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) q[m] = __ffma2_rn(y[m], z2, __fmul2_rn(y[m + 4], z2));
-    q[0] = __fadd2_rn(__fadd2_rn(q[0], q[1]), __fadd2_rn(q[2], q[3]));
-    if (__any_sync(0xffffffffu, q[0].x + q[0].y != 0.f)) {
-        uint32_t left = 0;
-#pragma unroll
-        for (int m = 0; m < 8; ++m)
-            left |= (finite_f(y[m].x) != finite_f(y[m].y) ? 1u : 0u) << m;
-        const uint32_t bad = str_nonfinite(left, sm, E, ne, base);
-        const float nan = __uint_as_float(0x7fc00000u);
-#pragma unroll
-        for (int m = 0; m < 8; ++m)
-            if (bad >> m & 1u) y[m] = make_float2(nan, nan);
-    }
-    win += ne;
-    if (win >= kSFold) {
-        win = 0;
-#pragma unroll
-        for (int m = 0; m < 8; ++m) y[m] = two_sum_carry2(hi[m], y[m]);
-    }
+    return ne;
 }
 
 __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
@@ -336,7 +352,14 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
             const uint64_t st = item / a.ntiles, q = item - st * a.ntiles;
             const uint32_t r0 = (uint32_t)(q << 12) | t << 1;
             const uint32_t rhi = WIDE ? (uint32_t)(q >> 20) << 24 : 0u;
-            uint32_t win = 0;
+            uint32_t win = 0, wb = b0;  // the window's strings and first block
+            auto fold = [&](uint32_t end) {
+                str_fold(y, hi, [&](uint32_t left) {
+                    return str_nonfinite_call(left, a.sblk, wb, end, a.ent,
+                                         static_cast<const float2 *>(a.psi) + st * a.N,
+                                         (q << 12) | (t << 1));
+                });
+            };
 #pragma unroll
             for (int m = 0; m < 8; ++m) y[m] = hi[m] = make_float2(0.f, 0.f);
             for (uint32_t b = b0; b < b1; ++b) {
@@ -356,8 +379,14 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
                 }
                 if (!skip) {
                     const uint4 *E = reinterpret_cast<const uint4 *>(s_ent + (size_t)s * kSEntBytes);
-                    str_block<WIDE>(y, hi, win, smem_raw, E, s * slot + t16,
-                                    static_cast<const float4 *>(a.diag) + (q << 11), t, r0, rhi);
+                    win += str_block<WIDE>(y, smem_raw, E, s * slot + t16,
+                                           static_cast<const float4 *>(a.diag) + (q << 11), t, r0,
+                                           rhi);
+                    if (win >= kSFold) {
+                        fold(b + 1);
+                        win = 0;
+                        wb = b + 1;
+                    }
                 }
                 __syncwarp();
                 if (lane == 0) arrive_local(&empty[s]);
@@ -366,8 +395,7 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings(const Ap
                     par ^= 1u;
                 }
             }
-#pragma unroll
-            for (int m = 0; m < 8; ++m) y[m] = two_sum_carry2(hi[m], y[m]);
+            fold(b1);
 
             float2 *yo = static_cast<float2 *>(a.y) + st * a.N + (q << 12);
             const float2 *vo = a.v ? static_cast<const float2 *>(a.v) + st * a.N + (q << 12) : nullptr;
@@ -445,7 +473,7 @@ __device__ __forceinline__ void str_batch_late(const StrBatchArgs &a) {
 // is the SMs its tiles do not cover (four states of 2^17 amplitudes are 128
 // tiles on 152 SMs; smaller ones are split over clusters, with a round of
 // exchange per tile) and its start and end; the ring runs on from item to
-// item.  24 operators of 10 to 17 qubits, 4 states: 1,366 us (1,428 with the
+// item.  24 operators of 10 to 17 qubits, 4 states: 1,335 us (1,428 with the
 // small ones in the table kernel and a launch per large one).  A string and
 // tile cost 390 clocks of an SM, as in a full launch of one operator, of which
 // the shared-memory wavefronts are 288.  A block's item travels with it: {operator, state, tile, first | last
@@ -526,6 +554,7 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings_batch(co
         asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
         float2 y[8], hi[8];
         uint32_t s = 0, par = 0, win = 0;
+        uint32_t b = 0, wb = 0;  // the item's block, the window's first
         for (;;) {
             // an expired wait sets the abort flag; every warp then leaves
             bool skip = false;
@@ -544,28 +573,38 @@ __global__ void __launch_bounds__(kSBlockThreads, 1) apply_c64c_strings_batch(co
             const uint4 me = s_meta[s];
             if (me.w & kEnd) break;
             if (me.w & 1u) {
-                win = 0;
+                win = b = wb = 0;
 #pragma unroll
                 for (int m = 0; m < 8; ++m) y[m] = hi[m] = make_float2(0.f, 0.f);
             }
-            str_block<false>(y, hi, win, smem_raw,
-                             reinterpret_cast<const uint4 *>(s_ent + (size_t)s * kSEntBytes),
-                             s * kSTileBytes + (t << 4),
-                             reinterpret_cast<const float4 *>(a.ops[me.x].diag) + ((uint64_t)me.z << 11),
-                             t, me.z << 12 | t << 1, 0u);
+            win += str_block<false>(
+                y, smem_raw, reinterpret_cast<const uint4 *>(s_ent + (size_t)s * kSEntBytes),
+                s * kSTileBytes + (t << 4),
+                reinterpret_cast<const float4 *>(a.ops[me.x].diag) + ((uint64_t)me.z << 11), t,
+                me.z << 12 | t << 1, 0u);
+            ++b;
+            const bool last = (me.w & 2u) != 0;
+            if (win >= kSFold || last) {
+                str_fold(y, hi, [&](uint32_t left) {
+                    const StrOp &op = a.ops[me.x];
+                    return str_nonfinite(left, op.sblk, wb, b, op.ent,
+                                         a.psi[me.x] + (uint64_t)me.y * op.N,
+                                         (uint64_t)me.z << 12 | t << 1);
+                });
+                win = 0;
+                wb = b;
+            }
             __syncwarp();
             if (lane == 0) arrive_local(&empty[s]);
             if (++s == kSMaxStages) {
                 s = 0;
                 par ^= 1u;
             }
-            if (!(me.w & 2u)) continue;
+            if (!last) continue;
             float2 *yo = a.y[me.x] + (uint64_t)me.y * a.ops[me.x].N + ((uint64_t)me.z << 12);
 #pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                y[m] = two_sum_carry2(hi[m], y[m]);
+            for (int m = 0; m < 8; ++m)
                 yo[2u * t + (m & 1u) + 1024u * (m >> 1)] = str_value(hi[m], y[m]);
-            }
         }
     }
     __syncthreads();

@@ -34,13 +34,14 @@ def _terms(n, strings, seed):
     return W.Terms(n, x, z, phase, rng.standard_normal(strings).astype(np.complex128))
 
 
-# one state of 14-18 qubits is split over a cluster, larger ones are not
-@pytest.mark.parametrize("n,strings", [(14, 300), (16, 1000), (18, 64), (20, 500)])
+# one state of 15-18 qubits is split over a cluster, larger ones are not
+@pytest.mark.parametrize("n,strings", [(15, 300), (16, 1000), (18, 64), (20, 500)])
 def test_rows_that_meet_one(cuda, oracle, n, strings):
     """They are NaN in both parts, every other row is what it was."""
     import torch
     t = _terms(n, strings, n)
     op = PauliOperator(n, t.x, t.z, t.phase, t.coeff)
+    assert op.apply_form(torch.complex64) == "strings"
     psi = W.random_state(np.random.default_rng(1), 1 << n).astype(np.complex64)
     clean = op.apply(torch.from_numpy(psi).to(cuda)).cpu().numpy()
     bad = np.array([3, 1 << 11, 1 << (n - 1), (1 << n) - 1])
@@ -56,7 +57,7 @@ def test_rows_that_meet_one(cuda, oracle, n, strings):
     op.sync_check()
 
 
-@pytest.mark.parametrize("n,strings", [(14, 300), (20, 500)])
+@pytest.mark.parametrize("n,strings", [(15, 300), (20, 500)])
 def test_overflow_stays_in_its_part(cuda, n, strings):
     """A finite amplitude whose products leave the range: NaN in the part that
     they are added to, the other part as with any real amplitude there."""
@@ -66,6 +67,7 @@ def test_overflow_stays_in_its_part(cuda, n, strings):
     t.phase[:] = 0
     t.coeff[:] = 2.0
     op = PauliOperator(n, t.x, t.z, t.phase, t.coeff)
+    assert op.apply_form(torch.complex64) == "strings"
     psi = W.random_state(np.random.default_rng(2), 1 << n).astype(np.complex64)
     at = 77
     psi[at] = complex(1.0, psi[at].imag)
