@@ -851,26 +851,29 @@ int build_cosets(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vecto
 
 // Rows up to which a complex64 call runs over rows, by what it would run on
 // otherwise: a tile kernel takes one SM per 4,096 rows.  Measured (us, tiles
-// against rows).  String kernel, which splits a tile over a cluster, 2^13 rows:
-// n = 12, 1,000 strings 33 / 25, 4,000 88 / 75, n = 13, 2,000 53 / 45; 2^14:
-// n = 12, 1,000 33 / 29, n = 14, 1,000 31 / 32, 5,000 128 / 121; 2^15: n = 12,
-// 2,000 51 / 76, n = 14, 5,000 128 / 194; 2^17: n = 12, 4,000 167 / 426.  Cosets
-// and per-tile tables, 2^17 rows: Jordan-Wigner of 92 x groups 25 / 25, 121 31 /
-// 31, molecular sums of 286 173 / 127, 981 507 / 377, 1,941 900 / 597, chain 13
-// / 9; 2^18: 121 31 / 55, 286 174 / 235, 981 507 / 707, 1,941 901 / 1,108.
-// Below 12 qubits a tile is smaller and costs 0.05-0.1 us per x group: n = 11,
-// 500 groups, 52 against 12 (one state), even at 2^15-2^16 rows.
-uint64_t c64_rows_limit(int n, bool strings) {
+// against rows).  String kernel, which splits a tile over a cluster, 2^14 rows:
+// n = 12, 1,000 strings 33 / 29, 4,000 88 / 90, n = 13, 2,000 53 / 53, n = 14,
+// 1,000 31 / 32, 5,000 128 / 121; 2^15: n = 12, 1,000 33 / 41, 2,000 51 / 76,
+// n = 14, 5,000 128 / 194; 2^17: n = 12, 4,000 167 / 426; it takes 12 us at
+// least, so few x groups run over more rows: 28 groups 2^17 12 / 8, 328 2^14
+// 21 / 16, 2^15 22 / 23.  Cosets and per-tile tables, 2^17 rows: Jordan-Wigner of
+// 92 x groups 25 / 25, 121 31 / 31, molecular sums of 286 173 / 127, 981 507 /
+// 377, 1,941 900 / 597, chain 13 / 9; 2^18: 121 31 / 55, 286 174 / 235, 981 507 /
+// 707, 1,941 901 / 1,108.  Below 12 qubits a tile is smaller and costs 0.05-0.1
+// us per x group: n = 11, 500 groups, 52 against 12 (one state), even at
+// 2^15-2^16 rows.
+uint64_t c64_rows_limit(int n, bool strings, uint64_t groups) {
     // a tile of fewer than 32 rows is less than a warp, which the per-tile-table
     // kernel does not run on
     if (n < 5) return ~0ull;
-    return strings ? 1ull << 13 : n >= 12 ? 1ull << 17 : 1ull << 15;
+    if (strings) return std::min(1ull << 17, std::max(1ull << 14, (1ull << 23) / groups));
+    return n >= 12 ? 1ull << 17 : 1ull << 15;
 }
 
 // Whether a call of this many states runs over rows.
 bool over_rows(const qr_op *op, const Plan &pl, int32_t call_states) {
     return pl.dtype == QR_C128 ||
-           (pl.rows && op->N * (uint64_t)call_states <= c64_rows_limit(op->n, pl.strings));
+           (pl.rows && op->N * (uint64_t)call_states <= c64_rows_limit(op->n, pl.strings, op->Ga));
 }
 
 int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
@@ -999,7 +1002,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     const size_t nstr = M - diag_terms.size();
     const double most = (pieces.size() <= (size_t)kTabCap ? 1.3 : 1.6) * (double)pieces.size();
     pl.strings = f32 && tile_bits < 0 && n >= 12 && nstr > 0 && (double)nstr <= most;
-    pl.rows = !f32 || (tile_bits < 0 && op->N <= c64_rows_limit(n, pl.strings));
+    pl.rows = !f32 || (tile_bits < 0 && op->N <= c64_rows_limit(n, pl.strings, op->Ga));
     pl.nsub = (uint32_t)pieces.size();
     // partner tiles, one with more than kTabCap sub-groups (the per-tile table's
     // size) visited as several consecutive blocks
@@ -2282,8 +2285,13 @@ int instantiate_mode(qr_batch *bt, int mode) {
         bt->str[i] = 0;
         if (mode != 0) rc = build_plan(bt->ops[i], QR_C64C, 0);
         const Plan &pl = bt->ops[i]->plans[QR_C64C][0];
+        // string plans of more than 2^13 rows, whatever a launch of their own would
+        // take: the operators share the SMs, so few tiles leave none idle (24
+        // operators of 10-18 qubits, four of several strings per group: 1,335 us,
+        // 1,347 with those in the persistent kernel)
         if (mode == 2 && !rc)
-            bt->str[i] = pl.strings && pl.str.tpb == 1 && !over_rows(bt->ops[i], pl, bt->nstates[i]);
+            bt->str[i] = pl.strings && pl.str.tpb == 1 &&
+                         bt->ops[i]->N * (uint64_t)bt->nstates[i] > (1ull << 13);
         bt->sel[i] = mode == 0 ? 1 : (mode == 1 ? 0 : bt->small[i] && !bt->str[i]);
     }
     if (!rc) rc = batch_build(bt, kBatchTileBits);

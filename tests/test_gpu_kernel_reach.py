@@ -43,7 +43,7 @@ def _letters(n, strings, seed):
 KERNELS = {
     "tables, one tile": ("tables", "complex64", 20, lambda: _letters(11, 200, 1), (0,)),
     "tables, several chunks": ("tables", "complex64", 1, lambda: _two_body(18, 250, 2), (0, 5, -1)),
-    "strings over a cluster": ("strings", "complex64", 1, lambda: _letters(14, 300, 3), (0, 3, 11)),
+    "strings over a cluster": ("strings", "complex64", 2, lambda: _letters(14, 300, 3), (0, 3, 11)),
     "strings, several rounds": ("strings", "complex64", 40, lambda: _letters(15, 200, 4), (0, 20)),
     "strings, two tiles a block": ("strings", "complex64", 1, lambda: _letters(20, 700, 5),
                                    (0, 3, 60)),
@@ -103,11 +103,11 @@ def test_wide_rows_are_identical(cuda, oracle, name, adjoint):
     assert np.linalg.norm(got - ref) <= 1e-6 * np.linalg.norm(ref)
 
 
-# string kernel: one partner tile (n = 12, three states are above the rows limit),
+# string kernel: one partner tile (n = 12, 33 states are above the rows limit),
 # blocks at their capacity of 255 strings (a 32nd of the strings below 19 qubits,
 # so from 8,160 on) and dense tiles at 19
-@pytest.mark.parametrize("n,states,strings", [(12, 3, k) for k in (1, 2, 3, 15, 16, 17, 33, 512)] +
-                         [(14, 1, 8159), (14, 1, 8160), (14, 3, 9000), (19, 1, 10000)])
+@pytest.mark.parametrize("n,states,strings", [(12, 33, k) for k in (1, 2, 3, 15, 16, 17, 33, 512)] +
+                         [(14, 2, 8159), (14, 2, 8160), (14, 3, 9000), (19, 1, 10000)])
 def test_string_blocks(cuda, oracle, n, states, strings):
     import torch
     t = _letters(n, strings, strings)

@@ -79,8 +79,9 @@ def test_capture_after_a_call_of_another_size(cuda, name, warm, call):
     assert torch.equal(torch.view_as_real(out), torch.view_as_real(want))
 
 
-# about one string per x group: the string kernel above 2^13 rows, whatever the
-# few groups of several strings and those on the diagonal
+# about one string per x group: the string kernel above 2^14 rows (2^23 over the
+# groups where they are few), whatever the few groups of several strings and those
+# on the diagonal
 @pytest.mark.parametrize("n,strings,diagonal", [(12, 400, 0), (12, 1000, 0), (12, 2000, 0),
                                                 (13, 2000, 0), (14, 2000, 0), (14, 900, 600)])
 def test_string_operators_leave_the_rows_kernel(cuda, oracle, n, strings, diagonal):
@@ -92,9 +93,9 @@ def test_string_operators_leave_the_rows_kernel(cuda, oracle, n, strings, diagon
         x[:diagonal], z[:diagonal] = 0, rng.choice(1 << n, diagonal, replace=False)
         t = W.Terms(n, x, z, np.zeros(strings, np.uint8), t.coeff)
     op = PauliOperator(n, t.x, t.z, t.phase, t.coeff)
-    states = 1 << (14 - n) if n < 14 else 1
+    states = 1 << (15 - n)
     assert op.apply_form(torch.complex64, states) == "strings"
-    assert op.apply_form(torch.complex64, max(1, states // 2)) == ("rows" if n < 14 else "strings")
+    assert op.apply_form(torch.complex64, states // 2) == "rows"
     psi = W.random_state(rng, 1 << n, nstates=2)[:1].astype(np.complex64)
     p = torch.from_numpy(np.repeat(psi, states, axis=0)).to(cuda)
     y = op.apply(p).cpu().numpy()
