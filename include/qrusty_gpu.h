@@ -123,7 +123,13 @@ int qr_csr_build(qr_op *op, uint64_t *indptr, uint64_t *indices, double *data,
  * QR_C128 computes in FP64 throughout.  QR_C64C keeps amplitudes and
  * products in FP32 and accumulates each amplitude's sum with compensated
  * (two-sum) additions; its relative error against the FP64 result is about
- * 2.5e-7 on a 26-qubit, 10,000-term operator (the tests bound it by 1e-6). */
+ * 1.7e-7 on a 26-qubit, 10,000-term operator (the tests bound it by 1e-6).
+ * Repeated calls of the same nstates give the same bits.  How a sum is split
+ * over the GPU depends on nstates, so a state may round differently in a call
+ * with another number of states.
+ * The first call per dtype and direction builds the plan (host work, device
+ * allocations, a synchronisation), which then serves every nstates: any later
+ * call of that dtype and direction can be captured into a CUDA graph. */
 int qr_apply(qr_op *op, int32_t dtype, const void *psi, void *y, int32_t nstates,
              int32_t adjoint, void *stream);
 
@@ -157,8 +163,9 @@ int qr_apply_host(qr_op *op, int32_t dtype, const void *psi_host, void *y_host,
 /* y = A v for a CSR matrix given by device arrays (replaces
  * spmat_dot_densevec, qrusty/src/accel.rs:338-370, and its binding
  * pyqrusty/src/lib.rs:476-491).  complex128; each row's products are summed
- * by 8 lanes (lane-strided partial sums, then a butterfly), so the result
- * matches a storage-order sum to rounding, not bit for bit.  v has ncols
+ * by 4 lanes (16 below 2^14 rows: lane-strided partial sums, then a butterfly),
+ * so the result matches a storage-order sum to rounding, not bit for bit.  The
+ * first row's length and entries choose the loop, not the result.  v has ncols
  * entries; a column index >= ncols is skipped.  indptr must be a valid
  * non-decreasing row-pointer array over data / indices. */
 int qr_csr_spmv(uint64_t nrows, uint64_t ncols, const uint64_t *indptr,
@@ -178,8 +185,9 @@ int qr_op_set_coeffs(qr_op *op, const double *coeff);
  * Replaces building a new SparsePauliOp (qrusty/src/lib.rs:354-376) like
  * qr_op_set_coeffs.  Kernels on `stream` recompute c' (make_params,
  * qrusty/src/accel.rs:141-157), the merged sums and every coefficient table
- * of the plans already built (qr_apply / qr_apply_axpby / qr_expect /
- * batches of this operator, and their diagonals), with the same FP64
+ * of the plans already built (one per dtype and direction of qr_apply /
+ * qr_apply_axpby / qr_expect, those of batches of this operator, and their
+ * diagonals), with the same FP64
  * operations in the same order as a host build, so results are bit for bit
  * those of an operator created with these coefficients.  Work on other
  * streams that reads the operator must be ordered after it by the caller;
@@ -202,7 +210,9 @@ int qr_op_set_coeffs_device(qr_op *op, const double *coeff, void *stream);
  *    it runs out after wait_ns.  The kernel then stops computing, waits for
  *    the copies it did issue, records the error word and returns; qr_check
  *    reports QR_EKERNEL.  -1 = off.
- * Hooks stay set until changed; (0, 0, -1) restores normal operation. */
+ * Hooks stay set until changed; (0, 0, -1) restores normal operation.  A batch
+ * reads its operators' hooks when it makes its graph (first call, new pointers or
+ * host coefficients). */
 enum { QR_TEST_FORCE_WIDE = 1 };
 int qr_op_set_test_hooks(qr_op *op, uint32_t flags, uint64_t wait_ns, int64_t withhold_step);
 /* TEST HOOK: the kernel family that qr_apply of nstates states runs on
@@ -253,8 +263,11 @@ int qr_expect(qr_op *op, int32_t dtype, const void *psi, int32_t nstates, double
  * coefficients the gradient is Re(out[k]).  FP32 products for QR_C64C,
  * FP64 accumulation across threads and tiles, every sum in a fixed order
  * (repeated calls and graph replays give the same bits).  Scratch is taken
- * from the stream-ordered allocator on `stream`.  New: no reference
- * counterpart (used by the autograd backward). */
+ * from the stream-ordered allocator on `stream`.  The first call per dtype
+ * uploads its string lists (synchronous); inside a stream capture it does
+ * without them (QR_C128, and QR_C64C with n < 12: the strings one by one, so it
+ * may round differently from later calls).  New: no reference counterpart (used
+ * by the autograd backward). */
 int qr_term_grad(qr_op *op, int32_t dtype, const void *psi, const void *g, int32_t nstates,
                  double *out, void *stream);
 
@@ -271,13 +284,16 @@ int qr_term_grad(qr_op *op, int32_t dtype, const void *psi, const void *g, int32
  * nstates[i] complex64 states (back to back).  The first call times, on the
  * given buffers (y is overwritten), (a) one persistent kernel over a work list
  * of (operator, state, amplitude tile) items, (b) a graph of one apply
- * kernel per operator on four parallel branches and, when the batch has
- * both, (c) the persistent kernel over the small operators (fewer work items
- * than half the SMs) beside per-operator kernels for the large ones; it
- * keeps the fastest, captured in a CUDA graph, and every call launches that
- * graph on `stream`.  A call whose pointers differ from the
- * previous call's synchronises `stream` first (and, for (b), captures the
- * graph again). */
+ * kernel per operator on four parallel branches and, when the batch has small
+ * operators (fewer work items than half the SMs) and large ones, (c) the
+ * persistent kernel over small operators beside one kernel that takes the
+ * (operator, state, tile) items of all operators of about one string per x mask
+ * and per-operator kernels for the others; it keeps the fastest, captured in a
+ * CUDA graph, and every call launches that graph on `stream`.  psi[i] and y[i]
+ * must not overlap.  A call whose pointers differ from
+ * the previous call's synchronises `stream` first (and, for (b) and (c), captures
+ * the graph again).  An expired wait is reported by qr_check of the operators,
+ * of all that share the item kernel. */
 typedef struct qr_batch qr_batch;
 int qr_batch_create(int32_t nops, qr_op *const *ops, const int32_t *nstates, qr_batch **out);
 int qr_batch_destroy(qr_batch *b);

@@ -29,7 +29,7 @@
 //
 // Measured (us, before -> after; before: rows t + 512 m, partner tiles in
 // pairs, the last warp out of a slot refilling it): Jordan-Wigner n = 26,
-// 10,000 terms 9,340 -> 7,270; n = 20, 4,000 103 -> 85; chain n = 22 110 -> 93,
+// 10,000 terms 9,340 -> 7,240; n = 20, 4,000 103 -> 84; chain n = 22 110 -> 93,
 // n = 24 464 -> 390.  Relative error at n = 26 2.1e-7 -> 1.7e-7 (a fold every 8
 // blocks instead of 16).
 #include "qr_common.cuh"

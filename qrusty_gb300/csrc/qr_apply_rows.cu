@@ -25,10 +25,10 @@
 //
 // Measured (us, before -> after; before: tiles of 4,096 amplitudes staged by
 // TMA, 4 multiply-adds per (amplitude, group)):
-//   random letters n = 12, 200 terms     848 ->  17   (was one CTA)
+//   random letters n = 12, 200 terms     848 ->  15   (was one CTA)
 //   Jordan-Wigner n = 18, 2,000 terms, 3 states   1,660 -> 820
-//   chain n = 22                       1,452 -> 640  (2 * 44 * 2^22
-//     multiply-adds: 1.15 of 1.26 TFLOP/s, the FP64 peak at 2,070 MHz)
+//   chain n = 22                       1,452 -> 623  (2 * 44 * 2^22
+//     multiply-adds: 1.18 of 1.26 TFLOP/s, the FP64 peak at 2,070 MHz)
 //   Jordan-Wigner n = 24, 4,000 terms 30,960 -> 29,940  (all factors complex:
 //     98 % of the FP64 peak)
 //
@@ -37,8 +37,8 @@
 // compensated fold every 16 groups of a slice (Kahan: the error opens the next
 // window) and the slices' compensated sums added in order.  Bound by latency
 // and, from 2^16 rows on, by L2 reads.  Measured (us, tiles -> rows): random
-// letters n = 10, 400 terms 28 -> 9.5; n = 11, 500 52 -> 12; Jordan-Wigner
-// n = 14, 1,400 25 -> 7.6; n = 16, 1,600 33 -> 18; chain n = 16 13 -> 6.
+// letters n = 10, 400 terms 28 -> 12; n = 11, 500 52 -> 15; Jordan-Wigner
+// n = 14, 1,400 25 -> 9.4; n = 16, 1,600 33 -> 21; chain n = 16 13 -> 8.5.
 #include <type_traits>
 
 #include "qr_common.cuh"

@@ -12,9 +12,10 @@
 // rows per thread (bits 0, 10 and 11 of the row are register bits, so one
 // 16-byte shared load brings two of a string's 8 partners) and take the
 // strings in turn: 4 loads, 8 sign XORs, 16 FMAs, since a string's
-// coefficient is real or imaginary (one with both parts takes 32).  Every 24
-// strings or more the sums are folded into a compensated pair (Kahan: the
-// error opens the next window).
+// coefficient is real or imaginary (one with both parts takes 32).  At the
+// end of a block, once the window holds 24 strings (278 at most, where blocks
+// are full), the sums are folded into a compensated pair (Kahan: the error opens
+// the next window).
 //
 // What bounds it: shared-memory wavefronts, 18 per warp and string (16 of
 // them partner amplitudes), 91 % busy (ncu, n = 18, 2,000 strings).  Hence
@@ -29,10 +30,11 @@
 // cluster of up to 8 CTAs, whose compensated sums meet through distributed
 // shared memory in rank order.
 //
-// Measured (us, before -> after; before: the per-tile table kernels): n = 12,
-// 200 strings 44 -> 17; n = 14, 500 98 -> 23; n = 16, 1,000, 3 states 212 ->
-// 82; n = 18, 2,000 463 -> 183; n = 20, 2,000 1,231 -> 735; n = 22, 500 1,770
-// -> 914.  Relative error of a random-letter product 1.0-1.4e-7 (was 1.3-3.0).
+// Measured (us, before -> after; before: the per-tile table kernels): n = 16,
+// 1,000 strings, 3 states 212 -> 88; n = 18, 2,000 463 -> 186; n = 20, 2,000 1,231
+// -> 741; n = 22, 500 1,770 -> 903.  Relative error of a random-letter product
+// 1.0-1.5e-7 with windows of few strings (was 1.3-3.0), 2.4-2.9e-7 with full
+// blocks (n = 14, 9,000 strings, n = 19, 10,000; was 4.2-8.0).
 #include <map>
 #include <mutex>
 #include <utility>
@@ -50,7 +52,7 @@ constexpr uint32_t kSTileBytes = 4096 * 8;
 constexpr uint32_t kSEntBytes = (kStrEntCap + 1) * 16;  // header and entries of a block
 constexpr uint32_t kSMaxStages = 4;
 constexpr float kFltMax = 3.402823466e38f;
-constexpr uint32_t kSFold = 24;  // strings per compensated fold, at least
+constexpr uint32_t kSFold = 24;  // strings per compensated fold, at least (23 + kStrEntCap at most)
 
 // partner amplitudes of one string: p[j] holds register indices 2 j, 2 j + 1
 __device__ __forceinline__ void str_load(float4 (&p)[4], const unsigned char *sm, uint32_t base,

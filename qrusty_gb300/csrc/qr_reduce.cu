@@ -263,8 +263,8 @@ __global__ void __launch_bounds__(kRedThreads) term_grad_finish_kernel(
 // is coefficient z & 255 up to the sign (-1)^popc(base & z).  A group of k
 // strings costs 4 + 16 operations per row and 2 k per 256 rows instead of 4 k
 // per row; complex128 is FP64-bound, so groups from kGradWhtMin strings take
-// this kernel (Jordan-Wigner n = 15, 500 terms, 95 of them on x = 0).
-// complex64: FP32 products and transform, FP64 sums.
+// this kernel where it saves enough (kGradWhtRows): Jordan-Wigner n = 15, 500
+// terms, 95 of them on x = 0, 110 us for the gradients (212).
 constexpr int kWhtPerLane = 8;  // strings per lane
 static_assert(kGradWhtBatch == 32 * kWhtPerLane, "strings of a batch");
 

@@ -20,8 +20,9 @@
 // The complex128 forms are bound by the FP64 pipe (2 operations per SM and
 // cycle): real scalars and real pivots, the rule for a Hermitian operator,
 // leave out the products of their zero part, and precond2 calls hypot only
-// near tol (2^20 elements: axpby with real scalars 34 -> 16 us, precond2 with
-// a real diagonal 92 -> 54, most of it the two divisions).
+// near tol (2^20 elements: axpby with real scalars 34 -> 16 us through the
+// binding, 12 on the device; precond2 with a real diagonal 92 -> 54, most of it
+// the two divisions).
 //
 // All element-wise kernels are streams: grid-stride over 16-byte
 // elements (one complex128 or two complex64), four elements in flight per
