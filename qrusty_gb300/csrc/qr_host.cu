@@ -1465,8 +1465,9 @@ int qr_csr_build(qr_op *op, uint64_t *indptr, uint64_t *indices, double *data, i
     // host destination: build in row chunks of <= ~1 GiB on the device
     const uint64_t per_row = op->G * 24;
     uint64_t rows = (1ull << 30) / (per_row ? per_row : 1);
-    // whole 256-row chunks, so that every launch starts on a chunk boundary
-    rows = rows < 256 ? 256 : rows & ~255ull;
+    // whole chunks (of 512 rows for one group, 256 at most otherwise), so that every
+    // launch starts on a chunk boundary
+    rows = rows < 512 ? 256 : rows & ~511ull;
     if (rows > op->N) rows = op->N;
     DevBuf d_ptr, d_idx, d_dat;
     QR_CUDA(d_ptr.alloc((op->N + 1) * sizeof(uint64_t)), "alloc indptr staging");
