@@ -1447,6 +1447,13 @@ int qr_csr_build(qr_op *op, uint64_t *indptr, uint64_t *indices, double *data, i
     auto fold_buffer = [&](uint64_t rows) {
         a.fvals = nullptr;
         if (op->nfold == 0 || op->G > 256 || a.inline_fold) return;
+        // One such group: in place after the fill, which costs a sector per entry,
+        // where the fill has many rows, or groups of several classes, whose stages
+        // the placing lengthens (us, placed by the fill / in place): Jordan-Wigner,
+        // 60 Z strings, n = 18 268 / 230, n = 19 534 / 454, n = 20 1,034 / 847; 60
+        // strings with x masks of their own and such a group n = 18 101 / 114, n = 20
+        // 342 / 331.  More groups: n = 18, 4 of 150 193 / 236, 16 322 / 475.
+        if (op->nfold == 1 && (op->n >= 20 || (op->n >= 18 && op->nctab >= 4 * op->G))) return;
         if (op->d_fv.alloc((size_t)op->nfold * rows * sizeof(double2)) == cudaSuccess)
             a.fvals = op->d_fv.as<double2>();
         else
