@@ -245,7 +245,8 @@ __device__ __forceinline__ double2 csr_fold_entry(const CsrArgs &a, uint64_t r, 
 // folds are computed first by csr_fold_kernel<true> into a row-major value
 // buffer and placed from there: their serial chains would hold the block at
 // the barrier, and stored in place after the fill each entry becomes a DRAM
-// read-modify-write of a line the bulk store has already evicted.  Without a
+// read-modify-write of a line the bulk store has already evicted (cheaper than
+// the placing for one group of many rows: qr_csr_build).  Without a
 // value buffer they are left unset and stored afterwards by
 // csr_fold_kernel<false>.  Which of these a launch needs is a template
 // argument: the code of all three in one body costs 10 %.
