@@ -143,7 +143,8 @@ struct Plan {
     int ebits = 0;  // log2 of the entries of the program's widest slot
     DevBuf prog;            // its slots, their members and coordinates
     size_t prog_mem = 0, prog_coord = 0;  // byte offsets of those
-    DevBuf dg_tz, dg_tc, dg_bz, dg_boff;
+    DevBuf dg;              // coefficients, z masks, bins' low masks and offsets, in turn
+    size_t dg_tz = 0, dg_bz = 0, dg_boff = 0;
     uint32_t dg_nbins = 0;
     int dg_db = 0;
 };
@@ -339,15 +340,6 @@ Span gf2_span(const std::vector<uint64_t> &zs, size_t dmax) {
     return sp;
 }
 
-template <typename Real>
-void push_cplx(std::vector<unsigned char> &buf, cd v) {
-    Cplx<Real> c;
-    c.re = (Real)v.re;
-    c.im = (Real)v.im;
-    const unsigned char *p = reinterpret_cast<const unsigned char *>(&c);
-    buf.insert(buf.end(), p, p + sizeof(c));
-}
-
 // One sub-group of a per-tile-table plan: merged strings sharing x and z on
 // the register bits, their z differences of rank <= 2, with their FP64 table.
 struct SubGroup {
@@ -378,30 +370,28 @@ int build_rows(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vector<
     std::stable_sort(ord.begin(), ord.end(),
                      [&](size_t a, size_t b) { return (gxs[a] >> 12) < (gxs[b] >> 12); });
     std::vector<GroupDesc> descs;
-    std::vector<unsigned char> tab, fc;
+    std::vector<Cplx<Real>> tab, fc;
     std::vector<uint64_t> fz;
-    struct Piece {
-        std::vector<uint32_t> mem;
-        std::vector<uint8_t> coord;
-        bool fat;
-    };
-    std::vector<Piece> pieces;  // of descs, for the coefficient program
-    uint32_t ntab = 0;
+    // strings of the descriptors in turn and their coordinates, for the
+    // coefficient program
+    std::vector<uint32_t> mem, first;
+    std::vector<uint8_t> coord;
     auto masks = [&](const std::vector<size_t> &part) {
         std::vector<uint64_t> zs;
+        zs.reserve(part.size());
         for (size_t k : part) zs.push_back(op->mz[k]);
         return zs;
     };
+    auto cplx = [](cd v) { return Cplx<Real>{(Real)v.re, (Real)v.im}; };
     auto push = [&](uint64_t x, const std::vector<size_t> &part, const Span &sp, bool fat) {
         GroupDesc d;
         memset(&d, 0, sizeof(d));
         d.z0 = op->mz[part[0]];
         d.x = x;
-        Piece pc;
-        pc.fat = fat;
+        first.push_back((uint32_t)mem.size());
         for (size_t kk = 0; kk < part.size(); ++kk) {
-            pc.mem.push_back((uint32_t)part[kk]);
-            pc.coord.push_back(fat ? 0 : (uint8_t)sp.coord[kk]);
+            mem.push_back((uint32_t)part[kk]);
+            coord.push_back(fat || sp.coord.empty() ? 0 : (uint8_t)sp.coord[kk]);
         }
         if (fat) {
             d.d = kFat;
@@ -409,18 +399,18 @@ int build_rows(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vector<
             d.cnt = (uint32_t)part.size();
             for (size_t k : part) {
                 fz.push_back(op->mz[k]);
-                push_cplx<Real>(fc, c[k]);
+                fc.push_back(cplx(c[k]));
             }
             pl.nfat++;
         } else {
             d.d = (uint32_t)sp.basis.size();
-            d.off = ntab;
+            d.off = (uint32_t)tab.size();
             for (size_t i = 0; i < sp.basis.size(); ++i) d.beta[i] = sp.basis[i];
             for (uint32_t u = 0; u < 1u << d.d; ++u) {
                 cd acc{0.0, 0.0};
                 for (size_t kk = 0; kk < part.size(); ++kk) {
                     const cd v = c[part[kk]];
-                    if (__builtin_popcountll(u & sp.coord[kk]) & 1) {
+                    if (__builtin_popcountll(u & coord[first.back() + kk]) & 1) {
                         acc.re -= v.re;
                         acc.im -= v.im;
                     } else {
@@ -428,15 +418,18 @@ int build_rows(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vector<
                         acc.im += v.im;
                     }
                 }
-                push_cplx<Real>(tab, acc);
+                tab.push_back(cplx(acc));
             }
-            ntab += 1u << d.d;
         }
         descs.push_back(d);
-        pieces.push_back(std::move(pc));
     };
+    const Span one;  // a single string: rank 0
     for (size_t g : ord) {
         if (skip_zero && gxs[g] == 0) continue;
+        if (members[g].size() == 1) {
+            push(gxs[g], members[g], one, false);
+            continue;
+        }
         const std::vector<uint64_t> zs = masks(members[g]);
         const Span sp = gf2_span(zs, kDMax);
         if (!sp.overflow || !f32) {
@@ -449,28 +442,29 @@ int build_rows(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vector<
             parts[full.coord[kk] >> kDMax].push_back(members[g][kk]);
         for (const auto &pt : parts) push(gxs[g], pt.second, gf2_span(masks(pt.second), kDMax), false);
     }
+    first.push_back((uint32_t)mem.size());
     pl.nrgroups = (uint32_t)descs.size();
     if (descs.empty()) descs.push_back(GroupDesc{});  // keep a valid pointer
     pl.rtables = descs.size() * sizeof(GroupDesc);
-    std::vector<unsigned char> img(pl.rtables + tab.size());
+    std::vector<unsigned char> img(pl.rtables + tab.size() * sizeof(Cplx<Real>));
     memcpy(img.data(), descs.data(), pl.rtables);
-    if (!tab.empty()) memcpy(img.data() + pl.rtables, tab.data(), tab.size());
+    if (!tab.empty()) memcpy(img.data() + pl.rtables, tab.data(), img.size() - pl.rtables);
     QR_CUDA(pl.groups.upload(img), "upload groups and tables");
     if constexpr (!f32) {
         QR_CUDA(pl.fat_z.upload(fz), "upload fat z");
         QR_CUDA(pl.fat_c.upload(fc), "upload fat c");
     }
-    for (size_t i = 0; i < pieces.size(); ++i) {
-        const Piece &pc = pieces[i];
+    for (size_t i = 0; i + 1 < first.size(); ++i) {
         const GroupDesc &d = descs[i];
-        if (!pc.fat) {
-            if (pc.mem.size() > 0xffff) return fail(QR_EINVAL, "plan: group too large");
-            add_slot((uint64_t)pl.groups.p + pl.rtables + (uint64_t)d.off * sizeof(Cplx<Real>), pc.mem.data(),
-                     pc.coord.data(), pc.mem.size(), d.d, f32 ? 0 : 1);
+        const uint32_t m0 = first[i], cnt = first[i + 1] - m0;
+        if (d.d != kFat) {
+            if (cnt > 0xffff) return fail(QR_EINVAL, "plan: group too large");
+            add_slot((uint64_t)pl.groups.p + pl.rtables + (uint64_t)d.off * sizeof(Cplx<Real>),
+                     &mem[m0], &coord[m0], cnt, d.d, f32 ? 0 : 1);
         } else {
-            for (size_t kk = 0; kk < pc.mem.size(); ++kk)
+            for (uint32_t kk = 0; kk < cnt; ++kk)
                 add_slot((uint64_t)pl.fat_c.p + (uint64_t)(d.off + kk) * sizeof(Cplx<Real>),
-                         &pc.mem[kk], nullptr, 1, 0, 2);
+                         &mem[m0 + kk], nullptr, 1, 0, 2);
         }
     }
     return QR_OK;
@@ -595,36 +589,38 @@ int build_cosets(qr_op *op, Plan &pl, const std::vector<cd> &c, const std::vecto
         return zs;
     };
     std::vector<Sub> subs;
+    std::vector<size_t> byzm[8];
     for (size_t g = 0; g < gxs.size(); ++g) {
         if (has_diag && gxs[g] == 0) continue;
         const uint32_t lo = (uint32_t)(gxs[g] & 4095u), xm = lo >> 9;
         const uint32_t off = ((lo & 511u) ^ ((__builtin_popcount(xm) & 1) ? 256u : 0u)) << 3;
-        std::vector<std::vector<size_t>> byzm(8);
+        auto push = [&](uint32_t zm, std::vector<size_t> part, Span sp) {
+            Sub sg;
+            sg.hi = gxs[g] >> 12;
+            sg.x = gxs[g];
+            sg.off = off;
+            sg.xm = xm;
+            sg.zm = zm;
+            sg.z0 = op->mz[part[0]] & ~0xe00ull;
+            sg.sp = std::move(sp);
+            sg.part = std::move(part);
+            subs.push_back(std::move(sg));
+        };
+        for (auto &v : byzm) v.clear();
         for (size_t k : members[g]) byzm[zm_of(k)].push_back(k);
         for (uint32_t zm = 0; zm < 8; ++zm) {
             if (byzm[zm].empty()) continue;
-            std::vector<std::vector<size_t>> pieces;
-            const Span full = gf2_span(masked(byzm[zm]), 64);
+            Span full = gf2_span(masked(byzm[zm]), 64);
             if (full.basis.size() <= 2) {
-                pieces.push_back(byzm[zm]);
-            } else {
-                std::map<uint64_t, std::vector<size_t>> parts;
-                for (size_t kk = 0; kk < byzm[zm].size(); ++kk)
-                    parts[full.coord[kk] >> 2].push_back(byzm[zm][kk]);
-                for (auto &pt : parts) pieces.push_back(std::move(pt.second));
+                push(zm, byzm[zm], std::move(full));
+                continue;
             }
-            for (auto &part : pieces) {
-                Sub sg;
-                sg.hi = gxs[g] >> 12;
-                sg.x = gxs[g];
-                sg.off = off;
-                sg.xm = xm;
-                sg.zm = zm;
-                const std::vector<uint64_t> zs = masked(part);
-                sg.z0 = zs[0];
-                sg.sp = gf2_span(zs, 2);
-                sg.part = std::move(part);
-                subs.push_back(std::move(sg));
+            std::map<uint64_t, std::vector<size_t>> parts;
+            for (size_t kk = 0; kk < byzm[zm].size(); ++kk)
+                parts[full.coord[kk] >> 2].push_back(byzm[zm][kk]);
+            for (auto &pt : parts) {
+                Span sp = gf2_span(masked(pt.second), 2);
+                push(zm, std::move(pt.second), std::move(sp));
             }
         }
     }
@@ -876,6 +872,16 @@ bool over_rows(const qr_op *op, const Plan &pl, int32_t call_states) {
            (pl.rows && op->N * (uint64_t)call_states <= c64_rows_limit(op->n, pl.strings, op->Ga));
 }
 
+// The plan's diagonal from its strings' coefficients on the device.
+cudaError_t run_diag(const qr_op *op, const Plan &pl, cudaStream_t st) {
+    const unsigned char *p = pl.dg.as<unsigned char>();
+    return launch_diag(pl.dtype, op->n, pl.dg_db, op->N >> pl.dg_db,
+                       reinterpret_cast<const uint64_t *>(p + pl.dg_bz),
+                       reinterpret_cast<const uint32_t *>(p + pl.dg_boff), pl.dg_nbins,
+                       reinterpret_cast<const uint64_t *>(p + pl.dg_tz),
+                       reinterpret_cast<const double *>(p), pl.diag.p, st);
+}
+
 int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     Plan &pl = tile_bits >= 0 ? op->bplans[tile_bits] : op->plans[dtype][adjoint];
     if (pl.built) return QR_OK;
@@ -941,7 +947,8 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
     while ((1 << abits) < pl.amps) ++abits;
     const uint64_t mmask = f32 ? (((1ull << abits) - 1) << pl.tb) : 0;
     std::vector<size_t> diag_terms;
-    std::vector<std::pair<size_t, std::vector<size_t>>> pieces;  // sub-groups: x group, strings
+    // sub-groups: x group, strings (none listed: all of the group's)
+    std::vector<std::pair<size_t, std::vector<size_t>>> pieces;
     for (size_t g = 0; g < gxs.size(); ++g) {
         if (gxs[g] == 0) {
             std::vector<uint64_t> zs;
@@ -953,7 +960,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
         }
         if (!f32) continue;  // whole groups (build_rows)
         if (members[g].size() == 1) {
-            pieces.push_back({g, members[g]});
+            pieces.emplace_back(g, std::vector<size_t>());
             continue;
         }
         std::vector<uint64_t> pkeys;
@@ -1045,7 +1052,7 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
             if (bhi[j] == 0) pl.diag_block = (int)j;
         std::vector<SubGroup> subs;
         for (const auto &pc : pieces) {
-            const std::vector<size_t> &part = pc.second;
+            const std::vector<size_t> &part = pc.second.empty() ? members[pc.first] : pc.second;
             std::vector<uint64_t> zs;
             for (size_t k : part) zs.push_back(op->mz[k]);
             const Span sp = gf2_span(zs, 2);
@@ -1192,22 +1199,24 @@ int build_plan(qr_op *op, int dtype, int adjoint, int tile_bits = -1) {
             tcv.push_back(c[dt[i]].im);
         }
         boff.push_back((uint32_t)dt.size());
-        QR_CUDA(pl.dg_tz.upload(tz), "upload diag z");
-        QR_CUDA(pl.dg_tc.upload(tcv), "upload diag c");
-        QR_CUDA(pl.dg_bz.upload(bz), "upload diag bins");
-        QR_CUDA(pl.dg_boff.upload(boff), "upload diag bin offsets");
+        pl.dg_tz = tcv.size() * sizeof(double);
+        pl.dg_bz = pl.dg_tz + tz.size() * sizeof(uint64_t);
+        pl.dg_boff = pl.dg_bz + bz.size() * sizeof(uint64_t);
+        std::vector<unsigned char> img(pl.dg_boff + boff.size() * sizeof(uint32_t));
+        memcpy(img.data(), tcv.data(), pl.dg_tz);
+        memcpy(img.data() + pl.dg_tz, tz.data(), pl.dg_bz - pl.dg_tz);
+        memcpy(img.data() + pl.dg_bz, bz.data(), pl.dg_boff - pl.dg_bz);
+        memcpy(img.data() + pl.dg_boff, boff.data(), img.size() - pl.dg_boff);
+        QR_CUDA(pl.dg.upload(img), "upload diagonal strings");
         pl.dg_nbins = (uint32_t)bz.size();
         pl.dg_db = db;
         for (size_t i = 0; i < dt.size(); ++i) {
             const uint32_t mi = (uint32_t)dt[i];
-            add_slot((uint64_t)pl.dg_tc.p + i * 2 * sizeof(double), &mi, nullptr, 1, 0, 2);
+            add_slot((uint64_t)pl.dg.p + i * 2 * sizeof(double), &mi, nullptr, 1, 0, 2);
         }
         const size_t esz = f32 ? sizeof(Cplx<float>) : sizeof(Cplx<double>);
         QR_CUDA(pl.diag.alloc(op->N * esz), "alloc diagonal");
-        QR_CUDA(launch_diag(dtype, n, db, op->N >> db, pl.dg_bz.as<uint64_t>(),
-                            pl.dg_boff.as<uint32_t>(), pl.dg_nbins, pl.dg_tz.as<uint64_t>(),
-                            pl.dg_tc.as<double>(), pl.diag.p, nullptr),
-                "diagonal kernel");
+        QR_CUDA(run_diag(op, pl, nullptr), "diagonal kernel");
         QR_CUDA(cudaDeviceSynchronize(), "diagonal kernel sync");
     }
     if (slots.empty()) slots.push_back(CoefSlot{});  // keep valid pointers
@@ -1813,10 +1822,7 @@ int qr_op_set_coeffs_device(qr_op *op, const double *coeff, void *stream) {
                                     op->d_madj.as<uint8_t>(), pl.adjoint, st),
                 "coefficient program");
         if (pl.has_diag)
-            QR_CUDA(launch_diag(pl.dtype, op->n, pl.dg_db, op->N >> pl.dg_db,
-                                pl.dg_bz.as<uint64_t>(), pl.dg_boff.as<uint32_t>(), pl.dg_nbins,
-                                pl.dg_tz.as<uint64_t>(), pl.dg_tc.as<double>(), pl.diag.p, st),
-                    "diagonal kernel");
+            QR_CUDA(run_diag(op, pl, st), "diagonal kernel");
         return QR_OK;
     };
     for (int d = 0; d < 2; ++d)
