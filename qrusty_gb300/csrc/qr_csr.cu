@@ -294,9 +294,11 @@ __host__ __device__ inline uint32_t csr_align(size_t b, uint32_t to) {
 }
 __host__ __device__ inline CsrStage csr_stage(uint32_t G, int n, uint32_t nctab, uint32_t nfv) {
     CsrStage s;
-    // 64 rows where they fill a stage, else 256; 512 for one group (one string, n =
-    // 20: 19 us with 256, 15 so)
-    s.L = (size_t)G * 24u << kCsrChunkBits >= kCsrStageBytes ? kCsrChunkBits : G == 1 ? 9 : 8;
+    // 64 rows where they fill a stage, else 256; 512 for one group of many rows (one
+    // string, n = 20: 19 us with 256, 15 so; n = 6 6.6 and 8.6)
+    s.L = (size_t)G * 24u << kCsrChunkBits >= kCsrStageBytes ? kCsrChunkBits
+          : G == 1 && n >= 18                                ? 9
+                                                             : 8;
     while (s.L > 1 && (size_t)G * ((1u << s.L) + 2) * 2u > kCsrLowBytes) --s.L;
     s.U = s.L > 1 ? s.L - 1 : 1;
     s.lsz = (1u << s.L) + 2;

@@ -1,5 +1,5 @@
-"""CSR of one x group (a single Pauli among them): chunks of 512 rows, bit for bit
-against the oracle, on the device and over the host."""
+"""CSR of one x group (a single Pauli among them), chunks of 512 rows from 18 qubits
+on: bit for bit against the oracle, on the device and over the host."""
 import numpy as np
 import pytest
 
@@ -8,7 +8,7 @@ from qrusty_gb300 import PauliOperator
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 8, 9, 10, 13])
+@pytest.mark.parametrize("n", [1, 8, 9, 10, 17, 18])
 @pytest.mark.parametrize("terms", [1, 3, 40])  # class tables, and folded term by term
 def test_one_group(cuda, oracle, n, terms):
     rng = np.random.default_rng(n + terms)
